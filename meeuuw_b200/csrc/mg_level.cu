@@ -1,0 +1,376 @@
+// A multigrid level's half of a V-cycle in one launch (sm_100a).
+//
+// The downward half smooths from a zero guess (Chebyshev-Jacobi, x0 = D^-1 b / theta, then deg - 1
+// steps), forms the residual b - K x and restricts it; the upward half adds the prolonged coarse
+// correction and smooths again.  A launch per operator apply and per transfer (three down, three
+// up in FP32) costs a level its launch latency six times over and writes x, d and r to memory in
+// between: every level of 128^2 elements and below took 25 us a cycle whatever its size.  Here a CTA
+// takes a tile with enough halo for all its applies (temporal blocking) and keeps every vector of
+// the tile in registers and shared memory; only b, x, the diagonal and the viscosity are read and x
+// and the coarse right-hand side written.
+//
+// Layout: a thread owns one cell, that is one element and the four lattice nodes of its lower-left
+// quadrant (corner, bottom midpoint, left midpoint, centre).  An apply exchanges, through shared
+// memory planes with unit stride over the threads, the values of the five nodes an element shares
+// with its right and upper neighbours, and afterwards the five sums it computed for them.  The halo
+// shrinks by one cell a side and apply; a tile of 16 x 16 cells owns 16 - 2 deg - 2 a side downward and
+// 16 - 2 deg upward.  Tiles of 32 x 16 cells repeat less (owning 26 x 10 and 28 x 12 of them in
+// FP32) but were slower at every size (V-cycle at 512^2 180 against 169 us, at 64^2 42 against 37).
+//
+// Measured, FP32 V-cycle from launch to launch (the separate launches before): 512^2 293 -> 169 us,
+// 256^2 184 -> 79, 128^2 139 -> 52, 64^2 107 -> 37, 8^2 31 -> 11; FP64, one smoothing step: 512^2 309 ->
+// 232, 128^2 104 -> 55.
+//
+// The arithmetic -- element products, node sums over the incident elements in ascending order,
+// smoothing steps, transfer taps -- is that of the kernels of stokes.cu in the same order, so the
+// results equal a cycle of separate launches.
+#include "mg_level.cuh"
+#include "q2_ref.cuh"
+
+namespace mw {
+
+namespace {
+
+// FP64 basis values come from the constant bank (an FP64 immediate costs registers and moves)
+__constant__ RefTables c_k;
+
+template <typename R, int Q, int K> MW_D R kdr() {
+  if constexpr (sizeof(R) == 4) return (float)RefD<Q, K>::r; else return c_k.dr[Q * 9 + K];
+}
+template <typename R, int Q, int K> MW_D R kdt() {
+  if constexpr (sizeof(R) == 4) return (float)RefD<Q, K>::t; else return c_k.dt[Q * 9 + K];
+}
+
+template <typename R, int Q> MW_D R kwq() {
+  constexpr double w = ref_wq(Q);
+  if constexpr (sizeof(R) == 4) return (float)w; else return c_k.wq[Q];
+}
+
+constexpr int CELLS = 16;                                   // cells of a tile, per side
+
+MW_D float2 fma2(float s, float2 a, float2 c) { return __ffma2_rn(make_float2(s, s), a, c); }
+MW_D double2 fma2(double s, double2 a, double2 c) { return make_double2(fma(s, a.x, c.x), fma(s, a.y, c.y)); }
+MW_D float2 pair(float a, float b) { return make_float2(a, b); }
+MW_D double2 pair(double a, double b) { return make_double2(a, b); }
+
+// K_el u on one element: the strain rate at each Gauss point, the stress, B^T back onto the nodes
+// (element_apply of stokes.cu without the pressure terms).
+template <typename R, typename R2>
+MW_D void k_element(R sx, R sz, R jac, const R2 (&u)[9], const R (&eq)[9], R2 (&y)[9]) {
+#pragma unroll
+  for (int k = 0; k < 9; ++k) y[k] = pair(R(0), R(0));
+  static_for<9>([&](auto qc) {
+    constexpr int Q = qc.value;
+    R2 gx = pair(R(0), R(0)), gz = pair(R(0), R(0));
+    static_for<9>([&](auto kc) {
+      constexpr int K = kc.value;
+      if constexpr (RefD<Q, K>::r != 0.0) gx = fma2(kdr<R, Q, K>(), u[K], gx);
+      if constexpr (RefD<Q, K>::t != 0.0) gz = fma2(kdt<R, Q, K>(), u[K], gz);
+    });
+    const R exx = sx * gx.x, ezz = sz * gz.y;
+    const R gg = sizeof(R) == 4 ? fma(sx, gx.y, sz * gz.x) : fma(sz, gz.x, sx * gx.y);
+    const R jw = jac * kwq<R, Q>();
+    const R e = eq[Q] * jw;
+    const R2 ar = pair((R(2) * e * exx) * sx, e * gg * sx);
+    const R2 at = pair(e * gg * sz, (R(2) * e * ezz) * sz);
+    static_for<9>([&](auto kc) {
+      constexpr int K = kc.value;
+      if constexpr (RefD<Q, K>::r != 0.0) y[K] = fma2(kdr<R, Q, K>(), ar, y[K]);
+      if constexpr (RefD<Q, K>::t != 0.0) y[K] = fma2(kdt<R, Q, K>(), at, y[K]);
+    });
+  });
+}
+
+// a / d from the rounded reciprocal y = 1 / d, correctly rounded as the division is: q = a y is
+// within two units, a first correction by the exact residual a - d q makes it faithful, and the
+// second rounds it correctly (Markstein, IBM J. Res. Dev. 34, 1990: a faithful quotient corrected
+// with a correctly rounded reciprocal).  Five packed multiply-adds for a node's two components in
+// place of two divisions.
+MW_D float2 div2(float2 a, float2 d, float2 y) {
+  const float2 nd = make_float2(-d.x, -d.y);
+  float2 q = __fmul2_rn(a, y);
+  float2 r = __ffma2_rn(nd, q, a);
+  q = __ffma2_rn(r, y, q);
+  r = __ffma2_rn(nd, q, a);
+  return __ffma2_rn(r, y, q);
+}
+MW_D double div1(double a, double d, double y) {
+  double q = a * y;
+  q = fma(fma(-d, q, a), y, q);
+  return fma(fma(-d, q, a), y, q);
+}
+MW_D double2 div2(double2 a, double2 d, double2 y) { return make_double2(div1(a.x, d.x, y.x), div1(a.y, d.y, y.y)); }
+
+// the restriction taps along one direction for a coarse node of parity P: fine offsets and weights
+template <int P> struct RTap;
+template <> struct RTap<0> {
+  static constexpr int n = 5;
+  MW_D static constexpr int off(int i) { return i == 0 ? -3 : (i == 1 ? -1 : (i == 2 ? 0 : (i == 3 ? 1 : 3))); }
+  MW_D static constexpr double w(int i) { return (i == 0 || i == 4) ? -0.125 : (i == 2 ? 1.0 : 0.375); }
+};
+template <> struct RTap<1> {
+  static constexpr int n = 3;
+  MW_D static constexpr int off(int i) { return i - 1; }
+  MW_D static constexpr double w(int i) { return i == 1 ? 1.0 : 0.75; }
+};
+
+// sum of the taps of the coarse node whose cell is at index c of the planes sr[4][NC] (row length CX)
+template <int PX, int PZ, int CX, int NC, typename R2>
+MW_D void restrict_taps(const R2* sr, int c, double* s0, double* s1) {
+  double a0 = 0, a1 = 0;
+  static_for<RTap<PZ>::n>([&](auto tz) {
+    constexpr int oz = RTap<PZ>::off(tz.value);
+    static_for<RTap<PX>::n>([&](auto tx) {
+      constexpr int ox = RTap<PX>::off(tx.value);
+      constexpr double w = RTap<PZ>::w(tz.value) * RTap<PX>::w(tx.value);
+      constexpr int plane = (oz & 1) * 2 + (ox & 1), dz = oz < 0 ? -((1 - oz) / 2) : oz / 2,
+                    dx = ox < 0 ? -((1 - ox) / 2) : ox / 2;
+      const R2 v = sr[plane * NC + c + dz * CX + dx];
+      a0 = fma(w, (double)v.x, a0);
+      a1 = fma(w, (double)v.y, a1);
+    });
+  });
+  *s0 = a0;
+  *s1 = a1;
+}
+
+// DOWN: pre-smoothing, residual, restriction; else correction and post-smoothing.  DEG: smoothing
+// steps.  PLANES: nine viscosity planes (else one value per element).
+template <typename R, int DEG, bool DOWN, bool PLANES>
+__global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_level(MgArgs<R> a) {
+  pdl_entry();
+  typedef typename Vec2<R>::T R2;
+  constexpr int CX = CELLS, CZ = CELLS, NC = CX * CZ;
+  constexpr int LO = DOWN ? DEG + 1 : DEG;                  // halo cells on the left and below
+  constexpr int TX = CX - (DOWN ? 2 * DEG + 2 : 2 * DEG), TZ = CZ - (DOWN ? 2 * DEG + 2 : 2 * DEG);
+  constexpr int WX = CX + 3, WZ = CZ + 3;                   // staged coarse nodes (upward)
+  static_assert(TX % 2 == 0 && TZ % 2 == 0, "tiles start at even cells (transfer parity)");
+  __shared__ __align__(16) R2 sx[4 * NC];                   // masked x (then the residual) by node type
+  __shared__ __align__(16) R2 se[5 * NC];                   // sums for the right and upper neighbours
+  __shared__ __align__(16) double2 sc[DOWN ? 1 : WX * WZ];
+  const int tid = threadIdx.x, lx = tid % CX, lz = tid / CX;
+  const int ex0 = blockIdx.x * TX, ez0 = blockIdx.y * TZ;
+  const int ex = ex0 + lx - LO, ez = ez0 + lz - LO;
+  const LevelGeo& g = a.g;
+  // which of the cell's nodes lie on the lattice (the cells past the last element own the right and
+  // top boundary nodes)
+  const bool cx0 = ex >= 0 && ex <= g.nx, cx1 = ex >= 0 && ex < g.nx;
+  const bool cz0 = ez >= 0 && ez <= g.nz, cz1 = ez >= 0 && ez < g.nz;
+  const bool has[4] = {cx0 && cz0, cx1 && cz0, cx0 && cz1, cx1 && cz1};
+  const int64_t n0 = (int64_t)(2 * ez) * g.nnx + 2 * ex;
+  const R2 zero = pair(R(0), R(0));
+  const double c1s = DEG > 1 ? a.cheb[2] : 0.0;
+  const R c20 = (R)a.cheb[1], c21 = DEG > 1 ? (R)a.cheb[3] : R(0);
+  R2 b[4], dg[4], di[4], x[4], d[4];
+  unsigned fx = 0;                                          // bit 2 t + c: component c of node t is fixed
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
+    b[t] = dg[t] = di[t] = x[t] = zero;
+    if (has[t]) {
+      b[t] = reinterpret_cast<const R2*>(a.b)[n];
+      dg[t] = reinterpret_cast<const R2*>(a.diag)[n];
+      di[t] = reinterpret_cast<const R2*>(a.dinv)[n];
+      const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n];
+      fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
+      if (!DOWN) x[t] = reinterpret_cast<const R2*>(a.xin)[n];
+    }
+  }
+  R eq[9];
+  if (has[3]) {
+    const int64_t e = (int64_t)ez * g.nx + ex, nel = (int64_t)g.nx * g.nz;
+    if (PLANES) {
+#pragma unroll
+      for (int q = 0; q < 9; ++q) eq[q] = a.eta[q * nel + e];
+    } else {
+      const R v = a.eta[e];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) eq[q] = v;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) eq[q] = R(0);
+  }
+  if constexpr (DOWN) {                                     // x0 = d0 = (1/theta) D^-1 b
+#pragma unroll
+    for (int t = 0; t < 4; ++t) d[t] = x[t] = div2(pair(c20 * b[t].x, c20 * b[t].y), dg[t], di[t]);
+  } else if (a.xc) {
+    // x + P x_c on the free components: the coarse nodes under the tile in shared memory, as
+    // doubles (converted once), the taps of prolong_taps in its order
+    const int bx = (ex0 - LO) & ~1, bz = (ez0 - LO) & ~1;
+    for (int i = tid; i < WX * WZ; i += NC) {
+      const int jx = bx + i % WX, jz = bz + i / WX;
+      R2 v = zero;
+      if (jx >= 0 && jx < a.gc.nnx && jz >= 0 && jz < a.gc.nnz)
+        v = reinterpret_cast<const R2*>(a.xc)[(int64_t)jz * a.gc.nnx + jx];
+      sc[i] = make_double2((double)v.x, (double)v.y);
+    }
+    __syncthreads();
+    const double wx0 = (ex & 1) ? -0.125 : 0.375, wx2 = (ex & 1) ? 0.375 : -0.125;
+    const double wz0 = (ez & 1) ? -0.125 : 0.375, wz2 = (ez & 1) ? 0.375 : -0.125;
+    const double wx[3] = {wx0, 0.75, wx2}, wz[3] = {wz0, 0.75, wz2};
+    const int ox = (ex & ~1) - bx, oz = (ez & ~1) - bz, mx = ex - bx, mz = ez - bz;
+    double s0[4], s1[4];
+    const double2 vc = sc[mz * WX + mx];
+    s0[0] = vc.x; s1[0] = vc.y;
+    s0[1] = s1[1] = s0[2] = s1[2] = s0[3] = s1[3] = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double2 v = sc[mz * WX + ox + i], w = sc[(oz + i) * WX + mx];
+      s0[1] = fma(wx[i], v.x, s0[1]); s1[1] = fma(wx[i], v.y, s1[1]);
+      s0[2] = fma(wz[i], w.x, s0[2]); s1[2] = fma(wz[i], w.y, s1[2]);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const double2 c = sc[(oz + i) * WX + ox + j];
+        const double p = wz[i] * wx[j];
+        s0[3] = fma(p, c.x, s0[3]); s1[3] = fma(p, c.y, s1[3]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (has[t]) {
+        if (!(fx & (1u << (2 * t)))) x[t].x += (R)s0[t];
+        if (!(fx & (2u << (2 * t)))) x[t].y += (R)s1[t];
+      }
+  }
+  const R sxe = R(2.0 / g.hx), sze = R(2.0 / g.hz), jace = R(g.hx * g.hz / 4.0);
+  auto masked = [&](int t) {
+    return pair((fx & (1u << (2 * t))) ? R(0) : x[t].x, (fx & (2u << (2 * t))) ? R(0) : x[t].y);
+  };
+#pragma unroll
+  for (int j = 0; j < DEG; ++j) {
+    // ---- y = K x at the cell's nodes ----
+    R2 u[9], y[9];
+    u[0] = masked(0); u[4] = masked(1); u[7] = masked(2); u[8] = masked(3);
+    sx[tid] = u[0]; sx[NC + tid] = u[4]; sx[2 * NC + tid] = u[7]; sx[3 * NC + tid] = u[8];
+    __syncthreads();
+    if (has[3] && lx >= j && lx <= CX - 2 - j && lz >= j && lz <= CZ - 2 - j) {
+      u[1] = sx[tid + 1];
+      u[5] = sx[2 * NC + tid + 1];
+      u[3] = sx[tid + CX];
+      u[6] = sx[NC + tid + CX];
+      u[2] = sx[tid + CX + 1];
+      k_element(sxe, sze, jace, u, eq, y);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) y[k] = zero;
+    }
+    se[tid] = y[1]; se[NC + tid] = y[5]; se[2 * NC + tid] = y[3]; se[3 * NC + tid] = y[6]; se[4 * NC + tid] = y[2];
+    __syncthreads();
+    // ascending element order: lower left, lower, left, own
+    const bool hl = lx > 0, hb = lz > 0;
+    const R2 p2 = hl && hb ? se[4 * NC + tid - CX - 1] : zero, p3 = hb ? se[2 * NC + tid - CX] : zero,
+             p1 = hl ? se[tid - 1] : zero, p6 = hb ? se[3 * NC + tid - CX] : zero, p5 = hl ? se[NC + tid - 1] : zero;
+    R2 s[4];
+    s[0] = pair(((p2.x + p3.x) + p1.x) + y[0].x, ((p2.y + p3.y) + p1.y) + y[0].y);
+    s[1] = pair(p6.x + y[4].x, p6.y + y[4].y);
+    s[2] = pair(p5.x + y[7].x, p5.y + y[7].y);
+    s[3] = y[8];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {                           // eliminated rows act as K_ii u_i
+      if (fx & (1u << (2 * t))) s[t].x = dg[t].x * x[t].x;
+      if (fx & (2u << (2 * t))) s[t].y = dg[t].y * x[t].y;
+    }
+    if (DOWN && j == DEG - 1) {                             // residual of the smoothed x
+#pragma unroll
+      for (int t = 0; t < 4; ++t) s[t] = has[t] ? pair(b[t].x - s[t].x, b[t].y - s[t].y) : zero;
+      const int ownx = min(ex0 + TX >= g.nx ? TX + 1 : TX, g.nx + 1 - ex0);
+      const int ownz = min(ez0 + TZ >= g.nz ? TZ + 1 : TZ, g.nz + 1 - ez0);
+      const bool own = lx >= LO && lx < LO + ownx && lz >= LO && lz < LO + ownz;
+      if (own) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          if (has[t]) {
+            const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
+            reinterpret_cast<R2*>(a.x)[n] = x[t];
+            if (!a.bc) reinterpret_cast<R2*>(a.r)[n] = s[t];
+          }
+      }
+      if (a.bc) {
+        // coarse node (I, J) sits on the corner of fine cell (I, J); the four parities have 9, 15,
+        // 15 and 25 taps, so each warp takes nodes of one parity
+#pragma unroll
+        for (int t = 0; t < 4; ++t) sx[t * NC + tid] = s[t];
+        __syncthreads();
+        const int warp = tid >> 5, px = warp & 1, pz = (warp >> 1) & 1;
+        const int mx = (ownx - px + 1) / 2, mz = (ownz - pz + 1) / 2;
+        for (int i = (warp >> 2) * 32 + (tid & 31); i < mx * mz; i += NC / 4) {
+          const int jx = 2 * (i % mx) + px, jz = 2 * (i / mx) + pz;
+          const int c = (jz + LO) * CX + jx + LO;
+          const int64_t n = (int64_t)(ez0 + jz) * a.gc.nnx + ex0 + jx;
+          const uchar2 f = reinterpret_cast<const uchar2*>(a.fixc)[n];
+          double s0, s1;
+          if (px) {
+            if (pz) restrict_taps<1, 1, CX, NC>(sx, c, &s0, &s1);
+            else restrict_taps<1, 0, CX, NC>(sx, c, &s0, &s1);
+          } else {
+            if (pz) restrict_taps<0, 1, CX, NC>(sx, c, &s0, &s1);
+            else restrict_taps<0, 0, CX, NC>(sx, c, &s0, &s1);
+          }
+          reinterpret_cast<R2*>(a.bc)[n] = pair(f.x ? R(0) : (R)s0, f.y ? R(0) : (R)s1);
+        }
+      }
+    } else {                                                // d = c1 d + c2 D^-1 (b - y); x += d
+      const bool first = !DOWN && j == 0;                   // the restart step reads no old direction
+      const R c2 = (DOWN || j > 0) ? c21 : c20;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        R2 dn = div2(pair(c2 * (b[t].x - s[t].x), c2 * (b[t].y - s[t].y)), dg[t], di[t]);
+        if (!first && c1s != 0.0) {
+          dn.x += R(c1s) * d[t].x;
+          dn.y += R(c1s) * d[t].y;
+        }
+        d[t] = dn;
+        x[t] = pair(x[t].x + dn.x, x[t].y + dn.y);
+      }
+    }
+  }
+  if constexpr (!DOWN) {
+    const int ownx = ex0 + TX >= g.nx ? TX + 1 : TX, ownz = ez0 + TZ >= g.nz ? TZ + 1 : TZ;
+    if (lx >= LO && lx < LO + ownx && lz >= LO && lz < LO + ownz) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (has[t]) reinterpret_cast<R2*>(a.x)[n0 + (t >> 1) * g.nnx + (t & 1)] = x[t];
+    }
+  }
+}
+
+template <typename R, int DEG, bool DOWN>
+void launch(const MgArgs<R>& a, bool planes, cudaStream_t s) {
+  constexpr int T = CELLS - (DOWN ? 2 * DEG + 2 : 2 * DEG);
+  const dim3 grid((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
+  if (planes) pdl_launch(k_mg_level<R, DEG, DOWN, true>, grid, CELLS * CELLS, 0, s, a);
+  else pdl_launch(k_mg_level<R, DEG, DOWN, false>, grid, CELLS * CELLS, 0, s, a);
+}
+
+template <typename R, bool DOWN>
+void by_degree(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
+  if (deg <= 1) launch<R, 1, DOWN>(a, planes, s);
+  else launch<R, MG_MAXDEG, DOWN>(a, planes, s);
+}
+
+}  // namespace
+
+int mg_ensure_tables() {
+  static bool ready = false;
+  if (ready) return MW_OK;
+  RefTables t;
+  host_ref_tables(&t);
+  if (cudaMemcpyToSymbol(c_k, &t, sizeof(t)) != cudaSuccess) return MW_ERR_CUDA;
+  ready = true;
+  return MW_OK;
+}
+
+template <typename R> void mg_down(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
+  by_degree<R, true>(a, deg, planes, s);
+}
+template <typename R> void mg_up(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
+  by_degree<R, false>(a, deg, planes, s);
+}
+
+template void mg_down<float>(const MgArgs<float>&, int, bool, cudaStream_t);
+template void mg_down<double>(const MgArgs<double>&, int, bool, cudaStream_t);
+template void mg_up<float>(const MgArgs<float>&, int, bool, cudaStream_t);
+template void mg_up<double>(const MgArgs<double>&, int, bool, cudaStream_t);
+
+}  // namespace mw

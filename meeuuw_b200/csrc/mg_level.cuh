@@ -1,0 +1,49 @@
+// One multigrid level's half of a V-cycle as one launch (mg_level.cu), and the level geometry it
+// shares with the operator and solver kernels of stokes.cu.
+#pragma once
+
+#include "common.cuh"
+
+namespace mw {
+
+struct LevelGeo {
+  int nx, nz;        // elements
+  int nnx, nnz;      // Q2 lattice nodes
+  double hx, hz;
+  double s;          // G scaling eta_ref / L_ref (build_matrix_stokes.py:157)
+};
+
+template <typename R> struct Vec2;
+template <> struct Vec2<float> { typedef float2 T; };
+template <> struct Vec2<double> { typedef double2 T; };
+
+// smoothing steps per sweep the level launches are built for
+constexpr int MG_MAXDEG = 2;
+
+// Arguments of a level's half cycle.  Velocity vectors are interleaved (u, w) pairs.
+template <typename R>
+struct MgArgs {
+  LevelGeo g, gc;      // this level, the coarser one
+  const R* eta;        // viscosity: nine planes of nel values (level 0), or one value per element
+  const uint8_t* fix;  // Dirichlet flags (2 per node)
+  const R *diag, *dinv;// diag(K) and its rounded reciprocal
+  const R* b;          // right-hand side
+  const R* xin;        // upward: x before the correction (not the output buffer)
+  R* x;                // downward: the smoothed x; upward: the result
+  const double* cheb;  // Chebyshev coefficient pairs {c1, c2} per step
+  // downward: the restricted residual goes to bc (fixed coarse entries zero), or -- bc null -- the
+  // residual itself to r
+  R* bc;
+  const uint8_t* fixc;
+  R* r;
+  const R* xc;         // upward: the coarse correction to prolong; null: xin already carries it
+};
+
+// The FP64 kernels' basis tables in the constant bank; called before the first level launch.
+int mg_ensure_tables();
+// Smoothing from a zero guess (`deg` Chebyshev-Jacobi steps), the residual and its restriction.
+template <typename R> void mg_down(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s);
+// The coarse correction and `deg` smoothing steps.
+template <typename R> void mg_up(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s);
+
+}  // namespace mw

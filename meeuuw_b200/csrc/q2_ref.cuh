@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cmath>
+#include <utility>
 
 #include "common.cuh"
 
@@ -38,6 +39,20 @@ MW_HD constexpr double ref_np(int q, int k) {
 MW_HD constexpr double ref_wq(int q) { return gwt(q / 3) * gwt(q % 3); }
 // N_V at Gauss point q: the product of the 1D functions (used for which terms vanish)
 MW_HD constexpr double ref_nv(int q, int k) { return lq(kdx(k), gpt(q / 3)) * lq(kdz(k), gpt(q % 3)); }
+
+// f(integral_constant<int, 0>) ... f(integral_constant<int, N - 1>): loops whose index is a constant
+// expression, so that the basis values are folded by the front end and not by the optimiser (a
+// translation unit of operator kernels compiles in seconds instead of minutes)
+template <int N, typename F, int... I>
+MW_D void static_for_impl(F&& f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>{}), ...);
+}
+template <int N, typename F>
+MW_D void static_for(F&& f) { static_for_impl<N>(f, std::make_integer_sequence<int, N>{}); }
+
+template <int Q, int K> struct RefD {
+  static constexpr double r = ref_dr(Q, K), t = ref_dt(Q, K);
+};
 
 inline void host_ref_tables(RefTables* T) {
   const double qc[3] = {-std::sqrt(3.0 / 5.0), 0.0, std::sqrt(3.0 / 5.0)};

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "mg_level.cuh"
 #include "q2_ref.cuh"
 
 namespace mw {
@@ -36,35 +37,28 @@ static bool g_ref_ready = false;
 // immediate would be materialised in registers for every use).  Which terms vanish is decided at
 // compile time in both cases (ref_dr / ref_dt of q2_ref.cuh).
 template <typename R> struct CT {
-  MW_D static constexpr R dr(int q, int k) { return (R)ref_dr(q, k); }
-  MW_D static constexpr R dt(int q, int k) { return (R)ref_dt(q, k); }
-  MW_D static constexpr R np(int q, int k) { return (R)ref_np(q, k); }
-  MW_D static constexpr R wq(int q) { return (R)ref_wq(q); }
+  template <int Q, int K> MW_D static constexpr R dr() { return (R)RefD<Q, K>::r; }
+  template <int Q, int K> MW_D static constexpr R dt() { return (R)RefD<Q, K>::t; }
+  template <int Q, int K> MW_D static constexpr R np() { constexpr double v = ref_np(Q, K); return (R)v; }
+  template <int Q> MW_D static constexpr R wq() { constexpr double v = ref_wq(Q); return (R)v; }
 };
 template <> struct CT<double> {
-  MW_D static double dr(int q, int k) { return c_ref.dr[q * 9 + k]; }
-  MW_D static double dt(int q, int k) { return c_ref.dt[q * 9 + k]; }
-  MW_D static double np(int q, int k) { return c_ref.NP[q * 4 + k]; }
-  MW_D static double wq(int q) { return c_ref.wq[q]; }
+  template <int Q, int K> MW_D static double dr() { return c_ref.dr[Q * 9 + K]; }
+  template <int Q, int K> MW_D static double dt() { return c_ref.dt[Q * 9 + K]; }
+  template <int Q, int K> MW_D static double np() { return c_ref.NP[Q * 4 + K]; }
+  template <int Q> MW_D static double wq() { return c_ref.wq[Q]; }
 };
 
 static int ensure_ref_tables() {
   if (g_ref_ready) return MW_OK;
   RefTables T;
   host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess) return MW_ERR_CUDA;
+  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables()) return MW_ERR_CUDA;
   g_ref_ready = true;
   return MW_OK;
 }
 
-// ---------------------------------------------------------------- level geometry
-struct LevelGeo {
-  int nx, nz;        // elements
-  int nnx, nnz;      // Q2 lattice nodes
-  double hx, hz;
-  double s;          // G scaling eta_ref / L_ref (build_matrix_stokes.py:157)
-};
-
+// ---------------------------------------------------------------- element tiles
 constexpr int TX = 16, TZ = 8;                 // owned element tile
 constexpr int EX = TX + 1, EZ = TZ + 1;        // with the left/bottom halo
 constexpr int NEL_T = EX * EZ;                 // 153 element computations per CTA
@@ -74,14 +68,7 @@ constexpr int APPLY_THREADS = 160;
 
 // AM_CHEB_Z: the second Chebyshev step of a sweep from a zero guess with the first one folded in:
 // the velocity staged is x0 = (1/theta) D^-1 b (the first step's x and d), computed on the fly
-// AM_CHEB_P: the first Chebyshev step after the coarse-grid correction with the prolongation folded
-// in: the velocity staged is x + P x_c (free dofs), computed from a staged tile of the coarse
-// correction with the taps and rounding of k_prolong_add, so the V-cycle needs no prolongation launch.
-enum ApplyMode { AM_APPLY = 0, AM_RESID = 1, AM_CHEB = 2, AM_CHEB_Z = 3, AM_CHEB_P = 4 };
-
-template <typename R> struct Vec2;
-template <> struct Vec2<float> { typedef float2 T; };
-template <> struct Vec2<double> { typedef double2 T; };
+enum ApplyMode { AM_APPLY = 0, AM_RESID = 1, AM_CHEB = 2, AM_CHEB_Z = 3 };
 
 template <typename R>
 struct ApplyArgs {
@@ -116,42 +103,53 @@ MW_D void element_apply(R sx, R sz, R jac, R s, const R* ue, const R* pe, const 
   for (int k = 0; k < 18; ++k) ye[k] = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) ype[k] = 0;
-#pragma unroll
-  for (int q = 0; q < 9; ++q) {
+  static_for<9>([&](auto qc) {
+    constexpr int Q = qc.value;
     R dxu = 0, dzw = 0, dzu = 0, dxw = 0;
-    if (HAS_U) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const R r = CT<R>::dr(q, k), t = CT<R>::dt(q, k);
-        if (ref_dr(q, k) != 0.0) { dxu += r * ue[2 * k]; if (NEED_V) dxw += r * ue[2 * k + 1]; }
-        if (ref_dt(q, k) != 0.0) { dzw += t * ue[2 * k + 1]; if (NEED_V) dzu += t * ue[2 * k]; }
-      }
+    if constexpr (HAS_U) {
+      static_for<9>([&](auto kc) {
+        constexpr int K = kc.value;
+        if constexpr (RefD<Q, K>::r != 0.0) {
+          const R r = CT<R>::template dr<Q, K>();
+          dxu += r * ue[2 * K];
+          if (NEED_V) dxw += r * ue[2 * K + 1];
+        }
+        if constexpr (RefD<Q, K>::t != 0.0) {
+          const R t = CT<R>::template dt<Q, K>();
+          dzw += t * ue[2 * K + 1];
+          if (NEED_V) dzu += t * ue[2 * K];
+        }
+      });
     }
-    const R exx = sx * dxu, ezz = sz * dzw, gg = sz * dzu + sx * dxw;   // gg = du/dz + dw/dx
-    const R jw = jac * CT<R>::wq(q);
-    if (NEED_V) {
-      const R e = eq[q] * jw;
+    // the shear rate du/dz + dw/dx, its rounding written out: every kernel that applies K rounds alike
+    const R exx = sx * dxu, ezz = sz * dzw, gg = fma(sz, dzu, sx * dxw);
+    const R jw = jac * CT<R>::template wq<Q>();
+    if constexpr (NEED_V) {
+      const R e = eq[Q] * jw;
       R pq = 0;
-      if (use_p) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) pq += CT<R>::np(q, k) * pe[k];
-      }
+      if (use_p) static_for<4>([&](auto kc) { pq += CT<R>::template np<Q, kc.value>() * pe[kc.value]; });
       const R sp = s * jw * pq;
       const R A = (R(2) * e * exx - sp) * sx, B = (R(2) * e * ezz - sp) * sz;
       const R Cx = e * gg * sx, Cz = e * gg * sz;
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const R r = CT<R>::dr(q, k), t = CT<R>::dt(q, k);
-        if (ref_dr(q, k) != 0.0) { ye[2 * k] += r * A; if (HAS_U) ye[2 * k + 1] += r * Cx; }
-        if (ref_dt(q, k) != 0.0) { if (HAS_U) ye[2 * k] += t * Cz; ye[2 * k + 1] += t * B; }
-      }
+      static_for<9>([&](auto kc) {
+        constexpr int K = kc.value;
+        if constexpr (RefD<Q, K>::r != 0.0) {
+          const R r = CT<R>::template dr<Q, K>();
+          ye[2 * K] += r * A;
+          if (HAS_U) ye[2 * K + 1] += r * Cx;
+        }
+        if constexpr (RefD<Q, K>::t != 0.0) {
+          const R t = CT<R>::template dt<Q, K>();
+          if (HAS_U) ye[2 * K] += t * Cz;
+          ye[2 * K + 1] += t * B;
+        }
+      });
     }
-    if (HAS_U) {
+    if constexpr (HAS_U) {
       const R dv = -s * jw * (exx + ezz);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) ype[k] += CT<R>::np(q, k) * dv;
+      static_for<4>([&](auto kc) { ype[kc.value] += CT<R>::template np<Q, kc.value>() * dv; });
     }
-  }
+  });
 }
 
 // FP32 variant on the packed two-lane FMA of sm_100 (__ffma2_rn): a node's (u, w) pair is one
@@ -166,36 +164,32 @@ MW_D void element_apply<float, true, true>(float sx, float sz, float jac, float 
   for (int k = 0; k < 9; ++k) y2[k] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int k = 0; k < 4; ++k) ype[k] = 0.f;
-#pragma unroll
-  for (int q = 0; q < 9; ++q) {
+  static_for<9>([&](auto qc) {
+    constexpr int Q = qc.value;
     float2 gx = make_float2(0.f, 0.f), gz = make_float2(0.f, 0.f);   // (du/dr, dw/dr), (du/dt, dw/dt)
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float r = CT<float>::dr(q, k), t = CT<float>::dt(q, k);
-      if (r != 0.f) gx = __ffma2_rn(make_float2(r, r), u2[k], gx);
-      if (t != 0.f) gz = __ffma2_rn(make_float2(t, t), u2[k], gz);
-    }
-    const float exx = sx * gx.x, ezz = sz * gz.y, gg = sz * gz.x + sx * gx.y;
-    const float jw = jac * CT<float>::wq(q);
-    const float e = eq[q] * jw;
+    static_for<9>([&](auto kc) {
+      constexpr int K = kc.value;
+      constexpr float r = (float)RefD<Q, K>::r, t = (float)RefD<Q, K>::t;
+      if constexpr (r != 0.f) gx = __ffma2_rn(make_float2(r, r), u2[K], gx);
+      if constexpr (t != 0.f) gz = __ffma2_rn(make_float2(t, t), u2[K], gz);
+    });
+    const float exx = sx * gx.x, ezz = sz * gz.y, gg = fma(sx, gx.y, sz * gz.x);
+    const float jw = jac * CT<float>::wq<Q>();
+    const float e = eq[Q] * jw;
     float pq = 0.f;
-    if (use_p) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pq += CT<float>::np(q, k) * pe[k];
-    }
+    if (use_p) static_for<4>([&](auto kc) { pq += CT<float>::np<Q, kc.value>() * pe[kc.value]; });
     const float sp = s * jw * pq;
     const float2 ar = make_float2((2.f * e * exx - sp) * sx, e * gg * sx);   // coefficients of dN/dr
     const float2 at = make_float2(e * gg * sz, (2.f * e * ezz - sp) * sz);   // coefficients of dN/dt
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float r = CT<float>::dr(q, k), t = CT<float>::dt(q, k);
-      if (r != 0.f) y2[k] = __ffma2_rn(make_float2(r, r), ar, y2[k]);
-      if (t != 0.f) y2[k] = __ffma2_rn(make_float2(t, t), at, y2[k]);
-    }
+    static_for<9>([&](auto kc) {
+      constexpr int K = kc.value;
+      constexpr float r = (float)RefD<Q, K>::r, t = (float)RefD<Q, K>::t;
+      if constexpr (r != 0.f) y2[K] = __ffma2_rn(make_float2(r, r), ar, y2[K]);
+      if constexpr (t != 0.f) y2[K] = __ffma2_rn(make_float2(t, t), at, y2[K]);
+    });
     const float dv = -s * jw * (exx + ezz);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) ype[k] += CT<float>::np(q, k) * dv;
-  }
+    static_for<4>([&](auto kc) { ype[kc.value] += CT<float>::np<Q, kc.value>() * dv; });
+  });
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     ye[2 * k] = y2[k].x;
@@ -329,8 +323,8 @@ MW_D int pw(int i, int* J, double* w) {
 }
 
 // (P x_c) at fine lattice node (ix, iz): the taps summed in double in a fixed order (z outer, x
-// inner) with explicit fused multiply-adds, so every path that prolongs (the prolongation kernel,
-// the cluster tail, the Chebyshev step with the prolongation folded in) rounds alike.
+// inner) with explicit fused multiply-adds, so every path that prolongs (the prolongation kernels,
+// the cluster tail, the level launches of mg_level.cu) rounds alike.
 // coarse(Jz, Jx) returns the coarse node's (u, w) pair.
 template <typename V>
 MW_D void prolong_taps(int ix, int iz, const V& coarse, double* s0, double* s1) {
@@ -408,11 +402,6 @@ MW_D void prolong_taps_g(const G& gf, const G& gc, int ix, int iz, const V& coar
   *s1 = a1;
 }
 
-// the coarse-correction tile the AM_CHEB_P staging reads: coarse lattice nodes [ex0 - 2, ex0 + 17]
-// x [ez0 - 2, ez0 + 9] cover every tap of the staged fine nodes [2 ex0 - 2, 2 ex0 + 32] x
-// [2 ez0 - 2, 2 ez0 + 16]
-constexpr int CLX = 20, CLZ = 12;
-
 #ifndef MW_APPLY_MINB
 #define MW_APPLY_MINB 5      // resident FP32 apply CTAs per SM the register budget is sized for
 #endif
@@ -433,8 +422,7 @@ MW_D void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory");
 template <typename R, int MODE>
 struct ApplySmem {
   typedef typename Vec2<R>::T R2;
-  static constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z || MODE == AM_CHEB_P;
-  static constexpr bool PRO = MODE == AM_CHEB_P;
+  static constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z;
   static constexpr int NPRE = sizeof(R) == 8 ? 0 : (CHEB ? 3 : (MODE == AM_RESID ? 1 : 0));
   static constexpr int NJ = APPLY_THREADS - TX * TZ;  // spare threads: right column and top row nodes
   __align__(16) R su[LZ * LX * 2];
@@ -443,7 +431,6 @@ struct ApplySmem {
   R sp[PZ * PX];
   R sye[NEL_T * 22];
   uchar2 sfix[LZ * LX];                              // Dirichlet flags of the staged nodes
-  __align__(16) R2 scx[PRO ? CLZ * CLX : 1];         // AM_CHEB_P: the coarse correction tile
 };
 
 // Where one tile's shared arrays are: the static arrays of k_apply, or an ApplySmem carved from
@@ -455,12 +442,11 @@ struct ApplyPtrs {
   R2 *spre, *sspare;
   R *sp, *sye;
   uchar2* sfix;
-  R2* scx;
 };
 
 template <typename R, int MODE>
 MW_D ApplyPtrs<R> apply_ptrs(ApplySmem<R, MODE>& sm) {
-  return ApplyPtrs<R>{sm.su, sm.spre, sm.sspare, sm.sp, sm.sye, sm.sfix, sm.scx};
+  return ApplyPtrs<R>{sm.su, sm.spre, sm.sspare, sm.sp, sm.sye, sm.sfix};
 }
 
 // One operator apply over element tile (bx, bz) by the APPLY_THREADS threads of a CTA, in the
@@ -470,7 +456,6 @@ template <typename R, int MODE>
 MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, const ApplyPtrs<R>& sm) {
   typedef typename Vec2<R>::T R2;
   constexpr bool CHEB = ApplySmem<R, MODE>::CHEB;
-  constexpr bool PRO = ApplySmem<R, MODE>::PRO;
   constexpr int NPRE = ApplySmem<R, MODE>::NPRE;
   constexpr int NJ = ApplySmem<R, MODE>::NJ;
   static_assert(2 * TZ + 1 + 2 * TX <= 2 * NJ, "the spare threads take at most two boundary nodes each");
@@ -480,7 +465,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   R* const sp = sm.sp;
   R* const sye = sm.sye;
   uchar2* const sfix = sm.sfix;
-  R2* const scx = sm.scx;
   const int ex0 = bx * TX, ez0 = bz * TZ;
   const int lx0 = 2 * ex0 - 2, lz0 = 2 * ez0 - 2;      // lattice origin of the staged nodes
   const int tid = threadIdx.x;
@@ -539,29 +523,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
       for (int q = 0; q < 9; ++q) eq[q] = eg[q];
     }
   }
-  // ---- AM_CHEB_P: the coarse correction tile (loaded now, stored after the fine loads) ----
-  constexpr int NCT = PRO ? (CLZ * CLX + APPLY_THREADS - 1) / APPLY_THREADS : 1;
-  R2 cv[NCT];
-  const int cx0 = ex0 - 2, cz0 = ez0 - 2;
-  if constexpr (PRO) {
-#pragma unroll
-    for (int k = 0; k < NCT; ++k) {
-      const int i = tid + k * APPLY_THREADS;
-      const int jz = i / CLX, jx = i - jz * CLX;
-      const int cx = cx0 + jx, cz = cz0 + jz;
-      cv[k].x = 0; cv[k].y = 0;
-      if (i < CLZ * CLX && cx >= 0 && cx < a.gc.nnx && cz >= 0 && cz < a.gc.nnz)
-        cv[k] = reinterpret_cast<const R2*>(a.xc)[(int64_t)cz * a.gc.nnx + cx];
-    }
-  }
-  // x + P x_c on the free dofs of fine node (ix, iz) (the arithmetic of k_prolong_add)
-  auto corrected = [&](int ix, int iz, R2 x, uchar2 ff) -> R2 {
-    double s0, s1;
-    prolong_taps(ix, iz, [&](int jz, int jx) { return scx[(jz - cz0) * CLX + (jx - cx0)]; }, &s0, &s1);
-    if (!ff.x) x.x += (R)s0;
-    if (!ff.y) x.y += (R)s1;
-    return x;
-  };
   // ---- stage velocity (masked; one vector load per node), pressure ----
   // A fixed number of nodes per thread, all loads issued before any shared-memory store, so the
   // staging costs one memory round trip rather than one per node.
@@ -574,12 +535,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   uchar2 sf[NST];
   R spv[NSP];
   if constexpr (sizeof(R) == 8) {                    // FP64: one node at a time (fewer live registers)
-    if constexpr (PRO) {
-#pragma unroll
-      for (int k = 0; k < NCT; ++k)
-        if (tid + k * APPLY_THREADS < CLZ * CLX) scx[tid + k * APPLY_THREADS] = cv[k];
-      __syncthreads();
-    }
     for (int i = tid; i < LZ * LX; i += APPLY_THREADS) {
       const int lz = i / LX, lx = i - lz * LX;
       const int ix = lx0 + lx, iz = lz0 + lz;
@@ -591,7 +546,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
         ff = f2[n];
         if (use_u) {
           R2 uu = u2[n];
-          if constexpr (PRO) uu = corrected(ix, iz, uu, ff);
           v.x = ff.x ? R(0) : uu.x;
           v.y = ff.y ? R(0) : uu.y;
         }
@@ -632,19 +586,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     const int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
     spv[k] = (use_p && i < PZ * PX && px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz)
                  ? a.p[(int64_t)pz * (g.nx + 1) + px] : R(0);
-  }
-  if constexpr (PRO) {
-#pragma unroll
-    for (int k = 0; k < NCT; ++k)
-      if (tid + k * APPLY_THREADS < CLZ * CLX) scx[tid + k * APPLY_THREADS] = cv[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NST; ++k) {
-      const int i = tid + k * APPLY_THREADS;
-      const int lz = i / LX, lx = i - lz * LX;
-      const int ix = lx0 + lx, iz = lz0 + lz;
-      if (i < LZ * LX && ix >= 0 && ix < g.nnx && iz >= 0 && iz < g.nnz) sv[k] = corrected(ix, iz, sv[k], sf[k]);
-    }
   }
 #pragma unroll
   for (int k = 0; k < NST; ++k) {
@@ -718,8 +659,8 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     if (CHEB) dg = pre ? pre_at(1, slot) : reinterpret_cast<const R2*>(a.diag)[n];
     else if (fixed) dg = reinterpret_cast<const R2*>(a.diag)[n];
     if (fixed && MODE != AM_CHEB_Z) {                // the fixed components' values (staged as 0);
-      const R2 raw = reinterpret_cast<const R2*>(a.u)[n];   // a free one keeps its staged value,
-      if (ff.x) uu.x = raw.x;                        // which under AM_CHEB_P carries P x_c
+      const R2 raw = reinterpret_cast<const R2*>(a.u)[n];   // a free one keeps its staged value
+      if (ff.x) uu.x = raw.x;
       if (ff.y) uu.y = raw.y;
     }
     if (MODE != AM_APPLY) bb = pre ? pre_at(0, slot) : reinterpret_cast<const R2*>(a.bV)[n];
@@ -872,8 +813,7 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
   // node vectors the epilogue reads for the four nodes each owned element emits (b; b, diag, d),
   // fetched asynchronously while the element products run (FP32; the FP64 kernel's shared memory
   // is already at the 48 KB static limit)
-  constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z || MODE == AM_CHEB_P;
-  constexpr bool PRO = MODE == AM_CHEB_P;
+  constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z;
   constexpr int NPRE = sizeof(R) == 8 ? 0 : (CHEB ? 3 : (MODE == AM_RESID ? 1 : 0));
   __shared__ __align__(16) R su[LZ * LX * 2];
   __shared__ __align__(16) R2 spre[(NPRE ? NPRE : 1) * 4 * TX * TZ];
@@ -883,7 +823,6 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
   __shared__ R sp[PZ * PX];
   __shared__ R sye[NEL_T * 22];
   __shared__ uchar2 sfix[LZ * LX];          // Dirichlet flags of the staged nodes
-  __shared__ __align__(16) R2 scx[PRO ? CLZ * CLX : 1];   // AM_CHEB_P: the coarse correction tile
   const int ex0 = blockIdx.x * TX, ez0 = blockIdx.y * TZ;
   const int lx0 = 2 * ex0 - 2, lz0 = 2 * ez0 - 2;      // lattice origin of the staged nodes
   const int tid = threadIdx.x;
@@ -942,29 +881,6 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
       for (int q = 0; q < 9; ++q) eq[q] = eg[q];
     }
   }
-  // ---- AM_CHEB_P: the coarse correction tile (loaded now, stored after the fine loads) ----
-  constexpr int NCT = PRO ? (CLZ * CLX + APPLY_THREADS - 1) / APPLY_THREADS : 1;
-  R2 cv[NCT];
-  const int cx0 = ex0 - 2, cz0 = ez0 - 2;
-  if constexpr (PRO) {
-#pragma unroll
-    for (int k = 0; k < NCT; ++k) {
-      const int i = tid + k * APPLY_THREADS;
-      const int jz = i / CLX, jx = i - jz * CLX;
-      const int cx = cx0 + jx, cz = cz0 + jz;
-      cv[k].x = 0; cv[k].y = 0;
-      if (i < CLZ * CLX && cx >= 0 && cx < a.gc.nnx && cz >= 0 && cz < a.gc.nnz)
-        cv[k] = reinterpret_cast<const R2*>(a.xc)[(int64_t)cz * a.gc.nnx + cx];
-    }
-  }
-  // x + P x_c on the free dofs of fine node (ix, iz) (the arithmetic of k_prolong_add)
-  auto corrected = [&](int ix, int iz, R2 x, uchar2 ff) -> R2 {
-    double s0, s1;
-    prolong_taps(ix, iz, [&](int jz, int jx) { return scx[(jz - cz0) * CLX + (jx - cx0)]; }, &s0, &s1);
-    if (!ff.x) x.x += (R)s0;
-    if (!ff.y) x.y += (R)s1;
-    return x;
-  };
   // ---- stage velocity (masked; one vector load per node), pressure ----
   // A fixed number of nodes per thread, all loads issued before any shared-memory store, so the
   // staging costs one memory round trip rather than one per node.
@@ -977,12 +893,6 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
   uchar2 sf[NST];
   R spv[NSP];
   if constexpr (sizeof(R) == 8) {                    // FP64: one node at a time (fewer live registers)
-    if constexpr (PRO) {
-#pragma unroll
-      for (int k = 0; k < NCT; ++k)
-        if (tid + k * APPLY_THREADS < CLZ * CLX) scx[tid + k * APPLY_THREADS] = cv[k];
-      __syncthreads();
-    }
     for (int i = tid; i < LZ * LX; i += APPLY_THREADS) {
       const int lz = i / LX, lx = i - lz * LX;
       const int ix = lx0 + lx, iz = lz0 + lz;
@@ -994,7 +904,6 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
         ff = f2[n];
         if (use_u) {
           R2 uu = u2[n];
-          if constexpr (PRO) uu = corrected(ix, iz, uu, ff);
           v.x = ff.x ? R(0) : uu.x;
           v.y = ff.y ? R(0) : uu.y;
         }
@@ -1035,19 +944,6 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
     const int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
     spv[k] = (use_p && i < PZ * PX && px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz)
                  ? a.p[(int64_t)pz * (g.nx + 1) + px] : R(0);
-  }
-  if constexpr (PRO) {
-#pragma unroll
-    for (int k = 0; k < NCT; ++k)
-      if (tid + k * APPLY_THREADS < CLZ * CLX) scx[tid + k * APPLY_THREADS] = cv[k];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NST; ++k) {
-      const int i = tid + k * APPLY_THREADS;
-      const int lz = i / LX, lx = i - lz * LX;
-      const int ix = lx0 + lx, iz = lz0 + lz;
-      if (i < LZ * LX && ix >= 0 && ix < g.nnx && iz >= 0 && iz < g.nnz) sv[k] = corrected(ix, iz, sv[k], sf[k]);
-    }
   }
 #pragma unroll
   for (int k = 0; k < NST; ++k) {
@@ -1121,8 +1017,8 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
     if (CHEB) dg = pre ? pre_at(1, slot) : reinterpret_cast<const R2*>(a.diag)[n];
     else if (fixed) dg = reinterpret_cast<const R2*>(a.diag)[n];
     if (fixed && MODE != AM_CHEB_Z) {                // the fixed components' values (staged as 0);
-      const R2 raw = reinterpret_cast<const R2*>(a.u)[n];   // a free one keeps its staged value,
-      if (ff.x) uu.x = raw.x;                        // which under AM_CHEB_P carries P x_c
+      const R2 raw = reinterpret_cast<const R2*>(a.u)[n];   // a free one keeps its staged value
+      if (ff.x) uu.x = raw.x;
       if (ff.y) uu.y = raw.y;
     }
     if (MODE != AM_APPLY) bb = pre ? pre_at(0, slot) : reinterpret_cast<const R2*>(a.bV)[n];
@@ -1261,9 +1157,10 @@ k_apply(LevelGeo g, ApplyArgs<R> a) {
   }
 }
 
-// diag(K): sum over incident elements of the element diagonal, ascending element order.
+// diag(K): sum over incident elements of the element diagonal, ascending element order; and its
+// rounded reciprocal (dinv may be null).
 template <typename R>
-__global__ void k_diag(LevelGeo g, const R* __restrict__ eta, R* __restrict__ diag) {
+__global__ void k_diag(LevelGeo g, const R* __restrict__ eta, R* __restrict__ diag, R* __restrict__ dinv) {
   pdl_entry();
   const int64_t nn = (int64_t)g.nnx * g.nnz;
   const double sx = 2.0 / g.hx, sz = 2.0 / g.hz, jac = g.hx * g.hz / 4.0;
@@ -1288,12 +1185,17 @@ __global__ void k_diag(LevelGeo g, const R* __restrict__ eta, R* __restrict__ di
       }
     diag[2 * n] = (R)d0;
     diag[2 * n + 1] = (R)d1;
+    if (dinv) {
+      dinv[2 * n] = R(1) / (R)d0;
+      dinv[2 * n + 1] = R(1) / (R)d1;
+    }
   }
 }
 
 // coarse viscosity: mean of the 36 fine qpoint values of the 2x2 children (element constant)
 template <typename R>
-__global__ void k_coarsen_eta(LevelGeo gf, LevelGeo gc, const R* __restrict__ fine, R* __restrict__ coarse) {
+__global__ void k_coarsen_eta(LevelGeo gf, LevelGeo gc, const R* __restrict__ fine, R* __restrict__ coarse,
+                              R* __restrict__ one) {
   pdl_entry();
   const int64_t nel = (int64_t)gc.nx * gc.nz;
   const int fnx = gf.nx;
@@ -1341,7 +1243,17 @@ __global__ void k_coarsen_eta(LevelGeo gf, LevelGeo gc, const R* __restrict__ fi
     }
     R v = (R)s;
     for (int q = 0; q < 9; ++q) coarse[e * 9 + q] = v;
+    one[e] = v;
   }
+}
+
+// the fine viscosity regrouped by Gauss point, so that a warp's elements read it coalesced
+template <typename R>
+__global__ void k_eta_planes(int64_t nel, const R* __restrict__ eta, R* __restrict__ planes) {
+  pdl_entry();
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nel; e += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) planes[q * nel + e] = eta[e * 9 + q];
 }
 
 // 1D Q2 restriction weights of coarse lattice node J from fine node 2J+o (o in -3..3)
@@ -2046,6 +1958,8 @@ struct Level {
   LevelGeo g;
   int64_t nn, ndof, nel;
   R *eta, *diag, *x, *b, *r, *d, *t;
+  R* dinv;            // 1 / diag, rounded
+  R* etap;            // level 0: the viscosity as nine planes of nel values; below: one value per element
   uint8_t* fix;
   double* cheb;       // 2*MAXDEG coefficients
   int deg;            // Chebyshev steps per smoothing sweep on this level
@@ -2184,7 +2098,9 @@ static void carve(Hierarchy<R>& H, Arena& A, const uint8_t* fine_fix) {
   for (int l = 0; l < H.nlev; ++l) {
     Level<R>& L = H.L[l];
     L.eta = (R*)A.take(sizeof(R) * L.nel * 9);
+    L.etap = (R*)A.take(sizeof(R) * L.nel * (l == 0 ? 9 : 1));
     L.diag = (R*)A.take(sizeof(R) * L.ndof);
+    L.dinv = (R*)A.take(sizeof(R) * L.ndof);
     L.x = (R*)A.take(sizeof(R) * L.ndof);
     L.b = (R*)A.take(sizeof(R) * L.ndof);
     L.r = (R*)A.take(sizeof(R) * L.ndof);
@@ -2665,20 +2581,6 @@ static void launch_tail(Hierarchy<R>& H, int l0, bool first_done, cudaStream_t s
   tail_swaps(H, l0, first_done);
 }
 
-// The prolongation runs as its own launch (k_prolong_add) before the post-smoothing by default;
-// MW_FUSED_PROLONG=1 in the environment (read at the first V-cycle) folds it into the first
-// smoothing step (AM_CHEB_P) instead: the same arithmetic and results, one launch fewer per level
-// and V-cycle, but the heavier smoothing kernel made the 512x512 FK step slower (26.50 against
-// 26.15 ms; on the levels of at most 128^2 or 256^2 elements only: 24.84 / 24.86 against 24.76 ms,
-// measured).
-static bool fused_prolongation() {
-  static const bool on = [] {
-    const char* e = getenv("MW_FUSED_PROLONG");
-    return e && e[0] == '1';
-  }();
-  return on;
-}
-
 template <typename R>
 static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = false) {
   Level<R>& L = H.L[l];
@@ -2696,12 +2598,31 @@ static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = fal
     return;
   }
   Level<R>& C = H.L[l + 1];
+  const bool nested = nested_levels(L.g, C.g);
+  if (L.deg <= MG_MAXDEG) {                        // each half of the level's cycle in one launch
+    MgArgs<R> a;
+    memset(&a, 0, sizeof(a));
+    a.g = L.g; a.gc = C.g; a.eta = L.etap; a.fix = L.fix; a.diag = L.diag; a.dinv = L.dinv; a.b = L.b;
+    a.cheb = L.cheb; a.x = L.t;
+    if (nested) { a.bc = C.b; a.fixc = C.fix; }
+    else a.r = L.r;
+    mg_down<R>(a, L.deg, l == 0, s);
+    if (!nested)
+      pdl_launch(k_restrict_g<R>, grid_for(C.nn, 256), 256, 0, s, L.g, C.g, L.r, C.fix, C.b, (const double*)nullptr,
+                 C.diag, C.x, C.d);
+    vcycle(H, l + 1, s);
+    if (!nested)
+      pdl_launch(k_prolong_g<R>, grid_for(L.nn, 256), 256, 0, s, L.g, C.g, (const R*)C.x, L.fix, L.t);
+    a.xin = L.t; a.x = L.x;
+    a.xc = nested ? C.x : nullptr;
+    mg_up<R>(a, L.deg, l == 0, s);
+    return;
+  }
   smooth(L, L.deg, !first_done, s, first_done);
   ApplyArgs<R> a = args0<R>();
   a.u = L.x; a.eta = L.eta; a.fix = L.fix; a.diag = L.diag; a.yV = L.r; a.bV = L.b;
   launch_apply<R, AM_RESID>(L.g, a, s);
-  const bool fuse = !(l + 1 == H.nlev - 1 && H.dense);
-  const bool nested = nested_levels(L.g, C.g);
+  const bool fuse = !(l + 1 == H.nlev - 1 && H.dense) && C.deg > MG_MAXDEG;
   if (nested)
     pdl_launch(k_restrict<R>, dim3((C.g.nnx + RTX - 1) / RTX, (C.g.nnz + RTZ - 1) / RTZ), RTX * RTZ, 0, s, L.g, C.g,
                L.r, C.fix, C.b, fuse ? C.cheb : nullptr, C.diag,
@@ -2710,32 +2631,12 @@ static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = fal
     pdl_launch(k_restrict_g<R>, grid_for(C.nn, 256), 256, 0, s, L.g, C.g, L.r, C.fix, C.b, fuse ? C.cheb : nullptr,
                C.diag, C.x, C.d);
   vcycle(H, l + 1, s, fuse);
-  if (!fused_prolongation() || !nested) {          // x += P x_c as its own launch, then the smoothing
-    if (nested)
-      pdl_launch(k_prolong_add<R>, dim3((L.g.nnx + PTX - 1) / PTX, (L.g.nnz + PTZ - 1) / PTZ), PTX * PTZ, 0, s, L.g,
-                 C.g, (const R*)C.x, L.fix, L.x);
-    else
-      pdl_launch(k_prolong_g<R>, grid_for(L.nn, 256), 256, 0, s, L.g, C.g, (const R*)C.x, L.fix, L.x);
-    smooth(L, L.deg, false, s);
-    return;
-  }
-  // x += P x_c folded into the first post-smoothing step (AM_CHEB_P: the restart step, which reads
-  // the corrected x only through its staging), then the remaining steps
-  {
-    ApplyArgs<R> a = args0<R>();
-    a.u = L.x; a.eta = L.eta; a.fix = L.fix; a.diag = L.diag; a.yV = L.d; a.bV = L.b; a.d = L.d; a.xo = L.t;
-    a.cheb = L.cheb;                    // step-0 pair {0, 1/theta}
-    a.xc = C.x; a.gc = C.g;
-    launch_apply<R, AM_CHEB_P>(L.g, a, s);
-    std::swap(L.x, L.t);
-  }
-  for (int k = 1; k < L.deg; ++k) {
-    ApplyArgs<R> a = args0<R>();
-    a.u = L.x; a.eta = L.eta; a.fix = L.fix; a.diag = L.diag; a.yV = L.d; a.bV = L.b; a.d = L.d; a.xo = L.t;
-    a.cheb = L.cheb + 2 * k;
-    launch_apply<R, AM_CHEB>(L.g, a, s);
-    std::swap(L.x, L.t);
-  }
+  if (nested)                                      // x += P x_c
+    pdl_launch(k_prolong_add<R>, dim3((L.g.nnx + PTX - 1) / PTX, (L.g.nnz + PTZ - 1) / PTZ), PTX * PTZ, 0, s, L.g,
+               C.g, (const R*)C.x, L.fix, L.x);
+  else
+    pdl_launch(k_prolong_g<R>, grid_for(L.nn, 256), 256, 0, s, L.g, C.g, (const R*)C.x, L.fix, L.x);
+  smooth(L, L.deg, false, s);
 }
 
 // Replays the kernels `record` issues on s from a CUDA graph cached under (kind, host state).
@@ -2839,15 +2740,16 @@ __global__ void k_normalize(int64_t n, const double* __restrict__ nrm2, R* __res
 template <typename R>
 static int setup_hierarchy(mw_stokes* S, Hierarchy<R>& H, cudaStream_t s) {
   const mw_stokes_params& prm = S->prm;
+  pdl_launch(k_eta_planes<R>, grid_for(H.L[0].nel, 256), 256, 0, s, H.L[0].nel, H.L[0].eta, H.L[0].etap);
   // coarse viscosities, fixed masks and diagonals of every level (a short chain)
   for (int l = 0; l < H.nlev; ++l) {
     Level<R>& L = H.L[l];
     if (l > 0) {
       Level<R>& F = H.L[l - 1];
-      pdl_launch(k_coarsen_eta<R>, grid_for(L.nel, 256), 256, 0, s, F.g, L.g, F.eta, L.eta);
+      pdl_launch(k_coarsen_eta<R>, grid_for(L.nel, 256), 256, 0, s, F.g, L.g, F.eta, L.eta, L.etap);
       pdl_launch(k_fix_coarse<R>, grid_for(L.nn, 256), 256, 0, s, F.g, L.g, F.fix, L.fix);
     }
-    pdl_launch(k_diag<R>, grid_for(L.nn, 128), 128, 0, s, L.g, L.eta, L.diag);
+    pdl_launch(k_diag<R>, grid_for(L.nn, 128), 128, 0, s, L.g, L.eta, L.diag, L.dinv);
   }
   // the coarsest level's dense inverse occupies one SM for most of a millisecond: it runs on a
   // side branch (forked from and joined back into s by events, which a stream capture records as
@@ -3585,7 +3487,7 @@ int mw_stokes_set_viscosity(mw_stokes* S, const double* etaq, const double* eta_
   if (S->has32) pdl_launch(k_cast<float>, grid_for(nel * 9, 256), 256, 0, s, nel * 9, etaq, S->etaq32);
   pdl_launch(k_inv_eta_e, grid_for(nel, 256), 256, 0, s, nel, etaq, eta_e, S->etae_w);
   pdl_launch(k_diag<double>, grid_for((int64_t)S->fine.nnx * S->fine.nnz, 128), 128, 0, s, S->fine, S->etaq64,
-             S->diag64);
+             S->diag64, (double*)nullptr);
   const int64_t np = (int64_t)(S->fine.nx + 1) * (S->fine.nz + 1);
   pdl_launch(k_mass_diag, grid_for(np, 256), 256, 0, s, S->fine, nullptr, S->mdiag);      // M
   pdl_launch(k_mass_diag, grid_for(np, 256), 256, 0, s, S->fine, S->etae_w, S->medi);     // M_eta
