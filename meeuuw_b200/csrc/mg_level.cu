@@ -24,82 +24,11 @@
 // The arithmetic -- element products, node sums over the incident elements in ascending order,
 // smoothing steps, transfer taps -- is that of the kernels of stokes.cu in the same order, so the
 // results equal a cycle of separate launches.
-#include "mg_level.cuh"
-#include "q2_ref.cuh"
+#include "cell_ops.cuh"
 
 namespace mw {
 
 namespace {
-
-// FP64 basis values come from the constant bank (an FP64 immediate costs registers and moves)
-__constant__ RefTables c_k;
-
-template <typename R, int Q, int K> MW_D R kdr() {
-  if constexpr (sizeof(R) == 4) return (float)RefD<Q, K>::r; else return c_k.dr[Q * 9 + K];
-}
-template <typename R, int Q, int K> MW_D R kdt() {
-  if constexpr (sizeof(R) == 4) return (float)RefD<Q, K>::t; else return c_k.dt[Q * 9 + K];
-}
-
-template <typename R, int Q> MW_D R kwq() {
-  constexpr double w = ref_wq(Q);
-  if constexpr (sizeof(R) == 4) return (float)w; else return c_k.wq[Q];
-}
-
-constexpr int CELLS = 16;                                   // cells of a tile, per side
-
-MW_D float2 fma2(float s, float2 a, float2 c) { return __ffma2_rn(make_float2(s, s), a, c); }
-MW_D double2 fma2(double s, double2 a, double2 c) { return make_double2(fma(s, a.x, c.x), fma(s, a.y, c.y)); }
-MW_D float2 pair(float a, float b) { return make_float2(a, b); }
-MW_D double2 pair(double a, double b) { return make_double2(a, b); }
-
-// K_el u on one element: the strain rate at each Gauss point, the stress, B^T back onto the nodes
-// (element_apply of stokes.cu without the pressure terms).
-template <typename R, typename R2>
-MW_D void k_element(R sx, R sz, R jac, const R2 (&u)[9], const R (&eq)[9], R2 (&y)[9]) {
-#pragma unroll
-  for (int k = 0; k < 9; ++k) y[k] = pair(R(0), R(0));
-  static_for<9>([&](auto qc) {
-    constexpr int Q = qc.value;
-    R2 gx = pair(R(0), R(0)), gz = pair(R(0), R(0));
-    static_for<9>([&](auto kc) {
-      constexpr int K = kc.value;
-      if constexpr (RefD<Q, K>::r != 0.0) gx = fma2(kdr<R, Q, K>(), u[K], gx);
-      if constexpr (RefD<Q, K>::t != 0.0) gz = fma2(kdt<R, Q, K>(), u[K], gz);
-    });
-    const R exx = sx * gx.x, ezz = sz * gz.y;
-    const R gg = sizeof(R) == 4 ? fma(sx, gx.y, sz * gz.x) : fma(sz, gz.x, sx * gx.y);
-    const R jw = jac * kwq<R, Q>();
-    const R e = eq[Q] * jw;
-    const R2 ar = pair((R(2) * e * exx) * sx, e * gg * sx);
-    const R2 at = pair(e * gg * sz, (R(2) * e * ezz) * sz);
-    static_for<9>([&](auto kc) {
-      constexpr int K = kc.value;
-      if constexpr (RefD<Q, K>::r != 0.0) y[K] = fma2(kdr<R, Q, K>(), ar, y[K]);
-      if constexpr (RefD<Q, K>::t != 0.0) y[K] = fma2(kdt<R, Q, K>(), at, y[K]);
-    });
-  });
-}
-
-// a / d from the rounded reciprocal y = 1 / d, correctly rounded as the division is: q = a y is
-// within two units, a first correction by the exact residual a - d q makes it faithful, and the
-// second rounds it correctly (Markstein, IBM J. Res. Dev. 34, 1990: a faithful quotient corrected
-// with a correctly rounded reciprocal).  Five packed multiply-adds for a node's two components in
-// place of two divisions.
-MW_D float2 div2(float2 a, float2 d, float2 y) {
-  const float2 nd = make_float2(-d.x, -d.y);
-  float2 q = __fmul2_rn(a, y);
-  float2 r = __ffma2_rn(nd, q, a);
-  q = __ffma2_rn(r, y, q);
-  r = __ffma2_rn(nd, q, a);
-  return __ffma2_rn(r, y, q);
-}
-MW_D double div1(double a, double d, double y) {
-  double q = a * y;
-  q = fma(fma(-d, q, a), y, q);
-  return fma(fma(-d, q, a), y, q);
-}
-MW_D double2 div2(double2 a, double2 d, double2 y) { return make_double2(div1(a.x, d.x, y.x), div1(a.y, d.y, y.y)); }
 
 // the restriction taps along one direction for a coarse node of parity P: fine offsets and weights
 template <int P> struct RTap;
@@ -351,15 +280,7 @@ void by_degree(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
 
 }  // namespace
 
-int mg_ensure_tables() {
-  static bool ready = false;
-  if (ready) return MW_OK;
-  RefTables t;
-  host_ref_tables(&t);
-  if (cudaMemcpyToSymbol(c_k, &t, sizeof(t)) != cudaSuccess) return MW_ERR_CUDA;
-  ready = true;
-  return MW_OK;
-}
+int mg_ensure_tables() { return ensure_cell_tables(); }
 
 template <typename R> void mg_down(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
   by_degree<R, true>(a, deg, planes, s);

@@ -1,0 +1,138 @@
+// The matrix-free Stokes operator y = [K G; G^T 0] (u, p) on a level, and residuals of it (sm_100a).
+//
+// A CTA takes a tile of 16 x 16 cells and owns 14 x 14 of them: one halo cell on the left and below for
+// the neighbours' sums, one on the right and above for their nodes.  Each thread loads its cell's four
+// nodes, hands the shared ones to its neighbours through shared memory, computes one element product and
+// exchanges the sums for shared nodes the same way; its own four nodes never leave its registers.  The
+// element-tile form this replaces staged the velocity and every element's 22 results in shared memory and
+// looked its indices up per node: 1065 warp instructions an element, of which 370 were the product.
+//
+// Measured, (u, p) -> (K u + G p, G^T u), before and now: FP32 512^2 16.5 -> 15.9 us, 128^2 5.0 -> 3.5, 8^2
+// 4.6 -> 3.4; FP64 512^2 40.8 -> 31, 256^2 13.8 -> 10.8.  At 512^2 the packed multiply-adds alone take 5.9 us
+// (they issue at half rate); the rest is the load and exchange latency that two tiles an SM leave open.
+#include "cell_ops.cuh"
+#include "op_apply.cuh"
+
+namespace mw {
+
+namespace {
+
+// Resident CTAs: two, or three where 80 registers do without spills (FP32 without pressure).  FP64
+// with two (128 registers, 156 bytes spilled with pressure) takes 31 us at 512^2 against 36 with one.
+template <typename R, bool PRESSURE>
+__global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3 : 2) k_op_apply(OpArgs<R> a) {
+  pdl_entry();
+  typedef typename Vec2<R>::T R2;
+  constexpr int CX = CELLS, NC = CELLS * CELLS, T = CELLS - 2;
+  __shared__ __align__(16) R2 sx[4 * NC];
+  __shared__ __align__(16) R2 se[5 * NC];
+  __shared__ R sp[PRESSURE ? 4 * NC : 1];
+  const int tid = threadIdx.x, lx = tid % CX, lz = tid / CX;
+  const int ex0 = blockIdx.x * T, ez0 = blockIdx.y * T;
+  const int ex = ex0 + lx - 1, ez = ez0 + lz - 1;
+  const LevelGeo& g = a.g;
+  const bool cx0 = ex >= 0 && ex <= g.nx, cx1 = ex >= 0 && ex < g.nx;
+  const bool cz0 = ez >= 0 && ez <= g.nz, cz1 = ez >= 0 && ez < g.nz;
+  const bool has[4] = {cx0 && cz0, cx1 && cz0, cx0 && cz1, cx1 && cz1};
+  const int64_t n0 = (int64_t)(2 * ez) * g.nnx + 2 * ex;
+  const int64_t np = (int64_t)ez * (g.nx + 1) + ex;
+  const R2 zero = pair(R(0), R(0));
+  const bool elem = has[3] && lx < CX - 1 && lz < CELLS - 1;
+  R2 x[4];
+  unsigned fx = 0;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    x[t] = zero;
+    if (has[t]) {
+      const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
+      if (a.u) x[t] = reinterpret_cast<const R2*>(a.u)[n];
+      const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n];
+      fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
+    }
+  }
+  R p0 = R(0);
+  if (PRESSURE && a.p && has[0]) p0 = a.p[np];
+  R eq[9];
+  if (elem) {
+    const R* e = a.eta + ((int64_t)ez * g.nx + ex) * a.es;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) eq[q] = e[q * a.qs];
+  }
+  R2 u[9], y[9];
+  R yp[4] = {R(0), R(0), R(0), R(0)};
+  auto masked = [&](int t) {
+    return pair((fx & (1u << (2 * t))) ? R(0) : x[t].x, (fx & (2u << (2 * t))) ? R(0) : x[t].y);
+  };
+  u[0] = masked(0); u[4] = masked(1); u[7] = masked(2); u[8] = masked(3);
+  sx[tid] = u[0]; sx[NC + tid] = u[4]; sx[2 * NC + tid] = u[7]; sx[3 * NC + tid] = u[8];
+  if (PRESSURE) sp[tid] = p0;
+  __syncthreads();
+  if (elem) {
+    u[1] = sx[tid + 1];
+    u[5] = sx[2 * NC + tid + 1];
+    u[3] = sx[tid + CX];
+    u[6] = sx[NC + tid + CX];
+    u[2] = sx[tid + CX + 1];
+    const R sxe = R(2.0 / g.hx), sze = R(2.0 / g.hz), jace = R(g.hx * g.hz / 4.0);
+    if constexpr (PRESSURE) {
+      const R pe[4] = {p0, sp[tid + 1], sp[tid + CX + 1], sp[tid + CX]};
+      k_element<true>(sxe, sze, jace, u, eq, y, R(g.s), pe, yp);
+    } else {
+      k_element(sxe, sze, jace, u, eq, y);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) y[k] = zero;
+  }
+  se[tid] = y[1]; se[NC + tid] = y[5]; se[2 * NC + tid] = y[3]; se[3 * NC + tid] = y[6]; se[4 * NC + tid] = y[2];
+  if (PRESSURE) { sp[NC + tid] = yp[1]; sp[2 * NC + tid] = yp[3]; sp[3 * NC + tid] = yp[2]; }
+  __syncthreads();
+  const int ownx = ex0 + T >= g.nx ? T + 1 : T, ownz = ez0 + T >= g.nz ? T + 1 : T;
+  if (lx < 1 || lx > ownx || lz < 1 || lz > ownz || !has[0]) return;
+  if (a.yV) {
+    // ascending element order: lower left, lower, left, own
+    const R2 p2 = se[4 * NC + tid - CX - 1], p3 = se[2 * NC + tid - CX], p1 = se[tid - 1],
+             p6 = se[3 * NC + tid - CX], p5 = se[NC + tid - 1];
+    R2 s[4];
+    s[0] = pair(((p2.x + p3.x) + p1.x) + y[0].x, ((p2.y + p3.y) + p1.y) + y[0].y);
+    s[1] = pair(p6.x + y[4].x, p6.y + y[4].y);
+    s[2] = pair(p5.x + y[7].x, p5.y + y[7].y);
+    s[3] = y[8];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (has[t]) {
+        const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
+        const unsigned f = (fx >> (2 * t)) & 3u;
+        if (f) {                                            // eliminated rows act as K_ii u_i
+          const R2 dg = a.u ? reinterpret_cast<const R2*>(a.diag)[n] : zero;
+          if (f & 1u) s[t].x = dg.x * x[t].x;
+          if (f & 2u) s[t].y = dg.y * x[t].y;
+        }
+        if (a.bV) {
+          const R2 b = reinterpret_cast<const R2*>(a.bV)[n];
+          s[t] = pair(b.x - s[t].x, b.y - s[t].y);
+        }
+        reinterpret_cast<R2*>(a.yV)[n] = s[t];
+      }
+  }
+  if (PRESSURE && a.yP) {                                   // the elements lower left, lower, left, own
+    const R v = ((sp[3 * NC + tid - CX - 1] + sp[2 * NC + tid - CX]) + sp[NC + tid - 1]) + yp[0];
+    a.yP[np] = a.bP ? a.bP[np] - v : v;
+  }
+}
+
+}  // namespace
+
+int op_ensure_tables() { return ensure_cell_tables(); }
+
+template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s) {
+  constexpr int T = CELLS - 2;
+  const dim3 grid((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
+  if (a.p || a.yP) pdl_launch(k_op_apply<R, true>, grid, CELLS * CELLS, 0, s, a);
+  else pdl_launch(k_op_apply<R, false>, grid, CELLS * CELLS, 0, s, a);
+}
+
+template void op_apply<float>(const OpArgs<float>&, cudaStream_t);
+template void op_apply<double>(const OpArgs<double>&, cudaStream_t);
+
+}  // namespace mw

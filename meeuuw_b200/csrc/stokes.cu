@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "mg_level.cuh"
+#include "op_apply.cuh"
 #include "q2_ref.cuh"
 
 namespace mw {
@@ -53,7 +54,8 @@ static int ensure_ref_tables() {
   if (g_ref_ready) return MW_OK;
   RefTables T;
   host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables()) return MW_ERR_CUDA;
+  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || op_ensure_tables())
+    return MW_ERR_CUDA;
   g_ref_ready = true;
   return MW_OK;
 }
@@ -2180,11 +2182,31 @@ static void div_u(mw_stokes* S, const double* u, double* y, cudaStream_t s) {
   pdl_launch(k_div_u, grid, 128, 0, s, g, u, S->fixV, y);
 }
 
+// y = K x on level l
 template <typename R>
-static void k_only_apply(const Level<R>& L, const R* x, R* y, cudaStream_t s) {
-  ApplyArgs<R> a = args0<R>();
-  a.u = x; a.eta = L.eta; a.fix = L.fix; a.diag = L.diag; a.yV = y;
-  launch_apply<R, AM_APPLY>(L.g, a, s);
+static OpArgs<R> op_args(const Level<R>& L, bool planes) {
+  OpArgs<R> a;
+  memset(&a, 0, sizeof(a));
+  a.g = L.g; a.eta = L.etap; a.fix = L.fix; a.diag = L.diag;
+  a.qs = planes ? L.nel : 0;                        // level 0: nine planes; below: one value per element
+  a.es = 1;
+  return a;
+}
+
+template <typename R>
+static void level_apply(const Level<R>& L, bool planes, const R* x, R* y, cudaStream_t s) {
+  OpArgs<R> a = op_args(L, planes);
+  a.u = x; a.yV = y;
+  op_apply<R>(a, s);
+}
+
+// the FP64 operator on the fine mesh (the caller's viscosity, element by element)
+static OpArgs<double> op_args64(const mw_stokes* S) {
+  OpArgs<double> a;
+  memset(&a, 0, sizeof(a));
+  a.g = S->fine; a.eta = S->etaq64; a.fix = S->fixV; a.diag = S->diag64;
+  a.qs = 1; a.es = 9;
+  return a;
 }
 
 // ---------------------------------------------------------------- coarse levels in one cluster
@@ -2810,7 +2832,7 @@ static int setup_hierarchy(mw_stokes* S, Hierarchy<R>& H, cudaStream_t s) {
     for (int it = 0; it < iters; ++it) {
       dot<R>(S, L.ndof, v, v, L.lam2 + 1, s);
       pdl_launch(k_normalize<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, L.lam2 + 1, v);
-      k_only_apply<R>(L, v, L.d, s);
+      level_apply<R>(L, l == 0, v, L.d, s);
       pdl_launch(k_dinv<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, L.d, L.diag, v);
     }
     dot<R>(S, L.ndof, v, v, L.lam2, s);          // ||D^-1 K v_prev||^2 with ||v_prev|| = 1
@@ -2865,7 +2887,7 @@ static int pcg_K(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double*
   int it = 0;
   double rr = bb;
   for (it = 1; it <= maxit; ++it) {
-    k_only_apply<R>(L, p, Ap, s);
+    level_apply<R>(L, true, p, Ap, s);
     dot<R>(S, n, p, Ap, sc + 1, s);
     pdl_launch(k_pcg_update_rr<R>, nb_for(n), 256, 0, s, n, sc + 0, sc + 1, p, Ap, xr, r, S->red, S->counter, sc + 2);
     rr = read_scalar(sc + 2, s);
@@ -2930,11 +2952,9 @@ static void remove_mean(mw_stokes* S, int64_t n, double* x, cudaStream_t s) {
 static double true_residual(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
                             double bnorm, cudaStream_t s) {
   const LevelGeo& g = S->fine;
-  ApplyArgs<double> a = args0<double>();
-  a.u = V; a.p = P; a.eta = S->etaq64; a.fix = S->fixV;
-  a.diag = S->diag64;
-  a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
-  launch_apply<double, AM_RESID>(g, a, s);
+  OpArgs<double> a = op_args64(S);
+  a.u = V; a.p = P; a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
+  op_apply<double>(a, s);
   const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
   dot<double>(S, nv, S->RV, S->RV, S->sc + 50, s);
   dot<double>(S, np, S->RP, S->RP, S->sc + 51, s);
@@ -3226,7 +3246,7 @@ static bool pcg_K_dev(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, do
   pdl_launch(k_dev_pcg_init, 1, 1, 0, s, sc, hw);
   if (!cond_node(s, b1, cudaGraphCondTypeWhile, hw)) return false;
   // body: one CG step and the convergence test, then (if continuing) the next search direction
-  k_only_apply<R>(L, p, Ap, b1);
+  level_apply<R>(L, true, p, Ap, b1);
   dot<R>(S, n, p, Ap, sc + P_PAP, b1);
   pdl_launch(k_pcg_update_rr<R>, nb_for(n), 256, 0, b1, n, sc + P_RZ, sc + P_PAP, p, Ap, xr, r, S->red, S->counter,
              sc + P_RR);
@@ -3253,11 +3273,9 @@ static bool solve_K_dev(mw_stokes* S, int prec, const double* b, double* x, doub
 static void true_residual_dev(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
                               cudaStream_t s) {
   const LevelGeo& g = S->fine;
-  ApplyArgs<double> a = args0<double>();
-  a.u = V; a.p = P; a.eta = S->etaq64; a.fix = S->fixV;
-  a.diag = S->diag64;
-  a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
-  launch_apply<double, AM_RESID>(g, a, s);
+  OpArgs<double> a = op_args64(S);
+  a.u = V; a.p = P; a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
+  op_apply<double>(a, s);
   const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
   dot<double>(S, nv, S->RV, S->RV, S->sc + T_RV, s);
   dot<double>(S, np, S->RP, S->RP, S->sc + T_RP, s);
@@ -3503,9 +3521,9 @@ static bool pair_aligned(const void* p, size_t pair_bytes) { return ((uintptr_t)
 
 int mw_stokes_apply(mw_stokes* S, const double* u, const double* p, double* yV, double* yP, void* stream) {
   if (!pair_aligned(u, 16) || !pair_aligned(yV, 16)) return MW_ERR_BAD_ARG;
-  ApplyArgs<double> a = args0<double>();
-  a.u = u; a.p = p; a.eta = S->etaq64; a.fix = S->fixV; a.diag = S->diag64; a.yV = yV; a.yP = yP;
-  launch_apply<double, AM_APPLY>(S->fine, a, (cudaStream_t)stream);
+  OpArgs<double> a = op_args64(S);
+  a.u = u; a.p = p; a.yV = yV; a.yP = yP;
+  op_apply<double>(a, (cudaStream_t)stream);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
@@ -3527,9 +3545,9 @@ int mw_stokes_div(mw_stokes* S, const double* u, double* yP, void* stream) {
 int mw_stokes_apply_f32(mw_stokes* S, const float* u, const float* p, float* yV, float* yP, void* stream) {
   if (!S->has32 || !pair_aligned(u, 8) || !pair_aligned(yV, 8)) return MW_ERR_BAD_ARG;
   if (ensure_hierarchy(S, MW_F32, (cudaStream_t)stream)) return MW_ERR_CUDA;
-  ApplyArgs<float> a = args0<float>();
-  a.u = u; a.p = p; a.eta = S->etaq32; a.fix = S->fixV; a.diag = S->H32.L[0].diag; a.yV = yV; a.yP = yP;
-  launch_apply<float, AM_APPLY>(S->fine, a, (cudaStream_t)stream);
+  OpArgs<float> a = op_args(S->H32.L[0], true);
+  a.u = u; a.p = p; a.yV = yV; a.yP = yP;
+  op_apply<float>(a, (cudaStream_t)stream);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
