@@ -256,11 +256,16 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
   }
   if constexpr (!DOWN) {
     const int ownx = ex0 + TX >= g.nx ? TX + 1 : TX, ownz = ez0 + TZ >= g.nz ? TZ + 1 : TZ;
+    double v = 0;
     if (lx >= LO && lx < LO + ownx && lz >= LO && lz < LO + ownz) {
 #pragma unroll
       for (int t = 0; t < 4; ++t)
-        if (has[t]) reinterpret_cast<R2*>(a.x)[n0 + (t >> 1) * g.nnx + (t & 1)] = x[t];
+        if (has[t]) {
+          reinterpret_cast<R2*>(a.x)[n0 + (t >> 1) * g.nnx + (t & 1)] = x[t];
+          if (a.bx.part) v += (double)b[t].x * (double)x[t].x + (double)b[t].y * (double)x[t].y;
+        }
     }
+    if (a.bx.part) grid_sum_parity(v, a.bx, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
   }
 }
 

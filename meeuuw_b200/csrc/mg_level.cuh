@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "reduce.cuh"
 
 namespace mw {
 
@@ -37,6 +38,7 @@ struct MgArgs {
   const uint8_t* fixc;
   R* r;
   const R* xc;         // upward: the coarse correction to prolong; null: xin already carries it
+  ParitySum bx;        // upward: (b, x) of the result (part null: not wanted)
 };
 
 // The FP64 kernels' basis tables in the constant bank; called before the first level launch.

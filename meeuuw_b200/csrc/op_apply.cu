@@ -19,8 +19,9 @@ namespace {
 
 // Resident CTAs: two, or three where 80 registers do without spills (FP32 without pressure).  FP64
 // with two (128 registers, 156 bytes spilled with pressure) takes 31 us at 512^2 against 36 with one.
-template <typename R, bool PRESSURE>
-__global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3 : 2) k_op_apply(OpArgs<R> a) {
+template <typename R, bool PRESSURE, bool PCG>
+__global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3 : 2) k_op_apply(OpArgs<R> a,
+                                                                                                 PcgDir<R> dir) {
   pdl_entry();
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, NC = CELLS * CELLS, T = CELLS - 2;
@@ -40,12 +41,30 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
   const bool elem = has[3] && lx < CX - 1 && lz < CELLS - 1;
   R2 x[4];
   unsigned fx = 0;
+  const R* pold = nullptr;
+  double beta = 0.0;
+  int k = 0;
+  if (PCG) {
+    k = (int)*dir.it;
+    if (k > 0) {
+      beta = dir.rz[k & 1] / dir.rz[(k & 1) ^ 1];
+      pold = (k & 1) ? dir.pbuf[0] : dir.pbuf[1];
+    }
+  }
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     x[t] = zero;
     if (has[t]) {
       const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
-      if (a.u) x[t] = reinterpret_cast<const R2*>(a.u)[n];
+      if (PCG) {
+        x[t] = reinterpret_cast<const R2*>(dir.z)[n];
+        if (pold) {
+          const R2 q = reinterpret_cast<const R2*>(pold)[n];
+          x[t] = pair((R)((double)x[t].x + beta * (double)q.x), (R)((double)x[t].y + beta * (double)q.y));
+        }
+      } else if (a.u) {
+        x[t] = reinterpret_cast<const R2*>(a.u)[n];
+      }
       const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n];
       fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
     }
@@ -88,8 +107,10 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
   if (PRESSURE) { sp[NC + tid] = yp[1]; sp[2 * NC + tid] = yp[3]; sp[3 * NC + tid] = yp[2]; }
   __syncthreads();
   const int ownx = ex0 + T >= g.nx ? T + 1 : T, ownz = ez0 + T >= g.nz ? T + 1 : T;
-  if (lx < 1 || lx > ownx || lz < 1 || lz > ownz || !has[0]) return;
-  if (a.yV) {
+  const bool own = lx >= 1 && lx <= ownx && lz >= 1 && lz <= ownz && has[0];
+  if (!PCG && !own) return;
+  double v = 0;
+  if (own && (PCG || a.yV)) {
     // ascending element order: lower left, lower, left, own
     const R2 p2 = se[4 * NC + tid - CX - 1], p3 = se[2 * NC + tid - CX], p1 = se[tid - 1],
              p6 = se[3 * NC + tid - CX], p5 = se[NC + tid - 1];
@@ -104,16 +125,24 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
         const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
         const unsigned f = (fx >> (2 * t)) & 3u;
         if (f) {                                            // eliminated rows act as K_ii u_i
-          const R2 dg = a.u ? reinterpret_cast<const R2*>(a.diag)[n] : zero;
+          const R2 dg = PCG || a.u ? reinterpret_cast<const R2*>(a.diag)[n] : zero;
           if (f & 1u) s[t].x = dg.x * x[t].x;
           if (f & 2u) s[t].y = dg.y * x[t].y;
         }
-        if (a.bV) {
+        if (PCG) {
+          reinterpret_cast<R2*>((k & 1) ? dir.pbuf[1] : dir.pbuf[0])[n] = x[t];
+          v += (double)x[t].x * (double)s[t].x + (double)x[t].y * (double)s[t].y;
+        } else if (a.bV) {
           const R2 b = reinterpret_cast<const R2*>(a.bV)[n];
           s[t] = pair(b.x - s[t].x, b.y - s[t].y);
         }
         reinterpret_cast<R2*>(a.yV)[n] = s[t];
       }
+  }
+  if constexpr (PCG) {
+    double sum;
+    if (grid_sum(v, dir.part, dir.counter, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, &sum))
+      *dir.pap = sum;
   }
   if (PRESSURE && a.yP) {                                   // the elements lower left, lower, left, own
     const R v = ((sp[3 * NC + tid - CX - 1] + sp[2 * NC + tid - CX]) + sp[NC + tid - 1]) + yp[0];
@@ -125,14 +154,28 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
 
 int op_ensure_tables() { return ensure_cell_tables(); }
 
-template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s) {
+template <typename R> static dim3 tiles(const OpArgs<R>& a) {
   constexpr int T = CELLS - 2;
-  const dim3 grid((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
-  if (a.p || a.yP) pdl_launch(k_op_apply<R, true>, grid, CELLS * CELLS, 0, s, a);
-  else pdl_launch(k_op_apply<R, false>, grid, CELLS * CELLS, 0, s, a);
+  return dim3((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
+}
+
+int cell_partials(int nx, int nz) {
+  constexpr int T = CELLS - 2 * MG_MAXDEG;           // the smallest tile among the launches that sum
+  return ((nx + T - 1) / T) * ((nz + T - 1) / T);
+}
+
+template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s) {
+  if (a.p || a.yP) pdl_launch(k_op_apply<R, true, false>, tiles(a), CELLS * CELLS, 0, s, a, PcgDir<R>());
+  else pdl_launch(k_op_apply<R, false, false>, tiles(a), CELLS * CELLS, 0, s, a, PcgDir<R>());
+}
+
+template <typename R> void op_pcg_direction(const OpArgs<R>& a, const PcgDir<R>& d, cudaStream_t s) {
+  pdl_launch(k_op_apply<R, false, true>, tiles(a), CELLS * CELLS, 0, s, a, d);
 }
 
 template void op_apply<float>(const OpArgs<float>&, cudaStream_t);
 template void op_apply<double>(const OpArgs<double>&, cudaStream_t);
+template void op_pcg_direction<float>(const OpArgs<float>&, const PcgDir<float>&, cudaStream_t);
+template void op_pcg_direction<double>(const OpArgs<double>&, const PcgDir<double>&, cudaStream_t);
 
 }  // namespace mw

@@ -19,7 +19,23 @@ struct OpArgs {
   const R *bV, *bP;
 };
 
+// One conjugate-gradient direction and its operator product: p = z + beta p, Ap = K p, (p, Ap).
+// p lives in pbuf[iteration & 1], so that a tile's halo can read the old direction while others
+// write the new one; rz holds (r, z) by the same parity, beta = rz[k] / rz[k - 1].
+template <typename R>
+struct PcgDir {
+  const R* z;
+  R* pbuf[2];
+  const double* rz;
+  const double* it;    // the iteration, 0 for the first (p = z)
+  double *part, *pap;  // partial sums, (p, Ap)
+  unsigned* counter;
+};
+
 int op_ensure_tables();
 template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s);
+template <typename R> void op_pcg_direction(const OpArgs<R>& a, const PcgDir<R>& d, cudaStream_t s);
+// the partial sums the level and direction launches of a level of nx x nz elements need
+int cell_partials(int nx, int nz);
 
 }  // namespace mw

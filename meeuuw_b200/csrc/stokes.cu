@@ -1518,6 +1518,29 @@ __global__ void k_fix_coarse(LevelGeo gf, LevelGeo gc, const uint8_t* __restrict
   }
 }
 
+// ---------------------------------------------------------------- scalars of the solver loops
+// Schur-residual reduction of a refinement sweep that starts at relative residual `rel`: the fixed
+// sweep_reduction, or with target > 0 the smaller reduction target * tol / rel (at most 0.5).
+MW_HD double sweep_target_reduction(double sweep_reduction, double target, double tol, double rel) {
+  if (!(target > 0) || !(rel > 0)) return sweep_reduction;
+  double r = target * tol / rel;
+  if (r > 0.5) r = 0.5;
+  return r > sweep_reduction ? r : sweep_reduction;
+}
+
+enum DevSlot {
+  P_PAP = 64, P_RR, P_BB, P_IT, P_RZ2,                       // inner PCG; (r, z) by iteration parity at
+                                                              // P_RZ2, P_RZ2 + 1
+  U_RW = 72, U_DSD, U_RWN, U_RR0, U_RR, U_IT, U_D2, U_Z2,    // Schur CG
+  T_RV = 84, T_RP, T_REL,                                     // true residual
+  S_BB = 88, S_BH, S_BNORM, S_REL0, S_NREF, S_RED,           // solve
+  I_OUTER = 96, I_INNER, I_STATUS                             // info
+};
+
+// Work caps of one solve on top of the per-loop caps: a stagnating solve ends with status 3 after
+// this many inner (multigrid-PCG) or outer (Schur) iterations in total.
+constexpr double DEV_INNER_BUDGET = 40000, DEV_OUTER_BUDGET = 4000;
+
 // ---------------------------------------------------------------- BLAS-1 with device scalars
 template <typename R>
 __global__ void k_dot_partial(int64_t n, const R* __restrict__ x, const R* __restrict__ y, double* __restrict__ part) {
@@ -1843,43 +1866,14 @@ __global__ void k_mass_cheb(LevelGeo g, const double* __restrict__ w, const doub
     mass_cheb_node(g, w, b, xin, xout, d, dg, c1, c2, first, Me, n);
 }
 
-// The grid-wide sum of one value per thread, finished in the same launch: block partials in
-// part[block], the last block to arrive adds them in block order into *out and resets the counter
-// (threadfence + arrival counter).  Called once, by every thread, at the end of a kernel.
+// the sum of one value per thread over a one-dimensional grid, into *out
 MW_D void grid_sum_last(double v, double* part, unsigned* counter, double* out) {
-  __shared__ double sh[32];
-  __shared__ bool last;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) {
-      part[blockIdx.x] = v;
-      __threadfence();
-      last = atomicAdd(counter, 1u) == gridDim.x - 1;
-    }
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double t = 0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += ((volatile double*)part)[i];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  if (lane == 0) sh[wid] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[k];
-    out[0] = s;
-    *counter = 0u;
-  }
+  double s;
+  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &s)) out[0] = s;
 }
 
 // Deterministic single-launch dot product: block partials, then the last block to finish sums
-// them in block order (threadfence + arrival counter, reset for the next call).
+// them in block order.
 template <typename R>
 __global__ void k_dot1(int64_t n, const R* __restrict__ x, const R* __restrict__ y, double* __restrict__ part,
                        unsigned* __restrict__ counter, double* __restrict__ out) {
@@ -1890,25 +1884,89 @@ __global__ void k_dot1(int64_t n, const R* __restrict__ x, const R* __restrict__
   grid_sum_last(v, part, counter, out);
 }
 
-// x += (num/den) p ; r -= (num/den) Ap, and (r, r) of the new residual into *rr, summed exactly as
-// k_dot1 sums it on the same grid (one launch for the CG step and its convergence norm)
+// ---- the inner PCG iteration (scalars in S->sc, slots P_*; buffers that change roles by iteration
+// parity): k_pcg_start, then { V-cycle with (r, z), op_pcg_direction with (p, Ap), k_pcg_update } until the
+// update's convergence test fails, then k_pcg_finish.
+
+// r = b, x = 0, (b, b); the loop condition (device loops)
 template <typename R>
-__global__ void k_pcg_update_rr(int64_t n, const double* __restrict__ num, const double* __restrict__ den,
-                                const R* __restrict__ p, const R* __restrict__ Ap, R* __restrict__ x,
-                                R* __restrict__ r, double* __restrict__ part, unsigned* __restrict__ counter,
-                                double* __restrict__ rr) {
+__global__ void k_pcg_start(int64_t n, const double* __restrict__ b, R* __restrict__ r, R* __restrict__ x,
+                            double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
+                            int device_loop, cudaGraphConditionalHandle hw) {
   pdl_entry();
-  const double a = *num / *den;
   double v = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] = (R)((double)x[i] + a * (double)p[i]);
-    const R ri = (R)((double)r[i] - a * (double)Ap[i]);
+    const R ri = (R)b[i];
     r[i] = ri;
+    x[i] = R(0);
     v += (double)ri * (double)ri;
   }
-  grid_sum_last(v, part, counter, rr);
+  double bb;
+  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &bb)) {
+    sc[P_BB] = bb;
+    sc[P_IT] = 0;
+    if (device_loop) cudaGraphSetConditional(hw, (bb > 0 && isfinite(bb)) ? 1u : 0u);
+  }
 }
 
+// x += alpha p, r -= alpha Ap, (r, r), and in the block that finishes the sum the iteration count and
+// -- device loops -- the convergence test: relative tolerance, iteration cap, total work cap
+template <typename R>
+__global__ void k_pcg_update(int64_t n, const R* __restrict__ p0, const R* __restrict__ p1, const R* __restrict__ Ap,
+                             R* __restrict__ x, R* __restrict__ r, double* __restrict__ part,
+                             unsigned* __restrict__ counter, double* __restrict__ sc, double rtol, int maxit,
+                             int device_loop, cudaGraphConditionalHandle hw) {
+  pdl_entry();
+  typedef typename Vec2<R>::T R2;
+  const int k = (int)sc[P_IT] & 1;
+  const double a = sc[P_RZ2 + k] / sc[P_PAP];
+  const R2* p = reinterpret_cast<const R2*>(k ? p1 : p0);
+  const R2* q = reinterpret_cast<const R2*>(Ap);
+  R2* x2 = reinterpret_cast<R2*>(x);
+  R2* r2 = reinterpret_cast<R2*>(r);
+  double v = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n / 2; i += (int64_t)gridDim.x * blockDim.x) {
+    const R2 pi = p[i], qi = q[i];
+    R2 xi = x2[i], ri = r2[i];
+    xi.x = (R)((double)xi.x + a * (double)pi.x);
+    xi.y = (R)((double)xi.y + a * (double)pi.y);
+    ri.x = (R)((double)ri.x - a * (double)qi.x);
+    ri.y = (R)((double)ri.y - a * (double)qi.y);
+    x2[i] = xi;
+    r2[i] = ri;
+    v += (double)ri.x * (double)ri.x + (double)ri.y * (double)ri.y;
+  }
+  double rr;
+  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &rr)) {
+    const double it = sc[P_IT] + 1;
+    sc[P_IT] = it;
+    sc[P_RR] = rr;
+    if (device_loop) {
+      bool go = isfinite(rr) && rr > rtol * rtol * sc[P_BB] && it < (double)maxit;
+      if (go && sc[I_INNER] + it >= DEV_INNER_BUDGET) { sc[I_STATUS] = 3; go = false; }
+      cudaGraphSetConditional(hw, go ? 1u : 0u);
+    }
+  }
+}
+
+// the result in double, and the solve's iteration count
+template <typename R>
+__global__ void k_pcg_finish(int64_t n, const R* __restrict__ xr, double* __restrict__ x, double* __restrict__ sc) {
+  pdl_entry();
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    x[i] = (double)xr[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc[I_INNER] += sc[P_IT];
+}
+
+// (x, y) into the slot of the iteration's parity (hierarchies whose V-cycle does not sum it)
+template <typename R>
+__global__ void k_dot_parity(int64_t n, const R* __restrict__ x, const R* __restrict__ y, ParitySum out) {
+  pdl_entry();
+  double v = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v += (double)x[i] * (double)y[i];
+  grid_sum_parity(v, out, blockIdx.x, gridDim.x);
+}
 
 // element weights 1/eta_e for M_eta (eta_e = mean of the qpoint viscosities of the element)
 __global__ void k_inv_eta_e(int64_t nel, const double* __restrict__ etaq, const double* __restrict__ eta_e,
@@ -2011,7 +2069,7 @@ struct mw_stokes {
   double* red;           // reduction partials
   double* sc;            // device scalars
   unsigned* counter;     // arrival counter of the single-launch dot products
-  // inner PCG vectors (precision of the hierarchy): x, r, z, p, Ap
+  // inner PCG vectors (precision of the hierarchy): x, r, p (two, by iteration parity), Ap
   double *pc64[5];
   float *pc32[5];
   const uint8_t* fixV;   // fine fixed mask (caller's)
@@ -2127,7 +2185,7 @@ static size_t layout(mw_stokes* S, Arena& A) {
                    &S->medi, &S->cP};
   for (auto p : pv) *p = (double*)A.take(sizeof(double) * np);
   S->etae_w = (double*)A.take(sizeof(double) * nel);
-  S->red = (double*)A.take(sizeof(double) * NB * 4);
+  S->red = (double*)A.take(sizeof(double) * std::max(NB * 4, cell_partials(g.nx, g.nz)));
   S->sc = (double*)A.take(sizeof(double) * 256);
   S->counter = (unsigned*)A.take(sizeof(unsigned) * 4);
   if (S->has64) {
@@ -2603,8 +2661,9 @@ static void launch_tail(Hierarchy<R>& H, int l0, bool first_done, cudaStream_t s
   tail_swaps(H, l0, first_done);
 }
 
+// bx: (L.b, result) of the finest level wanted there (summed in its upward launch, or on its own)
 template <typename R>
-static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = false) {
+static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = false, const ParitySum* bx = nullptr) {
   Level<R>& L = H.L[l];
   if (H.tail0 > 0 && l == H.tail0) {               // the coarse levels in one launch
     launch_tail(H, l, first_done, s);        // records the tail's pointer swaps too
@@ -2637,6 +2696,7 @@ static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = fal
       pdl_launch(k_prolong_g<R>, grid_for(L.nn, 256), 256, 0, s, L.g, C.g, (const R*)C.x, L.fix, L.t);
     a.xin = L.t; a.x = L.x;
     a.xc = nested ? C.x : nullptr;
+    if (bx) a.bx = *bx;
     mg_up<R>(a, L.deg, l == 0, s);
     return;
   }
@@ -2735,9 +2795,9 @@ static void vload(Hierarchy<R>& H, const std::vector<void*>& v) {
 
 // One V-cycle of hierarchy H (degree-`degree` Chebyshev smoothing) from a cached graph.
 template <typename R>
-static void vcycle_run(mw_stokes* S, Hierarchy<R>& H, cudaStream_t s) {
+static void vcycle_run(mw_stokes* S, Hierarchy<R>& H, const ParitySum* bx, cudaStream_t s) {
   const int kind = (sizeof(R) == 4 ? 1 : 2) * 64;
-  graph_run(S, kind, [&]() { vcycle(H, 0, s); }, [&]() { return vstate(H); },
+  graph_run(S, kind, [&]() { vcycle(H, 0, s, false, bx); }, [&]() { return vstate(H); },
             [&](const std::vector<void*>& v) { vload(H, v); }, s);
 }
 
@@ -2853,54 +2913,66 @@ static double read_scalar(const double* d, cudaStream_t s) {
   return h;
 }
 
-// Preconditioned CG for K x = b (b in double), MG V-cycle preconditioner at precision R.
-// x is written (overwritten) in double.  Returns iterations; *relres = ||r|| / ||b||.
+// The pieces of the inner PCG for K x = b (b in double), preconditioned by a V-cycle at precision R;
+// driven by the host (pcg_K) or recorded as a device loop (pcg_K_dev).
+template <typename R>
+struct Pcg {
+  mw_stokes* S;
+  Hierarchy<R>& H;
+  R** pc;              // x, r, p (two buffers, by iteration parity), Ap
+  int64_t n;
+  ParitySum rz() const { return ParitySum{S->red, S->counter, S->sc + P_RZ2, S->sc + P_IT}; }
+
+  void start(const double* b, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    pdl_launch(k_pcg_start<R>, nb_for(n), 256, 0, s, n, b, pc[1], pc[0], S->red, S->counter, S->sc, dev ? 1 : 0, hw);
+  }
+  // z = V(r) into the finest level's x, (r, z)
+  void precondition(bool graph, cudaStream_t s) const {
+    Level<R>& L = H.L[0];
+    const ParitySum out = rz();
+    R* saved_b = L.b;
+    L.b = pc[1];
+    const bool fused = H.nlev > 1 && L.deg <= MG_MAXDEG;
+    if (graph) vcycle_run(S, H, fused ? &out : nullptr, s);
+    else vcycle(H, 0, s, false, fused ? &out : nullptr);
+    L.b = saved_b;
+    if (!fused) pdl_launch(k_dot_parity<R>, nb_for(n), 256, 0, s, n, (const R*)pc[1], (const R*)L.x, out);
+  }
+  void step(double rtol, int maxit, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    OpArgs<R> a = op_args(H.L[0], true);
+    a.yV = pc[4];
+    PcgDir<R> d{H.L[0].x, {pc[2], pc[3]}, S->sc + P_RZ2, S->sc + P_IT, S->red, S->sc + P_PAP, S->counter};
+    op_pcg_direction<R>(a, d, s);
+    pdl_launch(k_pcg_update<R>, nb_for(n), 256, 0, s, n, (const R*)pc[2], (const R*)pc[3], (const R*)pc[4], pc[0],
+               pc[1], S->red, S->counter, S->sc, rtol, maxit, dev ? 1 : 0, hw);
+  }
+  void finish(double* x, cudaStream_t s) const {
+    pdl_launch(k_pcg_finish<R>, grid_for(n, 256), 256, 0, s, n, (const R*)pc[0], x, S->sc);
+  }
+};
+
+// K x = b with the loop on the host; x is overwritten.  Returns iterations; *relres = ||r|| / ||b||.
 template <typename R>
 static int pcg_K(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double* x, double rtol, int maxit,
                  double* relres, cudaStream_t s) {
-  Level<R>& L = H.L[0];
-  const int64_t n = L.ndof;
-  R *xr = pc[0], *r = pc[1], *p = pc[3], *Ap = pc[4];
-  R*& z = pc[2];
-  double* sc = S->sc;   // [0] rz, [1] pAp, [2] rr, [3] bb, [4] rz_new
-  pdl_launch(k_copy<R, double>, grid_for(n, 256), 256, 0, s, n, b, r);
-  pdl_launch(k_set<R>, grid_for(n, 256), 256, 0, s, n, R(0), xr);
-  dot<R>(S, n, r, r, sc + 3, s);
-  double bb = read_scalar(sc + 3, s);
-  if (!(bb > 0)) {
-    pdl_launch(k_set<double>, grid_for(n, 256), 256, 0, s, n, 0.0, x);
-    *relres = 0;
-    return 0;
-  }
-  // preconditioner z = V(r): the fine level reads r in place and the result buffer is exchanged
-  // with z (host pointers only, no copies)
-  auto precond = [&](R* rin, R*& zout) {
-    R* saved_b = L.b;
-    L.b = rin;
-    vcycle_run(S, H, s);
-    L.b = saved_b;
-    std::swap(zout, L.x);
-  };
-  precond(r, z);
-  pdl_launch(k_copy<R, R>, grid_for(n, 256), 256, 0, s, n, z, p);
-  dot<R>(S, n, r, z, sc + 0, s);
-  int it = 0;
+  const Pcg<R> P{S, H, pc, H.L[0].ndof};
+  P.start(b, false, 0, s);
+  const double bb = read_scalar(S->sc + P_BB, s);
   double rr = bb;
-  for (it = 1; it <= maxit; ++it) {
-    level_apply<R>(L, true, p, Ap, s);
-    dot<R>(S, n, p, Ap, sc + 1, s);
-    pdl_launch(k_pcg_update_rr<R>, nb_for(n), 256, 0, s, n, sc + 0, sc + 1, p, Ap, xr, r, S->red, S->counter, sc + 2);
-    rr = read_scalar(sc + 2, s);
-    if (!std::isfinite(rr)) break;
-    if (rr <= rtol * rtol * bb) break;
-    precond(r, z);
-    dot<R>(S, n, r, z, sc + 4, s);
-    pdl_launch(k_xpby_ratio<R>, grid_for(n, 256), 256, 0, s, n, z, sc + 4, sc + 0, p);
-    cudaMemcpyAsync(sc + 0, sc + 4, sizeof(double), cudaMemcpyDeviceToDevice, s);
+  int it = 0;
+  if (bb > 0) {
+    for (it = 1; it <= maxit; ++it) {
+      P.precondition(true, s);
+      P.step(rtol, maxit, false, 0, s);
+      rr = read_scalar(S->sc + P_RR, s);
+      if (!std::isfinite(rr)) break;
+      if (rr <= rtol * rtol * bb) break;
+    }
+    if (it > maxit) it = maxit;
   }
-  pdl_launch(k_copy<double, R>, grid_for(n, 256), 256, 0, s, n, xr, x);
-  *relres = std::sqrt(rr / bb);
-  return it > maxit ? maxit : it;
+  P.finish(x, s);
+  *relres = bb > 0 ? std::sqrt(rr / bb) : 0;
+  return it;
 }
 
 // Jacobi-PCG for the (weighted) Q1 mass matrix: M_w x = b.  weights NULL -> M (uzawa3),
@@ -3063,49 +3135,6 @@ static int uzawa(mw_stokes* S, const mw_solve_params& sp, int prec, const double
 // waits for the host.  Every loop is bounded by its iteration cap (max_inner, max_outer,
 // max_refine) and by a total work cap, both decided on the device.  Scalars live in S->sc from
 // slot 64 on.
-// Schur-residual reduction of a refinement sweep that starts at relative residual `rel`: the fixed
-// sweep_reduction, or with target > 0 the smaller reduction target * tol / rel (at most 0.5).
-MW_HD double sweep_target_reduction(double sweep_reduction, double target, double tol, double rel) {
-  if (!(target > 0) || !(rel > 0)) return sweep_reduction;
-  double r = target * tol / rel;
-  if (r > 0.5) r = 0.5;
-  return r > sweep_reduction ? r : sweep_reduction;
-}
-
-enum DevSlot {
-  P_RZ = 64, P_PAP, P_RR, P_BB, P_RZN, P_IT,                 // inner PCG
-  U_RW = 72, U_DSD, U_RWN, U_RR0, U_RR, U_IT, U_D2, U_Z2,    // Schur CG
-  T_RV = 84, T_RP, T_REL,                                     // true residual
-  S_BB = 88, S_BH, S_BNORM, S_REL0, S_NREF, S_RED,           // solve
-  I_OUTER = 96, I_INNER, I_STATUS                             // info
-};
-
-// Work caps of one solve on top of the per-loop caps: a stagnating solve ends with status 3 after
-// this many inner (multigrid-PCG) or outer (Schur) iterations in total.
-constexpr double DEV_INNER_BUDGET = 40000, DEV_OUTER_BUDGET = 4000;
-
-__global__ void k_dev_pcg_init(double* sc, cudaGraphConditionalHandle hw) {
-  pdl_entry();
-  sc[P_IT] = 0;
-  const double bb = sc[P_BB];
-  cudaGraphSetConditional(hw, (bb > 0 && isfinite(bb)) ? 1u : 0u);
-}
-
-__global__ void k_dev_pcg_check(double* sc, double rtol, int maxit, cudaGraphConditionalHandle hw,
-                                cudaGraphConditionalHandle hi) {
-  pdl_entry();
-  const double it = sc[P_IT] + 1;
-  sc[P_IT] = it;
-  const double rr = sc[P_RR];
-  bool go = isfinite(rr) && rr > rtol * rtol * sc[P_BB] && it < (double)maxit;
-  if (go && sc[I_INNER] + it >= DEV_INNER_BUDGET) { sc[I_STATUS] = 3; go = false; }
-  cudaGraphSetConditional(hw, go ? 1u : 0u);
-  cudaGraphSetConditional(hi, go ? 1u : 0u);
-}
-
-__global__ void k_dev_pcg_done(double* sc) {
-  pdl_entry(); sc[I_INNER] += sc[P_IT]; }
-
 __global__ void k_dev_uz_init(double* sc, int max_outer, cudaGraphConditionalHandle hw) {
   pdl_entry();
   sc[U_IT] = 0;
@@ -3217,49 +3246,21 @@ static bool cond_end(cudaStream_t bs) {
 static cudaStream_t lvl(mw_stokes* S, cudaStream_t s, int depth) { return depth == 0 ? s : S->bs[depth - 1]; }
 
 // Inner PCG for K x = b recorded with a device WHILE loop (capture only), at nesting level `depth`
-// (uses the body streams depth and depth + 1).  Adds its iteration count to sc[I_INNER].
+// (uses the body stream depth).  Adds its iteration count to sc[I_INNER].
 template <typename R>
 static bool pcg_K_dev(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double* x, double rtol, int maxit,
                       cudaStream_t s0, int depth) {
-  if (depth + 2 > 6) return false;
-  cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth], b2 = S->bs[depth + 1];
-  Level<R>& L = H.L[0];
-  const int64_t n = L.ndof;
-  R *xr = pc[0], *r = pc[1], *p = pc[3], *Ap = pc[4];
-  R*& z = pc[2];
-  double* sc = S->sc;
-  auto precond = [&](R* rin, R*& zout, cudaStream_t st) {
-    R* saved_b = L.b;
-    L.b = rin;
-    vcycle(H, 0, st);
-    L.b = saved_b;
-    std::swap(zout, L.x);
-  };
-  pdl_launch(k_copy<R, double>, grid_for(n, 256), 256, 0, s, n, b, r);
-  pdl_launch(k_set<R>, grid_for(n, 256), 256, 0, s, n, R(0), xr);
-  dot<R>(S, n, r, r, sc + P_BB, s);
-  precond(r, z, s);
-  pdl_launch(k_copy<R, R>, grid_for(n, 256), 256, 0, s, n, z, p);
-  dot<R>(S, n, r, z, sc + P_RZ, s);
-  cudaGraphConditionalHandle hw, hi;
+  if (depth + 1 > 6) return false;
+  cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth];
+  const Pcg<R> P{S, H, pc, H.L[0].ndof};
+  cudaGraphConditionalHandle hw;
   if (!cond_handle(s, &hw)) return false;
-  pdl_launch(k_dev_pcg_init, 1, 1, 0, s, sc, hw);
+  P.start(b, true, hw, s);
   if (!cond_node(s, b1, cudaGraphCondTypeWhile, hw)) return false;
-  // body: one CG step and the convergence test, then (if continuing) the next search direction
-  level_apply<R>(L, true, p, Ap, b1);
-  dot<R>(S, n, p, Ap, sc + P_PAP, b1);
-  pdl_launch(k_pcg_update_rr<R>, nb_for(n), 256, 0, b1, n, sc + P_RZ, sc + P_PAP, p, Ap, xr, r, S->red, S->counter,
-             sc + P_RR);
-  if (!cond_handle(b1, &hi)) return false;
-  pdl_launch(k_dev_pcg_check, 1, 1, 0, b1, sc, rtol, maxit, hw, hi);
-  if (!cond_node(b1, b2, cudaGraphCondTypeIf, hi)) return false;
-  precond(r, z, b2);
-  dot<R>(S, n, r, z, sc + P_RZN, b2);
-  pdl_launch(k_xpby_ratio<R>, grid_for(n, 256), 256, 0, b2, n, z, sc + P_RZN, sc + P_RZ, p);
-  pdl_launch(k_copy1, 1, 1, 0, b2, sc + P_RZN, sc + P_RZ);
-  if (!cond_end(b2) || !cond_end(b1)) return false;
-  pdl_launch(k_copy<double, R>, grid_for(n, 256), 256, 0, s, n, xr, x);
-  pdl_launch(k_dev_pcg_done, 1, 1, 0, s, sc);
+  P.precondition(false, b1);
+  P.step(rtol, maxit, true, hw, b1);
+  if (!cond_end(b1)) return false;
+  P.finish(x, s);
   return true;
 }
 
@@ -3283,10 +3284,10 @@ static void true_residual_dev(mw_stokes* S, const double* V, const double* P, co
 }
 
 // Schur-complement CG (the recurrences of the host version `uzawa`) recorded with a device WHILE
-// loop at nesting level `depth` (uses body streams depth .. depth + 3).
+// loop at nesting level `depth` (uses body streams depth .. depth + 1).
 static bool uzawa_dev(mw_stokes* S, const mw_solve_params& sp, int prec, const double* f, const double* h, double* V,
                       double* P, double reduction, bool check_true, cudaStream_t s0, int depth) {
-  if (depth + 4 > 6) return false;
+  if (depth + 2 > 6) return false;
   cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth];
   const LevelGeo& g = S->fine;
   const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
