@@ -19,12 +19,15 @@ namespace {
 
 // Resident CTAs: two, or three where 80 registers do without spills (FP32 without pressure).  FP64
 // with two (128 registers, 156 bytes spilled with pressure) takes 31 us at 512^2 against 36 with one.
-template <typename R, bool PRESSURE, bool PCG>
+enum { OP_PLAIN = 0, OP_PCG, OP_SUM };
+
+template <typename R, bool PRESSURE, int KIND, typename X>
 __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3 : 2) k_op_apply(OpArgs<R> a,
-                                                                                                 PcgDir<R> dir) {
+                                                                                                 X dir) {
   pdl_entry();
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, NC = CELLS * CELLS, T = CELLS - 2;
+  constexpr bool PCG = KIND == OP_PCG;
   __shared__ __align__(16) R2 sx[4 * NC];
   __shared__ __align__(16) R2 se[5 * NC];
   __shared__ R sp[PRESSURE ? 4 * NC : 1];
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
   const R* pold = nullptr;
   double beta = 0.0;
   int k = 0;
-  if (PCG) {
+  if constexpr (PCG) {
     k = (int)*dir.it;
     if (k > 0) {
       beta = dir.rz[k & 1] / dir.rz[(k & 1) ^ 1];
@@ -56,7 +59,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
     x[t] = zero;
     if (has[t]) {
       const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
-      if (PCG) {
+      if constexpr (PCG) {
         x[t] = reinterpret_cast<const R2*>(dir.z)[n];
         if (pold) {
           const R2 q = reinterpret_cast<const R2*>(pold)[n];
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
   __syncthreads();
   const int ownx = ex0 + T >= g.nx ? T + 1 : T, ownz = ez0 + T >= g.nz ? T + 1 : T;
   const bool own = lx >= 1 && lx <= ownx && lz >= 1 && lz <= ownz && has[0];
-  if (!PCG && !own) return;
+  if (KIND == OP_PLAIN && !own) return;
   double v = 0;
   if (own && (PCG || a.yV)) {
     // ascending element order: lower left, lower, left, own
@@ -129,24 +132,29 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
           if (f & 1u) s[t].x = dg.x * x[t].x;
           if (f & 2u) s[t].y = dg.y * x[t].y;
         }
-        if (PCG) {
+        if constexpr (PCG) {
           reinterpret_cast<R2*>((k & 1) ? dir.pbuf[1] : dir.pbuf[0])[n] = x[t];
           v += (double)x[t].x * (double)s[t].x + (double)x[t].y * (double)s[t].y;
         } else if (a.bV) {
           const R2 b = reinterpret_cast<const R2*>(a.bV)[n];
           s[t] = pair(b.x - s[t].x, b.y - s[t].y);
+          if (KIND == OP_SUM) v += (double)s[t].x * (double)s[t].x + (double)s[t].y * (double)s[t].y;
         }
         reinterpret_cast<R2*>(a.yV)[n] = s[t];
       }
   }
-  if constexpr (PCG) {
-    double sum;
-    if (grid_sum(v, dir.part, dir.counter, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, &sum))
-      *dir.pap = sum;
+  if (PRESSURE && own && a.yP) {                            // the elements lower left, lower, left, own
+    R r = ((sp[3 * NC + tid - CX - 1] + sp[2 * NC + tid - CX]) + sp[NC + tid - 1]) + yp[0];
+    if (a.bP) r = a.bP[np] - r;
+    a.yP[np] = r;
+    if (KIND == OP_SUM) v += (double)r * (double)r;
   }
-  if (PRESSURE && a.yP) {                                   // the elements lower left, lower, left, own
-    const R v = ((sp[3 * NC + tid - CX - 1] + sp[2 * NC + tid - CX]) + sp[NC + tid - 1]) + yp[0];
-    a.yP[np] = a.bP ? a.bP[np] - v : v;
+  if constexpr (KIND != OP_PLAIN) {
+    double sum;
+    if (grid_sum(v, dir.part, dir.counter, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, &sum)) {
+      if constexpr (PCG) *dir.pap = sum;
+      else residual_done(dir.sc, sum, dir.action, dir.test);
+    }
   }
 }
 
@@ -164,13 +172,19 @@ int cell_partials(int nx, int nz) {
   return ((nx + T - 1) / T) * ((nz + T - 1) / T);
 }
 
+struct NoExtra {};
+
 template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s) {
-  if (a.p || a.yP) pdl_launch(k_op_apply<R, true, false>, tiles(a), CELLS * CELLS, 0, s, a, PcgDir<R>());
-  else pdl_launch(k_op_apply<R, false, false>, tiles(a), CELLS * CELLS, 0, s, a, PcgDir<R>());
+  if (a.p || a.yP) pdl_launch(k_op_apply<R, true, OP_PLAIN, NoExtra>, tiles(a), CELLS * CELLS, 0, s, a, NoExtra());
+  else pdl_launch(k_op_apply<R, false, OP_PLAIN, NoExtra>, tiles(a), CELLS * CELLS, 0, s, a, NoExtra());
 }
 
 template <typename R> void op_pcg_direction(const OpArgs<R>& a, const PcgDir<R>& d, cudaStream_t s) {
-  pdl_launch(k_op_apply<R, false, true>, tiles(a), CELLS * CELLS, 0, s, a, d);
+  pdl_launch(k_op_apply<R, false, OP_PCG, PcgDir<R>>, tiles(a), CELLS * CELLS, 0, s, a, d);
+}
+
+void op_residual(const OpArgs<double>& a, const ResidSum& r, cudaStream_t s) {
+  pdl_launch(k_op_apply<double, true, OP_SUM, ResidSum>, tiles(a), CELLS * CELLS, 0, s, a, r);
 }
 
 template void op_apply<float>(const OpArgs<float>&, cudaStream_t);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "mg_level.cuh"
+#include "solve_scalars.cuh"
 
 namespace mw {
 
@@ -32,7 +33,16 @@ struct PcgDir {
   unsigned* counter;
 };
 
+// The FP64 residual (bV, bP) - A (u, p) with its sum of squares, and what follows from it.
+struct ResidSum {
+  double *part, *sc;
+  unsigned* counter;
+  int action;
+  LoopTest test;
+};
+
 int op_ensure_tables();
+void op_residual(const OpArgs<double>& a, const ResidSum& r, cudaStream_t s);
 template <typename R> void op_apply(const OpArgs<R>& a, cudaStream_t s);
 template <typename R> void op_pcg_direction(const OpArgs<R>& a, const PcgDir<R>& d, cudaStream_t s);
 // the partial sums the level and direction launches of a level of nx x nz elements need

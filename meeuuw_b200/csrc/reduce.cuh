@@ -5,21 +5,28 @@
 
 namespace mw {
 
-// The grid-wide sum of one value per thread: block partials in part[block], and the last block to
-// arrive adds them in block order and resets the counter (threadfence + arrival counter).  Called
-// once, by every thread, at the end of a kernel.  True for the one thread that holds the sum.
-MW_D bool grid_sum(double v, double* part, unsigned* counter, int block, int nblocks, double* sum) {
-  __shared__ double sh[32];
+// The grid-wide sums of NV values per thread: block partials in part[i * nblocks + block], and the last
+// block to arrive adds them in block order and resets the counter (threadfence + arrival counter).
+// Called once, by every thread, at the end of a kernel.  True for the one thread that holds the sums.
+template <int NV>
+MW_D bool grid_sums(double (&v)[NV], double* part, unsigned* counter, int block, int nblocks, double* sum) {
+  __shared__ double sh[NV][32];
   __shared__ bool last;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
+    if (lane == 0) sh[i][wid] = v[i];
+  }
   __syncthreads();
   if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      v[i] = lane < nw ? sh[i][lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
+      if (lane == 0) part[i * nblocks + block] = v[i];
+    }
     if (lane == 0) {
-      part[block] = v;
       __threadfence();
       last = atomicAdd(counter, 1u) == (unsigned)nblocks - 1;
     }
@@ -27,17 +34,32 @@ MW_D bool grid_sum(double v, double* part, unsigned* counter, int block, int nbl
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  double t = 0;
-  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) t += ((volatile double*)part)[i];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  if (lane == 0) sh[wid] = t;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double t = 0;
+    for (int k = threadIdx.x; k < nblocks; k += blockDim.x) t += ((volatile double*)part)[i * nblocks + k];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) sh[i][wid] = t;
+  }
   __syncthreads();
   if (threadIdx.x != 0) return false;
-  double s = 0;
-  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[k];
-  *sum = s;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    double s = 0;
+    for (int k = 0; k < nw; ++k) s += sh[i][k];
+    sum[i] = s;
+  }
   *counter = 0u;
   return true;
+}
+
+MW_D bool grid_sum(double v, double* part, unsigned* counter, int block, int nblocks, double* sum) {
+  double a[1] = {v};
+  return grid_sums<1>(a, part, counter, block, nblocks, sum);
+}
+MW_D bool grid_sum2(double v, double w, double* part, unsigned* counter, int block, int nblocks, double* sum) {
+  double a[2] = {v, w};
+  return grid_sums<2>(a, part, counter, block, nblocks, sum);
 }
 
 // Where a kernel leaves a sum that the iterations keep by parity: out[*it & 1].

@@ -214,8 +214,8 @@ MW_D int q2_local_idx(int dx, int dz) {
 // incident elements' entries in ascending element order.  Fixed velocity dofs: zero rows of G,
 // zeroed entries of u for G^T (the reference's Dirichlet elimination).
 // G p at velocity node (ix, iz) (f - G p with b): gx, gz are the GX, GZ tables, cx, cz the scalings.
-MW_D void grad_node(const LevelGeo& g, const double* p, const uint8_t* fix, const double* b, double* y, int ix,
-                    int iz, const double* gx, const double* gz, double cx, double cz) {
+MW_D double2 grad_value(const LevelGeo& g, const double* p, const uint8_t* fix, const double* b, int ix, int iz,
+                        const double* gx, const double* gz, double cx, double cz) {
   const int64_t n = (int64_t)iz * g.nnx + ix;
   const bool xo = ix & 1, zo = iz & 1;
   const int xa = xo ? (ix >> 1) : (ix >> 1) - 1, xb = ix >> 1;
@@ -243,13 +243,20 @@ MW_D void grad_node(const LevelGeo& g, const double* p, const uint8_t* fix, cons
     const double2 bb = reinterpret_cast<const double2*>(b)[n];
     r = double2{bb.x - r.x, bb.y - r.y};
   }
-  reinterpret_cast<double2*>(y)[n] = r;
+  return r;
+}
+
+MW_D void grad_node(const LevelGeo& g, const double* p, const uint8_t* fix, const double* b, double* y, int ix,
+                    int iz, const double* gx, const double* gz, double cx, double cz) {
+  reinterpret_cast<double2*>(y)[(int64_t)iz * g.nnx + ix] = grad_value(g, p, fix, b, ix, iz, gx, gz, cx, cz);
 }
 
 // G^T u at pressure node (px, pz)
-MW_D double div_node(const LevelGeo& g, const double* u, const uint8_t* fix, int px, int pz, const double* gx,
+template <typename R>
+MW_D double div_node(const LevelGeo& g, const R* u, const uint8_t* fix, int px, int pz, const double* gx,
                      const double* gz, double cx, double cz) {
-  const double2* u2 = reinterpret_cast<const double2*>(u);
+  typedef typename Vec2<R>::T R2;
+  const R2* u2 = reinterpret_cast<const R2*>(u);
   const uchar2* f2 = reinterpret_cast<const uchar2*>(fix);
   // incident elements in ascending order and this node's Q1 index in each
   const int exs[4] = {px - 1, px, px - 1, px}, ezs[4] = {pz - 1, pz - 1, pz, pz}, js[4] = {2, 3, 1, 0};
@@ -262,10 +269,10 @@ MW_D double div_node(const LevelGeo& g, const double* u, const uint8_t* fix, int
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const int64_t m = q2_node(ex, ez, k, g.nnx);
-      const double2 uu = u2[m];
+      const R2 uu = u2[m];
       const uchar2 ff = f2[m];
-      sx += gx[k * 4 + j] * (ff.x ? 0.0 : uu.x);
-      sz += gz[k * 4 + j] * (ff.y ? 0.0 : uu.y);
+      sx += gx[k * 4 + j] * (ff.x ? 0.0 : (double)uu.x);
+      sz += gz[k * 4 + j] * (ff.y ? 0.0 : (double)uu.y);
     }
     acc += cx * sx + cz * sz;
   }
@@ -1518,48 +1525,7 @@ __global__ void k_fix_coarse(LevelGeo gf, LevelGeo gc, const uint8_t* __restrict
   }
 }
 
-// ---------------------------------------------------------------- scalars of the solver loops
-// Schur-residual reduction of a refinement sweep that starts at relative residual `rel`: the fixed
-// sweep_reduction, or with target > 0 the smaller reduction target * tol / rel (at most 0.5).
-MW_HD double sweep_target_reduction(double sweep_reduction, double target, double tol, double rel) {
-  if (!(target > 0) || !(rel > 0)) return sweep_reduction;
-  double r = target * tol / rel;
-  if (r > 0.5) r = 0.5;
-  return r > sweep_reduction ? r : sweep_reduction;
-}
-
-enum DevSlot {
-  P_PAP = 64, P_RR, P_BB, P_IT, P_RZ2,                       // inner PCG; (r, z) by iteration parity at
-                                                              // P_RZ2, P_RZ2 + 1
-  U_RW = 72, U_DSD, U_RWN, U_RR0, U_RR, U_IT, U_D2, U_Z2,    // Schur CG
-  T_RV = 84, T_RP, T_REL,                                     // true residual
-  S_BB = 88, S_BH, S_BNORM, S_REL0, S_NREF, S_RED,           // solve
-  I_OUTER = 96, I_INNER, I_STATUS                             // info
-};
-
-// Work caps of one solve on top of the per-loop caps: a stagnating solve ends with status 3 after
-// this many inner (multigrid-PCG) or outer (Schur) iterations in total.
-constexpr double DEV_INNER_BUDGET = 40000, DEV_OUTER_BUDGET = 4000;
-
 // ---------------------------------------------------------------- BLAS-1 with device scalars
-template <typename R>
-__global__ void k_dot_partial(int64_t n, const R* __restrict__ x, const R* __restrict__ y, double* __restrict__ part) {
-  pdl_entry();
-  __shared__ double sh[32];
-  double v = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v += (double)x[i] * (double)y[i];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) part[blockIdx.x] = v;
-  }
-}
-
 __global__ void k_dot_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
   pdl_entry();
   __shared__ double sh[32];
@@ -1574,26 +1540,6 @@ __global__ void k_dot_final(const double* __restrict__ part, int nb, double* __r
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) out[0] = v;
   }
-}
-
-// y += sgn * (num/den) * x      (scalars on the device)
-template <typename R, typename S>
-__global__ void k_axpy_ratio(int64_t n, const double* __restrict__ num, const double* __restrict__ den, double sgn,
-                             const S* __restrict__ x, R* __restrict__ y) {
-  pdl_entry();
-  const double a = sgn * (*num / *den);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    y[i] = (R)((double)y[i] + a * (double)x[i]);
-}
-
-// p = z + (num/den) * p
-template <typename R>
-__global__ void k_xpby_ratio(int64_t n, const R* __restrict__ z, const double* __restrict__ num,
-                             const double* __restrict__ den, R* __restrict__ p) {
-  pdl_entry();
-  const double b = *num / *den;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = (R)((double)z[i] + b * (double)p[i]);
 }
 
 template <typename R>
@@ -1628,16 +1574,7 @@ __global__ void k_cheb_first(int64_t n, const double* __restrict__ cheb, const R
   }
 }
 
-// power iteration helpers for lambda_max(D^-1 K)
-template <typename R>
-__global__ void k_scale_dinv_norm(int64_t n, const R* __restrict__ y, const R* __restrict__ diag,
-                                  const double* __restrict__ nrm2, R* __restrict__ x) {
-  pdl_entry();
-  const double inv = 1.0 / sqrt(fmax(*nrm2, 1e-300));
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    x[i] = (R)((double)y[i] / (double)diag[i] * inv);
-}
-
+// power iteration helper for lambda_max(D^-1 K)
 template <typename R>
 __global__ void k_dinv(int64_t n, const R* __restrict__ y, const R* __restrict__ diag, R* __restrict__ x) {
   pdl_entry();
@@ -1763,37 +1700,8 @@ __global__ void k_dense_matvec(int nd, const double* __restrict__ Ainv, const R*
 }
 
 // ---------------------------------------------------------------- pressure mass matrices
-// y = M_w p with M_w the Q1 mass matrix weighted per element by w_e (w = NULL -> 1):
+// diag(M_w), M_w the Q1 mass matrix weighted per element by w_e (w = NULL -> 1):
 // M_el = sum_q N_P N_P^T JxW (build_matrix_stokes.py:147), M_eta = M_el / eta_e (:264).
-__global__ void k_mass_apply(LevelGeo g, const double* __restrict__ w, const double* __restrict__ p,
-                             double* __restrict__ y) {
-  pdl_entry();
-  const int ncx = g.nx + 1;
-  const int64_t np = (int64_t)ncx * (g.nz + 1);
-  const double jac = g.hx * g.hz / 4.0;
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np; n += (int64_t)gridDim.x * blockDim.x) {
-    int i = (int)(n % ncx), j = (int)(n / ncx);
-    const int exs[4] = {i - 1, i, i - 1, i};
-    const int ezs[4] = {j - 1, j - 1, j, j};
-    const int kk[4] = {2, 3, 1, 0};
-    double acc = 0;
-    for (int s = 0; s < 4; ++s) {
-      int ex = exs[s], ez = ezs[s];
-      if (ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
-      int64_t e = (int64_t)ez * g.nx + ex;
-      double we = w ? w[e] : 1.0;
-      double v = 0;
-      for (int k2 = 0; k2 < 4; ++k2) {
-        double m = 0;
-        for (int q = 0; q < 9; ++q) m += c_ref.NP[q * 4 + kk[s]] * c_ref.NP[q * 4 + k2] * jac * c_ref.wq[q];
-        v += m * p[q1_node(ex, ez, k2, g.nx)];
-      }
-      acc += we * v;
-    }
-    y[n] = acc;
-  }
-}
-
 __global__ void k_mass_diag(LevelGeo g, const double* __restrict__ w, double* __restrict__ d) {
   pdl_entry();
   const int ncx = g.nx + 1;
@@ -1854,16 +1762,30 @@ MW_D void mass_cheb_node(const LevelGeo& g, const double* w, const double* b, co
   xout[n] = (first ? 0.0 : xin[n]) + dn;
 }
 
-__global__ void k_mass_cheb(LevelGeo g, const double* __restrict__ w, const double* __restrict__ b,
+// m1 (first step): the sum of b, whose mean is removed from b before the step.  sum (last step, else
+// null): receives the sum of x.  zero (first step, may be null): a vector of np entries to clear.
+__global__ void k_mass_cheb(LevelGeo g, const double* __restrict__ w, double* __restrict__ b,
                             const double* __restrict__ xin, double* __restrict__ xout, double* __restrict__ d,
-                            const double* __restrict__ dg, double c1, double c2, int first) {
+                            const double* __restrict__ dg, double c1, double c2, int first,
+                            const double* __restrict__ m1, double* __restrict__ zero, double* __restrict__ part,
+                            unsigned* __restrict__ counter, double* __restrict__ sum) {
   pdl_entry();
   __shared__ double Me[16];
   if (threadIdx.x < 16) Me[threadIdx.x] = mass_entry(g, threadIdx.x / 4, threadIdx.x % 4);
   __syncthreads();
   const int64_t np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np; n += (int64_t)gridDim.x * blockDim.x)
+  const double mean = m1 ? *m1 / (double)np : 0.0;
+  double v = 0;
+  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np; n += (int64_t)gridDim.x * blockDim.x) {
+    if (m1) b[n] -= mean;
+    if (zero) zero[n] = 0.0;
     mass_cheb_node(g, w, b, xin, xout, d, dg, c1, c2, first, Me, n);
+    if (sum) v += xout[n];
+  }
+  if (sum) {
+    double t;
+    if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &t)) *sum = t;
+  }
 }
 
 // the sum of one value per thread over a one-dimensional grid, into *out
@@ -1888,7 +1810,14 @@ __global__ void k_dot1(int64_t n, const R* __restrict__ x, const R* __restrict__
 // parity): k_pcg_start, then { V-cycle with (r, z), op_pcg_direction with (p, Ap), k_pcg_update } until the
 // update's convergence test fails, then k_pcg_finish.
 
-// r = b, x = 0, (b, b); the loop condition (device loops)
+// (b, b) known: the loop's scalars and -- device loops -- its condition
+MW_D void pcg_started(double* sc, double bb, int device_loop, cudaGraphConditionalHandle hw) {
+  sc[P_BB] = bb;
+  sc[P_IT] = 0;
+  if (device_loop) cudaGraphSetConditional(hw, (bb > 0 && isfinite(bb)) ? 1u : 0u);
+}
+
+// r = b, x = 0, (b, b)
 template <typename R>
 __global__ void k_pcg_start(int64_t n, const double* __restrict__ b, R* __restrict__ r, R* __restrict__ x,
                             double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
@@ -1902,11 +1831,39 @@ __global__ void k_pcg_start(int64_t n, const double* __restrict__ b, R* __restri
     v += (double)ri * (double)ri;
   }
   double bb;
-  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &bb)) {
-    sc[P_BB] = bb;
-    sc[P_IT] = 0;
-    if (device_loop) cudaGraphSetConditional(hw, (bb > 0 && isfinite(bb)) ? 1u : 0u);
+  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &bb)) pcg_started(sc, bb, device_loop, hw);
+}
+
+// the same for b = G p, or f - G p with f (node stencils, one lattice row at a time)
+template <typename R>
+__global__ void k_pcg_start_grad(LevelGeo g, const double* __restrict__ p, const uint8_t* __restrict__ fix,
+                                 const double* __restrict__ f, R* __restrict__ r, R* __restrict__ x,
+                                 double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
+                                 int device_loop, cudaGraphConditionalHandle hw) {
+  pdl_entry();
+  typedef typename Vec2<R>::T R2;
+  __shared__ double gx[36], gz[36];
+  if (threadIdx.x < 36) {
+    gx[threadIdx.x] = c_ref.GX[threadIdx.x];
+    gz[threadIdx.x] = c_ref.GZ[threadIdx.x];
   }
+  __syncthreads();
+  double cx, cz, v = 0;
+  grad_scales(g, &cx, &cz);
+  for (int iz = blockIdx.y; iz < g.nnz; iz += gridDim.y)
+    for (int ix = blockIdx.x * blockDim.x + threadIdx.x; ix < g.nnx; ix += gridDim.x * blockDim.x) {
+      const double2 q = grad_value(g, p, fix, f, ix, iz, gx, gz, cx, cz);
+      R2 ri, zero;
+      ri.x = (R)q.x; ri.y = (R)q.y;
+      zero.x = zero.y = R(0);
+      const int64_t n = (int64_t)iz * g.nnx + ix;
+      reinterpret_cast<R2*>(r)[n] = ri;
+      reinterpret_cast<R2*>(x)[n] = zero;
+      v += (double)ri.x * (double)ri.x + (double)ri.y * (double)ri.y;
+    }
+  double bb;
+  if (grid_sum(v, part, counter, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, &bb))
+    pcg_started(sc, bb, device_loop, hw);
 }
 
 // x += alpha p, r -= alpha Ap, (r, r), and in the block that finishes the sum the iteration count and
@@ -1956,6 +1913,159 @@ __global__ void k_pcg_finish(int64_t n, const R* __restrict__ xr, double* __rest
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] = (double)xr[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) sc[I_INNER] += sc[P_IT];
+}
+
+// ---- the Schur-complement iteration around it (slots U_*): k_pcg_start_grad, the inner loop,
+// k_schur_div with (d, G^T z), k_schur_update with the sum of the new residual, the mass solve (which
+// removes that mean and sums its result), k_schur_dots with (r, w), (r, r) and the convergence test,
+// k_schur_direction.
+
+// G^T x of the inner solution x.  With V (the initial residual): V = x in double, out = G^T x - h and
+// its sum in U_M1; else (d, out) in U_DSD.  Adds the inner iteration count.
+template <typename R>
+__global__ void k_schur_div(LevelGeo g, const R* __restrict__ x, const uint8_t* __restrict__ fix,
+                            double* __restrict__ out, const double* __restrict__ h, double* __restrict__ V,
+                            const double* __restrict__ d, double* __restrict__ part, unsigned* __restrict__ counter,
+                            double* __restrict__ sc) {
+  pdl_entry();
+  __shared__ double gx[36], gz[36];
+  if (threadIdx.x < 36) {
+    gx[threadIdx.x] = c_ref.GX[threadIdx.x];
+    gz[threadIdx.x] = c_ref.GZ[threadIdx.x];
+  }
+  __syncthreads();
+  double cx, cz, v = 0;
+  grad_scales(g, &cx, &cz);
+  const int ncx = g.nx + 1;
+  for (int pz = blockIdx.y; pz <= g.nz; pz += gridDim.y)
+    for (int px = blockIdx.x * blockDim.x + threadIdx.x; px < ncx; px += gridDim.x * blockDim.x) {
+      const int64_t n = (int64_t)pz * ncx + px;
+      double y = div_node(g, x, fix, px, pz, gx, gz, cx, cz);
+      if (V && h) y -= h[n];
+      out[n] = y;
+      v += V ? y : d[n] * y;
+    }
+  const int block = blockIdx.y * gridDim.x + blockIdx.x, nblocks = gridDim.x * gridDim.y;
+  if (V) {
+    const int64_t nv = 2LL * g.nnx * g.nnz;
+    for (int64_t i = block * (int64_t)blockDim.x + threadIdx.x; i < nv; i += (int64_t)nblocks * blockDim.x)
+      V[i] = (double)x[i];
+  }
+  double s;
+  if (grid_sum(v, part, counter, block, nblocks, &s)) {
+    sc[V ? U_M1 : U_DSD] = s;
+    sc[I_INNER] += sc[P_IT];
+  }
+}
+
+// alpha = (r, w) / (d, G^T z): P += alpha d, V -= alpha z, r -= alpha G^T z, and the sum of r
+template <typename R>
+__global__ void k_schur_update(int64_t nv, int64_t np, const double* __restrict__ d, const R* __restrict__ z,
+                               const double* __restrict__ GTz, double* __restrict__ P, double* __restrict__ V,
+                               double* __restrict__ r, double* __restrict__ part, unsigned* __restrict__ counter,
+                               double* __restrict__ sc) {
+  pdl_entry();
+  typedef typename Vec2<R>::T R2;
+  const double a = sc[U_RW2 + ((int)sc[U_IT] & 1)] / sc[U_DSD];
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+  const R2* z2 = reinterpret_cast<const R2*>(z);
+  double2* V2 = reinterpret_cast<double2*>(V);
+  for (int64_t i = t0; i < nv / 2; i += nt) {
+    const R2 zi = z2[i];
+    double2 vi = V2[i];
+    vi.x += -a * (double)zi.x;
+    vi.y += -a * (double)zi.y;
+    V2[i] = vi;
+  }
+  double v = 0;
+  for (int64_t i = t0; i < np; i += nt) {
+    P[i] += a * d[i];
+    const double ri = r[i] + -a * GTz[i];
+    r[i] = ri;
+    v += ri;
+  }
+  double s;
+  if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &s)) sc[U_M1] = s;
+}
+
+// w -= its mean (sum in U_M2); (r, w) by the next iteration's parity, (r, r); then the start of the
+// loop (first) or the end of an iteration, with its test unless the true residual decides
+__global__ void k_schur_dots(int64_t np, double* __restrict__ w, const double* __restrict__ r, int first,
+                             double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
+                             LoopTest test) {
+  pdl_entry();
+  const double mean = sc[U_M2] / (double)np;
+  double a = 0, b = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+    const double wi = w[i] - mean, ri = r[i];
+    w[i] = wi;
+    a += ri * wi;
+    b += ri * ri;
+  }
+  double sum[2];
+  if (grid_sum2(a, b, part, counter, blockIdx.x, gridDim.x, sum)) {
+    const int k = first ? 0 : (int)sc[U_IT] + 1;
+    sc[U_RW2 + (k & 1)] = sum[0];
+    if (first) {
+      sc[U_RR0] = sum[1];
+      schur_start(sc, test);
+    } else {
+      sc[U_RR] = sum[1];
+      sc[U_IT] = k;
+      sc[I_OUTER] += 1;
+      if (!test.check_true) schur_test(sc, test);
+    }
+  }
+}
+
+// d = w + beta d, beta = (r, w) / (r, w) before; the first direction is w
+__global__ void k_schur_direction(int64_t np, const double* __restrict__ w, double* __restrict__ d,
+                                  const double* __restrict__ sc) {
+  pdl_entry();
+  const int k = (int)sc[U_IT];
+  const double b = k > 0 ? sc[U_RW2 + (k & 1)] / sc[U_RW2 + ((k & 1) ^ 1)] : 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x)
+    d[i] = k > 0 ? w[i] + b * d[i] : w[i];
+}
+
+// Convergence history of the iteration that k_schur_dots just ended, in the reference's terms
+// (uzawa3_solver_L2.py:85-88, cd_u_eta.py): xiV = ||alpha d_k||, xiP = ||alpha p_k||, alpha, beta.
+// hist is [4][len] (xiV, xiP, alpha, beta).
+__global__ void k_schur_history(const double* __restrict__ sc, double* __restrict__ hist, int len) {
+  pdl_entry();
+  const int row = (int)sc[I_OUTER] - 1, k = (int)sc[U_IT];
+  if (row < 0 || row >= len) return;
+  const double rw = sc[U_RW2 + ((k & 1) ^ 1)], alpha = rw / sc[U_DSD];
+  hist[row] = fabs(alpha) * sqrt(sc[U_Z2]);
+  hist[len + row] = fabs(alpha) * sqrt(sc[U_D2]);
+  hist[2 * len + row] = alpha;
+  hist[3 * len + row] = sc[U_RW2 + (k & 1)] / rw;
+}
+
+// (f, f) + (h, h) and the solve's counters; f or h of zero length
+__global__ void k_solve_init(int64_t nv, const double* __restrict__ f, int64_t np, const double* __restrict__ h,
+                             double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc) {
+  pdl_entry();
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+  double a = 0, b = 0;
+  for (int64_t i = t0; i < nv; i += nt) a += f[i] * f[i];
+  for (int64_t i = t0; i < np; i += nt) b += h[i] * h[i];
+  double sum[2];
+  if (grid_sum2(a, b, part, counter, blockIdx.x, gridDim.x, sum)) {
+    sc[S_BB] = sum[0];
+    sc[S_BH] = sum[1];
+    sc[S_BNORM] = sqrt(sum[0] + sum[1]);
+    sc[S_NREF] = sc[I_OUTER] = sc[I_INNER] = sc[I_STATUS] = 0;
+  }
+}
+
+// V += cV, P += cP
+__global__ void k_add_correction(int64_t nv, const double* __restrict__ cV, double* __restrict__ V, int64_t np,
+                                 const double* __restrict__ cP, double* __restrict__ P) {
+  pdl_entry();
+  const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t0; i < nv; i += nt) V[i] += cV[i];
+  for (int64_t i = t0; i < np; i += nt) P[i] += cP[i];
 }
 
 // (x, y) into the slot of the iteration's parity (hierarchies whose V-cycle does not sum it)
@@ -2906,308 +3016,6 @@ static int setup_hierarchy(mw_stokes* S, Hierarchy<R>& H, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? MW_OK : MW_ERR_CUDA;
 }
 
-static double read_scalar(const double* d, cudaStream_t s) {
-  double h = 0;
-  cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  return h;
-}
-
-// The pieces of the inner PCG for K x = b (b in double), preconditioned by a V-cycle at precision R;
-// driven by the host (pcg_K) or recorded as a device loop (pcg_K_dev).
-template <typename R>
-struct Pcg {
-  mw_stokes* S;
-  Hierarchy<R>& H;
-  R** pc;              // x, r, p (two buffers, by iteration parity), Ap
-  int64_t n;
-  ParitySum rz() const { return ParitySum{S->red, S->counter, S->sc + P_RZ2, S->sc + P_IT}; }
-
-  void start(const double* b, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
-    pdl_launch(k_pcg_start<R>, nb_for(n), 256, 0, s, n, b, pc[1], pc[0], S->red, S->counter, S->sc, dev ? 1 : 0, hw);
-  }
-  // z = V(r) into the finest level's x, (r, z)
-  void precondition(bool graph, cudaStream_t s) const {
-    Level<R>& L = H.L[0];
-    const ParitySum out = rz();
-    R* saved_b = L.b;
-    L.b = pc[1];
-    const bool fused = H.nlev > 1 && L.deg <= MG_MAXDEG;
-    if (graph) vcycle_run(S, H, fused ? &out : nullptr, s);
-    else vcycle(H, 0, s, false, fused ? &out : nullptr);
-    L.b = saved_b;
-    if (!fused) pdl_launch(k_dot_parity<R>, nb_for(n), 256, 0, s, n, (const R*)pc[1], (const R*)L.x, out);
-  }
-  void step(double rtol, int maxit, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
-    OpArgs<R> a = op_args(H.L[0], true);
-    a.yV = pc[4];
-    PcgDir<R> d{H.L[0].x, {pc[2], pc[3]}, S->sc + P_RZ2, S->sc + P_IT, S->red, S->sc + P_PAP, S->counter};
-    op_pcg_direction<R>(a, d, s);
-    pdl_launch(k_pcg_update<R>, nb_for(n), 256, 0, s, n, (const R*)pc[2], (const R*)pc[3], (const R*)pc[4], pc[0],
-               pc[1], S->red, S->counter, S->sc, rtol, maxit, dev ? 1 : 0, hw);
-  }
-  void finish(double* x, cudaStream_t s) const {
-    pdl_launch(k_pcg_finish<R>, grid_for(n, 256), 256, 0, s, n, (const R*)pc[0], x, S->sc);
-  }
-};
-
-// K x = b with the loop on the host; x is overwritten.  Returns iterations; *relres = ||r|| / ||b||.
-template <typename R>
-static int pcg_K(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double* x, double rtol, int maxit,
-                 double* relres, cudaStream_t s) {
-  const Pcg<R> P{S, H, pc, H.L[0].ndof};
-  P.start(b, false, 0, s);
-  const double bb = read_scalar(S->sc + P_BB, s);
-  double rr = bb;
-  int it = 0;
-  if (bb > 0) {
-    for (it = 1; it <= maxit; ++it) {
-      P.precondition(true, s);
-      P.step(rtol, maxit, false, 0, s);
-      rr = read_scalar(S->sc + P_RR, s);
-      if (!std::isfinite(rr)) break;
-      if (rr <= rtol * rtol * bb) break;
-    }
-    if (it > maxit) it = maxit;
-  }
-  P.finish(x, s);
-  *relres = bb > 0 ? std::sqrt(rr / bb) : 0;
-  return it;
-}
-
-// Jacobi-PCG for the (weighted) Q1 mass matrix: M_w x = b.  weights NULL -> M (uzawa3),
-// weights = 1/eta_e -> M_eta (cd_u_eta).
-// Solve M_w x = b (M_w = M for uzawa3, M_eta for cd_u_eta) by `iters` fixed-coefficient
-// Chebyshev-Jacobi steps on lambda(D^-1 M_w) in [0.25, 2.25] (see k_mass_cheb): error reduction
-// 2 (1/2)^iters, no dot products, no host synchronisation.  The diagonals are refreshed by
-// mw_stokes_set_viscosity.  Replaces the splu solves of uzawa3_solver_L2.py:46-47 / cd_u_eta.py:284-289.
-static void mass_solve_kernels(mw_stokes* S, const double* w, const double* b, double* x, int iters, cudaStream_t s);
-
-static int mass_solve(mw_stokes* S, const double* w, const double* b, double* x, int iters, cudaStream_t s) {
-  const int K = iters < 1 ? 1 : iters;
-  std::vector<void*> key = {(void*)w, (void*)b, (void*)x, (void*)(intptr_t)K};
-  graph_run(S, 1, [&]() { mass_solve_kernels(S, w, b, x, K, s); }, [&]() { return key; },
-            [&](const std::vector<void*>&) {}, s);
-  return K;
-}
-
-static void mass_solve_kernels(mw_stokes* S, const double* w, const double* b, double* x, int iters, cudaStream_t s) {
-  const LevelGeo& g = S->fine;
-  const int64_t n = (int64_t)(g.nx + 1) * (g.nz + 1);
-  const double* dg = w ? S->medi : S->mdiag;
-  const double a = 0.25 / 1.02, bb = 2.25 * 1.02;
-  const double theta = 0.5 * (bb + a), delta = 0.5 * (bb - a), sigma = theta / delta;
-  double rho = 1.0 / sigma;
-  double* bufs[2] = {x, S->tP};
-  const int K = iters < 1 ? 1 : iters;
-  for (int k = 0; k < K; ++k) {
-    double c1 = 0.0, c2 = 1.0 / theta;
-    if (k > 0) {
-      double rn = 1.0 / (2.0 * sigma - rho);
-      c1 = rn * rho;
-      c2 = 2.0 * rn / delta;
-      rho = rn;
-    }
-    double* xin = bufs[(K - k) % 2];
-    double* xout = bufs[(K - 1 - k) % 2];
-    pdl_launch(k_mass_cheb, grid_for(n, 256), 256, 0, s, g, w, b, xin, xout, S->tP2, dg, c1, c2, k == 0);
-  }
-}
-
-static void remove_mean(mw_stokes* S, int64_t n, double* x, cudaStream_t s) {
-  dsum(S, n, x, S->sc + 40, s);
-  pdl_launch(k_sub_mean, grid_for(n, 256), 256, 0, s, n, S->sc + 40, x);
-}
-
-// Full saddle residual in FP64: (RV, RP) = (f, h) - [K G; G^T 0] (V, P).  Returns ||R||/||b||
-// when bnorm > 0 (bnorm = ||(f, h)||), else ||R||.
-static double true_residual(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
-                            double bnorm, cudaStream_t s) {
-  const LevelGeo& g = S->fine;
-  OpArgs<double> a = op_args64(S);
-  a.u = V; a.p = P; a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
-  op_apply<double>(a, s);
-  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  dot<double>(S, nv, S->RV, S->RV, S->sc + 50, s);
-  dot<double>(S, np, S->RP, S->RP, S->sc + 51, s);
-  double a2[2];
-  cudaMemcpyAsync(a2, S->sc + 50, 2 * sizeof(double), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  double r = std::sqrt(a2[0] + a2[1]);
-  return bnorm > 0 ? r / bnorm : r;
-}
-
-// Inner K solve at the requested precision.
-static int ensure_hierarchy(mw_stokes* S, int prec, cudaStream_t s) {
-  if (prec == MW_F32) {
-    if (!S->has32) return MW_ERR_BAD_ARG;
-    if (S->dirty32) { int rc = setup_hierarchy<float>(S, S->H32, s); if (rc) return rc; S->dirty32 = false; }
-  } else {
-    if (!S->has64) return MW_ERR_BAD_ARG;
-    if (S->dirty64) { int rc = setup_hierarchy<double>(S, S->H64, s); if (rc) return rc; S->dirty64 = false; }
-  }
-  return MW_OK;
-}
-
-static int solve_K(mw_stokes* S, int prec, const double* b, double* x, double rtol, int maxit, double* relres,
-                   cudaStream_t s) {
-  if (prec == MW_F32) return pcg_K<float>(S, S->H32, S->pc32, b, x, rtol, maxit, relres, s);
-  return pcg_K<double>(S, S->H64, S->pc64, b, x, rtol, maxit, relres, s);
-}
-
-// Convergence history row k in the reference's terms (uzawa3_solver_L2.py:85-88, cd_u_eta.py):
-// xiV = ||alpha d_k||, xiP = ||alpha p_k||, alpha, beta.  hist is [4][len] (xiV, xiP, alpha, beta).
-__global__ void k_history(const double* __restrict__ sc, double* __restrict__ hist, int len, int k) {
-  pdl_entry();
-  const double alpha = sc[0] / sc[1];
-  hist[k] = fabs(alpha) * sqrt(sc[6]);
-  hist[len + k] = fabs(alpha) * sqrt(sc[5]);
-  hist[2 * len + k] = alpha;
-  hist[3 * len + k] = sc[2] / sc[0];
-}
-
-// Schur-complement PCG (uzawa3_solver_L2.py:21-99 / cd_u_eta.py:13-99) for the saddle system
-// with right-hand side (f, h), starting from (V, P) (V is recomputed from P).  Stops when the
-// Schur residual has dropped by `reduction` relative to its start, when the FP64 true residual
-// meets `tol` (checked each iteration if check_true), or after max_outer iterations.
-static int uzawa(mw_stokes* S, const mw_solve_params& sp, int prec, const double* f, const double* h, double* V,
-                 double* P, double reduction, bool check_true, double bnorm, mw_solve_info* info, cudaStream_t s) {
-  const LevelGeo& g = S->fine;
-  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  const double* w = sp.scheme == MW_SCHEME_UZAWA3 ? nullptr : S->etae_w;
-  double rel;
-  // V = K^-1 (f - G P)
-  grad_p(S, P, f, S->Gd, s);                                // Gd = f - G P
-  int inner = solve_K(S, prec, S->Gd, V, sp.inner_rtol, sp.max_inner, &rel, s);
-  info->inner_iters += inner;
-  // rho = G^T V - h
-  div_u(S, V, S->rP, s);                                    // rP = G^T V
-  if (h) pdl_launch(k_axpy<double>, grid_for(np, 256), 256, 0, s, np, -1.0, h, S->rP);
-  remove_mean(S, np, S->rP, s);
-  mass_solve(S, w, S->rP, S->wP, sp.mass_iters, s);
-  remove_mean(S, np, S->wP, s);
-  pdl_launch(k_copy<double, double>, grid_for(np, 256), 256, 0, s, np, S->wP, S->dP);
-  double* sc = S->sc + 24;    // [0] rw, [1] dSd, [2] rw_new, [3] rr0, [4] rr
-  dot<double>(S, np, S->rP, S->wP, sc + 0, s);
-  dot<double>(S, np, S->rP, S->rP, sc + 3, s);
-  const double rr0 = read_scalar(sc + 3, s);
-  int k;
-  for (k = 0; k < sp.max_outer; ++k) {
-    // z = K^-1 G d
-    grad_p(S, S->dP, nullptr, S->Gd, s);
-    inner = solve_K(S, prec, S->Gd, S->z, sp.inner_rtol, sp.max_inner, &rel, s);
-    info->inner_iters += inner;
-    // G^T z, step length alpha = (rho, w) / (d, G^T z)
-    div_u(S, S->z, S->GTz, s);
-    dot<double>(S, np, S->dP, S->GTz, sc + 1, s);
-    const bool hist = sp.history && info->outer_iters < sp.history_len;
-    if (hist) {                                               // ||d_k||^2, ||z_k||^2 before the updates
-      dot<double>(S, np, S->dP, S->dP, sc + 5, s);
-      dot<double>(S, nv, S->z, S->z, sc + 6, s);
-    }
-    pdl_launch(k_axpy_ratio<double, double>, grid_for(np, 256), 256, 0, s, np, sc + 0, sc + 1, 1.0, S->dP, P);
-    pdl_launch(k_axpy_ratio<double, double>, grid_for(nv, 256), 256, 0, s, nv, sc + 0, sc + 1, -1.0, S->z, V);
-    pdl_launch(k_axpy_ratio<double, double>, grid_for(np, 256), 256, 0, s, np, sc + 0, sc + 1, -1.0, S->GTz, S->rP);
-    remove_mean(S, np, S->rP, s);
-    mass_solve(S, w, S->rP, S->wP, sp.mass_iters, s);
-    remove_mean(S, np, S->wP, s);
-    dot<double>(S, np, S->rP, S->wP, sc + 2, s);
-    if (hist) pdl_launch(k_history, 1, 1, 0, s, sc, sp.history, sp.history_len, info->outer_iters);
-    pdl_launch(k_xpby_ratio<double>, grid_for(np, 256), 256, 0, s, np, S->wP, sc + 2, sc + 0, S->dP);
-    cudaMemcpyAsync(sc + 0, sc + 2, sizeof(double), cudaMemcpyDeviceToDevice, s);
-    info->outer_iters += 1;
-    dot<double>(S, np, S->rP, S->rP, sc + 4, s);
-    double rr = read_scalar(sc + 4, s);
-    if (!std::isfinite(rr)) return MW_ERR_NOT_CONVERGED;
-    if (check_true) {
-      double tr = true_residual(S, V, P, f, h, bnorm, s);
-      info->rel_residual = tr;
-      if (tr <= sp.tol) { ++k; break; }
-    }
-    if (rr <= reduction * reduction * rr0) { ++k; break; }
-  }
-  return MW_OK;
-}
-
-// ================================================================ device-side loops
-// The whole solve as one CUDA graph: the iterations run as conditional WHILE nodes whose bodies end
-// with a one-thread kernel that updates the loop scalars and sets the condition, so no iteration
-// waits for the host.  Every loop is bounded by its iteration cap (max_inner, max_outer,
-// max_refine) and by a total work cap, both decided on the device.  Scalars live in S->sc from
-// slot 64 on.
-__global__ void k_dev_uz_init(double* sc, int max_outer, cudaGraphConditionalHandle hw) {
-  pdl_entry();
-  sc[U_IT] = 0;
-  cudaGraphSetConditional(hw, (max_outer > 0 && isfinite(sc[U_RR0]) && sc[I_STATUS] == 0) ? 1u : 0u);
-}
-
-// one Schur iteration done: stop on a non-finite residual (status 2), on the FP64 true residual
-// (check_true), on the Schur residual reduction, at max_outer or at the work cap (status 3)
-__global__ void k_dev_uz_check(double* sc, double reduction, int check_true, double tol, int max_outer,
-                               cudaGraphConditionalHandle hw) {
-  pdl_entry();
-  const double it = sc[U_IT] + 1;
-  sc[U_IT] = it;
-  sc[I_OUTER] += 1;
-  const double rr = sc[U_RR];
-  if (reduction < 0) reduction = sc[S_RED];                   // this sweep's target (k_dev_sweep_red)
-  bool go = it < (double)max_outer;
-  if (!isfinite(rr)) { sc[I_STATUS] = 2; go = false; }
-  if (sc[I_OUTER] >= DEV_OUTER_BUDGET && sc[I_STATUS] == 0) sc[I_STATUS] = 3;
-  if (sc[I_STATUS] != 0) go = false;
-  if (check_true && sc[T_REL] <= tol) go = false;
-  if (rr <= reduction * reduction * sc[U_RR0]) go = false;
-  cudaGraphSetConditional(hw, go ? 1u : 0u);
-}
-
-__global__ void k_dev_hist(const double* sc, double* hist, int len) {
-  pdl_entry();
-  const int k = (int)sc[I_OUTER];
-  if (k < 0 || k >= len) return;
-  const double alpha = sc[U_RW] / sc[U_DSD];
-  hist[k] = fabs(alpha) * sqrt(sc[U_Z2]);
-  hist[len + k] = fabs(alpha) * sqrt(sc[U_D2]);
-  hist[2 * len + k] = alpha;
-  hist[3 * len + k] = sc[U_RWN] / sc[U_RW];
-}
-
-__global__ void k_dev_rel(double* sc) {
-  pdl_entry(); sc[T_REL] = sqrt(sc[T_RV] + sc[T_RP]) / sc[S_BNORM]; }
-
-__global__ void k_dev_solve_init(double* sc) {
-  pdl_entry();
-  sc[S_BNORM] = sqrt(sc[S_BB] + sc[S_BH]);
-  sc[S_NREF] = 0;
-  sc[I_OUTER] = 0;
-  sc[I_INNER] = 0;
-  sc[I_STATUS] = 0;
-}
-
-__global__ void k_dev_ref_init(double* sc, double tol, int max_refine, cudaGraphConditionalHandle hw) {
-  pdl_entry();
-  sc[S_REL0] = sc[T_REL];
-  const double r = sc[T_REL];
-  cudaGraphSetConditional(hw, (isfinite(r) && r > tol && max_refine > 0) ? 1u : 0u);
-}
-
-__global__ void k_dev_ref_check(double* sc, double tol, int max_refine, cudaGraphConditionalHandle hw) {
-  pdl_entry();
-  sc[S_NREF] += 1;
-  const double r = sc[T_REL];
-  const bool go = isfinite(r) && r > tol && sc[S_NREF] < (double)max_refine && sc[I_STATUS] == 0;
-  cudaGraphSetConditional(hw, go ? 1u : 0u);
-}
-
-// the reduction a refinement sweep's Schur iteration aims for: sweep_reduction, or -- with
-// target > 0 -- the smaller reduction that takes the current residual to target * tol
-__global__ void k_dev_sweep_red(double* sc, double sweep_reduction, double target, double tol) {
-  pdl_entry();
-  sc[S_RED] = sweep_target_reduction(sweep_reduction, target, tol, sc[T_REL]);
-}
-
-__global__ void k_copy1(const double* src, double* dst) {
-  pdl_entry(); *dst = *src; }
-
 // A conditional handle in the graph being captured on s (its value is set by kernels of that graph).
 static bool cond_handle(cudaStream_t s, cudaGraphConditionalHandle* h) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -3242,133 +3050,352 @@ static bool cond_end(cudaStream_t bs) {
   return cudaStreamEndCapture(bs, &g) == cudaSuccess;
 }
 
-// capture stream of nesting level `depth` (0: the solve's stream)
-static cudaStream_t lvl(mw_stokes* S, cudaStream_t s, int depth) { return depth == 0 ? s : S->bs[depth - 1]; }
+static double read_scalar(const double* d, cudaStream_t s) {
+  double h = 0;
+  cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, s);
+  cudaStreamSynchronize(s);
+  return h;
+}
 
-// Inner PCG for K x = b recorded with a device WHILE loop (capture only), at nesting level `depth`
-// (uses the body stream depth).  Adds its iteration count to sc[I_INNER].
+// rows of blocks of a kernel that sums over lattice rows: at most NB partial sums in all
+static int row_blocks(int rows, int gx) { return std::max(1, std::min(rows, NB / std::max(gx, 1))); }
+
+// The pieces of the inner PCG for K x = b (b in double), preconditioned by a V-cycle at precision R;
+// driven by the host (pcg_K) or recorded as a device loop (pcg_K_dev).
 template <typename R>
-static bool pcg_K_dev(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double* x, double rtol, int maxit,
-                      cudaStream_t s0, int depth) {
-  if (depth + 1 > 6) return false;
-  cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth];
-  const Pcg<R> P{S, H, pc, H.L[0].ndof};
-  cudaGraphConditionalHandle hw;
-  if (!cond_handle(s, &hw)) return false;
-  P.start(b, true, hw, s);
+struct Pcg {
+  mw_stokes* S;
+  Hierarchy<R>& H;
+  R** pc;              // x, r, p (two buffers, by iteration parity), Ap
+  int64_t n;
+  ParitySum rz() const { return ParitySum{S->red, S->counter, S->sc + P_RZ2, S->sc + P_IT}; }
+
+  void start(const double* b, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    pdl_launch(k_pcg_start<R>, nb_for(n), 256, 0, s, n, b, pc[1], pc[0], S->red, S->counter, S->sc, dev ? 1 : 0, hw);
+  }
+  // b = f - G p (f may be null: G p)
+  void start_grad(const double* p, const double* f, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    const LevelGeo& g = S->fine;
+    const int gx = (g.nnx + 127) / 128;
+    pdl_launch(k_pcg_start_grad<R>, dim3(gx, row_blocks(g.nnz, gx)), 128, 0, s, g, p, S->fixV, f, pc[1], pc[0], S->red,
+               S->counter, S->sc, dev ? 1 : 0, hw);
+  }
+  // z = V(r) into the finest level's x, (r, z)
+  void precondition(bool graph, cudaStream_t s) const {
+    Level<R>& L = H.L[0];
+    const ParitySum out = rz();
+    R* saved_b = L.b;
+    L.b = pc[1];
+    const bool fused = H.nlev > 1 && L.deg <= MG_MAXDEG;
+    if (graph) vcycle_run(S, H, fused ? &out : nullptr, s);
+    else vcycle(H, 0, s, false, fused ? &out : nullptr);
+    L.b = saved_b;
+    if (!fused) pdl_launch(k_dot_parity<R>, nb_for(n), 256, 0, s, n, (const R*)pc[1], (const R*)L.x, out);
+  }
+  void step(double rtol, int maxit, bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    OpArgs<R> a = op_args(H.L[0], true);
+    a.yV = pc[4];
+    PcgDir<R> d{H.L[0].x, {pc[2], pc[3]}, S->sc + P_RZ2, S->sc + P_IT, S->red, S->sc + P_PAP, S->counter};
+    op_pcg_direction<R>(a, d, s);
+    pdl_launch(k_pcg_update<R>, nb_for(n), 256, 0, s, n, (const R*)pc[2], (const R*)pc[3], (const R*)pc[4], pc[0],
+               pc[1], S->red, S->counter, S->sc, rtol, maxit, dev ? 1 : 0, hw);
+  }
+  void finish(double* x, cudaStream_t s) const {
+    pdl_launch(k_pcg_finish<R>, grid_for(n, 256), 256, 0, s, n, (const R*)pc[0], x, S->sc);
+  }
+};
+
+// The iterations of a started solve with the loop on the host.  Returns their number; *relres = ||r|| / ||b||.
+template <typename R>
+static int pcg_loop_host(const Pcg<R>& P, double rtol, int maxit, double* relres, cudaStream_t s) {
+  const double bb = read_scalar(P.S->sc + P_BB, s);
+  double rr = bb;
+  int it = 0;
+  if (bb > 0) {
+    for (it = 1; it <= maxit; ++it) {
+      P.precondition(true, s);
+      P.step(rtol, maxit, false, 0, s);
+      rr = read_scalar(P.S->sc + P_RR, s);
+      if (!std::isfinite(rr)) break;
+      if (rr <= rtol * rtol * bb) break;
+    }
+    if (it > maxit) it = maxit;
+  }
+  *relres = bb > 0 ? std::sqrt(rr / bb) : 0;
+  return it;
+}
+
+// The same as a device WHILE loop with handle hw (capture only), its body on stream b1.
+template <typename R>
+static bool pcg_loop_dev(const Pcg<R>& P, double rtol, int maxit, cudaGraphConditionalHandle hw, cudaStream_t s,
+                         cudaStream_t b1) {
   if (!cond_node(s, b1, cudaGraphCondTypeWhile, hw)) return false;
   P.precondition(false, b1);
   P.step(rtol, maxit, true, hw, b1);
-  if (!cond_end(b1)) return false;
+  return cond_end(b1);
+}
+
+// K x = b with the loop on the host; x is overwritten.
+template <typename R>
+static int pcg_K(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double* x, double rtol, int maxit,
+                 double* relres, cudaStream_t s) {
+  const Pcg<R> P{S, H, pc, H.L[0].ndof};
+  P.start(b, false, 0, s);
+  const int it = pcg_loop_host(P, rtol, maxit, relres, s);
   P.finish(x, s);
-  return true;
+  return it;
 }
 
-static bool solve_K_dev(mw_stokes* S, int prec, const double* b, double* x, double rtol, int maxit, cudaStream_t s0,
-                        int depth) {
-  if (prec == MW_F32) return pcg_K_dev<float>(S, S->H32, S->pc32, b, x, rtol, maxit, s0, depth);
-  return pcg_K_dev<double>(S, S->H64, S->pc64, b, x, rtol, maxit, s0, depth);
-}
-
-// FP64 true residual into sc[T_REL] (relative to sc[S_BNORM]); RV, RP hold the residual.
-static void true_residual_dev(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
-                              cudaStream_t s) {
+// Solve M_w x = b (M_w = M for uzawa3, weights null; M_eta for cd_u_eta, weights 1/eta_e) by `iters`
+// fixed-coefficient Chebyshev-Jacobi steps on lambda(D^-1 M_w) in [0.25, 2.25] (see mass_cheb_node): error
+// reduction 2 (1/2)^iters, no dot products, no host synchronisation.  The diagonals are refreshed by
+// mw_stokes_set_viscosity.  Replaces the splu solves of uzawa3_solver_L2.py:46-47 / cd_u_eta.py:284-289.
+// The first step removes b's mean (its sum in U_M1) and clears `zero` (may be null); the last leaves the
+// sum of x in U_M2.
+static void mass_solve(mw_stokes* S, const double* w, double* b, double* x, int iters, double* zero, cudaStream_t s) {
   const LevelGeo& g = S->fine;
+  const int64_t n = (int64_t)(g.nx + 1) * (g.nz + 1);
+  const double* dg = w ? S->medi : S->mdiag;
+  const double a = 0.25 / 1.02, bb = 2.25 * 1.02;
+  const double theta = 0.5 * (bb + a), delta = 0.5 * (bb - a), sigma = theta / delta;
+  double rho = 1.0 / sigma;
+  double* bufs[2] = {x, S->tP};
+  const int K = iters < 1 ? 1 : iters;
+  for (int k = 0; k < K; ++k) {
+    double c1 = 0.0, c2 = 1.0 / theta;
+    if (k > 0) {
+      double rn = 1.0 / (2.0 * sigma - rho);
+      c1 = rn * rho;
+      c2 = 2.0 * rn / delta;
+      rho = rn;
+    }
+    double* xin = bufs[(K - k) % 2];
+    double* xout = bufs[(K - 1 - k) % 2];
+    pdl_launch(k_mass_cheb, std::min(grid_for(n, 256), NB), 256, 0, s, g, w, b, xin, xout, S->tP2, dg, c1, c2, k == 0,
+               k == 0 ? (const double*)(S->sc + U_M1) : nullptr, k == 0 ? zero : nullptr, S->red, S->counter,
+               k == K - 1 ? S->sc + U_M2 : nullptr);
+  }
+}
+
+static void remove_mean(mw_stokes* S, int64_t n, double* x, cudaStream_t s) {
+  dsum(S, n, x, S->sc + 40, s);
+  pdl_launch(k_sub_mean, grid_for(n, 256), 256, 0, s, n, S->sc + 40, x);
+}
+
+// Full saddle residual in FP64: (RV, RP) = (f, h) - [K G; G^T 0] (V, P); T_RV = its sum of squares, T_REL
+// relative to S_BNORM, and what `action` asks for.
+static void true_residual(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
+                          int action, const LoopTest& test, cudaStream_t s) {
   OpArgs<double> a = op_args64(S);
   a.u = V; a.p = P; a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
-  op_apply<double>(a, s);
-  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  dot<double>(S, nv, S->RV, S->RV, S->sc + T_RV, s);
-  dot<double>(S, np, S->RP, S->RP, S->sc + T_RP, s);
-  pdl_launch(k_dev_rel, 1, 1, 0, s, S->sc);
+  op_residual(a, ResidSum{S->red, S->sc, S->counter, action, test}, s);
 }
 
+// Inner K solve at the requested precision.
+static int ensure_hierarchy(mw_stokes* S, int prec, cudaStream_t s) {
+  if (prec == MW_F32) {
+    if (!S->has32) return MW_ERR_BAD_ARG;
+    if (S->dirty32) { int rc = setup_hierarchy<float>(S, S->H32, s); if (rc) return rc; S->dirty32 = false; }
+  } else {
+    if (!S->has64) return MW_ERR_BAD_ARG;
+    if (S->dirty64) { int rc = setup_hierarchy<double>(S, S->H64, s); if (rc) return rc; S->dirty64 = false; }
+  }
+  return MW_OK;
+}
+
+static int solve_K(mw_stokes* S, int prec, const double* b, double* x, double rtol, int maxit, double* relres,
+                   cudaStream_t s) {
+  if (prec == MW_F32) return pcg_K<float>(S, S->H32, S->pc32, b, x, rtol, maxit, relres, s);
+  return pcg_K<double>(S, S->H64, S->pc64, b, x, rtol, maxit, relres, s);
+}
+
+// The pieces of the Schur-complement CG (uzawa3_solver_L2.py:21-99 / cd_u_eta.py:13-99) for the saddle
+// system with right-hand side (f, h), starting from pressure P (from_zero: from zero, whatever P holds);
+// V is recomputed from it.
+template <typename R>
+struct Schur {
+  mw_stokes* S;
+  const Pcg<R> pcg;
+  const mw_solve_params& sp;
+  const double *f, *h;
+  double *V, *P;
+  bool from_zero;
+  int64_t nv() const { return 2LL * S->fine.nnx * S->fine.nnz; }
+  int64_t np() const { return (int64_t)(S->fine.nx + 1) * (S->fine.nz + 1); }
+  const double* weights() const { return sp.scheme == MW_SCHEME_UZAWA3 ? nullptr : S->etae_w; }
+
+  void div(double* out, const double* hh, double* Vout, const double* d, cudaStream_t s) const {
+    const LevelGeo& g = S->fine;
+    const int gx = (g.nx + 1 + 127) / 128;
+    pdl_launch(k_schur_div<R>, dim3(gx, row_blocks(g.nz + 1, gx)), 128, 0, s, g, (const R*)pcg.pc[0], S->fixV, out, hh,
+               Vout, d, S->red, S->counter, S->sc);
+  }
+  void tail(bool first, const LoopTest& t, cudaStream_t s) const {
+    mass_solve(S, weights(), S->rP, S->wP, sp.mass_iters, first && from_zero ? P : nullptr, s);
+    pdl_launch(k_schur_dots, nb_for(np()), 256, 0, s, np(), S->wP, (const double*)S->rP, first ? 1 : 0, S->red,
+               S->counter, S->sc, t);
+    if (!first && sp.history && sp.history_len > 0)
+      pdl_launch(k_schur_history, 1, 1, 0, s, (const double*)S->sc, sp.history, sp.history_len);
+    pdl_launch(k_schur_direction, grid_for(np(), 256), 256, 0, s, np(), (const double*)S->wP, S->dP,
+               (const double*)S->sc);
+  }
+  // V = K^-1 (f - G P)
+  void start_initial(bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    if (from_zero) pcg.start(f, dev, hw, s);
+    else pcg.start_grad(P, f, dev, hw, s);
+  }
+  // rho = G^T V - h, w, d, and the loop's start
+  void begin(const LoopTest& t, cudaStream_t s) const {
+    div(S->rP, h, V, nullptr, s);
+    tail(true, t, s);
+  }
+  // z = K^-1 G d
+  void start_direction(bool dev, cudaGraphConditionalHandle hw, cudaStream_t s) const {
+    pcg.start_grad(S->dP, nullptr, dev, hw, s);
+  }
+  // the rest of an iteration; with check_true the FP64 true residual decides
+  void iterate(const LoopTest& t, cudaStream_t s) const {
+    div(S->GTz, nullptr, nullptr, S->dP, s);
+    if (sp.history && sp.history_len > 0) {                   // ||d_k||^2, ||z_k||^2 before the updates
+      dot<double>(S, np(), S->dP, S->dP, S->sc + U_D2, s);
+      dot<R>(S, nv(), pcg.pc[0], pcg.pc[0], S->sc + U_Z2, s);
+    }
+    pdl_launch(k_schur_update<R>, nb_for(nv()), 256, 0, s, nv(), np(), (const double*)S->dP, (const R*)pcg.pc[0],
+               (const double*)S->GTz, P, V, S->rP, S->red, S->counter, S->sc);
+    tail(false, t, s);
+    if (t.check_true) true_residual(S, V, P, f, h, RA_SCHUR, t, s);
+  }
+};
+
+static LoopTest schur_loop_test(const mw_solve_params& sp, double reduction, bool check_true, bool dev,
+                                cudaGraphConditionalHandle hw) {
+  LoopTest t;
+  memset(&t, 0, sizeof(t));
+  t.device = dev ? 1 : 0;
+  t.handle = hw;
+  t.tol = sp.tol;
+  t.max_count = sp.max_outer;
+  t.check_true = check_true ? 1 : 0;
+  t.reduction = reduction;
+  return t;
+}
+
+// Stops when the Schur residual has dropped by `reduction` relative to its start, when the FP64 true
+// residual meets `tol` (checked each iteration if check_true), or after max_outer iterations.
+template <typename R>
+static int uzawa(const Schur<R>& U, double reduction, bool check_true, mw_solve_info* info, cudaStream_t s) {
+  const mw_solve_params& sp = U.sp;
+  double* sc = U.S->sc;
+  double rel;
+  const LoopTest t = schur_loop_test(sp, reduction, check_true, false, 0);
+  U.start_initial(false, 0, s);
+  info->inner_iters += pcg_loop_host(U.pcg, sp.inner_rtol, sp.max_inner, &rel, s);
+  U.begin(t, s);
+  const double rr0 = read_scalar(sc + U_RR0, s);
+  for (int k = 0; k < sp.max_outer; ++k) {
+    U.start_direction(false, 0, s);
+    info->inner_iters += pcg_loop_host(U.pcg, sp.inner_rtol, sp.max_inner, &rel, s);
+    U.iterate(t, s);
+    info->outer_iters += 1;
+    const double rr = read_scalar(sc + U_RR, s);
+    if (!std::isfinite(rr)) return MW_ERR_NOT_CONVERGED;
+    if (check_true) {
+      info->rel_residual = read_scalar(sc + T_REL, s);
+      if (info->rel_residual <= sp.tol) break;
+    }
+    if (rr <= reduction * reduction * rr0) break;
+  }
+  return MW_OK;
+}
+
+// ================================================================ device-side loops
+// The whole solve as one CUDA graph: the iterations run as conditional WHILE nodes whose bodies end
+// with a one-thread kernel that updates the loop scalars and sets the condition, so no iteration
+// waits for the host.  Every loop is bounded by its iteration cap (max_inner, max_outer,
+// max_refine) and by a total work cap, both decided on the device.  Scalars live in S->sc from
+// slot 64 on.
+// capture stream of nesting level `depth` (0: the solve's stream)
+static cudaStream_t lvl(mw_stokes* S, cudaStream_t s, int depth) { return depth == 0 ? s : S->bs[depth - 1]; }
+
 // Schur-complement CG (the recurrences of the host version `uzawa`) recorded with a device WHILE
-// loop at nesting level `depth` (uses body streams depth .. depth + 1).
-static bool uzawa_dev(mw_stokes* S, const mw_solve_params& sp, int prec, const double* f, const double* h, double* V,
-                      double* P, double reduction, bool check_true, cudaStream_t s0, int depth) {
+// loop at nesting level `depth` (uses body streams depth and depth + 1).
+template <typename R>
+static bool uzawa_dev(const Schur<R>& U, double reduction, bool check_true, cudaStream_t s0, int depth) {
   if (depth + 2 > 6) return false;
-  cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth];
+  mw_stokes* S = U.S;
+  const mw_solve_params& sp = U.sp;
+  cudaStream_t s = lvl(S, s0, depth), b1 = S->bs[depth], b2 = S->bs[depth + 1];
+  cudaGraphConditionalHandle hi, hw, hz;
+  if (!cond_handle(s, &hi)) return false;
+  U.start_initial(true, hi, s);
+  if (!pcg_loop_dev(U.pcg, sp.inner_rtol, sp.max_inner, hi, s, b1)) return false;
+  if (!cond_handle(s, &hw)) return false;
+  const LoopTest t = schur_loop_test(sp, reduction, check_true, true, hw);
+  U.begin(t, s);
+  if (!cond_node(s, b1, cudaGraphCondTypeWhile, hw)) return false;
+  if (!cond_handle(b1, &hz)) return false;
+  U.start_direction(true, hz, b1);
+  if (!pcg_loop_dev(U.pcg, sp.inner_rtol, sp.max_inner, hz, b1, b2)) return false;
+  U.iterate(t, b1);
+  return cond_end(b1);
+}
+
+static LoopTest refine_test(const mw_solve_params& sp, int max_refine, bool dev, cudaGraphConditionalHandle hc) {
+  LoopTest t;
+  memset(&t, 0, sizeof(t));
+  t.device = dev ? 1 : 0;
+  t.handle = hc;
+  t.tol = sp.tol;
+  t.max_count = max_refine;
+  t.sweep_reduction = sp.sweep_reduction;
+  t.sweep_target = sp.sweep_target;
+  return t;
+}
+
+// The norm of (f, h), zeros for a solve without a guess
+static void solve_begin(mw_stokes* S, const double* f, const double* h, double* V, double* P,
+                        const mw_solve_params& sp, cudaStream_t s) {
   const LevelGeo& g = S->fine;
   const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  const double* w = sp.scheme == MW_SCHEME_UZAWA3 ? nullptr : S->etae_w;
-  double* sc = S->sc;
-  grad_p(S, P, f, S->Gd, s);                                // V = K^-1 (f - G P)
-  if (!solve_K_dev(S, prec, S->Gd, V, sp.inner_rtol, sp.max_inner, s0, depth)) return false;
-  div_u(S, V, S->rP, s);                                    // rho = G^T V - h
-  if (h) pdl_launch(k_axpy<double>, grid_for(np, 256), 256, 0, s, np, -1.0, h, S->rP);
-  remove_mean(S, np, S->rP, s);
-  mass_solve(S, w, S->rP, S->wP, sp.mass_iters, s);
-  remove_mean(S, np, S->wP, s);
-  pdl_launch(k_copy<double, double>, grid_for(np, 256), 256, 0, s, np, S->wP, S->dP);
-  dot<double>(S, np, S->rP, S->wP, sc + U_RW, s);
-  dot<double>(S, np, S->rP, S->rP, sc + U_RR0, s);
-  cudaGraphConditionalHandle hw;
-  if (!cond_handle(s, &hw)) return false;
-  pdl_launch(k_dev_uz_init, 1, 1, 0, s, sc, sp.max_outer, hw);
-  if (!cond_node(s, b1, cudaGraphCondTypeWhile, hw)) return false;
-  grad_p(S, S->dP, nullptr, S->Gd, b1);
-  if (!solve_K_dev(S, prec, S->Gd, S->z, sp.inner_rtol, sp.max_inner, s0, depth + 1)) return false;
-  div_u(S, S->z, S->GTz, b1);
-  dot<double>(S, np, S->dP, S->GTz, sc + U_DSD, b1);
-  const bool hist = sp.history && sp.history_len > 0;
-  if (hist) {
-    dot<double>(S, np, S->dP, S->dP, sc + U_D2, b1);
-    dot<double>(S, nv, S->z, S->z, sc + U_Z2, b1);
+  if (!sp.use_guess) {
+    pdl_launch(k_set<double>, grid_for(nv, 256), 256, 0, s, nv, 0.0, V);
+    pdl_launch(k_set<double>, grid_for(np, 256), 256, 0, s, np, 0.0, P);
   }
-  pdl_launch(k_axpy_ratio<double, double>, grid_for(np, 256), 256, 0, b1, np, sc + U_RW, sc + U_DSD, 1.0, S->dP, P);
-  pdl_launch(k_axpy_ratio<double, double>, grid_for(nv, 256), 256, 0, b1, nv, sc + U_RW, sc + U_DSD, -1.0, S->z, V);
-  pdl_launch(k_axpy_ratio<double, double>, grid_for(np, 256), 256, 0, b1, np, sc + U_RW, sc + U_DSD, -1.0, S->GTz,
-             S->rP);
-  remove_mean(S, np, S->rP, b1);
-  mass_solve(S, w, S->rP, S->wP, sp.mass_iters, b1);
-  remove_mean(S, np, S->wP, b1);
-  dot<double>(S, np, S->rP, S->wP, sc + U_RWN, b1);
-  if (hist) pdl_launch(k_dev_hist, 1, 1, 0, b1, sc, sp.history, sp.history_len);
-  pdl_launch(k_xpby_ratio<double>, grid_for(np, 256), 256, 0, b1, np, S->wP, sc + U_RWN, sc + U_RW, S->dP);
-  pdl_launch(k_copy1, 1, 1, 0, b1, sc + U_RWN, sc + U_RW);
-  dot<double>(S, np, S->rP, S->rP, sc + U_RR, b1);
-  if (check_true) true_residual_dev(S, V, P, f, h, b1);
-  pdl_launch(k_dev_uz_check, 1, 1, 0, b1, sc, reduction, check_true ? 1 : 0, sp.tol, sp.max_outer, hw);
-  return cond_end(b1);
+  pdl_launch(k_solve_init, nb_for(nv), 256, 0, s, nv, f, h ? np : (int64_t)0, h, S->red, S->counter, S->sc);
+}
+
+// A refinement sweep solves A (cV, cP) = (RV, RP) from zero: the residual is read where the last
+// true residual left it (the sweep's Schur iteration needs it only to start).
+static Schur<float> sweep(mw_stokes* S, const mw_solve_params& sp) {
+  return Schur<float>{S, Pcg<float>{S, S->H32, S->pc32, S->H32.L[0].ndof}, sp, S->RV, S->RP, S->cV, S->cP, true};
+}
+
+static void add_correction(mw_stokes* S, double* V, double* P, cudaStream_t s) {
+  const LevelGeo& g = S->fine;
+  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
+  pdl_launch(k_add_correction, grid_for(nv, 256), 256, 0, s, nv, (const double*)S->cV, V, np, (const double*)S->cP, P);
 }
 
 // The whole solve (FP64, or mixed: FP64 refinement around FP32-inner Schur sweeps), recorded.
 static bool stokes_solve_record(mw_stokes* S, const double* f, const double* h, double* V, double* P,
                                 const mw_solve_params& sp, cudaStream_t s) {
-  const LevelGeo& g = S->fine;
-  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  double* sc = S->sc;
-  if (!sp.use_guess) {
-    pdl_launch(k_set<double>, grid_for(nv, 256), 256, 0, s, nv, 0.0, V);
-    pdl_launch(k_set<double>, grid_for(np, 256), 256, 0, s, np, 0.0, P);
-  }
-  dot<double>(S, nv, f, f, sc + S_BB, s);
-  dot<double>(S, np, h, h, sc + S_BH, s);
-  pdl_launch(k_dev_solve_init, 1, 1, 0, s, sc);
-  true_residual_dev(S, V, P, f, h, s);
+  solve_begin(S, f, h, V, P, sp, s);
   cudaGraphConditionalHandle hc;
   if (!cond_handle(s, &hc)) return false;
-  if (sp.precision == MW_F64) {
-    pdl_launch(k_dev_ref_init, 1, 1, 0, s, sc, sp.tol, 1, hc);        // records the initial residual; gate on tol
-    if (!cond_node(s, S->bs[0], cudaGraphCondTypeIf, hc)) return false;
-    if (!uzawa_dev(S, sp, MW_F64, f, h, V, P, 0.0, true, s, 1)) return false;
-    if (!cond_end(S->bs[0])) return false;
-    true_residual_dev(S, V, P, f, h, s);
+  const bool f64 = sp.precision == MW_F64;
+  const LoopTest t = refine_test(sp, f64 ? 1 : sp.max_refine, true, hc);
+  true_residual(S, V, P, f, h, RA_FIRST, t, s);              // records the initial residual; gate on tol
+  cudaStream_t b = S->bs[0];
+  if (!cond_node(s, b, f64 ? cudaGraphCondTypeIf : cudaGraphCondTypeWhile, hc)) return false;
+  if (f64) {
+    const Schur<double> U{S, Pcg<double>{S, S->H64, S->pc64, S->H64.L[0].ndof}, sp, f, h, V, P, false};
+    if (!uzawa_dev(U, 0.0, true, s, 1)) return false;
+    if (!cond_end(b)) return false;
+    true_residual(S, V, P, f, h, RA_NONE, t, s);
   } else {
-    pdl_launch(k_dev_ref_init, 1, 1, 0, s, sc, sp.tol, sp.max_refine, hc);
-    if (!cond_node(s, S->bs[0], cudaGraphCondTypeWhile, hc)) return false;
-    cudaStream_t b = S->bs[0];
-    pdl_launch(k_copy<double, double>, grid_for(nv, 256), 256, 0, b, nv, S->RV, S->f);
-    pdl_launch(k_copy<double, double>, grid_for(np, 256), 256, 0, b, np, S->RP, S->h);
-    pdl_launch(k_set<double>, grid_for(nv, 256), 256, 0, b, nv, 0.0, S->cV);
-    pdl_launch(k_set<double>, grid_for(np, 256), 256, 0, b, np, 0.0, S->cP);
-    pdl_launch(k_dev_sweep_red, 1, 1, 0, b, sc, sp.sweep_reduction, sp.sweep_target, sp.tol);
-    if (!uzawa_dev(S, sp, MW_F32, S->f, S->h, S->cV, S->cP, -1.0, false, s, 1)) return false;
-    pdl_launch(k_axpy<double>, grid_for(nv, 256), 256, 0, b, nv, 1.0, S->cV, V);
-    pdl_launch(k_axpy<double>, grid_for(np, 256), 256, 0, b, np, 1.0, S->cP, P);
-    true_residual_dev(S, V, P, f, h, b);
-    pdl_launch(k_dev_ref_check, 1, 1, 0, b, sc, sp.tol, sp.max_refine, hc);
+    if (!uzawa_dev(sweep(S, sp), -1.0, false, s, 1)) return false;
+    add_correction(S, V, P, b);
+    true_residual(S, V, P, f, h, RA_SWEEP, t, b);
     if (!cond_end(b)) return false;
   }
   return true;
@@ -3658,7 +3685,8 @@ int mw_stokes_residual(mw_stokes* S, const double* V, const double* P, const dou
                        double* RP, double* norm_out, void* stream) {
   if (!f || !h || !pair_aligned(V, 16) || !pair_aligned(f, 16)) return MW_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  double r = true_residual(S, V, P, f, h, 0.0, s);
+  true_residual(S, V, P, f, h, RA_NONE, refine_test(mw_solve_params{}, 0, false, 0), s);
+  const double r = std::sqrt(read_scalar(S->sc + T_RV, s));
   if (RV) cudaMemcpyAsync(RV, S->RV, sizeof(double) * 2 * S->fine.nnx * S->fine.nnz, cudaMemcpyDeviceToDevice, s);
   if (RP) cudaMemcpyAsync(RP, S->RP, sizeof(double) * (S->fine.nx + 1) * (S->fine.nz + 1), cudaMemcpyDeviceToDevice, s);
   if (norm_out) *norm_out = r;
@@ -3840,58 +3868,42 @@ static int stokes_solve(mw_stokes* S, const double* f, const double* h, double* 
 
 static int stokes_solve_host(mw_stokes* S, const double* f, const double* h, double* solV, double* solP,
                              const mw_solve_params& sp, mw_solve_info* info, cudaStream_t s) {
-  const LevelGeo& g = S->fine;
-  const int64_t nv = 2LL * g.nnx * g.nnz, np = (int64_t)(g.nx + 1) * (g.nz + 1);
   mw_solve_info inf;
   memset(&inf, 0, sizeof(inf));
   if (!f || !h || !solV || !solP) return MW_ERR_BAD_ARG;
   if (int rc = ensure_hierarchy(S, sp.precision == MW_F32 ? MW_F32 : MW_F64, s)) return rc;
-  if (!sp.use_guess) {
-    pdl_launch(k_set<double>, grid_for(nv, 256), 256, 0, s, nv, 0.0, solV);
-    pdl_launch(k_set<double>, grid_for(np, 256), 256, 0, s, np, 0.0, solP);
-  }
-  // ||b||
-  dot<double>(S, nv, f, f, S->sc + 52, s);
-  if (h) dot<double>(S, np, h, h, S->sc + 53, s);
-  double bb[2] = {0, 0};
-  cudaMemcpyAsync(bb, S->sc + 52, (h ? 2 : 1) * sizeof(double), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  const double bnorm = std::sqrt(bb[0] + bb[1]);
+  solve_begin(S, f, h, solV, solP, sp, s);
+  const double bnorm = read_scalar(S->sc + S_BNORM, s);
   if (!std::isfinite(bnorm)) {
     inf.rel_residual = inf.initial_rel_residual = bnorm;
     if (info) *info = inf;
     return MW_ERR_NOT_CONVERGED;
   }
   if (!(bnorm > 0)) { if (info) *info = inf; return MW_OK; }
-  inf.initial_rel_residual = true_residual(S, solV, solP, f, h, bnorm, s);
+  const LoopTest t = refine_test(sp, sp.max_refine, false, 0);
+  auto residual = [&](int action) {
+    true_residual(S, solV, solP, f, h, action, t, s);
+    return read_scalar(S->sc + T_REL, s);
+  };
+  inf.initial_rel_residual = residual(RA_FIRST);
   int rc = MW_OK;
   if (sp.precision == MW_F64) {
     // plain FP64: one Schur-PCG run with the true residual checked every iteration
     inf.rel_residual = inf.initial_rel_residual;
     if (inf.rel_residual > sp.tol)
-      rc = uzawa(S, sp, MW_F64, f, h, solV, solP, 0.0, true, bnorm, &inf, s);
-    inf.rel_residual = true_residual(S, solV, solP, f, h, bnorm, s);
+      rc = uzawa(Schur<double>{S, Pcg<double>{S, S->H64, S->pc64, S->H64.L[0].ndof}, sp, f, h, solV, solP, false}, 0.0,
+                 true, &inf, s);
+    inf.rel_residual = residual(RA_NONE);
   } else {
-    // mixed: FP64 iterative refinement around an FP32-inner Uzawa correction solve
+    // mixed: FP64 iterative refinement around an FP32-inner Schur correction solve
     double rel = inf.initial_rel_residual;
     for (int it = 0; it < sp.max_refine && rel > sp.tol; ++it) {
-      // residual (RV, RP) is current in S->RV / S->RP from true_residual
-      double* cV = S->cV;
-      // solve A (cV, cP) = (RV, RP): copy the residual into f/h slots, zero guess
-      double* fr = S->f;
-      double* hr = S->h;
-      pdl_launch(k_copy<double, double>, grid_for(nv, 256), 256, 0, s, nv, S->RV, fr);
-      pdl_launch(k_copy<double, double>, grid_for(np, 256), 256, 0, s, np, S->RP, hr);
-      pdl_launch(k_set<double>, grid_for(nv, 256), 256, 0, s, nv, 0.0, cV);
-      double* cPr = S->cP;
-      pdl_launch(k_set<double>, grid_for(np, 256), 256, 0, s, np, 0.0, cPr);
-      rc = uzawa(S, sp, MW_F32, fr, hr, cV, cPr, sweep_target_reduction(sp.sweep_reduction, sp.sweep_target, sp.tol, rel),
-                 false, 0.0, &inf, s);
+      rc = uzawa(sweep(S, sp), sweep_target_reduction(sp.sweep_reduction, sp.sweep_target, sp.tol, rel), false, &inf,
+                 s);
       if (rc) break;
-      pdl_launch(k_axpy<double>, grid_for(nv, 256), 256, 0, s, nv, 1.0, cV, solV);
-      pdl_launch(k_axpy<double>, grid_for(np, 256), 256, 0, s, np, 1.0, cPr, solP);
+      add_correction(S, solV, solP, s);
       inf.refinements += 1;
-      rel = true_residual(S, solV, solP, f, h, bnorm, s);
+      rel = residual(RA_SWEEP);
       inf.rel_residual = rel;
     }
     inf.rel_residual = rel;

@@ -283,7 +283,7 @@ MW_D void ens_remove_mean(EnsCtx& c, double* x, int64_t n) {
   cluster_barrier();
 }
 
-// x = (the fixed-interval Chebyshev-Jacobi steps of mass_solve_kernels) M_w^-1 b
+// x = (the fixed-interval Chebyshev-Jacobi steps of mass_solve) M_w^-1 b
 MW_D void ens_mass_solve(EnsCtx& c, const double* w, const double* b, double* x, int iters) {
   const EnsMember& M = *c.M;
   const int64_t n = (int64_t)(M.g.nx + 1) * (M.g.nz + 1);
