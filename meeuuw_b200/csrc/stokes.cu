@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "mg_level.cuh"
+#include "mg_setup.cuh"
 #include "op_apply.cuh"
 #include "q2_ref.cuh"
 
@@ -54,7 +55,8 @@ static int ensure_ref_tables() {
   if (g_ref_ready) return MW_OK;
   RefTables T;
   host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || op_ensure_tables())
+  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || op_ensure_tables() ||
+      setup_ensure_tables())
     return MW_ERR_CUDA;
   g_ref_ready = true;
   return MW_OK;
@@ -1574,31 +1576,12 @@ __global__ void k_cheb_first(int64_t n, const double* __restrict__ cheb, const R
   }
 }
 
-// power iteration helper for lambda_max(D^-1 K)
-template <typename R>
-__global__ void k_dinv(int64_t n, const R* __restrict__ y, const R* __restrict__ diag, R* __restrict__ x) {
-  pdl_entry();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    x[i] = y[i] / diag[i];
-}
-
 // Chebyshev coefficients from lambda_max (stored at lam[0] as ||D^-1 K x||^2 with ||x|| = 1).
 __global__ void k_cheb_coeffs(const double* __restrict__ lam2, int degree, double ratio, double safety,
                               double* __restrict__ coef) {
   pdl_entry();
   if (threadIdx.x || blockIdx.x) return;
-  double lmax = sqrt(fmax(*lam2, 1e-300)) * safety;
-  double lmin = lmax / ratio;
-  double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin), sigma = theta / delta;
-  double rho = 1.0 / sigma;
-  coef[0] = 0.0;                             // step 0: d = (1/theta) D^-1 r
-  coef[1] = 1.0 / theta;
-  for (int k = 1; k < degree; ++k) {
-    double rn = 1.0 / (2.0 * sigma - rho);
-    coef[2 * k] = rn * rho;                  // c1: d = c1 d + c2 D^-1 r
-    coef[2 * k + 1] = 2.0 * rn / delta;
-    rho = rn;
-  }
+  cheb_coefficients(*lam2, degree, ratio, safety, coef);
 }
 
 // ---------------------------------------------------------------- coarsest level: dense inverse
@@ -1638,35 +1621,7 @@ __global__ void k_dense_assemble(LevelGeo g, const R* __restrict__ eta, const ui
   }
 }
 
-// In-place Gauss-Jordan inversion of an SPD matrix, one CTA.
-// Same inversion with the whole matrix held in shared memory (nd*nd doubles + a column).
-__global__ void k_gauss_jordan_smem(int nd, double* __restrict__ Ag) {
-  pdl_entry();
-  extern __shared__ double sm[];
-  double* A = sm;
-  double* col = sm + (size_t)nd * nd;
-  for (int t = threadIdx.x; t < nd * nd; t += blockDim.x) A[t] = Ag[t];
-  // rows over warps, columns over lanes: no index division in the elimination sweep
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int k = 0; k < nd; ++k) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < nd; i += blockDim.x) col[i] = A[i * nd + k];
-    __syncthreads();
-    const double piv = 1.0 / col[k];
-    for (int j = threadIdx.x; j < nd; j += blockDim.x) A[k * nd + j] = (j == k ? 1.0 : A[k * nd + j]) * piv;
-    __syncthreads();
-    const double* rk = A + k * nd;
-    for (int i = warp; i < nd; i += nwarp) {
-      if (i == k) continue;
-      const double ci = col[i];
-      double* ri = A + i * nd;
-      for (int j = lane; j < nd; j += 32) ri[j] = (j == k ? 0.0 : ri[j]) - ci * rk[j];
-    }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nd * nd; t += blockDim.x) Ag[t] = A[t];
-}
-
+// In-place Gauss-Jordan inversion of an SPD matrix too large for dense_inverse, one CTA.
 __global__ void k_gauss_jordan(int nd, double* __restrict__ A) {
   pdl_entry();
   extern __shared__ double col[];
@@ -2119,7 +2074,6 @@ constexpr int NB = 1184;          // reduction partials: up to 8 CTAs per SM
 // CTAs of a reduction over n values: enough to keep HBM busy on long vectors (at least 4 values
 // per thread), one on short ones
 static int nb_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(NB, (n + 1023) / 1024)); }
-constexpr int MAXLEV = 12;
 constexpr int MAXDEG = 8;
 constexpr int MAX_TAIL = 6;       // levels of the one-CTA V-cycle tail
 
@@ -2295,9 +2249,9 @@ static size_t layout(mw_stokes* S, Arena& A) {
                    &S->medi, &S->cP};
   for (auto p : pv) *p = (double*)A.take(sizeof(double) * np);
   S->etae_w = (double*)A.take(sizeof(double) * nel);
-  S->red = (double*)A.take(sizeof(double) * std::max(NB * 4, cell_partials(g.nx, g.nz)));
+  S->red = (double*)A.take(sizeof(double) * std::max(NB * 4, 2 * cell_partials(g.nx, g.nz) + 64));
   S->sc = (double*)A.take(sizeof(double) * 256);
-  S->counter = (unsigned*)A.take(sizeof(unsigned) * 4);
+  S->counter = (unsigned*)A.take(sizeof(unsigned) * (MAXLEV + 4));
   if (S->has64) {
     for (int i = 0; i < 5; ++i) S->pc64[i] = (double*)A.take(sizeof(double) * nv);
     carve(S->H64, A, S->fixV);
@@ -2918,14 +2872,6 @@ __global__ void k_power_init(int64_t n, R* __restrict__ v) {
     v[i] = (R)(1.0 + 0.5 * sin(0.7 * (double)i));
 }
 
-template <typename R>
-__global__ void k_normalize(int64_t n, const double* __restrict__ nrm2, R* __restrict__ v) {
-  pdl_entry();
-  const double inv = 1.0 / sqrt(fmax(*nrm2, 1e-300));
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v[i] = (R)((double)v[i] * inv);
-}
-
 // Build the hierarchy for the fine viscosity already in L[0].eta: coarse viscosities, fixed
 // masks, diagonals, lambda_max(D^-1 K) by power iteration and the Chebyshev coefficients, and the
 // dense inverse of the coarsest operator.  No host synchronisation.
@@ -2962,52 +2908,66 @@ static int setup_hierarchy(mw_stokes* S, Hierarchy<R>& H, cudaStream_t s) {
     else
       cudaGetLastError();
     Level<R>& L = H.L[H.nlev - 1];
-    pdl_launch(k_dense_assemble<R>, 1, 1024, 0, ds, L.g, L.eta, L.fix, H.Ainv);
-    const size_t smem = sizeof(double) * ((size_t)H.nd * H.nd + H.nd);
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    // the kernel's shared-memory limit is raised once per device, to the device's maximum and under
-    // a lock: solvers set up from several host threads never call it again (nor lower it under
-    // another thread's launch, which setting it per size allowed), and a setup recorded into a CUDA
-    // graph issues no attribute call after the first set-up
-    static std::mutex attr_mu;
-    static bool attr_set[64] = {false};
-    bool smem_ok = false;
-    if (smem <= (size_t)optin && dev >= 0 && dev < 64) {
-      std::lock_guard<std::mutex> lock(attr_mu);
-      if (!attr_set[dev])
-        attr_set[dev] = cudaFuncSetAttribute(k_gauss_jordan_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             optin) == cudaSuccess;
-      smem_ok = attr_set[dev];
-    }
-    if (smem_ok)
-      pdl_launch(k_gauss_jordan_smem, 1, 1024, smem, ds, H.nd, H.Ainv);
-    else
+    if (!dense_inverse<R>(L.g, L.eta, L.fix, H.nd, H.Ainv, ds)) {
+      pdl_launch(k_dense_assemble<R>, 1, 1024, 0, ds, L.g, L.eta, L.fix, H.Ainv);
       pdl_launch(k_gauss_jordan, 1, 1024, sizeof(double) * H.nd, ds, H.nd, H.Ainv);
+    }
   }
-  // Chebyshev intervals: power iteration v <- D^-1 K v / |v| per smoothed level, warm-started
-  // from the previous viscosity's vector
-  for (int l = 0; l < H.nlev - (dense ? 1 : 0); ++l) {
+  // Chebyshev intervals: power iteration v <- D^-1 K v / |v| on every smoothed level at once,
+  // warm-started from the previous viscosity's vectors
+  const int smoothed = H.nlev - (dense ? 1 : 0);
+  bool cold = false;
+  for (int l = 0; l < smoothed; ++l) {
     Level<R>& L = H.L[l];
-    const bool coarsest = l == H.nlev - 1;
-    R* v = L.ev;
-    int iters = prm.power_iters;
-    if (!L.ev_ready) {
-      pdl_launch(k_power_init<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, v);
-      L.ev_ready = true;
-    } else {
-      iters = prm.power_iters_warm > 0 ? prm.power_iters_warm : prm.power_iters;
+    if (L.ev_ready) continue;
+    pdl_launch(k_power_init<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, L.ev);
+    dot<R>(S, L.ndof, L.ev, L.ev, L.lam2, s);
+    L.ev_ready = cold = true;
+  }
+  const int iters = !cold && prm.power_iters_warm > 0 ? prm.power_iters_warm : prm.power_iters;
+  PowerArgs<R> pa;
+  memset(&pa, 0, sizeof(pa));
+  pa.n = smoothed;
+  pa.ratio = prm.cheb_ratio;
+  pa.safety = prm.cheb_safety;
+  int blocks = 0;
+  for (int l = 0; l < smoothed; ++l) {
+    const Level<R>& L = H.L[l];
+    PowerLevel<R>& P = pa.L[l];
+    P.g = L.g; P.eta = L.etap; P.qs = l == 0 ? L.nel : 0;
+    P.fix = L.fix; P.diag = L.diag; P.dinv = L.dinv;
+    P.lam2 = L.lam2; P.cheb = L.cheb;
+    P.deg = l == H.nlev - 1 ? MAXDEG : L.deg;
+    P.block0 = blocks;
+    P.tiles_x = power_tiles_x(L.g.nx);
+    P.part = S->red + blocks;
+    P.counter = S->counter + l;
+    blocks += power_blocks(L.g.nx, L.g.nz);
+  }
+  for (int it = 0; it < iters && blocks > 0; ++it) {
+    // the vector ends where it started: an odd count of three or more passes once through a third buffer
+    pa.it = it;
+    pa.last = it == iters - 1;
+    const bool odd = iters & 1;
+    int from = it & 1, to = 1 - from;                // ev -> d -> ev ...
+    if (odd) {                                       // ev -> d -> t -> ev -> d -> ev ...
+      from = it < 3 ? it : 1 - (it & 1);
+      to = it < 2 ? it + 1 : (it & 1);
     }
-    for (int it = 0; it < iters; ++it) {
-      dot<R>(S, L.ndof, v, v, L.lam2 + 1, s);
-      pdl_launch(k_normalize<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, L.lam2 + 1, v);
-      level_apply<R>(L, l == 0, v, L.d, s);
-      pdl_launch(k_dinv<R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, L.d, L.diag, v);
+    for (int l = 0; l < smoothed; ++l) {
+      const Level<R>& L = H.L[l];
+      R* const b[3] = {L.ev, L.d, L.t};
+      pa.L[l].vin = b[from];
+      pa.L[l].vout = b[to];
     }
-    dot<R>(S, L.ndof, v, v, L.lam2, s);          // ||D^-1 K v_prev||^2 with ||v_prev|| = 1
-    int deg = coarsest ? MAXDEG : L.deg;
-    pdl_launch(k_cheb_coeffs, 1, 32, 0, s, L.lam2, deg, prm.cheb_ratio, prm.cheb_safety, L.cheb);
+    power_step<R>(pa, blocks, s);
+  }
+  for (int l = 0; l < smoothed; ++l) {
+    Level<R>& L = H.L[l];
+    if (iters == 1) pdl_launch(k_copy<R, R>, grid_for(L.ndof, 256), 256, 0, s, L.ndof, (const R*)L.d, L.ev);
+    if (iters < 1)
+      pdl_launch(k_cheb_coeffs, 1, 32, 0, s, (const double*)L.lam2, l == H.nlev - 1 ? MAXDEG : L.deg, prm.cheb_ratio,
+                 prm.cheb_safety, L.cheb);
   }
   if (ds != s) {
     cudaEventRecord(S->ev_join, ds);
@@ -3487,7 +3447,7 @@ int mw_stokes_create(mw_box box, mw_stokes_params prm, const uint8_t* bc_fix_V, 
   size_t need = do_layout(S, nullptr, true);
   if (work_bytes < need) { delete S; return MW_ERR_WORKSPACE; }
   do_layout(S, (char*)work, false);
-  if (cudaMemset(S->counter, 0, sizeof(unsigned) * 4) != cudaSuccess) { delete S; return MW_ERR_CUDA; }
+  if (cudaMemset(S->counter, 0, sizeof(unsigned) * (MAXLEV + 4)) != cudaSuccess) { delete S; return MW_ERR_CUDA; }
   *out = S;
   return MW_OK;
 }

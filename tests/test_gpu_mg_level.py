@@ -47,3 +47,14 @@ def test_solve_K_converges(shape, precision, degree):
     if precision == "f64":
         y, _ = S.apply(x)
         assert float((y - b).norm() / b.norm()) < 10 * rtol
+
+
+@pytest.mark.parametrize("shape", [(2, 2), (3, 3), (4, 4), (3, 5), (2, 7), (2, 8)])
+def test_coarsest_inverse(shape):
+    """A hierarchy of one level is its dense inverse (50 ... 170 unknowns): K V(b) = b to FP64 rounding
+    times the condition number (about 1e4 here)."""
+    S, g = solver(*shape, "f64")
+    assert S.levels("f64") == 1
+    b = torch.randn(S.nv, generator=g, device="cuda", dtype=torch.float64)
+    y, _ = S.apply(S.vcycle(b, "f64"))
+    assert float((y - b).norm() / b.norm()) < 1e-10
