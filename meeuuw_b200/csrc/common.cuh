@@ -68,6 +68,11 @@ MW_D void pdl_entry() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A kernel may read, before pdl_entry(), what no kernel writes any more by the time its predecessor
+// starts: the predecessor let it be scheduled only after its own wait, so everything up to the
+// predecessor's predecessor is complete and visible.  The level and Krylov kernels load the diagonal,
+// the viscosity, the Dirichlet flags and their tables there (written at least two launches earlier, by
+// the set-up), so that a chain of short launches does not wait for them.
 bool pdl_enabled();        // false when the environment sets MW_PDL=0
 
 template <typename... KArgs, typename... Args>

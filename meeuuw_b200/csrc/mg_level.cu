@@ -67,7 +67,6 @@ MW_D void restrict_taps(const R2* sr, int c, double* s0, double* s1) {
 // steps.  PLANES: nine viscosity planes (else one value per element).
 template <typename R, int DEG, bool DOWN, bool PLANES>
 __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_level(MgArgs<R> a) {
-  pdl_entry();
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, CZ = CELLS, NC = CX * CZ;
   constexpr int LO = DOWN ? DEG + 1 : DEG;                  // halo cells on the left and below
@@ -88,21 +87,18 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
   const bool has[4] = {cx0 && cz0, cx1 && cz0, cx0 && cz1, cx1 && cz1};
   const int64_t n0 = (int64_t)(2 * ez) * g.nnx + 2 * ex;
   const R2 zero = pair(R(0), R(0));
-  const double c1s = DEG > 1 ? a.cheb[2] : 0.0;
-  const R c20 = (R)a.cheb[1], c21 = DEG > 1 ? (R)a.cheb[3] : R(0);
   R2 b[4], dg[4], di[4], x[4], d[4];
   unsigned fx = 0;                                          // bit 2 t + c: component c of node t is fixed
+  // what the set-up wrote, before the predecessor's results are waited for
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
     b[t] = dg[t] = di[t] = x[t] = zero;
     if (has[t]) {
-      b[t] = reinterpret_cast<const R2*>(a.b)[n];
       dg[t] = reinterpret_cast<const R2*>(a.diag)[n];
       di[t] = reinterpret_cast<const R2*>(a.dinv)[n];
       const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n];
       fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
-      if (!DOWN) x[t] = reinterpret_cast<const R2*>(a.xin)[n];
     }
   }
   R eq[9];
@@ -120,6 +116,16 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
 #pragma unroll
     for (int q = 0; q < 9; ++q) eq[q] = R(0);
   }
+  pdl_entry();
+  const double c1s = DEG > 1 ? a.cheb[2] : 0.0;
+  const R c20 = (R)a.cheb[1], c21 = DEG > 1 ? (R)a.cheb[3] : R(0);
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (has[t]) {
+      const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
+      b[t] = reinterpret_cast<const R2*>(a.b)[n];
+      if (!DOWN) x[t] = reinterpret_cast<const R2*>(a.xin)[n];
+    }
   if constexpr (DOWN) {                                     // x0 = d0 = (1/theta) D^-1 b
 #pragma unroll
     for (int t = 0; t < 4; ++t) d[t] = x[t] = div2(pair(c20 * b[t].x, c20 * b[t].y), dg[t], di[t]);

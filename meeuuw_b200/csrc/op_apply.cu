@@ -24,7 +24,7 @@ enum { OP_PLAIN = 0, OP_PCG, OP_SUM };
 template <typename R, bool PRESSURE, int KIND, typename X>
 __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3 : 2) k_op_apply(OpArgs<R> a,
                                                                                                  X dir) {
-  pdl_entry();
+  if (KIND != OP_PCG) pdl_entry();
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, NC = CELLS * CELLS, T = CELLS - 2;
   constexpr bool PCG = KIND == OP_PCG;
@@ -44,10 +44,23 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
   const bool elem = has[3] && lx < CX - 1 && lz < CELLS - 1;
   R2 x[4];
   unsigned fx = 0;
+  R eq[9];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (has[t]) {
+      const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n0 + (t >> 1) * g.nnx + (t & 1)];
+      fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
+    }
+  if (elem) {
+    const R* e = a.eta + ((int64_t)ez * g.nx + ex) * a.es;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) eq[q] = e[q * a.qs];
+  }
   const R* pold = nullptr;
   double beta = 0.0;
   int k = 0;
   if constexpr (PCG) {
+    pdl_entry();                                            // (the flags and the viscosity are the set-up's)
     k = (int)*dir.it;
     if (k > 0) {
       beta = dir.rz[k & 1] / dir.rz[(k & 1) ^ 1];
@@ -68,18 +81,10 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 && !PRESSURE ? 3
       } else if (a.u) {
         x[t] = reinterpret_cast<const R2*>(a.u)[n];
       }
-      const uchar2 f = reinterpret_cast<const uchar2*>(a.fix)[n];
-      fx |= ((f.x ? 1u : 0u) | (f.y ? 2u : 0u)) << (2 * t);
     }
   }
   R p0 = R(0);
   if (PRESSURE && a.p && has[0]) p0 = a.p[np];
-  R eq[9];
-  if (elem) {
-    const R* e = a.eta + ((int64_t)ez * g.nx + ex) * a.es;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) eq[q] = e[q * a.qs];
-  }
   R2 u[9], y[9];
   R yp[4] = {R(0), R(0), R(0), R(0)};
   auto masked = [&](int t) {

@@ -1724,9 +1724,9 @@ __global__ void k_mass_cheb(LevelGeo g, const double* __restrict__ w, double* __
                             const double* __restrict__ dg, double c1, double c2, int first,
                             const double* __restrict__ m1, double* __restrict__ zero, double* __restrict__ part,
                             unsigned* __restrict__ counter, double* __restrict__ sum) {
-  pdl_entry();
   __shared__ double Me[16];
   if (threadIdx.x < 16) Me[threadIdx.x] = mass_entry(g, threadIdx.x / 4, threadIdx.x % 4);
+  pdl_entry();
   __syncthreads();
   const int64_t np = (int64_t)(g.nx + 1) * (g.nz + 1);
   const double mean = m1 ? *m1 / (double)np : 0.0;
@@ -1795,13 +1795,13 @@ __global__ void k_pcg_start_grad(LevelGeo g, const double* __restrict__ p, const
                                  const double* __restrict__ f, R* __restrict__ r, R* __restrict__ x,
                                  double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
                                  int device_loop, cudaGraphConditionalHandle hw) {
-  pdl_entry();
   typedef typename Vec2<R>::T R2;
   __shared__ double gx[36], gz[36];
   if (threadIdx.x < 36) {
     gx[threadIdx.x] = c_ref.GX[threadIdx.x];
     gz[threadIdx.x] = c_ref.GZ[threadIdx.x];
   }
+  pdl_entry();
   __syncthreads();
   double cx, cz, v = 0;
   grad_scales(g, &cx, &cz);
@@ -1882,12 +1882,12 @@ __global__ void k_schur_div(LevelGeo g, const R* __restrict__ x, const uint8_t* 
                             double* __restrict__ out, const double* __restrict__ h, double* __restrict__ V,
                             const double* __restrict__ d, double* __restrict__ part, unsigned* __restrict__ counter,
                             double* __restrict__ sc) {
-  pdl_entry();
   __shared__ double gx[36], gz[36];
   if (threadIdx.x < 36) {
     gx[threadIdx.x] = c_ref.GX[threadIdx.x];
     gz[threadIdx.x] = c_ref.GZ[threadIdx.x];
   }
+  pdl_entry();
   __syncthreads();
   double cx, cz, v = 0;
   grad_scales(g, &cx, &cz);
