@@ -63,16 +63,22 @@ MW_D void restrict_taps(const R2* sr, int c, double* s0, double* s1) {
   *s1 = a1;
 }
 
+// owned cells a side of a tile.  Downward between levels that are not nested a coarse node's taps reach
+// up to four fine nodes to its right (three between nested ones), one cell more of halo.
+constexpr int owned_cells(bool down, int deg, bool nested) { return CELLS - (down ? 2 * deg + (nested ? 2 : 3) : 2 * deg); }
+
 // DOWN: pre-smoothing, residual, restriction; else correction and post-smoothing.  DEG: smoothing
-// steps.  PLANES: nine viscosity planes (else one value per element).
-template <typename R, int DEG, bool DOWN, bool PLANES>
+// steps.  PLANES: nine viscosity planes (else one value per element).  NESTED: both element counts
+// halve (compile-time taps); else the transfer tables.
+template <typename R, int DEG, bool DOWN, bool PLANES, bool NESTED>
 __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_level(MgArgs<R> a) {
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, CZ = CELLS, NC = CX * CZ;
   constexpr int LO = DOWN ? DEG + 1 : DEG;                  // halo cells on the left and below
-  constexpr int TX = CX - (DOWN ? 2 * DEG + 2 : 2 * DEG), TZ = CZ - (DOWN ? 2 * DEG + 2 : 2 * DEG);
-  constexpr int WX = CX + 3, WZ = CZ + 3;                   // staged coarse nodes (upward)
-  static_assert(TX % 2 == 0 && TZ % 2 == 0, "tiles start at even cells (transfer parity)");
+  constexpr int TX = owned_cells(DOWN, DEG, NESTED), TZ = TX;
+  constexpr int WX = NESTED ? CX + 3 : 26, WZ = WX;         // staged coarse nodes (upward): not nested, the 32
+                                                            // fine nodes span at most 25 (nf / nc >= 3 / 2)
+  static_assert(!NESTED || TX % 2 == 0, "tiles start at even cells (transfer parity)");
   __shared__ __align__(16) R2 sx[4 * NC];                   // masked x (then the residual) by node type
   __shared__ __align__(16) R2 se[5 * NC];                   // sums for the right and upper neighbours
   __shared__ __align__(16) double2 sc[DOWN ? 1 : WX * WZ];
@@ -129,7 +135,35 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
   if constexpr (DOWN) {                                     // x0 = d0 = (1/theta) D^-1 b
 #pragma unroll
     for (int t = 0; t < 4; ++t) d[t] = x[t] = div2(pair(c20 * b[t].x, c20 * b[t].y), dg[t], di[t]);
-  } else if (a.xc) {
+  } else if constexpr (!NESTED) {
+    // the same with the taps of the tables
+    const int i0 = max(2 * (ex0 - LO), 0), k0 = max(2 * (ez0 - LO), 0), bx = a.tx.pj[i0] & ~1, bz = a.tz.pj[k0] & ~1;
+    for (int i = tid; i < WX * WZ; i += NC) {
+      const int jx = bx + i % WX, jz = bz + i / WX;
+      R2 v = zero;
+      if (jx < a.gc.nnx && jz < a.gc.nnz) v = reinterpret_cast<const R2*>(a.xc)[(int64_t)jz * a.gc.nnx + jx];
+      sc[i] = make_double2((double)v.x, (double)v.y);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (has[t]) {
+        const int i = 2 * ex + (t & 1), k = 2 * ez + (t >> 1);
+        const int c0 = (a.tz.pj[k] - bz) * WX + a.tx.pj[i] - bx;
+        double s0 = 0, s1 = 0;
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            const double w = a.tz.pw[3 * k + p] * a.tx.pw[3 * i + q];
+            const double2 c = sc[c0 + p * WX + q];
+            s0 = fma(w, c.x, s0);
+            s1 = fma(w, c.y, s1);
+          }
+        if (!(fx & (1u << (2 * t)))) x[t].x += (R)s0;
+        if (!(fx & (2u << (2 * t)))) x[t].y += (R)s1;
+      }
+  } else {
     // x + P x_c on the free components: the coarse nodes under the tile in shared memory, as
     // doubles (converted once), the taps of prolong_taps in its order
     const int bx = (ex0 - LO) & ~1, bz = (ez0 - LO) & ~1;
@@ -218,10 +252,38 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
           if (has[t]) {
             const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
             reinterpret_cast<R2*>(a.x)[n] = x[t];
-            if (!a.bc) reinterpret_cast<R2*>(a.r)[n] = s[t];
           }
       }
-      if (a.bc) {
+      if constexpr (!NESTED) {
+        // the tile restricts to the coarse nodes that lie on its owned cells: coarse node J at fine
+        // lattice position J nf / nc
+#pragma unroll
+        for (int t = 0; t < 4; ++t) sx[t * NC + tid] = s[t];
+        __syncthreads();
+        auto first = [](int c, int nf, int nc) { return (int)((2LL * c * nc + nf - 1) / nf); };
+        const int j0 = first(ex0, g.nx, a.gc.nx), k0 = first(ez0, g.nz, a.gc.nz);
+        const int mx = (ex0 + TX >= g.nx ? a.gc.nnx : first(ex0 + TX, g.nx, a.gc.nx)) - j0;
+        const int mz = (ez0 + TZ >= g.nz ? a.gc.nnz : first(ez0 + TZ, g.nz, a.gc.nz)) - k0;
+        for (int i = tid; i < mx * mz; i += NC) {
+          const int jx = j0 + i % mx, jz = k0 + i / mx;
+          const int64_t n = (int64_t)jz * a.gc.nnx + jx;
+          const uchar2 f = reinterpret_cast<const uchar2*>(a.fixc)[n];
+          const int fx0 = a.tx.ri[jx] - 2 * (ex0 - LO), fz0 = a.tz.ri[jz] - 2 * (ez0 - LO), nx = a.tx.rn[jx],
+                    nz = a.tz.rn[jz];
+          double s0 = 0, s1 = 0;
+          for (int p = 0; p < nz; ++p) {
+            const double wz = a.tz.rw[RTAPS * jz + p];
+            const int row = ((fz0 + p) & 1) * 2 * NC + ((fz0 + p) >> 1) * CX;
+            for (int q = 0; q < nx; ++q) {
+              const double w = wz * a.tx.rw[RTAPS * jx + q];
+              const R2 v = sx[row + ((fx0 + q) & 1) * NC + ((fx0 + q) >> 1)];
+              s0 = fma(w, (double)v.x, s0);
+              s1 = fma(w, (double)v.y, s1);
+            }
+          }
+          reinterpret_cast<R2*>(a.bc)[n] = pair(f.x ? R(0) : (R)s0, f.y ? R(0) : (R)s1);
+        }
+      } else {
         // coarse node (I, J) sits on the corner of fine cell (I, J); the four parities have 9, 15,
         // 15 and 25 taps, so each warp takes nodes of one parity
 #pragma unroll
@@ -275,18 +337,24 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
   }
 }
 
-template <typename R, int DEG, bool DOWN>
+template <typename R, int DEG, bool DOWN, bool NESTED>
 void launch(const MgArgs<R>& a, bool planes, cudaStream_t s) {
-  constexpr int T = CELLS - (DOWN ? 2 * DEG + 2 : 2 * DEG);
+  constexpr int T = owned_cells(DOWN, DEG, NESTED);
   const dim3 grid((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
-  if (planes) pdl_launch(k_mg_level<R, DEG, DOWN, true>, grid, CELLS * CELLS, 0, s, a);
-  else pdl_launch(k_mg_level<R, DEG, DOWN, false>, grid, CELLS * CELLS, 0, s, a);
+  if (planes) pdl_launch(k_mg_level<R, DEG, DOWN, true, NESTED>, grid, CELLS * CELLS, 0, s, a);
+  else pdl_launch(k_mg_level<R, DEG, DOWN, false, NESTED>, grid, CELLS * CELLS, 0, s, a);
 }
 
 template <typename R, bool DOWN>
-void by_degree(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
-  if (deg <= 1) launch<R, 1, DOWN>(a, planes, s);
-  else launch<R, MG_MAXDEG, DOWN>(a, planes, s);
+void pick(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
+  const bool nested = a.g.nx == 2 * a.gc.nx && a.g.nz == 2 * a.gc.nz;
+  if (deg <= 1) {
+    if (nested) launch<R, 1, DOWN, true>(a, planes, s);
+    else launch<R, 1, DOWN, false>(a, planes, s);
+  } else {
+    if (nested) launch<R, MG_MAXDEG, DOWN, true>(a, planes, s);
+    else launch<R, MG_MAXDEG, DOWN, false>(a, planes, s);
+  }
 }
 
 }  // namespace
@@ -294,10 +362,10 @@ void by_degree(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
 int mg_ensure_tables() { return ensure_cell_tables(); }
 
 template <typename R> void mg_down(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
-  by_degree<R, true>(a, deg, planes, s);
+  pick<R, true>(a, deg, planes, s);
 }
 template <typename R> void mg_up(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
-  by_degree<R, false>(a, deg, planes, s);
+  pick<R, false>(a, deg, planes, s);
 }
 
 template void mg_down<float>(const MgArgs<float>&, int, bool, cudaStream_t);

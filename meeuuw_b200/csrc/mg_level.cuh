@@ -21,6 +21,17 @@ template <> struct Vec2<double> { typedef double2 T; };
 // smoothing steps per sweep the level launches are built for
 constexpr int MG_MAXDEG = 2;
 
+// The transfer between a level of nf elements a side and the coarser one of nc along one direction, as
+// tables: fine lattice node i takes coarse nodes pj[i] .. pj[i] + 2 with weights pw[3 i ...] (nodes past the
+// end with weight zero); coarse node J takes fine nodes ri[J] .. ri[J] + rn[J] - 1 with weights rw[RTAPS J ...].
+constexpr int RTAPS = 8;
+struct Transfer1D {
+  const int* pj;
+  const double* pw;
+  const int *ri, *rn;
+  const double* rw;
+};
+
 // Arguments of a level's half cycle.  Velocity vectors are interleaved (u, w) pairs.
 template <typename R>
 struct MgArgs {
@@ -32,12 +43,10 @@ struct MgArgs {
   const R* xin;        // upward: x before the correction (not the output buffer)
   R* x;                // downward: the smoothed x; upward: the result
   const double* cheb;  // Chebyshev coefficient pairs {c1, c2} per step
-  // downward: the restricted residual goes to bc (fixed coarse entries zero), or -- bc null -- the
-  // residual itself to r
-  R* bc;
+  R* bc;               // downward: the restricted residual (fixed coarse entries zero)
   const uint8_t* fixc;
-  R* r;
-  const R* xc;         // upward: the coarse correction to prolong; null: xin already carries it
+  const R* xc;         // upward: the coarse correction
+  Transfer1D tx, tz;   // levels that are not nested: the transfer along each direction
   ParitySum bx;        // upward: (b, x) of the result (part null: not wanted)
 };
 

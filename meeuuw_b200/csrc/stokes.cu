@@ -2084,6 +2084,8 @@ struct Level {
   R *eta, *diag, *x, *b, *r, *d, *t;
   R* dinv;            // 1 / diag, rounded
   R* etap;            // level 0: the viscosity as nine planes of nel values; below: one value per element
+  int* tj[2];         // transfer tables to the next level along x, z: pj, ri, rn ...
+  double* tw[2];      // ... pw, rw (Transfer1D)
   uint8_t* fix;
   double* cheb;       // 2*MAXDEG coefficients
   int deg;            // Chebyshev steps per smoothing sweep on this level
@@ -2217,6 +2219,68 @@ static void plan_levels(Hierarchy<R>& H, const LevelGeo& fine, const mw_stokes_p
 
 
 
+// The transfer of one direction between nf and nc elements on the device tables (host-built; the
+// weights of pw_g and restrict_taps_1d).
+static int fill_transfer(int nf, int nc, int* dj, double* dw) {
+  const int nnf = 2 * nf + 1, nnc = 2 * nc + 1;
+  std::vector<int> j(nnf + 2 * nnc);
+  std::vector<double> w(3 * (size_t)nnf + RTAPS * (size_t)nnc, 0.0);
+  for (int i = 0; i < nnf; ++i) {
+    double* q = &w[3 * (size_t)i];
+    if (nested_1d(nf, nc)) {
+      if (i & 1) {
+        const int E = i / 4;
+        j[i] = 2 * E;
+        q[0] = (i & 3) == 1 ? 0.375 : -0.125; q[1] = 0.75; q[2] = (i & 3) == 1 ? -0.125 : 0.375;
+      } else {
+        j[i] = i / 2;
+        q[0] = 1.0;
+      }
+    } else {
+      int E = (int)(((int64_t)i * nc) / (2LL * nf));
+      if (E > nc - 1) E = nc - 1;
+      const double xi = (double)((int64_t)i * nc - 2LL * nf * E - nf) / (double)nf;
+      j[i] = 2 * E;
+      q[0] = 0.5 * xi * (xi - 1.0); q[1] = (1.0 - xi) * (1.0 + xi); q[2] = 0.5 * xi * (xi + 1.0);
+    }
+  }
+  for (int J = 0; J < nnc; ++J) {           // the transpose: the fine nodes with a weight on J
+    int first = -1, last = -1;
+    const int lo = std::max(0, (int)(((int64_t)(J - 2) * nf) / nc) - 1), hi = std::min(nnf - 1, (int)(((int64_t)(J + 2) * nf) / nc) + 1);
+    for (int i = lo; i <= hi; ++i) {
+      const int o = J - j[i];
+      if (o < 0 || o > 2 || w[3 * (size_t)i + o] == 0.0) continue;
+      if (first < 0) first = i;
+      last = i;
+      if (i - first >= RTAPS) return MW_ERR_BAD_ARG;
+      w[3 * (size_t)nnf + RTAPS * (size_t)J + (i - first)] = w[3 * (size_t)i + o];
+    }
+    if (first < 0) return MW_ERR_BAD_ARG;
+    j[nnf + J] = first;
+    j[nnf + nnc + J] = last - first + 1;
+  }
+  if (cudaMemcpy(dj, j.data(), sizeof(int) * j.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(dw, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    return MW_ERR_CUDA;
+  return MW_OK;
+}
+
+template <typename R>
+static int fill_transfers(Hierarchy<R>& H) {
+  for (int l = 0; l + 1 < H.nlev; ++l)
+    for (int d = 0; d < 2; ++d) {
+      const LevelGeo &f = H.L[l].g, &c = H.L[l + 1].g;
+      if (int rc = fill_transfer(d ? f.nz : f.nx, d ? c.nz : c.nx, H.L[l].tj[d], H.L[l].tw[d])) return rc;
+    }
+  return MW_OK;
+}
+
+template <typename R>
+static Transfer1D transfer_of(const Level<R>& F, const Level<R>& C, int d) {
+  const int nnf = d ? F.g.nnz : F.g.nnx, nnc = d ? C.g.nnz : C.g.nnx;
+  return Transfer1D{F.tj[d], F.tw[d], F.tj[d] + nnf, F.tj[d] + nnf + nnc, F.tw[d] + 3 * (size_t)nnf};
+}
+
 template <typename R>
 static void carve(Hierarchy<R>& H, Arena& A, const uint8_t* fine_fix) {
   for (int l = 0; l < H.nlev; ++l) {
@@ -2235,6 +2299,11 @@ static void carve(Hierarchy<R>& H, Arena& A, const uint8_t* fine_fix) {
     L.lam2 = (double*)A.take(sizeof(double) * 4);
     L.ev = (R*)A.take(sizeof(R) * L.ndof);
     L.ev_ready = false;
+    for (int d = 0; d < 2 && l + 1 < H.nlev; ++d) {
+      const int nf = d ? L.g.nnz : L.g.nnx, nc = d ? H.L[l + 1].g.nnz : H.L[l + 1].g.nnx;
+      L.tj[d] = (int*)A.take(sizeof(int) * (nf + 2 * nc));
+      L.tw[d] = (double*)A.take(sizeof(double) * (3 * nf + RTAPS * nc));
+    }
   }
   H.Ainv = H.dense ? (double*)A.take(sizeof(double) * (size_t)H.nd * H.nd) : nullptr;
   H.tail_ye = H.tail0 ? (R*)A.take(sizeof(R) * H.tail_len) : nullptr;
@@ -2749,17 +2818,13 @@ static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = fal
     memset(&a, 0, sizeof(a));
     a.g = L.g; a.gc = C.g; a.eta = L.etap; a.fix = L.fix; a.diag = L.diag; a.dinv = L.dinv; a.b = L.b;
     a.cheb = L.cheb; a.x = L.t;
-    if (nested) { a.bc = C.b; a.fixc = C.fix; }
-    else a.r = L.r;
+    a.bc = C.b; a.fixc = C.fix; a.xc = C.x;
+    a.tx = transfer_of(L, C, 0);
+    a.tz = transfer_of(L, C, 1);
     mg_down<R>(a, L.deg, l == 0, s);
-    if (!nested)
-      pdl_launch(k_restrict_g<R>, grid_for(C.nn, 256), 256, 0, s, L.g, C.g, L.r, C.fix, C.b, (const double*)nullptr,
-                 C.diag, C.x, C.d);
     vcycle(H, l + 1, s);
-    if (!nested)
-      pdl_launch(k_prolong_g<R>, grid_for(L.nn, 256), 256, 0, s, L.g, C.g, (const R*)C.x, L.fix, L.t);
+    a.xc = C.x;                                    // (deeper levels may exchange their buffers)
     a.xin = L.t; a.x = L.x;
-    a.xc = nested ? C.x : nullptr;
     if (bx) a.bx = *bx;
     mg_up<R>(a, L.deg, l == 0, s);
     return;
@@ -3447,6 +3512,7 @@ int mw_stokes_create(mw_box box, mw_stokes_params prm, const uint8_t* bc_fix_V, 
   size_t need = do_layout(S, nullptr, true);
   if (work_bytes < need) { delete S; return MW_ERR_WORKSPACE; }
   do_layout(S, (char*)work, false);
+  if ((S->has64 && fill_transfers(S->H64)) || (S->has32 && fill_transfers(S->H32))) { delete S; return MW_ERR_CUDA; }
   if (cudaMemset(S->counter, 0, sizeof(unsigned) * (MAXLEV + 4)) != cudaSuccess) { delete S; return MW_ERR_CUDA; }
   *out = S;
   return MW_OK;
