@@ -82,6 +82,9 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
   __shared__ __align__(16) R2 sx[4 * NC];                   // masked x (then the residual) by node type
   __shared__ __align__(16) R2 se[5 * NC];                   // sums for the right and upper neighbours
   __shared__ __align__(16) double2 sc[DOWN ? 1 : WX * WZ];
+  constexpr int CN = DOWN && !NESTED ? 16 : 1;              // coarse nodes a tile restricts to, per side (at most 13)
+  __shared__ double sw[2][CN][RTAPS];                       // their weights, first fine nodes and counts
+  __shared__ int si[2][CN], sn[2][CN];
   const int tid = threadIdx.x, lx = tid % CX, lz = tid / CX;
   const int ex0 = blockIdx.x * TX, ez0 = blockIdx.y * TZ;
   const int ex = ex0 + lx - LO, ez = ez0 + lz - LO;
@@ -122,6 +125,39 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
 #pragma unroll
     for (int q = 0; q < 9; ++q) eq[q] = R(0);
   }
+  int j0 = 0, k0 = 0, mx = 0, mz = 0;                       // the coarse nodes on the tile's owned cells: coarse
+  if constexpr (DOWN && !NESTED) {                          // node J lies at fine lattice position J nf / nc
+    auto first = [](int c, int nf, int nc) { return (int)((2LL * c * nc + nf - 1) / nf); };
+    j0 = first(ex0, g.nx, a.gc.nx);
+    k0 = first(ez0, g.nz, a.gc.nz);
+    mx = (ex0 + TX >= g.nx ? a.gc.nnx : first(ex0 + TX, g.nx, a.gc.nx)) - j0;
+    mz = (ez0 + TZ >= g.nz ? a.gc.nnz : first(ez0 + TZ, g.nz, a.gc.nz)) - k0;
+    for (int i = tid; i < 2 * CN * RTAPS; i += NC) {
+      const int dir = i / (CN * RTAPS), j = i / RTAPS % CN, q = i % RTAPS;
+      if (j >= (dir ? mz : mx)) continue;
+      const Transfer1D& t = dir ? a.tz : a.tx;
+      const int J = (dir ? k0 : j0) + j;
+      sw[dir][j][q] = t.rw[RTAPS * J + q];
+      if (q == 0) {
+        si[dir][j] = t.ri[J];
+        sn[dir][j] = t.rn[J];
+      }
+    }
+  }
+  int pj[2][2] = {{0, 0}, {0, 0}};                          // the taps of the cell's two columns and two rows
+  double pw[2][2][3];
+  if constexpr (!DOWN && !NESTED) {
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir)
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const Transfer1D& tr = dir ? a.tz : a.tx;
+        const int i = min(max(2 * (dir ? ez : ex) + t, 0), (dir ? g.nnz : g.nnx) - 1);
+        pj[dir][t] = tr.pj[i];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) pw[dir][t][q] = tr.pw[3 * i + q];
+      }
+  }
   pdl_entry();
   const double c1s = DEG > 1 ? a.cheb[2] : 0.0;
   const R c20 = (R)a.cheb[1], c21 = DEG > 1 ? (R)a.cheb[3] : R(0);
@@ -148,14 +184,13 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
 #pragma unroll
     for (int t = 0; t < 4; ++t)
       if (has[t]) {
-        const int i = 2 * ex + (t & 1), k = 2 * ez + (t >> 1);
-        const int c0 = (a.tz.pj[k] - bz) * WX + a.tx.pj[i] - bx;
+        const int c0 = (pj[1][t >> 1] - bz) * WX + pj[0][t & 1] - bx;
         double s0 = 0, s1 = 0;
 #pragma unroll
         for (int p = 0; p < 3; ++p)
 #pragma unroll
           for (int q = 0; q < 3; ++q) {
-            const double w = a.tz.pw[3 * k + p] * a.tx.pw[3 * i + q];
+            const double w = pw[1][t >> 1][p] * pw[0][t & 1][q];
             const double2 c = sc[c0 + p * WX + q];
             s0 = fma(w, c.x, s0);
             s1 = fma(w, c.y, s1);
@@ -255,31 +290,29 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
           }
       }
       if constexpr (!NESTED) {
-        // the tile restricts to the coarse nodes that lie on its owned cells: coarse node J at fine
-        // lattice position J nf / nc
 #pragma unroll
         for (int t = 0; t < 4; ++t) sx[t * NC + tid] = s[t];
         __syncthreads();
-        auto first = [](int c, int nf, int nc) { return (int)((2LL * c * nc + nf - 1) / nf); };
-        const int j0 = first(ex0, g.nx, a.gc.nx), k0 = first(ez0, g.nz, a.gc.nz);
-        const int mx = (ex0 + TX >= g.nx ? a.gc.nnx : first(ex0 + TX, g.nx, a.gc.nx)) - j0;
-        const int mz = (ez0 + TZ >= g.nz ? a.gc.nnz : first(ez0 + TZ, g.nz, a.gc.nz)) - k0;
         for (int i = tid; i < mx * mz; i += NC) {
-          const int jx = j0 + i % mx, jz = k0 + i / mx;
-          const int64_t n = (int64_t)jz * a.gc.nnx + jx;
+          const int jx = i % mx, jz = i / mx;
+          const int64_t n = (int64_t)(k0 + jz) * a.gc.nnx + j0 + jx;
           const uchar2 f = reinterpret_cast<const uchar2*>(a.fixc)[n];
-          const int fx0 = a.tx.ri[jx] - 2 * (ex0 - LO), fz0 = a.tz.ri[jz] - 2 * (ez0 - LO), nx = a.tx.rn[jx],
-                    nz = a.tz.rn[jz];
+          const int fx0 = si[0][jx] - 2 * (ex0 - LO), fz0 = si[1][jz] - 2 * (ez0 - LO), nx = sn[0][jx], nz = sn[1][jz];
+          double wx[RTAPS];
+#pragma unroll
+          for (int q = 0; q < RTAPS; ++q) wx[q] = sw[0][jx][q];
           double s0 = 0, s1 = 0;
           for (int p = 0; p < nz; ++p) {
-            const double wz = a.tz.rw[RTAPS * jz + p];
+            const double wz = sw[1][jz][p];
             const int row = ((fz0 + p) & 1) * 2 * NC + ((fz0 + p) >> 1) * CX;
-            for (int q = 0; q < nx; ++q) {
-              const double w = wz * a.tx.rw[RTAPS * jx + q];
-              const R2 v = sx[row + ((fx0 + q) & 1) * NC + ((fx0 + q) >> 1)];
-              s0 = fma(w, (double)v.x, s0);
-              s1 = fma(w, (double)v.y, s1);
-            }
+#pragma unroll
+            for (int q = 0; q < RTAPS; ++q)
+              if (q < nx) {
+                const double w = wz * wx[q];
+                const R2 v = sx[row + ((fx0 + q) & 1) * NC + ((fx0 + q) >> 1)];
+                s0 = fma(w, (double)v.x, s0);
+                s1 = fma(w, (double)v.y, s1);
+              }
           }
           reinterpret_cast<R2*>(a.bc)[n] = pair(f.x ? R(0) : (R)s0, f.y ? R(0) : (R)s1);
         }
