@@ -54,6 +54,12 @@ MW_D void set_flag(int32_t* err, int32_t bit) {
 // Grid size: enough CTAs to cover n work items, capped at a multiple of the SM count.
 int grid_for(int64_t n, int threads, int waves = 8);
 int num_sms();
+// One thread per work item (up to a large cap): for kernels of a few resident CTAs an SM, whose last wave
+// over a capped grid would leave much of the chip idle.
+inline unsigned grid_all(int64_t n, int threads) {
+  const int64_t need = (n + threads - 1) / threads;
+  return (unsigned)(need < 1 ? 1 : (need < (1 << 20) ? need : (1 << 20)));
+}
 
 // Programmatic dependent launch.  The solver loops are long chains of short kernels on one stream;
 // launched through pdl_launch(), a kernel's CTAs are scheduled while its predecessor is still

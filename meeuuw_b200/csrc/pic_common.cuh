@@ -21,6 +21,15 @@ MW_D bool element_of(const mw_box& b, double x, double z, int64_t* e) {
 MW_D double xv0(const mw_box& b, int ex) { return ((double)(2 * ex) * b.hx) / 2; }
 MW_D double zv0(const mw_box& b, int ez) { return ((double)(2 * ez) * b.hz) / 2; }
 
+// a / h from the rounded reciprocal ih = 1 / h, rounded as the division is (a product corrected twice
+// by its exact residual: Markstein, IBM J. Res. Dev. 34, 1990).  Not finite where the product
+// overflows: locate refuses such a position either way.
+MW_D double quotient_exact(double a, double h, double ih) {
+  double q = a * ih;
+  q = fma(fma(-h, q, a), ih, q);
+  return fma(fma(-h, q, a), ih, q);
+}
+
 template <typename F>
 MW_D double q2_dot(const double* N, const F& nodal, int ex, int ez, int nnx) {
   double acc = N[0] * nodal(q2_node(ex, ez, 0, nnx));
