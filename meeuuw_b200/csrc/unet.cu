@@ -2,7 +2,10 @@
 // themselves are implicit GEMMs on the tcgen05 GEMM (gemm_tc.cu) over the im2col matrices built
 // here.  Activations are NHWC; convolution K index = tap * C + c with tap = (dy+1)*3 + (dx+1),
 // zero-padded to a multiple of 64.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -10,44 +13,102 @@ namespace mw {
 
 typedef __nv_bfloat16 bf16;
 
-// X [B,H,W,C] (bf16) -> col [M = B*H*W, Kp] (bf16), 'same' 3x3 patches, zeros outside
-__global__ void k_im2col(int B, int H, int W, int C, int Kp, const bf16* __restrict__ X, bf16* __restrict__ col) {
-  const int64_t M = (int64_t)B * H * W;
-  const int64_t total = M * Kp;
+// V bf16 values at a time (16 bytes for eight)
+template <int V> struct __align__(2 * V) Bf { bf16 v[V]; };
+template <int V> struct __align__(4 * V) Fl { float v[V]; };
+
+// quotient and remainder of index i of an [.., n] array (32-bit indices divide several times faster)
+template <typename I> MW_D void split(I i, I n, I* q, I* r) { *q = i / n; *r = i - *q * n; }
+
+// X [B,H,W,C] (bf16) -> col [M = B*H*W, Kp] (bf16), 'same' 3x3 patches, zeros outside; eight K entries a
+// thread, one 16-byte store (an entry a thread with 64-bit index divisions: 104 us for 262144 pixels of two
+// channels)
+template <int V>
+__global__ void __launch_bounds__(256) k_im2col(int B, int H, int W, int C, int Kp, const bf16* __restrict__ X,
+                                                bf16* __restrict__ col) {
+  const int64_t M = (int64_t)B * H * W, total = M * (Kp / V);
   const bf16 z = __float2bfloat16(0.f);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / Kp;
-    const int k = (int)(i - p * Kp);
-    bf16 v = z;
-    if (k < 9 * C) {
-      const int tap = k / C, c = k - tap * C;
-      const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((int64_t)W * H));
-      const int yy = y + tap / 3 - 1, xx = x + tap % 3 - 1;
-      if (yy >= 0 && yy < H && xx >= 0 && xx < W) v = X[(((int64_t)b * H + yy) * W + xx) * C + c];
+    const int64_t p = i / (Kp / V);
+    const int k0 = (int)(i - p * (Kp / V)) * V;
+    const int q = (int)(p % ((int64_t)H * W)), y = q / W, x = q - y * W;
+    Bf<V> o;
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      const int k = k0 + j;
+      bf16 v = z;
+      if (k < 9 * C) {
+        const int tap = k / C, c = k - tap * C, dy = tap / 3 - 1, dx = tap % 3 - 1;
+        if (y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W) v = X[(p + dy * W + dx) * C + c];
+      }
+      o.v[j] = v;
     }
-    col[i] = v;
+    reinterpret_cast<Bf<V>*>(col)[i] = o;
   }
 }
 
 // transposed im2col: colT [Kp, ldT] (ldT >= M; columns p >= M are zero so the pixel dimension can
-// be padded to the GEMM's K granularity)
-__global__ void k_im2col_T(int B, int H, int W, int C, int Kp, int64_t ldT, const bf16* __restrict__ X,
-                           bf16* __restrict__ colT) {
-  const int64_t M = (int64_t)B * H * W;
-  const int64_t total = ldT * Kp;
+// be padded to the GEMM's K granularity).  A block takes 128 pixels and 32 channels: per row offset dy it
+// loads the pixels shifted by dy W (one to either side too) once, transposed into shared memory, and writes
+// the three taps of each channel from there, eight pixels a store where VEC (ldT a multiple of eight, 16-byte
+// base).  An output entry a thread read X with a stride of C entries and divided its 64-bit index per entry:
+// 387 us a layer on average, half of a training step; 1.6 GB are written a step of 16 128 x 128 snapshots,
+// 0.5 ms at the memory's write rate.
+constexpr int TP = 128, TC = 32, TPS = TP + 6;             // row of 67 words: channels fall on different banks
+template <bool VEC, bool PAIR>
+__global__ void __launch_bounds__(256) k_im2col_T(int B, int H, int W, int C, int Kp, int64_t ldT,
+                                                  const bf16* __restrict__ X, bf16* __restrict__ colT) {
+  __shared__ bf16 sx[TC][TPS];
+  __shared__ uint8_t sok[9][TP];                           // the tap's source lies in the image
+  const int64_t M = (int64_t)B * H * W, p0 = (int64_t)blockIdx.x * TP;
+  const int c0 = blockIdx.y * TC, nc = min(TC, C - c0), tid = threadIdx.x;
   const bf16 z = __float2bfloat16(0.f);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int k = (int)(i / ldT);
-    const int64_t p = i - (int64_t)k * ldT;
-    bf16 v = z;
-    if (k < 9 * C && p < M) {
-      const int tap = k / C, c = k - tap * C;
-      const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((int64_t)W * H));
-      const int yy = y + tap / 3 - 1, xx = x + tap % 3 - 1;
-      if (yy >= 0 && yy < H && xx >= 0 && xx < W) v = X[(((int64_t)b * H + yy) * W + xx) * C + c];
+  for (int j = tid; j < TP; j += 256) {
+    const int64_t p = p0 + j;
+    const int q = (int)(p % ((int64_t)H * W)), y = q / W, x = q - y * W;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const int dy = t / 3 - 1, dx = t % 3 - 1;
+      sok[t][j] = p < M && y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W;
     }
-    colT[i] = v;
   }
+  const int np = (int)min((int64_t)TP, ldT - p0);          // columns of the tile
+  for (int dy = -1; dy <= 1; ++dy) {
+    __syncthreads();
+    const int64_t s0 = p0 + (int64_t)dy * W - 1;           // the pixel at column 0
+    if (PAIR) {
+      const int half = nc / 2;
+      for (int i = tid; i < (TP + 2) * half; i += 256) {
+        const int j = i / half, c = 2 * (i - j * half);
+        const int64_t sp = s0 + j;
+        __nv_bfloat162 v{z, z};
+        if (sp >= 0 && sp < M) v = *reinterpret_cast<const __nv_bfloat162*>(X + sp * C + c0 + c);
+        sx[c][j] = v.x;
+        sx[c + 1][j] = v.y;
+      }
+    } else {
+      for (int i = tid; i < (TP + 2) * nc; i += 256) {
+        const int j = i / nc, c = i - j * nc;
+        const int64_t sp = s0 + j;
+        sx[c][j] = sp >= 0 && sp < M ? X[sp * C + c0 + c] : z;
+      }
+    }
+    __syncthreads();
+    constexpr int V = VEC ? 8 : 1;
+    for (int i = tid; i < 3 * nc * (TP / V); i += 256) {
+      const int j = (i % (TP / V)) * V, r = i / (TP / V), c = r % nc, dx = r / nc - 1, tap = 3 * (dy + 1) + dx + 1;
+      if (j >= np) continue;
+      Bf<V> o;
+#pragma unroll
+      for (int k = 0; k < V; ++k) o.v[k] = sok[tap][j + k] ? sx[c][j + k + dx + 1] : z;
+      *reinterpret_cast<Bf<V>*>(colT + (int64_t)(tap * C + c0 + c) * ldT + p0 + j) = o;
+    }
+  }
+  if (c0 + TC >= C)                                        // the padding rows
+    for (int i = tid; i < (Kp - 9 * C) * TP; i += 256) {
+      const int j = i % TP;
+      if (j < np) colT[(int64_t)(9 * C + i / TP) * ldT + p0 + j] = z;
+    }
 }
 
 // fp32 master weights W [Cout, Kp_in] -> bf16 copy
@@ -70,115 +131,178 @@ __global__ void k_w_bwd(int Cout, int Cin, int Kp_in, int Kp_out, const float* _
   }
 }
 
-// dZ = dA * (A > 0 or !relu): bf16 [M, C], bf16 transposed [C, ldT] (columns >= M untouched), fp32 [M, C]
-__global__ void k_relu_grad(int64_t M, int C, int relu, int64_t ldT, const float* __restrict__ dA,
-                            const bf16* __restrict__ A, bf16* __restrict__ dZ, bf16* __restrict__ dZT,
-                            float* __restrict__ dZ32) {
-  const int64_t total = M * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / C;
-    const int c = (int)(i - p * C);
-    float g = dA[i];
-    if (relu && !(__bfloat162float(A[i]) > 0.f)) g = 0.f;
+// dZ = dA * (A > 0 or !relu): bf16 [M, C], bf16 transposed [C, ldT] (columns >= M untouched), fp32 [M, C];
+// 64 pixels x 32 channels a block, the transposed copy through shared memory (written entry by entry it
+// touched a cache line per value)
+constexpr int RP = 64, RC = 32;
+__global__ void __launch_bounds__(256) k_relu_grad(int64_t M, int C, int relu, int64_t ldT,
+                                                   const float* __restrict__ dA, const bf16* __restrict__ A,
+                                                   bf16* __restrict__ dZ, bf16* __restrict__ dZT,
+                                                   float* __restrict__ dZ32) {
+  __shared__ bf16 sg[RC][RP + 2];
+  const int64_t p0 = (int64_t)blockIdx.x * RP;
+  const int c0 = blockIdx.y * RC, nc = min(RC, C - c0), np = (int)min((int64_t)RP, M - p0);
+  for (int i = threadIdx.x; i < np * nc; i += 256) {
+    const int j = i / nc, c = i - j * nc;
+    const int64_t n = (p0 + j) * C + c0 + c;
+    float g = dA[n];
+    if (relu && !(__bfloat162float(A[n]) > 0.f)) g = 0.f;
     const bf16 gb = __float2bfloat16(g);
-    dZ[i] = gb;
-    dZT[(int64_t)c * ldT + p] = gb;
-    dZ32[i] = g;
+    dZ[n] = gb;
+    dZ32[n] = g;
+    sg[c][j] = gb;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nc * RP; i += 256) {
+    const int c = i / RP, j = i % RP;
+    if (j < np) dZT[(int64_t)(c0 + c) * ldT + p0 + j] = sg[c][j];
   }
 }
 
-// column sums of X [M, C] (fp32): one block per column, deterministic
-__global__ void k_colsum(int64_t M, int C, const float* __restrict__ X, float* __restrict__ out) {
-  __shared__ double sh[32];
-  const int c = blockIdx.x;
+// column sums of X [M, C] (fp32), deterministic: a cluster of eight blocks per eight columns (a 32-byte
+// sector of each row), each block its share of the rows, the blocks' sums added in rank order (a block per
+// column fetched every sector eight times and left most of the chip idle)
+constexpr int SC = 8, SB = 8;
+__global__ void __cluster_dims__(SB, 1, 1) __launch_bounds__(1024) k_colsum(int64_t M, int C,
+                                                                           const float* __restrict__ X,
+                                                                           float* __restrict__ out) {
+  __shared__ double sh[32][SC], tot[SC];
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  const int rank = (int)cl.block_rank(), c = (blockIdx.x / SB) * SC + threadIdx.x % SC;
+  constexpr int ROWS = 1024 / SC;
   double s = 0;
-  for (int64_t p = threadIdx.x; p < M; p += blockDim.x) s += X[p * C + c];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  if (c < C)
+    for (int64_t p = rank * ROWS + threadIdx.x / SC; p < M; p += SB * ROWS) s += X[p * C + c];
+  // lanes 8 apart hold the same column
+  for (int o = 16; o >= SC; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) < SC) sh[threadIdx.x >> 5][threadIdx.x & 31] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < SC) {
     double t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
+    for (int w = 0; w < 32; ++w) t += sh[w][threadIdx.x];
+    tot[threadIdx.x] = t;
+  }
+  cl.sync();
+  if (rank == 0 && threadIdx.x < SC && c < C) {
+    double t = 0;
+    for (int r = 0; r < SB; ++r) t += cl.map_shared_rank(tot, r)[threadIdx.x];
     out[c] = (float)t;
   }
+  cl.sync();                                               // no block leaves while its sums may be read
 }
 
+// The element-wise kernels below take V channels a thread (eight bf16 or four fp32: 16 bytes) where the
+// channel counts, offsets and base addresses allow it, else one, and index in 32 bits below 2^31 groups.  An
+// element a thread with three 64-bit divisions each: 62 us for an upsampling that moves 0.1 GB.
+
 // 2x2 average pooling, NHWC bf16
+template <int V, typename I>
 __global__ void k_avgpool2(int B, int H, int W, int C, const bf16* __restrict__ X, bf16* __restrict__ Y) {
-  const int h = H / 2, w = W / 2;
-  const int64_t total = (int64_t)B * h * w * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t q = i / C;
-    const int x = (int)(q % w), y = (int)((q / w) % h), b = (int)(q / ((int64_t)w * h));
-    const bf16* s = X + (((int64_t)b * H + 2 * y) * W + 2 * x) * C + c;
-    float v = __bfloat162float(s[0]) + __bfloat162float(s[C]) + __bfloat162float(s[(int64_t)W * C]) +
-              __bfloat162float(s[(int64_t)W * C + C]);
-    Y[i] = __float2bfloat16(0.25f * v);
+  const I h = H / 2, w = W / 2, cv = C / V, total = (I)B * h * w * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I q, c, t, x, b, y;
+    split(i, cv, &q, &c);
+    split(q, w, &t, &x);
+    split(t, h, &b, &y);
+    const bf16* s = X + (((int64_t)b * H + 2 * y) * W + 2 * x) * C + c * V;
+    const Bf<V> a0 = *reinterpret_cast<const Bf<V>*>(s), a1 = *reinterpret_cast<const Bf<V>*>(s + C),
+                a2 = *reinterpret_cast<const Bf<V>*>(s + (int64_t)W * C),
+                a3 = *reinterpret_cast<const Bf<V>*>(s + (int64_t)W * C + C);
+    Bf<V> o;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const float v = __bfloat162float(a0.v[k]) + __bfloat162float(a1.v[k]) + __bfloat162float(a2.v[k]) +
+                      __bfloat162float(a3.v[k]);
+      o.v[k] = __float2bfloat16(0.25f * v);
+    }
+    reinterpret_cast<Bf<V>*>(Y)[i] = o;
   }
 }
 
 // gradient of avg pooling: dX[b,y,x,c] (+)= dY[b,y/2,x/2,c] / 4   (fp32)
+template <int V, typename I>
 __global__ void k_avgpool2_bwd(int B, int H, int W, int C, const float* __restrict__ dY, float* __restrict__ dX,
                                int accumulate) {
-  const int64_t total = (int64_t)B * H * W * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t q = i / C;
-    const int x = (int)(q % W), y = (int)((q / W) % H), b = (int)(q / ((int64_t)W * H));
-    const float g = 0.25f * dY[(((int64_t)b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c];
-    dX[i] = accumulate ? dX[i] + g : g;
+  const I cv = C / V, total = (I)B * H * W * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I q, c, t, x, b, y;
+    split(i, cv, &q, &c);
+    split(q, (I)W, &t, &x);
+    split(t, (I)H, &b, &y);
+    const Fl<V> g = *reinterpret_cast<const Fl<V>*>(
+        dY + (((int64_t)b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c * V);
+    Fl<V>* d = reinterpret_cast<Fl<V>*>(dX) + i;
+    Fl<V> o;
+    if (accumulate) o = *d;
+#pragma unroll
+    for (int k = 0; k < V; ++k) o.v[k] = accumulate ? o.v[k] + 0.25f * g.v[k] : 0.25f * g.v[k];
+    *d = o;
   }
 }
 
 // nearest 2x upsampling of X [B,h,w,C] into channels [c0, c0+C) of Y [B,2h,2w,Ctot]
+template <int V, typename I>
 __global__ void k_upsample2_into(int B, int h, int w, int C, int Ctot, int c0, const bf16* __restrict__ X,
                                  bf16* __restrict__ Y) {
-  const int H = 2 * h, W = 2 * w;
-  const int64_t total = (int64_t)B * H * W * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t q = i / C;
-    const int x = (int)(q % W), y = (int)((q / W) % H), b = (int)(q / ((int64_t)W * H));
-    Y[q * Ctot + c0 + c] = X[(((int64_t)b * h + y / 2) * w + x / 2) * C + c];
+  const I H = 2 * h, W = 2 * w, cv = C / V, total = (I)B * H * W * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I q, c, t, x, b, y;
+    split(i, cv, &q, &c);
+    split(q, (I)W, &t, &x);
+    split(t, (I)H, &b, &y);
+    *reinterpret_cast<Bf<V>*>(Y + (int64_t)q * Ctot + c0 + c * V) =
+        *reinterpret_cast<const Bf<V>*>(X + (((int64_t)b * h + y / 2) * w + x / 2) * C + c * V);
   }
 }
 
 // copy X [.., C] into channels [c0, c0+C) of Y [.., Ctot]
-__global__ void k_copy_channels(int64_t P, int C, int Ctot, int c0, const bf16* __restrict__ X, bf16* __restrict__ Y) {
-  const int64_t total = P * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / C;
-    const int c = (int)(i - p * C);
-    Y[p * Ctot + c0 + c] = X[i];
+template <int V, typename I>
+__global__ void k_copy_channels(int64_t P, int C, int Ctot, int c0, const bf16* __restrict__ X,
+                                bf16* __restrict__ Y) {
+  const I cv = C / V, total = (I)P * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I p, c;
+    split(i, cv, &p, &c);
+    *reinterpret_cast<Bf<V>*>(Y + (int64_t)p * Ctot + c0 + c * V) = reinterpret_cast<const Bf<V>*>(X)[i];
   }
 }
 
 // gradient of the upsample into a concat: dX[b,y,x,c] = sum of the 4 fine cells' dY[.., c0+c]
+template <int V, typename I>
 __global__ void k_upsample2_bwd(int B, int h, int w, int C, int Ctot, int c0, const float* __restrict__ dY,
                                 float* __restrict__ dX) {
-  const int W = 2 * w;
-  const int64_t total = (int64_t)B * h * w * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % C);
-    const int64_t q = i / C;
-    const int x = (int)(q % w), y = (int)((q / w) % h), b = (int)(q / ((int64_t)w * h));
-    const int64_t r0 = ((int64_t)b * 2 * h + 2 * y) * W + 2 * x;
-    float s = dY[r0 * Ctot + c0 + c] + dY[(r0 + 1) * Ctot + c0 + c] + dY[(r0 + W) * Ctot + c0 + c] +
-              dY[(r0 + W + 1) * Ctot + c0 + c];
-    dX[i] = s;
+  const I W = 2 * w, cv = C / V, total = (I)B * h * w * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I q, c, t, x, b, y;
+    split(i, cv, &q, &c);
+    split(q, (I)w, &t, &x);
+    split(t, (I)h, &b, &y);
+    const float* g = dY + (((int64_t)b * 2 * h + 2 * y) * W + 2 * x) * Ctot + c0 + c * V;
+    const Fl<V> a0 = *reinterpret_cast<const Fl<V>*>(g), a1 = *reinterpret_cast<const Fl<V>*>(g + Ctot),
+                a2 = *reinterpret_cast<const Fl<V>*>(g + (int64_t)W * Ctot),
+                a3 = *reinterpret_cast<const Fl<V>*>(g + (int64_t)(W + 1) * Ctot);
+    Fl<V> o;
+#pragma unroll
+    for (int k = 0; k < V; ++k) o.v[k] = a0.v[k] + a1.v[k] + a2.v[k] + a3.v[k];
+    reinterpret_cast<Fl<V>*>(dX)[i] = o;
   }
 }
 
 // dX[.., c] (+)= dY[.., c0 + c]   (channel slice of a concat gradient)
-__global__ void k_slice_grad(int64_t P, int C, int Ctot, int c0, const float* __restrict__ dY, float* __restrict__ dX,
-                             int accumulate) {
-  const int64_t total = P * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = i / C;
-    const int c = (int)(i - p * C);
-    const float g = dY[p * Ctot + c0 + c];
-    dX[i] = accumulate ? dX[i] + g : g;
+template <int V, typename I>
+__global__ void k_slice_grad(int64_t P, int C, int Ctot, int c0, const float* __restrict__ dY,
+                             float* __restrict__ dX, int accumulate) {
+  const I cv = C / V, total = (I)P * cv;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
+    I p, c;
+    split(i, cv, &p, &c);
+    const Fl<V> g = *reinterpret_cast<const Fl<V>*>(dY + (int64_t)p * Ctot + c0 + c * V);
+    Fl<V>* d = reinterpret_cast<Fl<V>*>(dX) + i;
+    Fl<V> o;
+    if (accumulate) o = *d;
+#pragma unroll
+    for (int k = 0; k < V; ++k) o.v[k] = accumulate ? o.v[k] + g.v[k] : g.v[k];
+    *d = o;
   }
 }
 
@@ -187,10 +311,24 @@ __global__ void k_mse(int64_t n, const float* __restrict__ y, const float* __res
                       double* __restrict__ loss_part) {
   __shared__ double sh[32];
   double s = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float d = y[i] - t[i];
-    dy[i] = 2.f * d / (float)n;
-    s += (double)d * d;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  // eight terms in flight a thread, added in order
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 8 * step) {
+    float a[8], b[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int64_t i = i0 + k * step;
+      a[k] = i < n ? y[i] : 0.f;
+      b[k] = i < n ? t[i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int64_t i = i0 + k * step;
+      if (i >= n) continue;
+      const float d = a[k] - b[k];
+      dy[i] = 2.f * d / (float)n;
+      s += (double)d * d;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
@@ -392,6 +530,22 @@ __global__ void k_to_fields(mw_box b, int f, int gxp, const float* __restrict__ 
 
 using namespace mw;
 
+// Runs go(integral_constant<V>, index type) for `n` values: V = WIDE when `wide` (alignment) holds, 32-bit
+// indices when the group count fits.
+template <int WIDE, typename G>
+static int launch_wide(bool wide, int64_t n, const G& go) {
+  if (n <= 0) return MW_OK;
+  auto one = [&](auto v) {
+    const int64_t groups = n / v.value;
+    if (groups < (1LL << 31)) go(v, (uint32_t)0, grid_all(groups, 256));
+    else go(v, (uint64_t)0, grid_all(groups, 256));
+  };
+  if (wide) one(std::integral_constant<int, WIDE>{});
+  else one(std::integral_constant<int, 1>{});
+  return cudaGetLastError() == cudaSuccess ? MW_OK : MW_ERR_CUDA;
+}
+static bool on16(const void* a, const void* b) { return ((uintptr_t)a | (uintptr_t)b) % 16 == 0; }
+
 extern "C" {
 
 #define MW_GRID(n) grid_for((n), 256), 256, 0, (cudaStream_t)stream
@@ -402,9 +556,21 @@ int mw_unet_im2col(int32_t B, int32_t H, int32_t W, int32_t C, int32_t Kp, int32
   const int64_t M = (int64_t)B * H * W;
   if (transposed) {
     if (ldT < M) return MW_ERR_BAD_ARG;
-    k_im2col_T<<<MW_GRID(ldT * Kp)>>>(B, H, W, C, Kp, ldT, (const bf16*)X, (bf16*)col);
+    if (ldT <= 0) return MW_OK;
+    const dim3 grid((unsigned)((ldT + TP - 1) / TP), (C + TC - 1) / TC);
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool vec = ldT % 8 == 0 && (uintptr_t)col % 16 == 0, two = C % 2 == 0 && (uintptr_t)X % 4 == 0;
+    const bf16* x = (const bf16*)X;
+    bf16* o = (bf16*)col;
+    if (vec && two) k_im2col_T<true, true><<<grid, 256, 0, s>>>(B, H, W, C, Kp, ldT, x, o);
+    else if (vec) k_im2col_T<true, false><<<grid, 256, 0, s>>>(B, H, W, C, Kp, ldT, x, o);
+    else if (two) k_im2col_T<false, true><<<grid, 256, 0, s>>>(B, H, W, C, Kp, ldT, x, o);
+    else k_im2col_T<false, false><<<grid, 256, 0, s>>>(B, H, W, C, Kp, ldT, x, o);
+  } else if ((uintptr_t)col % 16 == 0) {
+    k_im2col<8><<<grid_all(M * (Kp / 8), 256), 256, 0, (cudaStream_t)stream>>>(B, H, W, C, Kp, (const bf16*)X,
+                                                                             (bf16*)col);
   } else {
-    k_im2col<<<MW_GRID(M * Kp)>>>(B, H, W, C, Kp, (const bf16*)X, (bf16*)col);
+    k_im2col<1><<<grid_all(M * Kp, 256), 256, 0, (cudaStream_t)stream>>>(B, H, W, C, Kp, (const bf16*)X, (bf16*)col);
   }
   MW_CHECK_LAUNCH();
   return MW_OK;
@@ -427,55 +593,69 @@ int mw_unet_weights_bwd(int32_t Cout, int32_t Cin, int32_t Kp_in, int32_t Kp_out
 int mw_unet_relu_grad(int64_t M, int32_t C, int32_t relu, int64_t ldT, const float* dA, const void* A, void* dZ,
                       void* dZT, float* dZ32, void* stream) {
   if (ldT < M) return MW_ERR_BAD_ARG;
-  k_relu_grad<<<MW_GRID(M * C)>>>(M, C, relu, ldT, dA, (const bf16*)A, (bf16*)dZ, (bf16*)dZT, dZ32);
+  if (M <= 0 || C <= 0) return MW_OK;
+  k_relu_grad<<<dim3((unsigned)((M + RP - 1) / RP), (C + RC - 1) / RC), 256, 0, (cudaStream_t)stream>>>(M, C, relu, ldT, dA, (const bf16*)A, (bf16*)dZ, (bf16*)dZT, dZ32);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
 
 int mw_unet_colsum(int64_t M, int32_t C, const float* X, float* out, void* stream) {
-  k_colsum<<<C, 256, 0, (cudaStream_t)stream>>>(M, C, X, out);
+  if (C <= 0) return MW_OK;
+  k_colsum<<<(C + SC - 1) / SC * SB, 1024, 0, (cudaStream_t)stream>>>(M, C, X, out);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
 
 int mw_unet_avgpool2(int32_t B, int32_t H, int32_t W, int32_t C, const void* X, void* Y, void* stream) {
-  k_avgpool2<<<MW_GRID((int64_t)B * (H / 2) * (W / 2) * C)>>>(B, H, W, C, (const bf16*)X, (bf16*)Y);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 8 == 0 && on16(X, Y);
+  return launch_wide<8>(wide, (int64_t)B * (H / 2) * (W / 2) * C, [&](auto v, auto idx, unsigned grid) {
+    k_avgpool2<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        B, H, W, C, (const bf16*)X, (bf16*)Y);
+  });
 }
 
 int mw_unet_avgpool2_bwd(int32_t B, int32_t H, int32_t W, int32_t C, const float* dY, float* dX, int32_t accumulate,
                          void* stream) {
-  k_avgpool2_bwd<<<MW_GRID((int64_t)B * H * W * C)>>>(B, H, W, C, dY, dX, accumulate);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 4 == 0 && on16(dY, dX);
+  return launch_wide<4>(wide, (int64_t)B * H * W * C, [&](auto v, auto idx, unsigned grid) {
+    k_avgpool2_bwd<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        B, H, W, C, dY, dX, accumulate);
+  });
 }
 
 int mw_unet_upsample2_into(int32_t B, int32_t h, int32_t w, int32_t C, int32_t Ctot, int32_t c0, const void* X,
                            void* Y, void* stream) {
-  k_upsample2_into<<<MW_GRID((int64_t)B * 4 * h * w * C)>>>(B, h, w, C, Ctot, c0, (const bf16*)X, (bf16*)Y);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 8 == 0 && Ctot % 8 == 0 && c0 % 8 == 0 && on16(X, Y);
+  return launch_wide<8>(wide, (int64_t)B * 4 * h * w * C, [&](auto v, auto idx, unsigned grid) {
+    k_upsample2_into<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        B, h, w, C, Ctot, c0, (const bf16*)X, (bf16*)Y);
+  });
 }
 
 int mw_unet_copy_channels(int64_t P, int32_t C, int32_t Ctot, int32_t c0, const void* X, void* Y, void* stream) {
-  k_copy_channels<<<MW_GRID(P * C)>>>(P, C, Ctot, c0, (const bf16*)X, (bf16*)Y);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 8 == 0 && Ctot % 8 == 0 && c0 % 8 == 0 && on16(X, Y);
+  return launch_wide<8>(wide, P * C, [&](auto v, auto idx, unsigned grid) {
+    k_copy_channels<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        P, C, Ctot, c0, (const bf16*)X, (bf16*)Y);
+  });
 }
 
 int mw_unet_upsample2_bwd(int32_t B, int32_t h, int32_t w, int32_t C, int32_t Ctot, int32_t c0, const float* dY,
                           float* dX, void* stream) {
-  k_upsample2_bwd<<<MW_GRID((int64_t)B * h * w * C)>>>(B, h, w, C, Ctot, c0, dY, dX);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 4 == 0 && Ctot % 4 == 0 && c0 % 4 == 0 && on16(dY, dX);
+  return launch_wide<4>(wide, (int64_t)B * h * w * C, [&](auto v, auto idx, unsigned grid) {
+    k_upsample2_bwd<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        B, h, w, C, Ctot, c0, dY, dX);
+  });
 }
 
 int mw_unet_slice_grad(int64_t P, int32_t C, int32_t Ctot, int32_t c0, const float* dY, float* dX, int32_t accumulate,
                        void* stream) {
-  k_slice_grad<<<MW_GRID(P * C)>>>(P, C, Ctot, c0, dY, dX, accumulate);
-  MW_CHECK_LAUNCH();
-  return MW_OK;
+  const bool wide = C % 4 == 0 && Ctot % 4 == 0 && c0 % 4 == 0 && on16(dY, dX);
+  return launch_wide<4>(wide, P * C, [&](auto v, auto idx, unsigned grid) {
+    k_slice_grad<decltype(v)::value, decltype(idx)><<<grid, 256, 0, (cudaStream_t)stream>>>(
+        P, C, Ctot, c0, dY, dX, accumulate);
+  });
 }
 
 int mw_unet_mse(int64_t n, const float* y, const float* t, float* dy, double* loss_part, int32_t nparts,
