@@ -20,6 +20,7 @@
 
 #include "common.cuh"
 #include "q2_ref.cuh"
+#include "reduce.cuh"
 #include "tma.cuh"
 
 namespace mw {
@@ -144,97 +145,86 @@ __global__ void k_energy_rows(mw_box b, RowPlanes P, const double* __restrict__ 
   }
 }
 
-__global__ void k_edot_partial(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                               double* __restrict__ part) {
-  pdl_entry();
-  __shared__ double sh[32];
-  double v = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    v += a[i] * b[i];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) part[blockIdx.x] = v;
+// ---------------------------------------------------------------- the iteration's scalars
+// Slots (sc): 0 rho = (r0, r), 1 rho of the previous iteration, 2 alpha and 3 omega of the previous
+// iteration, 4 (r0, v), 5 (t, s), 6 (t, t), 10 (b, b), 11 (r, r), 12 iteration count, 13 the flag word.
+// Each kernel that ends in a sum finishes it in its last block, which also takes the decisions that
+// follow from it: no launch has a scalar to compute alone.
+enum EnergyKind {
+  EK_APPLY,      // y = A x
+  EK_START,      // r = r0 = b - A x, (b, b), (r, r); first loop condition
+  EK_P,          // p = r + beta (p - omega v), v = A D^-1 p, (r0, v)
+  EK_S,          // s = r - alpha v, t = A D^-1 s, (t, s), (t, t)
+  EK_X           // x += alpha D^-1 p + omega D^-1 s, r = s - omega t, (r, r), (r0, r); loop condition
+};
+
+struct BicgEnd {
+  double *sc, *part;
+  unsigned* counter;
+  double rtol;
+  int maxit, use_h;                    // use_h: the loop is a conditional node of a recorded graph
+  cudaGraphConditionalHandle h;
+};
+
+// continue while the residual is finite, above rtol * ||b|| and the count is below maxit
+MW_D void bicg_condition(const BicgEnd& E) {
+  const double rr = E.sc[11];
+  if (E.use_h)
+    cudaGraphSetConditional(E.h, (isfinite(rr) && rr > E.rtol * E.rtol * E.sc[10] && E.sc[12] < (double)E.maxit) ? 1u : 0u);
+}
+
+// The sums of a kernel of KIND (a, and b where it has two) and what follows from them.  Called once,
+// by every thread, at the end of the kernel.
+template <int KIND>
+MW_D void bicg_end(const BicgEnd& E, double a, double b) {
+  double s[2] = {0.0, 0.0};
+  if (KIND == EK_P) {
+    if (grid_sum(a, E.part, E.counter, blockIdx.x, gridDim.x, s)) E.sc[4] = s[0];
+    return;
+  }
+  if (!grid_sum2(a, b, E.part, E.counter, blockIdx.x, gridDim.x, s)) return;
+  double* sc = E.sc;
+  if (KIND == EK_S) {
+    sc[5] = s[0];
+    sc[6] = s[1];
+  } else if (KIND == EK_START) {
+    sc[10] = s[0] > 0 ? s[0] : 1.0;
+    sc[11] = s[1];
+    sc[12] = 0;
+    sc[0] = s[1];                      // rho = (r0, r) = (r, r): r0 = r
+    bicg_condition(E);
+  } else {                             // EK_X: keep alpha, omega and rho, count the iteration
+    sc[2] = sc[0] / sc[4];
+    sc[3] = sc[6] != 0.0 ? sc[5] / sc[6] : 0.0;
+    sc[1] = sc[0];
+    sc[0] = s[1];
+    sc[11] = s[0];
+    sc[12] += 1;
+    bicg_condition(E);
   }
 }
 
-__global__ void k_edot_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-  pdl_entry();
-  __shared__ double sh[32];
-  double v = 0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) v += part[i];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) out[0] = v;
-  }
-}
+// The vectors of a solve.  The matrix-free kernels compute p and s of a tile's surrounding nodes
+// themselves, so they write p and v of an iteration beside the previous one's (p[it & 1], v[it & 1]):
+// another tile may still have to read the old ones.  The element-matrix kernels update in place (both
+// pointers the same) and take D^-1 p and D^-1 s from ph and sh.
+struct BicgVecs {
+  double *r, *r0, *p[2], *v[2], *sv, *t, *ph, *sh, *dg;
+};
 
-// BiCGSTAB vector updates with device scalars s[]: see the host loop for the slot meaning.
-// Deterministic grid-wide sums of K values per thread: block sums go to part[k * gridDim.x + block],
-// the last block to arrive adds them in block order, writes *out[k] and resets the counter.  Called
-// once, by every thread, at the end of a kernel.
-template <int K>
-MW_D void grid_sums(double (&v)[K], double* part, unsigned* counter, double* const (&out)[K]) {
-  __shared__ double sh[K][32];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double t = v[k];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0) sh[k][wid] = t;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      double t = 0;
-      for (int w = 0; w < nw; ++w) t += sh[k][w];
-      part[k * gridDim.x + blockIdx.x] = t;
-    }
-    __threadfence();
-    last = atomicAdd(counter, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double t = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += ((volatile double*)part)[k * gridDim.x + i];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    __syncthreads();
-    if (lane == 0) sh[k][wid] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double u = 0;
-      for (int w = 0; w < nw; ++w) u += sh[k][w];
-      *out[k] = u;
-    }
-  }
-  if (threadIdx.x == 0) *counter = 0u;
-}
+MW_D double bicg_beta(const double* sc) { return (sc[0] / sc[1]) * (sc[2] / sc[3]); }
+MW_D double bicg_alpha(const double* sc) { return sc[0] / sc[4]; }
+MW_D double bicg_omega(const double* sc) { return sc[6] != 0.0 ? sc[5] / sc[6] : 0.0; }
 
-// k_energy_matvec on the coefficient planes: the same products summed in the same order.  ND = 1
-// also sums (a0, y) (the iteration's (r0, v)), ND = 2 sums (y, a0) and (y, y) ((t, s), (t, t)).
-template <int ND>
+// k_energy_matvec on the coefficient planes: the same products summed in the same order.  EK_START
+// also writes the diagonal; EK_P and EK_S multiply ph and sh.
+template <int KIND>
 __global__ void k_energy_matvec_rows(mw_box b, RowPlanes P, const double* __restrict__ coef,
-                                     const double* __restrict__ x, const double* __restrict__ rhs,
-                                     double* __restrict__ y, double* __restrict__ diag, int mode,
-                                     const double* __restrict__ a0, double* __restrict__ part,
-                                     unsigned* __restrict__ counter, double* o0, double* o1) {
+                                     const double* __restrict__ x, const double* __restrict__ rhs, BicgVecs V,
+                                     BicgEnd E) {
   pdl_entry();
   const int nnx = 2 * b.nelx + 1;
-  double v[ND > 0 ? ND : 1] = {};
+  double d0 = 0.0, d1 = 0.0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < P.m0[4]; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t m;
     const int c = class_of(P, t, &m);
@@ -256,21 +246,23 @@ __global__ void k_energy_matvec_rows(mw_box b, RowPlanes P, const double* __rest
       }
     }
     const int64_t n = (int64_t)iz * nnx + ix;
-    y[n] = mode == 1 ? rhs[n] - acc : acc;
-    if (diag) diag[n] = dg;
-    if (ND == 1) v[0] += a0[n] * acc;
-    if (ND == 2) {
-      v[0] += acc * a0[n];
-      v[ND - 1] += acc * acc;
+    if (KIND == EK_START) {
+      const double bn = rhs[n], rn = bn - acc;
+      V.r[n] = rn;
+      V.r0[n] = rn;
+      V.dg[n] = dg;
+      d0 += bn * bn;
+      d1 += rn * rn;
+    } else if (KIND == EK_P) {
+      V.v[0][n] = acc;
+      d0 += V.r0[n] * acc;
+    } else {
+      V.t[n] = acc;
+      d0 += acc * V.sv[n];
+      d1 += acc * acc;
     }
   }
-  if (ND == 1) {
-    double* const out[1] = {o0};
-    grid_sums<1>(*reinterpret_cast<double(*)[1]>(v), part, counter, out);
-  } else if (ND == 2) {
-    double* const out[2] = {o0, o1};
-    grid_sums<2>(*reinterpret_cast<double(*)[2]>(v), part, counter, out);
-  }
+  bicg_end<KIND>(E, d0, d1);
 }
 
 // ---------------------------------------------------------------- matrix-free operator
@@ -286,22 +278,24 @@ __global__ void k_energy_matvec_rows(mw_box b, RowPlanes P, const double* __rest
 // products and fixed rows return diag_i x_i, diag the summed element diagonals.  A CTA owns the
 // nodes of an ETX x ETZ tile of elements, recomputes a one-element halo on the left and bottom,
 // and sums every owned node's incident elements in ascending element order from shared memory.
-constexpr int ETX = 16, ETZ = 8;
-constexpr int EEX = ETX + 1, EEZ = ETZ + 1, ENEL = EEX * EEZ;   // 153 element computations
-constexpr int ELX = 2 * ETX + 3, ELZ = 2 * ETZ + 3;           // 35 x 19 staged nodes
-constexpr int E_THREADS = 160;
+constexpr int ETX = 16, ETZ = 7;
+constexpr int EEX = ETX + 1, EEZ = ETZ + 1, ENEL = EEX * EEZ;   // 136 element computations
+constexpr int ELX = 2 * ETX + 3, ELZ = 2 * ETZ + 3;           // 35 x 17 staged nodes
+constexpr int E_THREADS = 160, E_CTAS_PER_SM = 4;
 constexpr int E_PLANES = 5;
 
 __constant__ RefTables c_eref;
 
 struct EnergyOp {
-  const double* planes;   // [(c * 9 + q) * nel + e], c = cM, au, aw, dr, ds
+  const double* planes;   // [(c * 9 + q) * nelz + ez] rows of eop_row(b) elements, c = cM, au, aw, dr, ds
   const double* diag;     // summed element diagonals (nn)
   const uint8_t* fix;     // Dirichlet flags (nn)
   int32_t* flag;          // flag word of standalone applies (after the flags, 16-byte aligned)
 };
 
-inline int64_t eop_plane_doubles(mw_box b) { return (int64_t)E_PLANES * 9 * b.nelx * b.nelz; }
+// elements of a plane's row: even, so that every row starts on a 16-byte boundary (TMA)
+MW_HD int eop_row(const mw_box& b) { return (b.nelx + 1) & ~1; }
+inline int64_t eop_plane_doubles(mw_box b) { return (int64_t)E_PLANES * 9 * eop_row(b) * b.nelz; }
 inline int64_t eop_nodes(mw_box b) { return (int64_t)(2 * b.nelx + 1) * (2 * b.nelz + 1); }
 inline EnergyOp eop_view(mw_box b, const void* op) {
   EnergyOp o;
@@ -384,21 +378,58 @@ MW_D double enode_sum(const mw_box& b, const ETile& T, int ix, int iz, const dou
 //           nodes, 0 elsewhere: the lifting of the fixed columns)
 //   rhs_i = diag_i bc_val_i                                        (fixed rows)
 // i.e. the element products of mass input T_old - x_bc and stiffness input -(T_old + x_bc).
-__global__ void __launch_bounds__(E_THREADS) k_energy_op_setup(mw_box b, mw_energy_in in, double* __restrict__ planes,
-                                                                double* __restrict__ diag, uint8_t* __restrict__ fix,
-                                                                double* __restrict__ rhs) {
+//
+// The Gauss-point inputs are [element][9]: a thread a point reads them in whole lines (a thread an
+// element read 72 bytes apart, 45 dependent rounds), forms the point's coefficients in shared memory,
+// and the element products run from there: half of the threads the right-hand side, half the diagonal.
+// 300x200 elements with the EBA terms 46 -> 32 us, 512^2 122 -> 108; bounded by latency: two CTAs an SM
+// (three, at 72 registers, spill and take 47 us).
+constexpr int ES_THREADS = 320;
+constexpr int ES_PLANES = E_PLANES + 1;                 // the heat source rides along
+constexpr size_t E_SMEM_SETUP = (size_t)(ES_PLANES * 9 * ENEL + 2 * ELZ * ELX) * sizeof(double);
+
+__global__ void __launch_bounds__(ES_THREADS, 2) k_energy_op_setup(mw_box b, mw_energy_in in,
+                                                                    double* __restrict__ planes,
+                                                                    double* __restrict__ diag, uint8_t* __restrict__ fix,
+                                                                    double* __restrict__ rhs, int32_t* flag) {
   pdl_entry();
-  __shared__ double sa[ELZ * ELX], sb[ELZ * ELX];
-  __shared__ double sy[ENEL * 9], sd[ENEL * 9];
+  extern __shared__ __align__(128) double esm[];
+  double* sc = esm;                                     // [c * 9 + q][element], then the products
+  double* sa = sc + ES_PLANES * 9 * ENEL;
+  double* sb = sa + ELZ * ELX;
+  double *sy = sc, *sd = sc + 9 * ENEL;
   const int tid = threadIdx.x;
-  const int nnx = 2 * b.nelx + 1, nnz = 2 * b.nelz + 1;
-  const int64_t nel = (int64_t)b.nelx * b.nelz;
+  const int nnx = 2 * b.nelx + 1, nnz = 2 * b.nelz + 1, row = eop_row(b);
   const int64_t ntile = (int64_t)((b.nelx + ETX - 1) / ETX) * ((b.nelz + ETZ - 1) / ETZ);
   const double dt = in.dt_dev ? *in.dt_dev : in.dt;
   const double h = dt * 0.5;
+  if (blockIdx.x == 0 && tid < 4) flag[tid] = 0;
   for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x) {
     const ETile T = etile(b, t);
-    for (int i = tid; i < ELZ * ELX; i += E_THREADS) {
+#pragma unroll 2
+    for (int i = tid; i < ENEL * 9; i += ES_THREADS) {
+      const int le = i / 9, q = i - le * 9, lez = le / EEX, lex = le - lez * EEX;
+      const int ex = T.ex0 - 1 + lex, ez = T.ez0 - 1 + lez;
+      if (ex < 0 || ex >= b.nelx || ez < 0 || ez >= b.nelz) continue;
+      const int64_t g = ((int64_t)ez * b.nelx + ex) * 9 + q;
+      const double jxw = in.JxWq[g], j00 = in.jcbi00q[g], j11 = in.jcbi11q[g], w = in.wq[g];
+      const double cM = in.rho0 * in.hcapaq[g] * jxw, cK = h * in.hcondq[g] * jxw;
+      double sq = in.hprodq[g] * jxw;                                           // :83
+      if (in.formulation == 1) {                                                // :85-110 (EBA)
+        const double exx = in.exxq[g], ezz = in.ezzq[g], exz = in.exzq[g];
+        sq += 2 * in.etaq[g] *
+              (2.0 / 3.0 * exx * exx + 2.0 / 3.0 * ezz * ezz - 2.0 / 3.0 * exx * ezz + 2 * exz * exz) * jxw;
+        sq += in.alphaq[g] * in.Tq[g] * (-w * in.rho0 * 10) * jxw;
+      }
+      double* o = sc + q * ENEL + le;
+      o[0] = cM;
+      o[9 * ENEL] = h * cM * in.uq[g] * j00;
+      o[18 * ENEL] = h * cM * w * j11;
+      o[27 * ENEL] = cK * j00 * j00;
+      o[36 * ENEL] = cK * j11 * j11;
+      o[45 * ENEL] = sq;
+    }
+    for (int i = tid; i < ELZ * ELX; i += ES_THREADS) {
       const int ix = T.lx0 + i % ELX, iz = T.lz0 + i / ELX;
       double a = 0.0, c = 0.0;
       if (ix >= 0 && ix < nnx && iz >= 0 && iz < nnz) {
@@ -411,62 +442,73 @@ __global__ void __launch_bounds__(E_THREADS) k_energy_op_setup(mw_box b, mw_ener
       sb[i] = c;
     }
     __syncthreads();
-    if (tid < ENEL) {
-      const int lex = tid % EEX, lez = tid / EEX;
+    {  // the owned elements' coefficients, a row of the tile at a time
+      const int nx = min(ETX, b.nelx - T.ex0), nz = min(ETZ, b.nelz - T.ez0);
+      for (int i = tid; i < E_PLANES * 9 * ETZ * ETX; i += ES_THREADS) {
+        const int lx = i % ETX, lz = i / ETX % ETZ, pl = i / (ETX * ETZ);
+        if (lx < nx && lz < nz)
+          planes[((int64_t)pl * b.nelz + T.ez0 + lz) * row + T.ex0 + lx] = sc[pl * ENEL + (lz + 1) * EEX + lx + 1];
+      }
+    }
+    const bool isd = tid >= ES_THREADS / 2;
+    const int le = isd ? tid - ES_THREADS / 2 : tid;
+    double y[9] = {};
+    if (le < ENEL) {
+      const int lex = le % EEX, lez = le / EEX;
       const int ex = T.ex0 - 1 + lex, ez = T.ez0 - 1 + lez;
       if (ex >= 0 && ex < b.nelx && ez >= 0 && ez < b.nelz) {
-        const int64_t e = (int64_t)ez * b.nelx + ex;
-        const bool own = lex > 0 && lez > 0;
-        double xa[9], xb[9], y[9], sk[9], dk[9];
-        const int bx = 2 * lex, bz = 2 * lez;
+        if (!isd) {
+          double xa[9], xb[9], sk[9] = {};
+          const int bx = 2 * lex, bz = 2 * lez;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          const int li = (bz + q2_dz(k)) * ELX + bx + q2_dx(k);
-          xa[k] = sa[li];
-          xb[k] = sb[li];
-          y[k] = 0.0; sk[k] = 0.0; dk[k] = 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-          const int64_t g = e * 9 + q;
-          const double jxw = in.JxWq[g], j00 = in.jcbi00q[g], j11 = in.jcbi11q[g];
-          const double cM = in.rho0 * in.hcapaq[g] * jxw, cK = h * in.hcondq[g] * jxw;
-          const double c[E_PLANES] = {cM, h * cM * in.uq[g] * j00, h * cM * in.wq[g] * j11, cK * j00 * j00,
-                                      cK * j11 * j11};
-          double sq = in.hprodq[g] * jxw;                                       // :83
-          if (in.formulation == 1) {                                            // :85-110 (EBA)
-            const double exx = in.exxq[g], ezz = in.ezzq[g], exz = in.exzq[g];
-            sq += 2 * in.etaq[g] *
-                  (2.0 / 3.0 * exx * exx + 2.0 / 3.0 * ezz * ezz - 2.0 / 3.0 * exx * ezz + 2 * exz * exz) * jxw;
-            sq += in.alphaq[g] * in.Tq[g] * (-in.wq[g] * in.rho0 * 10) * jxw;
+          for (int k = 0; k < 9; ++k) {
+            const int li = (bz + q2_dz(k)) * ELX + bx + q2_dx(k);
+            xa[k] = sa[li];
+            xb[k] = sb[li];
           }
-          if (own)
 #pragma unroll
-            for (int cc = 0; cc < E_PLANES; ++cc) planes[(int64_t)(cc * 9 + q) * nel + e] = c[cc];
-          energy_point(q, c, xa, xb, y);
+          for (int q = 0; q < 9; ++q) {
+            double c[E_PLANES];
 #pragma unroll
-          for (int k = 0; k < 9; ++k) {                 // element diagonal A_kk and heat source
-            if (ref_nv(q, k) != 0.0) {
-              sk[k] += eN(q, k) * sq;
-              double a = c[0] * eN(q, k);
-              if (ref_dr(q, k) != 0.0) a += c[1] * eR(q, k);
-              if (ref_dt(q, k) != 0.0) a += c[2] * eS(q, k);
-              dk[k] += eN(q, k) * a;
+            for (int cc = 0; cc < E_PLANES; ++cc) c[cc] = sc[(cc * 9 + q) * ENEL + le];
+            const double sq = sc[(E_PLANES * 9 + q) * ENEL + le];
+            energy_point(q, c, xa, xb, y);
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+              if (ref_nv(q, k) != 0.0) sk[k] += eN(q, k) * sq;
+          }
+#pragma unroll
+          for (int k = 0; k < 9; ++k) y[k] = dt * sk[k] + y[k];
+        } else {                                        // element diagonal A_kk
+#pragma unroll
+          for (int q = 0; q < 9; ++q) {
+            double c[E_PLANES];
+#pragma unroll
+            for (int cc = 0; cc < E_PLANES; ++cc) c[cc] = sc[(cc * 9 + q) * ENEL + le];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+              if (ref_nv(q, k) != 0.0) {
+                double a = c[0] * eN(q, k);
+                if (ref_dr(q, k) != 0.0) a += c[1] * eR(q, k);
+                if (ref_dt(q, k) != 0.0) a += c[2] * eS(q, k);
+                y[k] += eN(q, k) * a;
+              }
+              if (ref_dr(q, k) != 0.0) y[k] += c[3] * eR(q, k) * eR(q, k);
+              if (ref_dt(q, k) != 0.0) y[k] += c[4] * eS(q, k) * eS(q, k);
             }
-            if (ref_dr(q, k) != 0.0) dk[k] += c[3] * eR(q, k) * eR(q, k);
-            if (ref_dt(q, k) != 0.0) dk[k] += c[4] * eS(q, k) * eS(q, k);
           }
-        }
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          sy[tid * 9 + k] = dt * sk[k] + y[k];
-          sd[tid * 9 + k] = dk[k];
         }
       }
     }
+    __syncthreads();                                    // the coefficients are read: their room is reused
+    if (le < ENEL) {
+      double* o = (isd ? sd : sy) + le * 9;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) o[k] = y[k];
+    }
     __syncthreads();
     const int nox = T.ix1 - T.ix0, noz = T.iz1 - T.iz0;
-    for (int i = tid; i < nox * noz; i += E_THREADS) {
+    for (int i = tid; i < nox * noz; i += ES_THREADS) {
       const int ix = T.ix0 + i % nox, iz = T.iz0 + i / nox;
       const int64_t n = (int64_t)iz * nnx + ix;
       const double d = enode_sum(b, T, ix, iz, sd);
@@ -479,82 +521,132 @@ __global__ void __launch_bounds__(E_THREADS) k_energy_op_setup(mw_box b, mw_ener
   }
 }
 
-// Coefficients of one tile for the TMA path: planes [45][nelz][nelx] read as a 3D box of 18 x 9 x
+// Coefficients of one tile for the TMA path: planes [45][nelz][eop_row] read as a 3D box of 18 x 8 x
 // 45 starting at element (ex0 - 2, ez0 - 1) -- x even, so the box starts on a 16-byte boundary --
-// into shared memory [45][9][18]; elements off the mesh read as zero.
-constexpr int EBX = ETX + 2, EBZ = EEZ;                 // 18 x 9 elements per box
+// into shared memory [45][8][18]; elements off the planes read as zero.
+constexpr int EBX = ETX + 2, EBZ = EEZ;                 // 18 x 8 elements per box
 constexpr int EP_TILE = E_PLANES * 9 * EBZ * EBX;       // doubles
 constexpr long long E_SPIN = 1LL << 22;                 // mbarrier polls before a tile load is given up
-constexpr size_t E_SMEM_TMA = (size_t)(EP_TILE + ELZ * ELX + ENEL * 9) * sizeof(double) + 16;
-constexpr size_t E_SMEM = (size_t)(ELZ * ELX + ENEL * 9) * sizeof(double);
+constexpr size_t E_SMEM_TMA = (size_t)(EP_TILE + ELZ * ELX) * sizeof(double) + 16;
+constexpr size_t E_SMEM = (size_t)(ENEL * 9 + ELZ * ELX) * sizeof(double) + 16;
 
-// y = A x (MODE 0) or y = rhs - A x (MODE 1) on the owned nodes of each tile; ND = 1 also sums
-// (a0, Ax), ND = 2 sums (Ax, a0) and (Ax, Ax), as k_energy_matvec_rows.  TMA: each tile's
-// coefficients arrive in shared memory by one TMA box (one thread issues it, all wait on an
-// mbarrier while the staging of x runs), so a CTA has its 58 KB of coefficients in flight at once
-// instead of one element's 45 loads at a time; a load not complete after E_SPIN polls sets
+// A launch of KIND on the matrix-free operator, a tile of elements a CTA.  EK_APPLY and EK_START read x;
+// EK_P and EK_S compute their vector at the tile's nodes and the surrounding ones as they stage it
+// (owners store it), so that a BiCGSTAB iteration is this kernel twice and k_bicg_x.  Between them
+// they replace six launches: a solve of 300x200 elements (7 iterations) 452 -> 340 us, 64^2 (11) 403 -> 342,
+// 512^2 (8) 1217 -> 1037.  What bounds it: 64^2 the chain of a tile (8 us a launch: scalars, vectors,
+// Gauss points, sums) and the loop's own 5 us; 512^2 the 94 MB of coefficients a launch (36 us where a
+// copy of them takes 15: one box a CTA, no second one in flight).
+//
+// TMA: each tile's coefficients arrive in shared memory by one TMA box (one thread issues it, all wait
+// on an mbarrier while the staging runs), so a CTA has its 52 KB of coefficients in flight at once.
+// The first box of EK_P and EK_S, the flags and the diagonal are requested before the predecessor is
+// waited for: the set-up that wrote them is at least two launches back.  The products overwrite the
+// coefficients and the tile is 7 elements high, which leaves room for four CTAs an SM (16 x 8: three;
+// 300x200 elements are 551 tiles, one wave instead of two, 17.6 -> 13.9 us a product).  A load not complete after E_SPIN polls sets
 // MW_FLAG_ITER_LIMIT in *flag (when given), waits for it once more (bounded) and stops computing.
-// Without TMA (odd nelx: the planes' rows are not 16-byte multiples) the coefficients are read
-// from global memory.
-template <int MODE, int ND, bool TMA>
-__global__ void __launch_bounds__(E_THREADS) k_energy_op_apply(const __grid_constant__ CUtensorMap tmP, mw_box b,
-                                                                EnergyOp op, const double* __restrict__ x,
-                                                                const double* __restrict__ rhs, double* __restrict__ y,
-                                                                const double* __restrict__ a0, double* __restrict__ part,
-                                                                unsigned* __restrict__ counter, double* o0, double* o1,
-                                                                int32_t* flag) {
-  pdl_entry();
+// Without TMA (an operator buffer that is not 16-byte aligned) the coefficients are read from global
+// memory.
+template <int KIND, bool TMA>
+__global__ void __launch_bounds__(E_THREADS, E_CTAS_PER_SM) k_energy_op_apply(const __grid_constant__ CUtensorMap tmP, mw_box b,
+                                                                   EnergyOp op, const double* __restrict__ x,
+                                                                   const double* __restrict__ rhs,
+                                                                   double* __restrict__ y, BicgVecs V, BicgEnd E,
+                                                                   int32_t* flag) {
+  constexpr bool ITER = KIND == EK_P || KIND == EK_S;
   extern __shared__ __align__(128) double esm[];
-  double* sc = esm;                                     // TMA: the tile's coefficients
-  double* sx = esm + (TMA ? EP_TILE : 0);
-  double* sy = sx + ELZ * ELX;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sy + ENEL * 9);
+  double* sc = esm;                                     // TMA: the tile's coefficients; then the products
+  double* sy = esm;
+  double* sx = esm + (TMA ? EP_TILE : ENEL * 9);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sx + ELZ * ELX);
   const int tid = threadIdx.x;
-  const int nnx = 2 * b.nelx + 1, nnz = 2 * b.nelz + 1;
-  const int64_t nel = (int64_t)b.nelx * b.nelz;
+  const int nnx = 2 * b.nelx + 1, nnz = 2 * b.nelz + 1, row = eop_row(b);
+  const int64_t plane = (int64_t)row * b.nelz;
   const int64_t ntile = (int64_t)((b.nelx + ETX - 1) / ETX) * ((b.nelz + ETZ - 1) / ETZ);
-  double v[ND > 0 ? ND : 1] = {};
-  if (TMA) {
-    if (tid == 0) {
-      mbar_init(bar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
+  if (!ITER) pdl_entry();
+  auto request = [&](const ETile& T) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // earlier uses of sc before the copy
+    mbar_expect_tx(bar, (uint32_t)(EP_TILE * sizeof(double)));
+    tma_load_3d(sc, &tmP, bar, T.ex0 - 2, T.ez0 - 1, 0);
+  };
+  if (TMA && tid == 0) {
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    request(etile(b, blockIdx.x));
   }
+  double d0 = 0.0, d1 = 0.0;
+  double beta = 0.0, om = 0.0, alpha = 0.0;
+  bool first = false;
+  const double *pold = nullptr, *vold = nullptr;
+  double *pnew = nullptr, *vnew = nullptr;
   uint32_t parity = 0;
+  constexpr int NS = (ELZ * ELX + E_THREADS - 1) / E_THREADS;
   for (int64_t t = blockIdx.x; t < ntile; t += gridDim.x) {
     const ETile T = etile(b, t);
-    if (TMA && tid == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier reads of sc before the copy
-      mbar_expect_tx(bar, (uint32_t)(EP_TILE * sizeof(double)));
-      tma_load_3d(sc, &tmP, bar, T.ex0 - 2, T.ez0 - 1, 0);
-    }
-    {  // stage x (fixed entries zeroed): every load issued before any store, one round trip
-      constexpr int NS = (ELZ * ELX + E_THREADS - 1) / E_THREADS;
-      double xv[NS];
+    const bool head = t == blockIdx.x;
+    if (TMA && !head && tid == 0) request(T);
+    {  // stage the vector (fixed entries zeroed): every load issued before any use, one round trip
+      double g[NS];
       uint8_t fv[NS];
+      int64_t nn[NS];
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
         const int i = tid + k * E_THREADS;
         const int ix = T.lx0 + i % ELX, iz = T.lz0 + i / ELX;
-        xv[k] = 0.0;
+        nn[k] = -1;
         fv[k] = 1;
+        g[k] = 1.0;
         if (i < ELZ * ELX && ix >= 0 && ix < nnx && iz >= 0 && iz < nnz) {
-          const int64_t n = (int64_t)iz * nnx + ix;
-          fv[k] = op.fix[n];
-          xv[k] = x[n];
+          nn[k] = (int64_t)iz * nnx + ix;
+          fv[k] = op.fix[nn[k]];
+          if (ITER) g[k] = op.diag[nn[k]];
         }
+      }
+      if (ITER && head) {
+        pdl_entry();
+        const int it = (int)E.sc[12];
+        if (KIND == EK_P) {
+          first = it == 0;
+          if (!first) {
+            beta = bicg_beta(E.sc);
+            om = E.sc[3];
+          }
+          pnew = it & 1 ? V.p[1] : V.p[0];
+          pold = it & 1 ? V.p[0] : V.p[1];
+          vold = it & 1 ? V.v[0] : V.v[1];
+          vnew = it & 1 ? V.v[1] : V.v[0];
+        } else {
+          alpha = bicg_alpha(E.sc);
+          vold = it & 1 ? V.v[1] : V.v[0];
+        }
+      }
+      double a[NS], c[NS], d[NS];
+#pragma unroll
+      for (int k = 0; k < NS; ++k) {
+        a[k] = c[k] = d[k] = 0.0;
+        if (nn[k] < 0) continue;
+        if (!ITER) a[k] = x[nn[k]];
+        else a[k] = V.r[nn[k]];
+        if (KIND == EK_S || (KIND == EK_P && !first)) c[k] = vold[nn[k]];     // the first pass never reads p, v
+        if (KIND == EK_P && !first) d[k] = pold[nn[k]];
       }
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
         const int i = tid + k * E_THREADS;
-        if (i < ELZ * ELX) sx[i] = fv[k] ? 0.0 : xv[k];
+        if (KIND == EK_P && !first) a[k] = a[k] + beta * (d[k] - om * c[k]);
+        if (KIND == EK_S) a[k] = a[k] - alpha * c[k];
+        if (ITER && nn[k] >= 0) {
+          const int ix = T.lx0 + i % ELX, iz = T.lz0 + i / ELX;
+          if (ix >= T.ix0 && ix < T.ix1 && iz >= T.iz0 && iz < T.iz1) (KIND == EK_P ? pnew : V.sv)[nn[k]] = a[k];
+        }
+        if (i < ELZ * ELX) sx[i] = fv[k] ? 0.0 : (ITER ? a[k] / g[k] : a[k]);
       }
     }
     if (TMA) {
+      __syncthreads();                                  // the barrier is initialised, the vector staged
       const bool ok = mbar_wait_bounded(bar, parity, E_SPIN);
       parity ^= 1u;
-      if (__syncthreads_or(!ok)) {                     // give up: flag, drain the copy, stop
+      if (__syncthreads_or(!ok)) {                      // give up: flag, drain the copy, stop
         if (tid == 0) {
           if (flag) atomicOr(flag, MW_FLAG_ITER_LIMIT);
           mbar_wait_bounded(bar, parity ^ 1u, E_SPIN);
@@ -565,36 +657,36 @@ __global__ void __launch_bounds__(E_THREADS) k_energy_op_apply(const __grid_cons
     } else {
       __syncthreads();
     }
+    double ye[9] = {};
     if (tid < ENEL) {
       const int lex = tid % EEX, lez = tid / EEX;
       const int ex = T.ex0 - 1 + lex, ez = T.ez0 - 1 + lez;
       if (ex >= 0 && ex < b.nelx && ez >= 0 && ez < b.nelz) {
-        const int64_t e = (int64_t)ez * b.nelx + ex;
-        double xe[9], ye[9];
+        double xe[9];
         const int bx = 2 * lex, bz = 2 * lez;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-          xe[k] = sx[(bz + q2_dz(k)) * ELX + bx + q2_dx(k)];
-          ye[k] = 0.0;
-        }
-        const double* pl = op.planes + e;
+        for (int k = 0; k < 9; ++k) xe[k] = sx[(bz + q2_dz(k)) * ELX + bx + q2_dx(k)];
+        const double* pl = op.planes + (int64_t)ez * row + ex;
         const double* ps = sc + lez * EBX + lex + 1;
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
           double c[E_PLANES];
 #pragma unroll
           for (int cc = 0; cc < E_PLANES; ++cc)
-            c[cc] = TMA ? ps[(cc * 9 + q) * EBZ * EBX] : __ldg(pl + (int64_t)(cc * 9 + q) * nel);
+            c[cc] = TMA ? ps[(cc * 9 + q) * EBZ * EBX] : __ldg(pl + (cc * 9 + q) * plane);
           energy_point(q, c, xe, xe, ye);
         }
-#pragma unroll
-        for (int k = 0; k < 9; ++k) sy[tid * 9 + k] = ye[k];
       }
+    }
+    if (TMA) __syncthreads();                           // the coefficients are read
+    if (tid < ENEL) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) sy[tid * 9 + k] = ye[k];
     }
     __syncthreads();
     {  // owned nodes: the loads of every node first, then the (rare) fixed rows, then the stores
-      const int nox = T.ix1 - T.ix0, noz = T.iz1 - T.iz0;
-      constexpr int NO = ((2 * ETX + 1) * (2 * ETZ + 1) + E_THREADS - 1) / E_THREADS;
+      constexpr int OX = 2 * ETX + 1, OZ = 2 * ETZ + 1;
+      constexpr int NO = (OX * OZ + E_THREADS - 1) / E_THREADS;
       int64_t nk[NO];
       uint8_t fk[NO];
       double acc[NO], bk[NO], ak[NO];
@@ -604,47 +696,68 @@ __global__ void __launch_bounds__(E_THREADS) k_energy_op_apply(const __grid_cons
         nk[k] = -1;
         fk[k] = 0;
         acc[k] = bk[k] = ak[k] = 0.0;
-        if (i < nox * noz) {
-          const int ix = T.ix0 + i % nox, iz = T.iz0 + i / nox;
+        const int ix = T.ix0 + i % OX, iz = T.iz0 + i / OX;
+        if (i < OX * OZ && ix < T.ix1 && iz < T.iz1) {
           const int64_t n = (int64_t)iz * nnx + ix;
           nk[k] = n;
           fk[k] = op.fix[n];
-          if (MODE == 1) bk[k] = rhs[n];
-          if (ND > 0) ak[k] = a0[n];
+          if (KIND == EK_START) ak[k] = rhs[n];
+          if (KIND == EK_P) ak[k] = V.r0[n];
+          if (KIND == EK_S) {
+            ak[k] = V.r[n];
+            bk[k] = vold[n];
+          }
           acc[k] = enode_sum(b, T, ix, iz, sy);
         }
       }
 #pragma unroll
-      for (int k = 0; k < NO; ++k)
-        if (nk[k] >= 0 && fk[k]) acc[k] = op.diag[nk[k]] * x[nk[k]];
+      for (int k = 0; k < NO; ++k) {
+        const int64_t n = nk[k];
+        if (KIND == EK_S) ak[k] = ak[k] - alpha * bk[k];
+        if (n >= 0 && fk[k]) {
+          const double dg = op.diag[n];
+          double xn;
+          if (!ITER) xn = x[n];
+          else if (KIND == EK_S) xn = ak[k] / dg;
+          else xn = (first ? V.r[n] : V.r[n] + beta * (pold[n] - om * vold[n])) / dg;
+          acc[k] = dg * xn;
+        }
+      }
 #pragma unroll
       for (int k = 0; k < NO; ++k) {
-        if (nk[k] < 0) continue;
-        y[nk[k]] = MODE == 1 ? bk[k] - acc[k] : acc[k];
-        if (ND == 1) v[0] += ak[k] * acc[k];
-        if (ND == 2) {
-          v[0] += acc[k] * ak[k];
-          v[ND - 1] += acc[k] * acc[k];
+        const int64_t n = nk[k];
+        if (n < 0) continue;
+        if (KIND == EK_APPLY) {
+          y[n] = acc[k];
+        } else if (KIND == EK_START) {
+          const double rn = ak[k] - acc[k];
+          V.r[n] = rn;
+          V.r0[n] = rn;
+          d0 += ak[k] * ak[k];
+          d1 += rn * rn;
+        } else if (KIND == EK_P) {
+          vnew[n] = acc[k];
+          d0 += ak[k] * acc[k];
+        } else {
+          V.t[n] = acc[k];
+          d0 += acc[k] * ak[k];
+          d1 += acc[k] * acc[k];
         }
       }
     }
+    if (TMA) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the products, before the next box
     __syncthreads();
   }
-  if (ND == 1) {
-    double* const out[1] = {o0};
-    grid_sums<1>(*reinterpret_cast<double(*)[1]>(v), part, counter, out);
-  } else if (ND == 2) {
-    double* const out[2] = {o0, o1};
-    grid_sums<2>(*reinterpret_cast<double(*)[2]>(v), part, counter, out);
-  }
+  if (KIND != EK_APPLY) bicg_end<KIND>(E, d0, d1);
 }
 
-// The coefficient-plane map of the TMA path; false when the planes cannot be described (odd nelx).
+// The coefficient-plane map of the TMA path; false when the planes cannot be described (not 16-byte aligned).
 static bool eop_plane_map(CUtensorMap* m, mw_box b, const void* op) {
   auto enc = get_encode();
-  if (!enc || (b.nelx & 1) || ((uintptr_t)op & 15)) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)b.nelx, (cuuint64_t)b.nelz, (cuuint64_t)(E_PLANES * 9)};
-  cuuint64_t strides[2] = {(cuuint64_t)b.nelx * 8, (cuuint64_t)b.nelx * b.nelz * 8};
+  if (!enc || ((uintptr_t)op & 15)) return false;
+  const cuuint64_t row = (cuuint64_t)eop_row(b);
+  cuuint64_t dims[3] = {row, (cuuint64_t)b.nelz, (cuuint64_t)(E_PLANES * 9)};
+  cuuint64_t strides[2] = {row * 8, row * b.nelz * 8};
   cuuint32_t box[3] = {(cuuint32_t)EBX, (cuuint32_t)EBZ, (cuuint32_t)(E_PLANES * 9)};
   cuuint32_t estr[3] = {1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void*>(op), dims, strides, box, estr,
@@ -652,107 +765,84 @@ static bool eop_plane_map(CUtensorMap* m, mw_box b, const void* op) {
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launches k_energy_op_apply<MODE, ND> on the TMA path when the map could be made.
-template <int MODE, int ND>
+// Launches k_energy_op_apply<KIND> on the TMA path when the map could be made.
+template <int KIND>
 static void launch_eop_apply(bool tma, const CUtensorMap& tm, int grid, cudaStream_t s, mw_box b, const EnergyOp& op,
-                             const double* x, const double* rhs, double* y, const double* a0, double* part,
-                             unsigned* counter, double* o0, double* o1, int32_t* flag) {
+                             const double* x, const double* rhs, double* y, const BicgVecs& V, const BicgEnd& E,
+                             int32_t* flag) {
   if (tma) {
     static bool attr = false;
     if (!attr) {
-      cudaFuncSetAttribute(k_energy_op_apply<MODE, ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(k_energy_op_apply<KIND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)E_SMEM_TMA);
       attr = true;
     }
-    pdl_launch(k_energy_op_apply<MODE, ND, true>, grid, E_THREADS, E_SMEM_TMA, s, tm, b, op, x, rhs, y, a0, part, counter,
-               o0, o1, flag);
+    pdl_launch(k_energy_op_apply<KIND, true>, grid, E_THREADS, E_SMEM_TMA, s, tm, b, op, x, rhs, y, V, E, flag);
   } else {
-    pdl_launch(k_energy_op_apply<MODE, ND, false>, grid, E_THREADS, E_SMEM, s, tm, b, op, x, rhs, y, a0, part, counter,
-               o0, o1, flag);
+    pdl_launch(k_energy_op_apply<KIND, false>, grid, E_THREADS, E_SMEM, s, tm, b, op, x, rhs, y, V, E, flag);
   }
 }
 
-// Scalar slots of the iteration (sc): 0 rho = (r0, r), 1 rho of the previous iteration, 2 alpha,
-// 3 omega, 4 (r0, v), 5 (t, s), 6 (t, t), 7 (r0, r) of the new residual, 10 (b, b), 11 (r, r),
-// 12 iteration count.  Each iteration is six launches: the direction update, A p^ with (r0, v),
-// the s update, A s^ with (t, s) and (t, t), the x / r update with (r, r) and (r0, r), the scalar
-// roll with the loop test.
-
+// ---- the element-matrix path's vector updates ----
 // p = r + beta (p - omega v), beta = (rho/rho_old) (alpha/omega) (p = r on the first iteration);
 // p^ = D^-1 p
-__global__ void k_bicg_p(int64_t n, const double* __restrict__ sc, const double* __restrict__ r,
-                         const double* __restrict__ v, double* __restrict__ p, const double* __restrict__ dg,
-                         double* __restrict__ ph) {
+__global__ void k_bicg_p(int64_t n, const double* __restrict__ sc, BicgVecs V) {
   pdl_entry();
   const bool first = sc[12] == 0.0;
-  const double beta = first ? 0.0 : (sc[0] / sc[1]) * (sc[2] / sc[3]);
+  const double beta = first ? 0.0 : bicg_beta(sc);
   const double om = first ? 0.0 : sc[3];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double pi = first ? r[i] : r[i] + beta * (p[i] - om * v[i]);   // the first pass never reads p, v
-    p[i] = pi;
-    ph[i] = pi / dg[i];
+    const double pi = first ? V.r[i] : V.r[i] + beta * (V.p[0][i] - om * V.v[0][i]);   // the first pass never reads p, v
+    V.p[0][i] = pi;
+    V.ph[i] = pi / V.dg[i];
   }
 }
 
 // s = r - alpha v, alpha = rho / (r0, v); s^ = D^-1 s
-__global__ void k_bicg_s(int64_t n, const double* __restrict__ sc, const double* __restrict__ r,
-                         const double* __restrict__ v, double* __restrict__ sv, const double* __restrict__ dg,
-                         double* __restrict__ sh) {
+__global__ void k_bicg_s(int64_t n, const double* __restrict__ sc, BicgVecs V) {
   pdl_entry();
-  const double alpha = sc[0] / sc[4];
+  const double alpha = bicg_alpha(sc);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double si = r[i] - alpha * v[i];
-    sv[i] = si;
-    sh[i] = si / dg[i];
+    const double si = V.r[i] - alpha * V.v[0][i];
+    V.sv[i] = si;
+    V.sh[i] = si / V.dg[i];
   }
 }
 
-// x += alpha p^ + omega s^ ; r = s - omega t ; omega = (t, s) / (t, t); then (r, r) -> sc[11] and
-// (r0, r) -> sc[7]
-__global__ void k_bicg_x(int64_t n, double* __restrict__ sc, const double* __restrict__ ph,
-                         const double* __restrict__ sh, const double* __restrict__ sv, const double* __restrict__ t,
-                         const double* __restrict__ r0, double* __restrict__ x, double* __restrict__ r,
-                         double* __restrict__ part, unsigned* __restrict__ counter) {
+// x += alpha p^ + omega s^ ; r = s - omega t ; (r, r) and (r0, r), then the iteration's end.  Two nodes
+// a pass have their loads in flight together; one wave of four CTAs an SM (at three the launch was two
+// waves: 300x200 elements, 15 -> 11 us).
+constexpr int EX_THREADS = 256, EX_CTAS_PER_SM = 4;
+__global__ void __launch_bounds__(EX_THREADS, EX_CTAS_PER_SM) k_bicg_x(int64_t n, BicgVecs V, double* __restrict__ x, BicgEnd E) {
   pdl_entry();
-  const double alpha = sc[0] / sc[4];
-  const double omega = sc[6] != 0.0 ? sc[5] / sc[6] : 0.0;
-  double v[2] = {0.0, 0.0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += alpha * ph[i] + omega * sh[i];
-    const double ri = sv[i] - omega * t[i];
-    r[i] = ri;
-    v[0] += ri * ri;
-    v[1] += r0[i] * ri;
+  const double alpha = bicg_alpha(E.sc), omega = bicg_omega(E.sc);
+  const double* __restrict__ p = (int)E.sc[12] & 1 ? V.p[1] : V.p[0];
+  const double *__restrict__ sv = V.sv, *__restrict__ tt = V.t, *__restrict__ r0 = V.r0, *__restrict__ dg = V.dg;
+  double d0 = 0.0, d1 = 0.0;
+  const int64_t step = (int64_t)gridDim.x * EX_THREADS;
+  for (int64_t i = blockIdx.x * (int64_t)EX_THREADS + threadIdx.x; i < n; i += 2 * step) {
+    double pi[2], si[2], ti[2], ri[2], gi[2], xi[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t j = i + k * step;
+      pi[k] = si[k] = ti[k] = ri[k] = xi[k] = 0.0;
+      gi[k] = 1.0;
+      if (j < n) {
+        pi[k] = p[j]; si[k] = sv[j]; ti[k] = tt[j]; ri[k] = r0[j]; gi[k] = dg[j]; xi[k] = x[j];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int64_t j = i + k * step;
+      if (j >= n) continue;
+      x[j] = xi[k] + (alpha * (pi[k] / gi[k]) + omega * (si[k] / gi[k]));
+      const double r = si[k] - omega * ti[k];
+      V.r[j] = r;
+      d0 += r * r;
+      d1 += ri[k] * r;
+    }
   }
-  double* const out[2] = {sc + 11, sc + 7};
-  grid_sums<2>(v, part, counter, out);
-}
-
-// keep alpha (slot 2) and omega (slot 3) of this iteration, rho_old <- rho, rho <- (r0, r);
-// count the iteration and, inside a recorded graph (use_h), set the loop condition: continue while
-// the residual is finite, above rtol * ||b|| and the count is below maxit
-__global__ void k_bicg_roll(double* sc, double rtol, int maxit, cudaGraphConditionalHandle h, int use_h) {
-  pdl_entry();
-  if (threadIdx.x || blockIdx.x) return;
-  sc[2] = sc[0] / sc[4];
-  sc[3] = sc[6] != 0.0 ? sc[5] / sc[6] : 0.0;
-  sc[1] = sc[0];
-  sc[0] = sc[7];
-  const double it = sc[12] + 1;
-  sc[12] = it;
-  const double rr = sc[11];
-  if (use_h) cudaGraphSetConditional(h, (isfinite(rr) && rr > rtol * rtol * sc[10] && it < (double)maxit) ? 1u : 0u);
-}
-
-// ---- the iteration as a recorded CUDA graph with a device WHILE loop ----
-// sc[12] = iteration count; rho = (r0, r) = (r, r) to start with (r0 = r)
-__global__ void k_bicg_init(double* sc, double rtol, int maxit, cudaGraphConditionalHandle h, int use_h) {
-  pdl_entry();
-  if (!(sc[10] > 0)) sc[10] = 1.0;
-  sc[12] = 0;
-  sc[0] = sc[11];
-  const double rr = sc[11];
-  if (use_h) cudaGraphSetConditional(h, (isfinite(rr) && rr > rtol * rtol * sc[10] && maxit > 0) ? 1u : 0u);
+  bicg_end<EK_X>(E, d0, d1);
 }
 
 // Workspace of the solve (doubles): nine node vectors, then the dot-product partials, the device
@@ -809,12 +899,12 @@ size_t mw_energy_solve_workspace_bytes(mw_box box) {
 int mw_energy_device_info(mw_box box, const void* work, int32_t* iters, double* relres, void* stream) {
   const int64_t n = (int64_t)(2 * box.nelx + 1) * (2 * box.nelz + 1);
   const double* sc = (const double*)work + 9 * n + E_SC;
-  double q[3];
+  double q[4];
   int32_t flag = 0;
   cudaStream_t s = (cudaStream_t)stream;
   cudaMemcpyAsync(q, sc + 10, sizeof(q), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&flag, sc + 202, sizeof(flag), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return MW_ERR_CUDA;
+  memcpy(&flag, q + 3, sizeof(flag));
   if (iters) *iters = (int32_t)q[2];
   if (relres) *relres = flag ? NAN : std::sqrt(q[1] / q[0]);     // a tile load given up: no result
   return MW_OK;
@@ -827,15 +917,17 @@ int mw_energy_matvec(mw_box box, const double* VV_T, const double* x, double* y,
   return MW_OK;
 }
 
-// The buffers of the solve in its workspace (doubles): r, r0, p, v, s, t, p^, s^, diag, the
-// dot-product partials, the scalar slots (the arrival counter of the fused dot products in slot
-// 200) and the row planes.
+// The buffers of the solve in its workspace (doubles): r, r0, p, v, s, t, then p^, s^ and diag (element
+// matrices) or the second p and v (matrix-free), the dot-product partials, the scalar slots (the
+// arrival counter of the sums in slot 200) and the row planes.
 struct EnergyBufs {
   int64_t n;
-  double *r, *r0, *p, *v, *sv, *t, *ph, *sh, *dg, *part, *sc, *coef;
-  unsigned* counter;
+  BicgVecs V;
+  BicgEnd end;
+  double *sc, *coef;
   RowPlanes RP;
   int grid;               // CTAs of the node kernels (at most E_NB: one partial slot each)
+  int grid_x;             // CTAs of k_bicg_x
   EnergyA A;
   EnergyOp op;            // the matrix-free operator's view (A.op set)
   int grid_op;            // CTAs of the matrix-free apply (tile loop; at most E_NB)
@@ -844,26 +936,29 @@ struct EnergyBufs {
   int32_t* flag;          // device flag word of the solve (a tile load given up)
 };
 
-static EnergyBufs energy_bufs(mw_box box, void* work, EnergyA A) {
+static EnergyBufs energy_bufs(mw_box box, void* work, EnergyA A, double rtol, int maxit) {
   EnergyBufs E;
   E.A = A;
   E.n = (int64_t)(2 * box.nelx + 1) * (2 * box.nelz + 1);
   double* w = (double*)work;
   const int64_t n = E.n;
-  E.r = w; E.r0 = w + n; E.p = w + 2 * n; E.v = w + 3 * n; E.sv = w + 4 * n; E.t = w + 5 * n;
-  E.ph = w + 6 * n; E.sh = w + 7 * n; E.dg = w + 8 * n;
-  E.part = w + 9 * n;
+  BicgVecs& V = E.V;
+  V.r = w; V.r0 = w + n; V.p[0] = V.p[1] = w + 2 * n; V.v[0] = V.v[1] = w + 3 * n; V.sv = w + 4 * n; V.t = w + 5 * n;
+  V.ph = w + 6 * n; V.sh = w + 7 * n; V.dg = w + 8 * n;
   E.sc = w + 9 * n + E_SC;
-  E.counter = reinterpret_cast<unsigned*>(E.sc + 200);
   E.coef = w + 9 * n + E_COEF;
   E.RP = row_planes(box);
   E.grid = std::min(grid_for(n, 256), E_NB);
-  E.flag = reinterpret_cast<int32_t*>(E.sc + 202);
+  E.grid_x = (int)std::min<int64_t>({(n + EX_THREADS - 1) / EX_THREADS, (int64_t)EX_CTAS_PER_SM * num_sms(), E_NB});
+  E.flag = reinterpret_cast<int32_t*>(E.sc + 13);
+  E.end = BicgEnd{E.sc, w + 9 * n, reinterpret_cast<unsigned*>(E.sc + 200), rtol, maxit, 0, cudaGraphConditionalHandle(0)};
   E.tma = false;
   memset(&E.tm, 0, sizeof(E.tm));
   if (A.op) {
     E.op = eop_view(box, A.op);
-    E.dg = const_cast<double*>(E.op.diag);
+    V.p[1] = V.ph;
+    V.v[1] = V.sh;
+    V.dg = const_cast<double*>(E.op.diag);
     const int64_t ntile = (int64_t)((box.nelx + ETX - 1) / ETX) * ((box.nelz + ETZ - 1) / ETZ);
     E.grid_op = (int)std::min<int64_t>(ntile, E_NB);
     E.tma = eop_plane_map(&E.tm, box, A.op);
@@ -871,46 +966,31 @@ static EnergyBufs energy_bufs(mw_box box, void* work, EnergyA A) {
   return E;
 }
 
-// Row planes from VV_T, r = b - A T (T holds the initial guess) with diag(A), r0 = r, (b, b) and
-// (r, r) into sc[10], sc[11].
+// Row planes from VV_T, r = r0 = b - A T (T holds the initial guess) with diag(A), (b, b) and (r, r)
+// into sc[10], sc[11], the loop's first condition.
 static void energy_start(const EnergyBufs& E, mw_box box, const double* rhs, double* T, cudaStream_t s) {
-  cudaMemsetAsync(E.counter, 0, 4 * sizeof(double), s);        // arrival counter and flag word (slots 200-203)
+  cudaMemsetAsync(E.sc + 13, 0, (200 - 13 + 1) * sizeof(double), s);    // flag word to arrival counter
   if (E.A.op) {
-    launch_eop_apply<1, 0>(E.tma, E.tm, E.grid_op, s, box, E.op, T, rhs, E.r, nullptr, nullptr, nullptr, nullptr,
-                           nullptr, E.flag);
+    launch_eop_apply<EK_START>(E.tma, E.tm, E.grid_op, s, box, E.op, T, rhs, nullptr, E.V, E.end, E.flag);
   } else {
     pdl_launch(k_energy_rows, grid_for(E.RP.total / 9, 256), 256, 0, s, box, E.RP, E.A.VV, E.coef);
-    pdl_launch(k_energy_matvec_rows<0>, E.grid, 256, 0, s, box, E.RP, E.coef, T, rhs, E.r, E.dg, 1, nullptr,
-               nullptr, nullptr, nullptr, nullptr);
-  }
-  cudaMemcpyAsync(E.r0, E.r, sizeof(double) * E.n, cudaMemcpyDeviceToDevice, s);
-  const double* a[2] = {rhs, E.r};
-  for (int k = 0; k < 2; ++k) {
-    pdl_launch(k_edot_partial, E_NB, 256, 0, s, E.n, a[k], a[k], E.part);
-    pdl_launch(k_edot_final, 1, 256, 0, s, E.part, E_NB, E.sc + 10 + k);
+    pdl_launch(k_energy_matvec_rows<EK_START>, E.grid, 256, 0, s, box, E.RP, E.coef, T, rhs, E.V, E.end);
   }
 }
 
-// One BiCGSTAB iteration (Jacobi-preconditioned), six launches; with use_h the last one sets the
-// WHILE condition of the recorded loop.
-static void energy_iteration(const EnergyBufs& E, mw_box box, double* T, double rtol, int maxit,
-                             cudaGraphConditionalHandle h, int use_h, cudaStream_t s) {
-  pdl_launch(k_bicg_p, E.grid, 256, 0, s, E.n, E.sc, E.r, E.v, E.p, E.dg, E.ph);
-  if (E.A.op)
-    launch_eop_apply<0, 1>(E.tma, E.tm, E.grid_op, s, box, E.op, E.ph, nullptr, E.v, E.r0, E.part, E.counter, E.sc + 4,
-                           nullptr, E.flag);
-  else
-    pdl_launch(k_energy_matvec_rows<1>, E.grid, 256, 0, s, box, E.RP, E.coef, E.ph, nullptr, E.v, nullptr, 0, E.r0,
-               E.part, E.counter, E.sc + 4, nullptr);
-  pdl_launch(k_bicg_s, E.grid, 256, 0, s, E.n, E.sc, E.r, E.v, E.sv, E.dg, E.sh);
-  if (E.A.op)
-    launch_eop_apply<0, 2>(E.tma, E.tm, E.grid_op, s, box, E.op, E.sh, nullptr, E.t, E.sv, E.part, E.counter, E.sc + 5,
-                           E.sc + 6, E.flag);
-  else
-    pdl_launch(k_energy_matvec_rows<2>, E.grid, 256, 0, s, box, E.RP, E.coef, E.sh, nullptr, E.t, nullptr, 0, E.sv,
-               E.part, E.counter, E.sc + 5, E.sc + 6);
-  pdl_launch(k_bicg_x, E.grid, 256, 0, s, E.n, E.sc, E.ph, E.sh, E.sv, E.t, E.r0, T, E.r, E.part, E.counter);
-  pdl_launch(k_bicg_roll, 1, 32, 0, s, E.sc, rtol, maxit, h, use_h);
+// One BiCGSTAB iteration (Jacobi-preconditioned): three launches matrix-free, five on element matrices;
+// inside a recorded loop the last one sets the WHILE condition.
+static void energy_iteration(const EnergyBufs& E, mw_box box, double* T, cudaStream_t s) {
+  if (E.A.op) {
+    launch_eop_apply<EK_P>(E.tma, E.tm, E.grid_op, s, box, E.op, nullptr, nullptr, nullptr, E.V, E.end, E.flag);
+    launch_eop_apply<EK_S>(E.tma, E.tm, E.grid_op, s, box, E.op, nullptr, nullptr, nullptr, E.V, E.end, E.flag);
+  } else {
+    pdl_launch(k_bicg_p, E.grid, 256, 0, s, E.n, E.sc, E.V);
+    pdl_launch(k_energy_matvec_rows<EK_P>, E.grid, 256, 0, s, box, E.RP, E.coef, E.V.ph, nullptr, E.V, E.end);
+    pdl_launch(k_bicg_s, E.grid, 256, 0, s, E.n, E.sc, E.V);
+    pdl_launch(k_energy_matvec_rows<EK_S>, E.grid, 256, 0, s, box, E.RP, E.coef, E.V.sh, nullptr, E.V, E.end);
+  }
+  pdl_launch(k_bicg_x, E.grid_x, EX_THREADS, 0, s, E.n, E.V, T, E.end);
 }
 
 // Records the BiCGSTAB solve on the capturing stream s (body captured on b); false on failure.
@@ -972,11 +1052,11 @@ static bool energy_solve_graph(mw_box box, EnergyA A, const double* rhs, double*
   if (!legacy && cudaGraphLaunch(exec, s) != cudaSuccess) { cudaGetLastError(); return false; }
   const int64_t n = (int64_t)(2 * box.nelx + 1) * (2 * box.nelz + 1);
   const double* sc = (const double*)work + 9 * n + E_SC;
-  double q[3];
+  double q[4];
   int32_t flag = 0;
   cudaMemcpyAsync(q, sc + 10, sizeof(q), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&flag, sc + 202, sizeof(flag), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return false;
+  memcpy(&flag, q + 3, sizeof(flag));
   if (iters) *iters = (int32_t)q[2];
   if (relres) *relres = flag ? NAN : std::sqrt(q[1] / q[0]);
   return true;
@@ -1014,7 +1094,7 @@ static int energy_solve(mw_box box, EnergyA A, const double* rhs, double* T, dou
     }
   }
   cudaStream_t s = (cudaStream_t)stream;
-  const EnergyBufs E = energy_bufs(box, work, A);
+  const EnergyBufs E = energy_bufs(box, work, A, rtol, maxit);
   auto rd = [&](const double* d) {
     double h = 0;
     cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -1022,12 +1102,11 @@ static int energy_solve(mw_box box, EnergyA A, const double* rhs, double* T, dou
     return h;
   };
   energy_start(E, box, rhs, T, s);
-  pdl_launch(k_bicg_init, 1, 1, 0, s, E.sc, rtol, maxit, cudaGraphConditionalHandle(0), 0);
   double bb = rd(E.sc + 10);
   double rr = rd(E.sc + 11);
   int it = 0;
   for (it = 1; it <= maxit && rr > rtol * rtol * bb; ++it) {
-    energy_iteration(E, box, T, rtol, maxit, cudaGraphConditionalHandle(0), 0, s);
+    energy_iteration(E, box, T, s);
     rr = rd(E.sc + 11);
     if (!std::isfinite(rr)) break;
   }
@@ -1067,9 +1146,13 @@ int mw_energy_op_setup(mw_box box, mw_energy_in in, void* op, size_t op_bytes, d
   double* diag = planes + eop_plane_doubles(box);
   uint8_t* fix = reinterpret_cast<uint8_t*>(diag + eop_nodes(box));
   const int64_t ntile = (int64_t)((box.nelx + ETX - 1) / ETX) * ((box.nelz + ETZ - 1) / ETZ);
-  if (cudaMemsetAsync(eop_view(box, op).flag, 0, 16, (cudaStream_t)stream) != cudaSuccess) return MW_ERR_CUDA;
-  pdl_launch(k_energy_op_setup, (int)std::min<int64_t>(ntile, 8 * num_sms()), E_THREADS, 0, (cudaStream_t)stream, box,
-             in, planes, diag, fix, rhs);
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_energy_op_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E_SMEM_SETUP);
+    attr = true;
+  }
+  pdl_launch(k_energy_op_setup, (int)std::min<int64_t>(ntile, 8 * num_sms()), ES_THREADS, E_SMEM_SETUP,
+             (cudaStream_t)stream, box, in, planes, diag, fix, rhs, eop_view(box, op).flag);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
@@ -1082,8 +1165,8 @@ int mw_energy_op_apply(mw_box box, const void* op, const double* x, double* y, v
   memset(&tm, 0, sizeof(tm));
   const bool tma = eop_plane_map(&tm, box, op);
   const EnergyOp o = eop_view(box, op);
-  launch_eop_apply<0, 0>(tma, tm, (int)std::min<int64_t>(ntile, E_NB), (cudaStream_t)stream, box, o, x, nullptr, y,
-                         nullptr, nullptr, nullptr, nullptr, nullptr, o.flag);
+  launch_eop_apply<EK_APPLY>(tma, tm, (int)std::min<int64_t>(ntile, E_NB), (cudaStream_t)stream, box, o, x, nullptr, y,
+                             BicgVecs{}, BicgEnd{}, o.flag);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
@@ -1104,8 +1187,7 @@ int mw_energy_op_solve(mw_box box, const void* op, const double* rhs, double* T,
 
 static bool energy_record(mw_box box, EnergyA A, const double* rhs, double* T, double rtol, int maxit, void* work,
                           cudaStream_t s, cudaStream_t b) {
-  const EnergyBufs E = energy_bufs(box, work, A);
-  energy_start(E, box, rhs, T, s);
+  EnergyBufs E = energy_bufs(box, work, A, rtol, maxit);
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   cudaGraph_t g = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -1113,7 +1195,9 @@ static bool energy_record(mw_box box, EnergyA A, const double* rhs, double* T, d
   if (cudaStreamGetCaptureInfo(s, &st, nullptr, &g, nullptr, nullptr) != cudaSuccess) return false;
   cudaGraphConditionalHandle h;
   if (cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault) != cudaSuccess) return false;
-  pdl_launch(k_bicg_init, 1, 1, 0, s, E.sc, rtol, maxit, h, 1);
+  E.end.use_h = 1;
+  E.end.h = h;
+  energy_start(E, box, rhs, T, s);
   if (cudaStreamGetCaptureInfo(s, &st, nullptr, &g, &deps, &nd) != cudaSuccess) return false;
   cudaGraphNodeParams prm = {cudaGraphNodeTypeConditional};
   prm.conditional.handle = h;
@@ -1125,7 +1209,7 @@ static bool energy_record(mw_box box, EnergyA A, const double* rhs, double* T, d
   if (cudaStreamBeginCaptureToGraph(b, prm.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                     cudaStreamCaptureModeThreadLocal) != cudaSuccess)
     return false;
-  energy_iteration(E, box, T, rtol, maxit, h, 1, b);         // the body: one iteration and the loop test
+  energy_iteration(E, box, T, b);         // the body: one iteration and the loop test
   cudaGraph_t gb = nullptr;
   return cudaStreamEndCapture(b, &gb) == cudaSuccess;
 }
