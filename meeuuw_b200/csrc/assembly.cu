@@ -1,10 +1,10 @@
 // Element assembly kernels (sm_100a): Q2xQ1 Stokes and Q2 Crank-Nicolson energy.
 //
 // Reference: build_matrix_stokes.py:18-278 (box, plane strain) and build_matrix_energy.py:12-141.
-// One CTA per batch of EB elements; 18 (Stokes) or 9 (energy) threads per element, one element
+// A CTA works on batches of EB elements; 18 (Stokes) or 9 (energy) threads per element, one element
 // matrix row each.  The 3x3 Gauss basis tables and the batch's per-qpoint inputs are staged in
-// shared memory; the element outputs are staged in shared memory too and leave with coalesced
-// stores in the reference's VV order (build_matrix_stokes.py:235-276, build_matrix_energy.py:133-137).
+// shared memory; the element outputs are staged in shared memory too and leave in whole lines
+// in the reference's VV order (build_matrix_stokes.py:235-276, build_matrix_energy.py:133-137).
 //
 // Dirichlet elimination (build_matrix_stokes.py:206-217, build_matrix_energy.py:118-130) is done
 // row-locally: eliminating fixed dofs in ascending order leaves a free row i with
@@ -14,6 +14,8 @@
 // Right-hand sides: each element writes its local vector to a scratch buffer; a node-centric
 // gather then sums the (up to 4) element contributions in ascending element order, the order of
 // the reference's scatter loop.  No atomics; results are run-to-run identical.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace mw {
@@ -28,184 +30,259 @@ MW_HD int q2_local(int dx, int dz) {
   return dx == 0 ? 3 : (dx == 1 ? 6 : 2);
 }
 
-template <typename R, typename S>
-__global__ void __launch_bounds__(EB_S * 18)
-k_assemble_stokes(mw_box b, mw_stokes_in in, int blocks, S* __restrict__ vv_full, S* __restrict__ vv_K,
-                  S* __restrict__ vv_G, S* __restrict__ vv_GT, S* __restrict__ vv_M, S* __restrict__ vv_Meta,
-                  S* __restrict__ vv_H, double* __restrict__ f_el, double* __restrict__ h_el) {
+// One matrix row (element, dof) a thread, EB_S elements a pass, CTAs that stay for many passes.  A point's
+// weighted coefficients are formed once per element, so that an entry of K costs three multiply-adds (two
+// for its diagonal component, one for the other) from one 16-byte load of (dN/dx, dN/dz).  The results
+// take the room of the derivatives and leave as bulk copies.  BLOCKS writes K, G, GT, M, M_eta and H,
+// otherwise [K | G G]; both skip what they do not write.
+// Bounds: the 245 MB written (256^2 elements, FP64) take 37 us; the FP64 multiply-adds about 24, the
+// loads that feed them as much; the phases of a batch overlap only across the three CTAs of an SM:
+// 325 -> 128 us (8 elements a batch, 5 or 6 CTAs: 139, 146; 16 and 2: 139).
+template <typename R>
+struct alignas(2 * sizeof(R)) Pair {
+  R x, z;
+};
+
+template <typename R, bool BLOCKS>
+struct StokesSmem {                        // R values per CTA, by offset
+  static constexpr int Q = EB_S * 9;
+  static constexpr int DV = 0;                                   // pairs (dN/dx, dN/dz) of the velocity
+  static constexpr int DP = DV + 2 * EB_S * 81;                  // of the pressure
+  static constexpr int W = DP + (BLOCKS ? 2 * EB_S * 36 : 0);    // eta JxW, JxW, rho gx JxW, rho gz JxW
+  static constexpr int J = W + 4 * Q;                            // the four entries of the Jacobian
+  static constexpr int IN_END = J + 4 * Q;
+  static constexpr int G0 = 0;                                   // rows of G before the elimination
+  static constexpr int OUT = BLOCKS ? 572 : 468;                 // results per element
+  static constexpr int ROOM = IN_END > EB_S * OUT ? IN_END : EB_S * OUT;
+  static constexpr int NV = ROOM, NP = NV + 81, DRV = NP + 37, DRP = DRV + 162;
+  static constexpr int BCV = (DRP + 72 + 3) / 4 * 4;             // doubles, then one flag word an element
+  static constexpr int CTAS = BLOCKS ? 2 : 3;                    // an SM (FP64: 78 and 65 KB a CTA)
+  static constexpr size_t bytes = BCV * sizeof(R) + EB_S * 18 * sizeof(double) + EB_S * sizeof(unsigned);
+};
+
+// n bytes (a multiple of 16) from shared to global memory, by one thread, both 16-byte aligned
+MW_D void bulk_store(void* dst, const void* src, unsigned n) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+               :: "l"(dst), "r"((unsigned)__cvta_generic_to_shared(src)), "r"(n) : "memory");
+}
+
+template <typename R, bool BLOCKS>
+__global__ void __launch_bounds__(EB_S * 18, StokesSmem<R, BLOCKS>::CTAS)
+k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict__ vv_full, R* __restrict__ vv_K,
+                  R* __restrict__ vv_G, R* __restrict__ vv_GT, R* __restrict__ vv_M, R* __restrict__ vv_Meta,
+                  R* __restrict__ vv_H, double* __restrict__ f_el, double* __restrict__ h_el) {
+  using L = StokesSmem<R, BLOCKS>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  R* tab = reinterpret_cast<R*>(smem_raw);                 // 351 table values
-  R* NV = tab;            // 81
-  R* NP = tab + 81;       // 36
-  R* dNdx_V = tab + 117;  // EB*81  (per element, per q, per node)
-  R* dNdz_V = dNdx_V + EB_S * 81;
-  R* dNdx_P = dNdz_V + EB_S * 81;  // EB*36
-  R* dNdz_P = dNdx_P + EB_S * 36;
-  R* qin = dNdz_P + EB_S * 36;     // 5 arrays * EB*9 : rho, eta, JxW, gx, gz
-  R* G0 = qin + 5 * EB_S * 9;      // EB*18*4 (fixed rows of G, for h)
-  // the float instantiation ends G0 at a 4-byte boundary: realign before the double array
-  double* bcv = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(G0 + EB_S * 72) + 15) & ~uintptr_t(15));
-  int* bcf = reinterpret_cast<int*>(bcv + EB_S * 18);        // EB*18 flags
-  S* outs = reinterpret_cast<S*>(bcf + EB_S * 18);           // staged element outputs
+  R* sm = reinterpret_cast<R*>(smem_raw);
+  Pair<R>* dV = reinterpret_cast<Pair<R>*>(sm + L::DV);
+  Pair<R>* dP = reinterpret_cast<Pair<R>*>(sm + L::DP);
+  R *wq = sm + L::W, *jc = sm + L::J, *G0 = sm + L::G0, *outs = sm;
+  R *NV = sm + L::NV, *NP = sm + L::NP, *drV = sm + L::DRV, *drP = sm + L::DRP;
+  double* bcv = reinterpret_cast<double*>(sm + L::BCV);
+  unsigned* bcf = reinterpret_cast<unsigned*>(bcv + EB_S * 18);
 
   const int64_t nel = (int64_t)b.nelx * b.nelz;
-  const int64_t e0 = (int64_t)blockIdx.x * EB_S;
-  const int ne = (int)((nel - e0) < EB_S ? (nel - e0) : EB_S);
+  const int64_t nbatch = (nel + EB_S - 1) / EB_S;
   const int tid = threadIdx.x;
   const int nnx = 2 * b.nelx + 1;
-
-  __shared__ R dNdr_V[81], dNdt_V[81], dNdr_P[36], dNdt_P[36];
-  for (int i = tid; i < 81; i += blockDim.x) {
-    NV[i] = (R)in.N_V[i]; dNdr_V[i] = (R)in.dNdr_V[i]; dNdt_V[i] = (R)in.dNdt_V[i];
+  constexpr int NT = EB_S * 18;
+  for (int i = tid; i < 81; i += NT) {
+    NV[i] = (R)in.N_V[i]; drV[2 * i] = (R)in.dNdr_V[i]; drV[2 * i + 1] = (R)in.dNdt_V[i];
   }
-  for (int i = tid; i < 36; i += blockDim.x) {
-    NP[i] = (R)in.N_P[i]; dNdr_P[i] = (R)in.dNdr_P[i]; dNdt_P[i] = (R)in.dNdt_P[i];
+  for (int i = tid; i < 36; i += NT) {
+    NP[i] = (R)in.N_P[i]; drP[2 * i] = (R)in.dNdr_P[i]; drP[2 * i + 1] = (R)in.dNdt_P[i];
   }
-  for (int i = tid; i < ne * 9; i += blockDim.x) {
-    int64_t g = e0 * 9 + i;
-    qin[i] = (R)in.rhoq[g];
-    qin[EB_S * 9 + i] = (R)in.etaq[g];
-    qin[2 * EB_S * 9 + i] = (R)in.JxWq[g];
-    qin[3 * EB_S * 9 + i] = (R)in.gxq[g];
-    qin[4 * EB_S * 9 + i] = (R)in.gzq[g];
-  }
-  for (int i = tid; i < ne * 18; i += blockDim.x) {
-    int el = i / 18, ikk = i % 18;
-    int64_t e = e0 + el;
-    int ex = (int)(e % b.nelx), ez = (int)(e / b.nelx);
-    int64_t dof = 2 * q2_node(ex, ez, ikk / 2, nnx) + (ikk & 1);     // local_to_globalV, meeuuw.py:874-882
-    bcf[i] = in.bc_fix_V[dof] ? 1 : 0;
-    bcv[i] = in.bc_val_V[dof];
-  }
-  __syncthreads();
-  // derivatives at qpoints: build_matrix_stokes.py:131-134
-  for (int i = tid; i < ne * 9; i += blockDim.x) {
-    int el = i / 9, q = i % 9;
-    int64_t g = (e0 + el) * 9 + q;
-    R j00 = (R)in.jcbi00q[g], j01 = (R)in.jcbi01q[g], j10 = (R)in.jcbi10q[g], j11 = (R)in.jcbi11q[g];
-    for (int k = 0; k < 9; ++k) {
-      dNdx_V[el * 81 + q * 9 + k] = j00 * dNdr_V[q * 9 + k] + j01 * dNdt_V[q * 9 + k];
-      dNdz_V[el * 81 + q * 9 + k] = j10 * dNdr_V[q * 9 + k] + j11 * dNdt_V[q * 9 + k];
-    }
-    for (int k = 0; k < 4; ++k) {
-      dNdx_P[el * 36 + q * 4 + k] = j00 * dNdr_P[q * 4 + k] + j01 * dNdt_P[q * 4 + k];
-      dNdz_P[el * 36 + q * 4 + k] = j10 * dNdr_P[q * 4 + k] + j11 * dNdt_P[q * 4 + k];
-    }
-  }
-  __syncthreads();
-
-  const int el = tid / 18, ikk = tid % 18;
-  const bool live = el < ne;
+  const R s = (R)(in.eta_ref / in.L_ref);                                // build_matrix_stokes.py:157
+  const int el = tid / 18, ikk = tid - el * 18;
   const int i = ikk >> 1, c = ikk & 1;
-  R K[18], G[4], H[4], Mv = 0, f = 0;
-#pragma unroll
-  for (int j = 0; j < 18; ++j) K[j] = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) { G[k] = 0; H[k] = 0; }
-  if (live) {
-    for (int q = 0; q < 9; ++q) {
-      const R eta = qin[EB_S * 9 + el * 9 + q], jxw = qin[2 * EB_S * 9 + el * 9 + q];
-      const R rho = qin[el * 9 + q];
-      const R g = c == 0 ? qin[3 * EB_S * 9 + el * 9 + q] : qin[4 * EB_S * 9 + el * 9 + q];
-      const R* dx = dNdx_V + el * 81 + q * 9;
-      const R* dz = dNdz_V + el * 81 + q * 9;
-      const R dxi = dx[i], dzi = dz[i];
-#pragma unroll
-      for (int j = 0; j < 9; ++j) {
-        R a, bb;   // B^T C B entries (build_matrix_stokes.py:140), C = diag(2, 2, 1)
-        if (c == 0) { a = dxi * (R(2) * dx[j]) + dzi * dz[j]; bb = dzi * dx[j]; }
-        else        { a = dxi * dz[j]; bb = dzi * (R(2) * dz[j]) + dxi * dx[j]; }
-        K[2 * j] += a * eta * jxw;
-        K[2 * j + 1] += bb * eta * jxw;
-      }
-      f += NV[q * 9 + i] * jxw * rho * g;                              // :142-143
-      const R d = c == 0 ? dxi : dzi;
-      const R* dP = (c == 0 ? dNdx_P : dNdz_P) + el * 36 + q * 4;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        G[k] -= d * NP[q * 4 + k] * jxw;                                 // :144-146
-        H[k] += dP[k] * NV[q * 9 + i] * jxw;                             // :148-153
-      }
-      if (ikk < 16) Mv += NP[q * 4 + (ikk >> 2)] * NP[q * 4 + (ikk & 3)] * jxw;   // :147
+
+  for (int64_t batch = blockIdx.x; batch < nbatch; batch += gridDim.x) {
+    const int64_t e0 = batch * EB_S;
+    const int ne = (int)((nel - e0) < EB_S ? (nel - e0) : EB_S);
+    const bool live = el < ne;
+    if (tid < EB_S) bcf[tid] = 0;
+    if (tid < ne * 9) {
+      const int64_t g = e0 * 9 + tid;
+      const R jxw = (R)in.JxWq[g], eta = (R)in.etaq[g], rj = jxw * (R)in.rhoq[g];
+      wq[tid] = eta * jxw;
+      wq[L::Q + tid] = jxw;
+      wq[2 * L::Q + tid] = rj * (R)in.gxq[g];
+      wq[3 * L::Q + tid] = rj * (R)in.gzq[g];
+      jc[tid] = (R)in.jcbi00q[g];
+      jc[L::Q + tid] = (R)in.jcbi01q[g];
+      jc[2 * L::Q + tid] = (R)in.jcbi10q[g];
+      jc[3 * L::Q + tid] = (R)in.jcbi11q[g];
     }
-    const R s = (R)(in.eta_ref / in.L_ref);                                // :157
-#pragma unroll
-    for (int k = 0; k < 4; ++k) G[k] *= s;
-  }
-  // ---- Dirichlet elimination (row-local form) ----
-  const int* fx = bcf + el * 18;
-  const double* fv = bcv + el * 18;
-  bool fixed_row = live && fx[ikk];
-  R frow = f;
-  if (live) {
-    if (fixed_row) {
-      R kd = 0;
-#pragma unroll
-      for (int j = 0; j < 18; ++j) if (j == ikk) kd = K[j];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) G0[el * 72 + ikk * 4 + k] = G[k];
-#pragma unroll
-      for (int j = 0; j < 18; ++j) K[j] = (j == ikk) ? kd : R(0);
-      frow = kd * (R)fv[ikk];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) G[k] = 0;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 18; ++j)
-        if (fx[j]) { frow -= K[j] * (R)fv[j]; K[j] = 0; }
-    }
-  }
-  __syncthreads();
-  if (live) {
-    f_el[(e0 + el) * 18 + ikk] = (double)frow;
-    if (ikk < 4) {
-      R h = 0;
-      for (int r2 = 0; r2 < 18; ++r2)
-        if (fx[r2]) h -= G0[el * 72 + r2 * 4 + ikk] * (R)fv[r2];
-      h_el[(e0 + el) * 4 + ikk] = (double)h;
-    }
-  }
-  // ---- stage outputs and store coalesced (skipped in rhs-only mode) ----
-  if (vv_full == nullptr && vv_K == nullptr) return;
-  if (!blocks) {
+    bool flag = false;
+    int64_t dof = 0;
     if (live) {
-      S* o = outs + el * 468 + ikk * 26;                                   // :268-276
-#pragma unroll
-      for (int j = 0; j < 18; ++j) o[j] = (S)K[j];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { o[18 + 2 * k] = (S)G[k]; o[19 + 2 * k] = (S)G[k]; }
+      const int64_t e = e0 + el;
+      dof = 2 * q2_node((int)(e % b.nelx), (int)(e / b.nelx), i, nnx) + c;     // local_to_globalV, meeuuw.py:874-882
+      flag = in.bc_fix_V[dof] != 0;
     }
     __syncthreads();
-    S* dst = vv_full + e0 * 468;
-    for (int x = tid; x < ne * 468; x += blockDim.x) dst[x] = outs[x];
-  } else {
-    S* oK = outs;                    // EB*324
-    S* oG = oK + EB_S * 324;         // EB*72
-    S* oGT = oG + EB_S * 72;
-    S* oH = oGT + EB_S * 72;
-    S* oM = oH + EB_S * 72;          // EB*16
-    S* oMe = oM + EB_S * 16;
-    if (live) {
+    if (flag) {
+      bcv[tid] = in.bc_val_V[dof];
+      atomicOr(bcf + el, 1u << ikk);
+    }
+    // derivatives at the Gauss points: build_matrix_stokes.py:131-134
+    for (int t = tid; t < ne * 81; t += NT) {
+      const int q = t / 9, k = t % 81;                                   // q: point of the batch
+      const R r = drV[2 * k], u = drV[2 * k + 1];
+      dV[t] = Pair<R>{jc[q] * r + jc[L::Q + q] * u, jc[2 * L::Q + q] * r + jc[3 * L::Q + q] * u};
+    }
+    if (BLOCKS)
+      for (int t = tid; t < ne * 36; t += NT) {
+        const int q = t / 4, k = t % 36;
+        const R r = drP[2 * k], u = drP[2 * k + 1];
+        dP[t] = Pair<R>{jc[q] * r + jc[L::Q + q] * u, jc[2 * L::Q + q] * r + jc[3 * L::Q + q] * u};
+      }
+    __syncthreads();
+
+    R K[18], G[4], H[4], Mv = 0, f = 0;
 #pragma unroll
-      for (int j = 0; j < 18; ++j) oK[el * 324 + ikk * 18 + j] = (S)K[j];       // :237-240
+    for (int j = 0; j < 18; ++j) K[j] = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { G[k] = 0; H[k] = 0; }
+    if (live) {
+#pragma unroll 1
+      for (int q = 0; q < 9; ++q) {
+        const int eq = el * 9 + q;
+        const R w = wq[eq], jxw = wq[L::Q + eq];
+        const Pair<R>* d = dV + el * 81 + q * 9;
+        const Pair<R> di = d[i];
+        // B^T C B (build_matrix_stokes.py:140), C = diag(2, 2, 1): with (o, t) the row's own direction and
+        // the other one, K_own = 2 o o_j + t t_j, K_other = t o_j
+        const R own = c == 0 ? di.x : di.z, oth = c == 0 ? di.z : di.x;
+        const R wo = R(2) * w * own, wt = w * oth;
+        if (c == 0) {
+#pragma unroll
+          for (int j = 0; j < 9; ++j) {
+            const Pair<R> dj = d[j];
+            K[2 * j] += wo * dj.x;
+            K[2 * j] += wt * dj.z;
+            K[2 * j + 1] += wt * dj.x;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 9; ++j) {
+            const Pair<R> dj = d[j];
+            K[2 * j + 1] += wo * dj.z;
+            K[2 * j + 1] += wt * dj.x;
+            K[2 * j] += wt * dj.z;
+          }
+        }
+        const R n = NV[q * 9 + i];
+        f += n * wq[(2 + c) * L::Q + eq];                                // :142-143
+        const R oj = own * jxw;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) G[k] -= oj * NP[q * 4 + k];          // :144-146
+        if (BLOCKS) {
+          const R nj = n * jxw;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const Pair<R> dk = dP[eq * 4 + k];
+            H[k] += (c == 0 ? dk.x : dk.z) * nj;                         // :148-153
+          }
+          if (ikk < 16) Mv += NP[q * 4 + (ikk >> 2)] * NP[q * 4 + (ikk & 3)] * jxw;   // :147
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) G[k] *= s;
+    }
+    // ---- Dirichlet elimination (row-local form) ----
+    const unsigned fx = live ? bcf[el] : 0;
+    const double* fv = bcv + el * 18;
+    R frow = f;
+    R G1[4] = {G[0], G[1], G[2], G[3]};
+    if (fx) {
+      if (fx >> ikk & 1) {
+        R kd = 0;
+#pragma unroll
+        for (int j = 0; j < 18; ++j) {
+          if (j == ikk) kd = K[j];
+          else K[j] = 0;
+        }
+        frow = kd * (R)fv[ikk];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) G[k] = 0;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 18; ++j)
+          if (fx >> j & 1) { frow -= K[j] * (R)fv[j]; K[j] = 0; }
+      }
+    }
+    __syncthreads();                                       // the derivatives are read: their room is reused
+    if (fx >> ikk & 1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) G0[el * 72 + ikk * 4 + k] = G1[k];
+    }
+    __syncthreads();
+    if (live) {
+      f_el[(e0 + el) * 18 + ikk] = (double)frow;
+      if (ikk < 4) {
+        R h = 0;
+        for (unsigned m = fx; m; m &= m - 1) {
+          const int r2 = __ffs(m) - 1;
+          h -= G0[el * 72 + r2 * 4 + ikk] * (R)fv[r2];
+        }
+        h_el[(e0 + el) * 4 + ikk] = (double)h;
+      }
+    }
+    __syncthreads();
+    if (!write) continue;                                  // right-hand sides only
+    // ---- the element results in the reference's order ----
+    if (!BLOCKS) {
+      if (live) {
+        Pair<R>* o = reinterpret_cast<Pair<R>*>(outs + el * 468 + ikk * 26);    // :268-276
+#pragma unroll
+        for (int j = 0; j < 9; ++j) o[j] = Pair<R>{K[2 * j], K[2 * j + 1]};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[9 + k] = Pair<R>{G[k], G[k]};
+      }
+    } else if (live) {
+      R* oK = outs + el * 324 + ikk * 18;
+      R *oG = outs + EB_S * 324, *oGT = oG + EB_S * 72, *oH = oGT + EB_S * 72, *oM = oH + EB_S * 72, *oMe = oM + EB_S * 16;
+#pragma unroll
+      for (int j = 0; j < 18; ++j) oK[j] = K[j];                                // :237-240
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        oG[el * 72 + ikk * 4 + k] = (S)G[k];                                    // :243-246
-        oGT[el * 72 + k * 18 + ikk] = (S)G[k];                                  // :249-252
-        oH[el * 72 + k * 18 + ikk] = (S)H[k];                                   // :255-258
+        oG[el * 72 + ikk * 4 + k] = G[k];                                       // :243-246
+        oGT[el * 72 + k * 18 + ikk] = G[k];                                     // :249-252
+        oH[el * 72 + k * 18 + ikk] = H[k];                                      // :255-258
       }
       if (ikk < 16) {
-        oM[el * 16 + ikk] = (S)Mv;                                              // :261-265
-        oMe[el * 16 + ikk] = (S)(Mv / (R)in.eta_e[e0 + el]);
+        oM[el * 16 + ikk] = Mv;                                                 // :261-265
+        oMe[el * 16 + ikk] = Mv / (R)in.eta_e[e0 + el];
       }
     }
+    if (bulk) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the results, before the copies
     __syncthreads();
-    for (int x = tid; x < ne * 324; x += blockDim.x) vv_K[e0 * 324 + x] = oK[x];
-    for (int x = tid; x < ne * 72; x += blockDim.x) {
-      vv_G[e0 * 72 + x] = oG[x]; vv_GT[e0 * 72 + x] = oGT[x]; vv_H[e0 * 72 + x] = oH[x];
+    auto put = [&](R* dst, const R* src, int per) {
+      if (bulk) {
+        if (tid == 0) bulk_store(dst + e0 * per, src, (unsigned)(ne * per * sizeof(R)));
+      } else {
+        for (int x = tid; x < ne * per; x += NT) dst[e0 * per + x] = src[x];
+      }
+    };
+    if (!BLOCKS) {
+      put(vv_full, outs, 468);
+    } else {
+      const R *oG = outs + EB_S * 324, *oGT = oG + EB_S * 72, *oH = oGT + EB_S * 72, *oM = oH + EB_S * 72;
+      put(vv_K, outs, 324);
+      put(vv_G, oG, 72);
+      put(vv_GT, oGT, 72);
+      put(vv_H, oH, 72);
+      put(vv_M, oM, 16);
+      put(vv_Meta, oM + EB_S * 16, 16);
     }
-    for (int x = tid; x < ne * 16; x += blockDim.x) { vv_M[e0 * 16 + x] = oM[x]; vv_Meta[e0 * 16 + x] = oMe[x]; }
+    if (bulk && tid == 0) {                                // the room is free once the copies have read it
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    __syncthreads();
   }
+  if (bulk && tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // Sum element-local vectors onto Q2 nodes (ndof per node) in ascending element order.
@@ -372,27 +449,22 @@ __global__ void k_body_force(mw_box b, const double* __restrict__ rhoq, const do
   }
 }
 
-template <typename R>
-static size_t stokes_smem_bytes() {
-  size_t n = 117 + 2 * EB_S * 81 + 2 * EB_S * 36 + 5 * EB_S * 9 + EB_S * 72;
-  size_t bytes = n * sizeof(R);
-  bytes = ((bytes + 15) & ~size_t(15)) + 16;
-  bytes += EB_S * 18 * sizeof(double) + EB_S * 18 * sizeof(int);
-  bytes += (size_t)EB_S * 572 * sizeof(double);   // largest staged output (blocks layout, f64)
-  return bytes;
-}
-
-template <typename R, typename S>
-static int launch_stokes(const mw_box& b, const mw_stokes_in& in, const mw_stokes_out& out, int blocks, double* fel,
-                         double* hel, cudaStream_t s) {
-  int64_t nel = (int64_t)b.nelx * b.nelz;
-  size_t sm = stokes_smem_bytes<R>();
-  auto kern = k_assemble_stokes<R, S>;
+template <typename R, bool BLOCKS>
+static int launch_stokes(const mw_box& b, const mw_stokes_in& in, const mw_stokes_out& out, double* fel, double* hel,
+                         cudaStream_t s) {
+  const int64_t nel = (int64_t)b.nelx * b.nelz;
+  auto kern = k_assemble_stokes<R, BLOCKS>;
+  constexpr size_t sm = StokesSmem<R, BLOCKS>::bytes;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
     return MW_ERR_CUDA;
-  unsigned grid = (unsigned)((nel + EB_S - 1) / EB_S);
-  kern<<<grid, EB_S * 18, sm, s>>>(b, in, blocks, (S*)out.VV_Stokes, (S*)out.VV_K, (S*)out.VV_G, (S*)out.VV_GT,
-                                   (S*)out.VV_M, (S*)out.VV_M_eta, (S*)out.VV_H, fel, hel);
+  const void* const all[7] = {out.VV_Stokes, out.VV_K, out.VV_G, out.VV_GT, out.VV_M, out.VV_M_eta, out.VV_H};
+  const int write = BLOCKS ? out.VV_K != nullptr : out.VV_Stokes != nullptr;
+  int bulk = 1;                            // an element's results are a multiple of 16 bytes in every array
+  for (int k = BLOCKS ? 1 : 0; k < (BLOCKS ? 7 : 1); ++k)
+    if ((uintptr_t)all[k] & 15) bulk = 0;
+  const unsigned grid = (unsigned)std::min<int64_t>((nel + EB_S - 1) / EB_S, StokesSmem<R, BLOCKS>::CTAS * num_sms());
+  kern<<<grid, EB_S * 18, sm, s>>>(b, in, write, bulk, (R*)out.VV_Stokes, (R*)out.VV_K, (R*)out.VV_G, (R*)out.VV_GT,
+                                   (R*)out.VV_M, (R*)out.VV_M_eta, (R*)out.VV_H, fel, hel);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }
@@ -419,8 +491,11 @@ int mw_assemble_stokes(mw_box box, int32_t blocks, int32_t precision, mw_stokes_
   int64_t nel = (int64_t)box.nelx * box.nelz;
   double* fel = (double*)work;
   double* hel = fel + nel * 18;
-  int rc = precision == MW_F32 ? launch_stokes<float, float>(box, in, out, blocks, fel, hel, s)
-                               : launch_stokes<double, double>(box, in, out, blocks, fel, hel, s);
+  const bool f32 = precision == MW_F32;
+  int rc = blocks ? (f32 ? launch_stokes<float, true>(box, in, out, fel, hel, s)
+                         : launch_stokes<double, true>(box, in, out, fel, hel, s))
+                  : (f32 ? launch_stokes<float, false>(box, in, out, fel, hel, s)
+                         : launch_stokes<double, false>(box, in, out, fel, hel, s));
   if (rc) return rc;
   int64_t nn = (int64_t)(2 * box.nelx + 1) * (2 * box.nelz + 1);
   k_gather_q2<<<grid_for(nn, 256), 256, 0, s>>>(box, 2, fel, out.rhs_f);

@@ -543,8 +543,9 @@ constexpr size_t E_SMEM = (size_t)(ENEL * 9 + ELZ * ELX) * sizeof(double) + 16;
 // The first box of EK_P and EK_S, the flags and the diagonal are requested before the predecessor is
 // waited for: the set-up that wrote them is at least two launches back.  The products overwrite the
 // coefficients and the tile is 7 elements high, which leaves room for four CTAs an SM (16 x 8: three;
-// 300x200 elements are 551 tiles, one wave instead of two, 17.6 -> 13.9 us a product).  A load not complete after E_SPIN polls sets
-// MW_FLAG_ITER_LIMIT in *flag (when given), waits for it once more (bounded) and stops computing.
+// 300x200 elements are 551 tiles, one wave instead of two, 17.6 -> 13.9 us a product).  A load not
+// complete after E_SPIN polls sets MW_FLAG_ITER_LIMIT in *flag (when given), waits for it once more
+// (bounded) and stops computing.
 // Without TMA (an operator buffer that is not 16-byte aligned) the coefficients are read from global
 // memory.
 template <int KIND, bool TMA>
