@@ -242,7 +242,8 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       }
     } else if (live) {
       R* oK = outs + el * 324 + ikk * 18;
-      R *oG = outs + EB_S * 324, *oGT = oG + EB_S * 72, *oH = oGT + EB_S * 72, *oM = oH + EB_S * 72, *oMe = oM + EB_S * 16;
+      R *oG = outs + EB_S * 324, *oGT = oG + EB_S * 72, *oH = oGT + EB_S * 72, *oM = oH + EB_S * 72;
+      R* oMe = oM + EB_S * 16;
 #pragma unroll
       for (int j = 0; j < 18; ++j) oK[j] = K[j];                                // :237-240
 #pragma unroll

@@ -58,7 +58,7 @@ def workspace(tag="default"):
     if owner is not None:
         key = (tag, "model", owner)
     else:
-        key = (tag, torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else 0)
+        key = (tag, L.stream_handle() if torch.cuda.is_available() else 0)
     if key not in _ws:
         _ws[key] = Workspace()
     return _ws[key]

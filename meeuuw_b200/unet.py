@@ -131,7 +131,7 @@ _bufs = {}
 def _buf(key, shape, dtype, zero=False):
     """Scratch tensor reused across calls with the same key on the same stream (consumed in stream
     order; models advanced concurrently on different streams never share one)."""
-    k = (key, dtype, torch.cuda.current_stream().cuda_stream)
+    k = (key, dtype, L.stream_handle())
     b = _bufs.get(k)
     if b is None or tuple(b.shape) != tuple(shape):
         b = (torch.zeros if zero else torch.empty)(shape, dtype=dtype, device="cuda")
