@@ -57,4 +57,29 @@ template <typename R> void mg_down(const MgArgs<R>& a, int deg, bool planes, cud
 // The coarse correction and `deg` smoothing steps.
 template <typename R> void mg_up(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s);
 
+// The coarse end of a V-cycle in one launch (mg_tail.cu): `n` smoothed levels of at most MG_TAIL_CELLS cells
+// ((nx + 1)(nz + 1)) and the coarsest level's dense inverse.
+constexpr int MG_TAIL_CELLS = 384, MG_TAIL_LEVELS = 5;
+template <typename R>
+struct MgTailLevel {
+  LevelGeo g;
+  const R *eta, *diag, *dinv;          // eta: one value per element
+  const uint8_t* fix;
+  const double* cheb;
+  Transfer1D tx, tz;                   // to the next level
+};
+template <typename R>
+struct MgTailArgs {
+  MgTailLevel<R> L[MG_TAIL_LEVELS];
+  int n, nd;
+  LevelGeo gd;                         // the coarsest level: nd unknowns, Ainv
+  const uint8_t* fixd;
+  const double* Ainv;
+  const R* b;                          // the first level's right-hand side ...
+  R* x;                                // ... and result
+};
+int mg_tail_ensure_tables();
+// false when the levels' vectors do not fit one CTA's shared memory (nothing is launched)
+template <typename R> bool mg_tail(const MgTailArgs<R>& a, int deg, cudaStream_t s);
+
 }  // namespace mw

@@ -55,8 +55,8 @@ static int ensure_ref_tables() {
   if (g_ref_ready) return MW_OK;
   RefTables T;
   host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || op_ensure_tables() ||
-      setup_ensure_tables())
+  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || mg_tail_ensure_tables() ||
+      op_ensure_tables() || setup_ensure_tables())
     return MW_ERR_CUDA;
   g_ref_ready = true;
   return MW_OK;
@@ -2794,6 +2794,32 @@ static void launch_tail(Hierarchy<R>& H, int l0, bool first_done, cudaStream_t s
   tail_swaps(H, l0, first_done);
 }
 
+// The cycle from level l down in one launch where every level fits a CTA (mg_tail.cu) and some transfer
+// there is not nested; false when it goes level by level.  One CTA takes 3000 clocks an apply at 20 x 14
+// cells and 1800 at one warp; the level launches spread theirs over several SMs and cost 2.9 us each when
+// nested (64^2: 37 us a cycle by levels, 46 with the tail), 4 to 5 when not (150x97, from 19 x 13: 31 us in
+// the tail, 40 by levels).
+template <typename R>
+static bool vcycle_tail(Hierarchy<R>& H, int l, cudaStream_t s) {
+  const int n = H.nlev - 1 - l;
+  if (l < 1 || n < 1 || n > MG_TAIL_LEVELS || !H.dense || H.L[l].deg > MG_MAXDEG) return false;
+  if ((int64_t)(H.L[l].g.nx + 1) * (H.L[l].g.nz + 1) > MG_TAIL_CELLS) return false;
+  bool nested = true;
+  for (int i = l; i + 1 < H.nlev; ++i) nested = nested && nested_levels(H.L[i].g, H.L[i + 1].g);
+  if (nested) return false;
+  MgTailArgs<R> a;
+  memset(&a, 0, sizeof(a));
+  for (int i = 0; i < n; ++i) {
+    const Level<R>& L = H.L[l + i];
+    a.L[i] = MgTailLevel<R>{L.g, L.etap, L.diag, L.dinv, L.fix, L.cheb, transfer_of(L, H.L[l + i + 1], 0),
+                            transfer_of(L, H.L[l + i + 1], 1)};
+  }
+  const Level<R>& D = H.L[H.nlev - 1];
+  a.n = n; a.nd = H.nd; a.gd = D.g; a.fixd = D.fix; a.Ainv = H.Ainv;
+  a.b = H.L[l].b; a.x = H.L[l].x;
+  return mg_tail<R>(a, H.L[l].deg, s);
+}
+
 // bx: (L.b, result) of the finest level wanted there (summed in its upward launch, or on its own)
 template <typename R>
 static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = false, const ParitySum* bx = nullptr) {
@@ -2802,6 +2828,7 @@ static void vcycle(Hierarchy<R>& H, int l, cudaStream_t s, bool first_done = fal
     launch_tail(H, l, first_done, s);        // records the tail's pointer swaps too
     return;
   }
+  if (!first_done && H.tail0 == 0 && vcycle_tail(H, l, s)) return;
   if (l == H.nlev - 1) {
     if (H.dense) {
       int nd = H.nd;
