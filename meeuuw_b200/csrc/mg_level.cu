@@ -17,7 +17,7 @@
 // 16 - 2 deg upward.  Tiles of 32 x 16 cells repeat less (owning 26 x 10 and 28 x 12 of them in
 // FP32) but were slower at every size (V-cycle at 512^2 180 against 169 us, at 64^2 42 against 37).
 //
-// Measured, FP32 V-cycle from launch to launch (the separate launches before): 512^2 293 -> 169 us,
+// Measured, FP32 V-cycle from launch to launch (the separate launches before): 512^2 293 -> 158 us,
 // 256^2 184 -> 79, 128^2 139 -> 52, 64^2 107 -> 37, 8^2 31 -> 11; FP64, one smoothing step: 512^2 309 ->
 // 232, 128^2 104 -> 55.
 //
@@ -65,24 +65,32 @@ MW_D void restrict_taps(const R2* sr, int c, double* s0, double* s1) {
 
 // owned cells a side of a tile.  Downward between levels that are not nested a coarse node's taps reach
 // up to four fine nodes to its right (three between nested ones), one cell more of halo.
-constexpr int owned_cells(bool down, int deg, bool nested) { return CELLS - (down ? 2 * deg + (nested ? 2 : 3) : 2 * deg); }
+constexpr int owned_cells(bool restricts, int applies, bool nested) {
+  return CELLS - 2 * applies - (restricts ? (nested ? 2 : 3) : 0);
+}
 
 // DOWN: pre-smoothing, residual, restriction; else correction and post-smoothing.  DEG: smoothing
 // steps.  PLANES: nine viscosity planes (else one value per element).  NESTED: both element counts
-// halve (compile-time taps); else the transfer tables.
-template <typename R, int DEG, bool DOWN, bool PLANES, bool NESTED>
+// halve (compile-time taps); else the transfer tables.  PART: downward with DEG = 2, the smoothing
+// (PART_SMOOTH) or the residual of a.xin and its restriction (PART_RESID) alone.
+enum { PART_ALL = 0, PART_SMOOTH, PART_RESID };
+template <typename R, int DEG, bool DOWN, bool PLANES, bool NESTED, int PART = PART_ALL>
 __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_level(MgArgs<R> a) {
   typedef typename Vec2<R>::T R2;
   constexpr int CX = CELLS, CZ = CELLS, NC = CX * CZ;
-  constexpr int LO = DOWN ? DEG + 1 : DEG;                  // halo cells on the left and below
-  constexpr int TX = owned_cells(DOWN, DEG, NESTED), TZ = TX;
+  constexpr int J0 = PART == PART_RESID ? DEG - 1 : 0, J1 = PART == PART_SMOOTH ? DEG - 1 : DEG;   // applies
+  constexpr int AP = J1 - J0;
+  constexpr bool RESTRICT = DOWN && PART != PART_SMOOTH;
+  constexpr int LO = RESTRICT ? AP + 1 : AP;                // halo cells on the left and below
+  constexpr int TX = owned_cells(RESTRICT, AP, NESTED), TZ = TX;
   constexpr int WX = NESTED ? CX + 3 : 26, WZ = WX;         // staged coarse nodes (upward): not nested, the 32
                                                             // fine nodes span at most 25 (nf / nc >= 3 / 2)
+  static_assert(PART == PART_ALL || (DOWN && DEG > 1), "only a smoothing step and a residual are split");
   static_assert(!NESTED || TX % 2 == 0, "tiles start at even cells (transfer parity)");
   __shared__ __align__(16) R2 sx[4 * NC];                   // masked x (then the residual) by node type
   __shared__ __align__(16) R2 se[5 * NC];                   // sums for the right and upper neighbours
   __shared__ __align__(16) double2 sc[DOWN ? 1 : WX * WZ];
-  constexpr int CN = DOWN && !NESTED ? 16 : 1;              // coarse nodes a tile restricts to, per side (at most 13)
+  constexpr int CN = RESTRICT && !NESTED ? 16 : 1;          // coarse nodes a tile restricts to, per side (at most 16)
   __shared__ double sw[2][CN][RTAPS];                       // their weights, first fine nodes and counts
   __shared__ int si[2][CN], sn[2][CN];
   const int tid = threadIdx.x, lx = tid % CX, lz = tid / CX;
@@ -126,7 +134,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
     for (int q = 0; q < 9; ++q) eq[q] = R(0);
   }
   int j0 = 0, k0 = 0, mx = 0, mz = 0;                       // the coarse nodes on the tile's owned cells: coarse
-  if constexpr (DOWN && !NESTED) {                          // node J lies at fine lattice position J nf / nc
+  if constexpr (RESTRICT && !NESTED) {                      // node J lies at fine lattice position J nf / nc
     auto first = [](int c, int nf, int nc) { return (int)((2LL * c * nc + nf - 1) / nf); };
     j0 = first(ex0, g.nx, a.gc.nx);
     k0 = first(ez0, g.nz, a.gc.nz);
@@ -166,9 +174,10 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
     if (has[t]) {
       const int64_t n = n0 + (t >> 1) * g.nnx + (t & 1);
       b[t] = reinterpret_cast<const R2*>(a.b)[n];
-      if (!DOWN) x[t] = reinterpret_cast<const R2*>(a.xin)[n];
+      if (!DOWN || PART == PART_RESID) x[t] = reinterpret_cast<const R2*>(a.xin)[n];
     }
-  if constexpr (DOWN) {                                     // x0 = d0 = (1/theta) D^-1 b
+  if constexpr (PART == PART_RESID) {
+  } else if constexpr (DOWN) {                              // x0 = d0 = (1/theta) D^-1 b
 #pragma unroll
     for (int t = 0; t < 4; ++t) d[t] = x[t] = div2(pair(c20 * b[t].x, c20 * b[t].y), dg[t], di[t]);
   } else if constexpr (!NESTED) {
@@ -242,13 +251,14 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
     return pair((fx & (1u << (2 * t))) ? R(0) : x[t].x, (fx & (2u << (2 * t))) ? R(0) : x[t].y);
   };
 #pragma unroll
-  for (int j = 0; j < DEG; ++j) {
+  for (int j = J0; j < J1; ++j) {
     // ---- y = K x at the cell's nodes ----
+    const int in = j - J0;                                  // cells the halo has shrunk by
     R2 u[9], y[9];
     u[0] = masked(0); u[4] = masked(1); u[7] = masked(2); u[8] = masked(3);
     sx[tid] = u[0]; sx[NC + tid] = u[4]; sx[2 * NC + tid] = u[7]; sx[3 * NC + tid] = u[8];
     __syncthreads();
-    if (has[3] && lx >= j && lx <= CX - 2 - j && lz >= j && lz <= CZ - 2 - j) {
+    if (has[3] && lx >= in && lx <= CX - 2 - in && lz >= in && lz <= CZ - 2 - in) {
       u[1] = sx[tid + 1];
       u[5] = sx[2 * NC + tid + 1];
       u[3] = sx[tid + CX];
@@ -281,7 +291,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
       const int ownx = min(ex0 + TX >= g.nx ? TX + 1 : TX, g.nx + 1 - ex0);
       const int ownz = min(ez0 + TZ >= g.nz ? TZ + 1 : TZ, g.nz + 1 - ez0);
       const bool own = lx >= LO && lx < LO + ownx && lz >= LO && lz < LO + ownz;
-      if (own) {
+      if (own && PART != PART_RESID) {
 #pragma unroll
         for (int t = 0; t < 4; ++t)
           if (has[t]) {
@@ -355,7 +365,7 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
       }
     }
   }
-  if constexpr (!DOWN) {
+  if constexpr (!RESTRICT) {
     const int ownx = ex0 + TX >= g.nx ? TX + 1 : TX, ownz = ez0 + TZ >= g.nz ? TZ + 1 : TZ;
     double v = 0;
     if (lx >= LO && lx < LO + ownx && lz >= LO && lz < LO + ownz) {
@@ -363,19 +373,37 @@ __global__ void __launch_bounds__(CELLS * CELLS, sizeof(R) == 4 ? 2 : 1) k_mg_le
       for (int t = 0; t < 4; ++t)
         if (has[t]) {
           reinterpret_cast<R2*>(a.x)[n0 + (t >> 1) * g.nnx + (t & 1)] = x[t];
-          if (a.bx.part) v += (double)b[t].x * (double)x[t].x + (double)b[t].y * (double)x[t].y;
+          if (!DOWN && a.bx.part) v += (double)b[t].x * (double)x[t].x + (double)b[t].y * (double)x[t].y;
         }
     }
-    if (a.bx.part) grid_sum_parity(v, a.bx, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
+    if (!DOWN && a.bx.part) grid_sum_parity(v, a.bx, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
   }
 }
 
-template <typename R, int DEG, bool DOWN, bool NESTED>
+template <typename R, int DEG, bool DOWN, bool NESTED, int PART = PART_ALL>
 void launch(const MgArgs<R>& a, bool planes, cudaStream_t s) {
-  constexpr int T = owned_cells(DOWN, DEG, NESTED);
+  constexpr int T = owned_cells(DOWN && PART != PART_SMOOTH, PART == PART_ALL ? DEG : 1, NESTED);
   const dim3 grid((a.g.nx + T - 1) / T, (a.g.nz + T - 1) / T);
-  if (planes) pdl_launch(k_mg_level<R, DEG, DOWN, true, NESTED>, grid, CELLS * CELLS, 0, s, a);
-  else pdl_launch(k_mg_level<R, DEG, DOWN, false, NESTED>, grid, CELLS * CELLS, 0, s, a);
+  if (planes) pdl_launch(k_mg_level<R, DEG, DOWN, true, NESTED, PART>, grid, CELLS * CELLS, 0, s, a);
+  else pdl_launch(k_mg_level<R, DEG, DOWN, false, NESTED, PART>, grid, CELLS * CELLS, 0, s, a);
+}
+
+// Downward with two smoothing steps on large levels: the smoothing and the residual with its restriction as
+// two launches.  Together they repeat 256 / 100 of the element products (a tile owns 10 x 10 cells), apart
+// 256 / 196 and 256 / 144; in exchange x is read back and there is one more launch.  FP32 V-cycle with every
+// level above the line split, against none: 512^2 165.5 -> 158 us, 384^2 111.5 -> 107; splitting 256^2 as
+// well changes nothing there (77.5, 77.3), 128^2 and below lose (77.5 -> 78.9 with all of them).
+constexpr int64_t SPLIT_ELEMENTS = 1 << 16;
+template <typename R, bool NESTED>
+void down2(const MgArgs<R>& a, bool planes, cudaStream_t s) {
+  if ((int64_t)a.g.nx * a.g.nz <= SPLIT_ELEMENTS) {
+    launch<R, MG_MAXDEG, true, NESTED>(a, planes, s);
+    return;
+  }
+  launch<R, MG_MAXDEG, true, NESTED, PART_SMOOTH>(a, planes, s);
+  MgArgs<R> r = a;
+  r.xin = a.x;
+  launch<R, MG_MAXDEG, true, NESTED, PART_RESID>(r, planes, s);
 }
 
 template <typename R, bool DOWN>
@@ -385,8 +413,13 @@ void pick(const MgArgs<R>& a, int deg, bool planes, cudaStream_t s) {
     if (nested) launch<R, 1, DOWN, true>(a, planes, s);
     else launch<R, 1, DOWN, false>(a, planes, s);
   } else {
-    if (nested) launch<R, MG_MAXDEG, DOWN, true>(a, planes, s);
-    else launch<R, MG_MAXDEG, DOWN, false>(a, planes, s);
+    if constexpr (DOWN) {
+      if (nested) down2<R, true>(a, planes, s);
+      else down2<R, false>(a, planes, s);
+    } else {
+      if (nested) launch<R, MG_MAXDEG, false, true>(a, planes, s);
+      else launch<R, MG_MAXDEG, false, false>(a, planes, s);
+    }
   }
 }
 
