@@ -1688,12 +1688,26 @@ MW_D double mass_entry(const LevelGeo& g, int a, int c) {
   return m;
 }
 
-// One fused Chebyshev-Jacobi step for M_w x = b:  r = b - M_w x_in ; d = c1 d + c2 D^-1 r ;
-// x_out = x_in + d.  `first` means x_in = 0 (no product, no old direction).  For Q1 mass matrices
-// with positive element weights, lambda(D^-1 M_w) lies in [0.25, 2.25] whatever the weights
-// (element-by-element bound; the exactly integrated bilinear element matrix has D_e^-1 M_e eigenvalues
-// 9/4, 3/4, 3/4, 1/4), so the coefficients are fixed and need no dot products.
-// (the step at pressure node n; Me: the element mass matrix)
+// Chebyshev-Jacobi steps for M_w x = b:  r = b - M_w x ; d = c1 d + c2 D^-1 r ; x += d, the first one from
+// x = 0 (no product, no old direction).  For Q1 mass matrices with positive element weights,
+// lambda(D^-1 M_w) lies in [0.25, 2.25] whatever the weights (element-by-element bound; the exactly
+// integrated bilinear element matrix has D_e^-1 M_e eigenvalues 9/4, 3/4, 3/4, 1/4), so the coefficients are
+// fixed and need no dot products.
+//
+// A launch does up to MASS_STEPS of them: a thread keeps its node's b, d, x and weights, a tile of 32 x 32
+// nodes exchanges x through shared memory and loses a ring of nodes to every product (it owns 22 x 22 after
+// six steps from zero).  A launch a step cost a Schur iteration six launches of 3 us (64^2 elements) to 12
+// (512^2, where every step read its six vectors back): a solve of six steps 73 -> 38 us at 512^2, 22 -> 9 at
+// 64^2, whose time step (19 solves) goes 4.85 -> 4.61 ms.  Bounds: shared-memory loads (nine values and the
+// exchange a step) and FP64 issue, 0.7 us a step and SM; one CTA of 64 registers a thread.
+constexpr int MASS_TILE = 32, MASS_STEPS = 6;
+struct MassSteps {
+  int n, first;                    // steps; the first one starts from x = 0
+  double c1[MASS_STEPS], c2[MASS_STEPS];
+};
+
+// one step at pressure node n from global memory (the ensemble's clusters); Me: the element mass matrix, `first`
+// means x_in = 0
 MW_D void mass_cheb_node(const LevelGeo& g, const double* w, const double* b, const double* xin, double* xout,
                          double* d, const double* dg, double c1, double c2, int first, const double* Me, int64_t n) {
   const int ncx = g.nx + 1;
@@ -1717,29 +1731,83 @@ MW_D void mass_cheb_node(const LevelGeo& g, const double* w, const double* b, co
   xout[n] = (first ? 0.0 : xin[n]) + dn;
 }
 
-// m1 (first step): the sum of b, whose mean is removed from b before the step.  sum (last step, else
-// null): receives the sum of x.  zero (first step, may be null): a vector of np entries to clear.
-__global__ void k_mass_cheb(LevelGeo g, const double* __restrict__ w, double* __restrict__ b,
-                            const double* __restrict__ xin, double* __restrict__ xout, double* __restrict__ d,
-                            const double* __restrict__ dg, double c1, double c2, int first,
-                            const double* __restrict__ m1, double* __restrict__ zero, double* __restrict__ part,
-                            unsigned* __restrict__ counter, double* __restrict__ sum) {
-  __shared__ double Me[16];
-  if (threadIdx.x < 16) Me[threadIdx.x] = mass_entry(g, threadIdx.x / 4, threadIdx.x % 4);
+// m1: the sum of b, whose mean the steps take off b.  sum (may be null): receives the sum of x.  dout (may be
+// null): the direction, for a launch that goes on from xout.  zero (may be null): np entries to clear.
+__global__ void __launch_bounds__(MASS_TILE * MASS_TILE)
+    k_mass_steps(LevelGeo g, const double* __restrict__ w, const double* __restrict__ b, const double* __restrict__ m1,
+                 const double* __restrict__ xin, double* __restrict__ xout, const double* __restrict__ din,
+                 double* __restrict__ dout, const double* __restrict__ dg, const __grid_constant__ MassSteps st,
+                 double* __restrict__ zero, double* __restrict__ part, unsigned* __restrict__ counter,
+                 double* __restrict__ sum) {
+  constexpr int T = MASS_TILE;
+  __shared__ double Me[16], sx[2][T * T];
+  const int tid = threadIdx.x, lx = tid % T, lz = tid / T;
+  const int halo = st.n - (st.first ? 1 : 0), own = T - 2 * halo;
+  const int i = (int)blockIdx.x * own + lx - halo, j = (int)blockIdx.y * own + lz - halo;
+  const bool in = i >= 0 && i <= g.nx && j >= 0 && j <= g.nz;
+  const int64_t n = (int64_t)j * (g.nx + 1) + i;
+  if (tid < 16) Me[tid] = mass_entry(g, tid / 4, tid % 4);
+  // incident elements (j-1,i-1) k=2, (j-1,i) k=3, (j,i-1) k=1, (j,i) k=0
+  double we[4], dgn = 1.0;                                  // (missing elements: weight zero)
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int ex = (s & 1) ? i : i - 1, ez = (s & 2) ? j : j - 1;
+    we[s] = 0.0;
+    if (ex < 0 || ex >= g.nx || ez < 0 || ez >= g.nz) continue;
+    we[s] = w ? w[(int64_t)ez * g.nx + ex] : 1.0;
+  }
+  if (in) dgn = dg[n];
   pdl_entry();
+  const double mean = *m1 / (double)((int64_t)(g.nx + 1) * (g.nz + 1));
+  double bn = 0.0, x = 0.0, d = 0.0;
+  if (in) {
+    bn = b[n] - mean;
+    if (!st.first) {
+      x = xin[n];
+      d = din[n];
+    }
+  }
   __syncthreads();
-  const int64_t np = (int64_t)(g.nx + 1) * (g.nz + 1);
-  const double mean = m1 ? *m1 / (double)np : 0.0;
+  double me[16];
+#pragma unroll
+  for (int a = 0; a < 16; ++a) me[a] = Me[a];
+  int ring = 0;                                             // rings of the tile lost to products
+#pragma unroll 1
+  for (int k = 0; k < st.n; ++k) {
+    double y = 0;
+    if (k > 0 || !st.first) {
+      double* p = sx[ring & 1];
+      p[tid] = x;
+      ++ring;
+      __syncthreads();
+      if (lz < ring || lz >= T - ring || lx < ring || lx >= T - ring || !in) continue;
+      double q[9];
+#pragma unroll
+      for (int a = 0; a < 9; ++a) q[a] = a == 4 ? x : p[tid + (a / 3 - 1) * T + a % 3 - 1];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int kl = s == 0 ? 2 : (s == 1 ? 3 : (s == 2 ? 1 : 0)), c = (s >> 1) * 3 + (s & 1);   // lower left
+        double v = 0;
+#pragma unroll
+        for (int k2 = 0; k2 < 4; ++k2)
+          v += me[kl * 4 + k2] * q[c + (k2 == 1 || k2 == 2 ? 1 : 0) + (k2 >= 2 ? 3 : 0)];
+        y += we[s] * v;
+      }
+    }
+    const double r = bn - y;
+    d = k == 0 && st.first ? st.c2[k] * r / dgn : st.c1[k] * d + st.c2[k] * r / dgn;
+    x += d;
+  }
   double v = 0;
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < np; n += (int64_t)gridDim.x * blockDim.x) {
-    if (m1) b[n] -= mean;
+  if (in && lx >= halo && lx < halo + own && lz >= halo && lz < halo + own) {
+    xout[n] = x;
+    if (dout) dout[n] = d;
     if (zero) zero[n] = 0.0;
-    mass_cheb_node(g, w, b, xin, xout, d, dg, c1, c2, first, Me, n);
-    if (sum) v += xout[n];
+    v = x;
   }
   if (sum) {
     double t;
-    if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &t)) *sum = t;
+    if (grid_sum(v, part, counter, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, &t)) *sum = t;
   }
 }
 
@@ -1871,9 +1939,8 @@ __global__ void k_pcg_finish(int64_t n, const R* __restrict__ xr, double* __rest
 }
 
 // ---- the Schur-complement iteration around it (slots U_*): k_pcg_start_grad, the inner loop,
-// k_schur_div with (d, G^T z), k_schur_update with the sum of the new residual, the mass solve (which
-// removes that mean and sums its result), k_schur_dots with (r, w), (r, r) and the convergence test,
-// k_schur_direction.
+// k_schur_div with (d, G^T z), k_schur_update with the sum of the new residual, the mass solve of it less
+// its mean, k_schur_dots with (r, w), (r, r) and the convergence test, k_schur_direction.
 
 // G^T x of the inner solution x.  With V (the initial residual): V = x in double, out = G^T x - h and
 // its sum in U_M1; else (d, out) in U_DSD.  Adds the inner iteration count.
@@ -1943,17 +2010,18 @@ __global__ void k_schur_update(int64_t nv, int64_t np, const double* __restrict_
   if (grid_sum(v, part, counter, blockIdx.x, gridDim.x, &s)) sc[U_M1] = s;
 }
 
-// w -= its mean (sum in U_M2); (r, w) by the next iteration's parity, (r, r); then the start of the
+// r and w lose their means (sums in U_M1, U_M2); (r, w) by the next iteration's parity, (r, r); then the start of the
 // loop (first) or the end of an iteration, with its test unless the true residual decides
-__global__ void k_schur_dots(int64_t np, double* __restrict__ w, const double* __restrict__ r, int first,
+__global__ void k_schur_dots(int64_t np, double* __restrict__ w, double* __restrict__ r, int first,
                              double* __restrict__ part, unsigned* __restrict__ counter, double* __restrict__ sc,
                              LoopTest test) {
   pdl_entry();
-  const double mean = sc[U_M2] / (double)np;
+  const double mean = sc[U_M2] / (double)np, rmean = sc[U_M1] / (double)np;
   double a = 0, b = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-    const double wi = w[i] - mean, ri = r[i];
+    const double wi = w[i] - mean, ri = r[i] - rmean;
     w[i] = wi;
+    r[i] = ri;
     a += ri * wi;
     b += ri * ri;
   }
@@ -3199,33 +3267,41 @@ static int pcg_K(mw_stokes* S, Hierarchy<R>& H, R** pc, const double* b, double*
 }
 
 // Solve M_w x = b (M_w = M for uzawa3, weights null; M_eta for cd_u_eta, weights 1/eta_e) by `iters`
-// fixed-coefficient Chebyshev-Jacobi steps on lambda(D^-1 M_w) in [0.25, 2.25] (see mass_cheb_node): error
+// fixed-coefficient Chebyshev-Jacobi steps on lambda(D^-1 M_w) in [0.25, 2.25] (k_mass_steps): error
 // reduction 2 (1/2)^iters, no dot products, no host synchronisation.  The diagonals are refreshed by
 // mw_stokes_set_viscosity.  Replaces the splu solves of uzawa3_solver_L2.py:46-47 / cd_u_eta.py:284-289.
-// The first step removes b's mean (its sum in U_M1) and clears `zero` (may be null); the last leaves the
-// sum of x in U_M2.
-static void mass_solve(mw_stokes* S, const double* w, double* b, double* x, int iters, double* zero, cudaStream_t s) {
+// The right-hand side is b less its mean (its sum in U_M1; b itself keeps it).  Clears `zero` (may be null);
+// leaves the sum of x in U_M2.  Overwrites tP, tP2 and GTz.
+static void mass_solve(mw_stokes* S, const double* w, const double* b, double* x, int iters, double* zero,
+                       cudaStream_t s) {
   const LevelGeo& g = S->fine;
-  const int64_t n = (int64_t)(g.nx + 1) * (g.nz + 1);
   const double* dg = w ? S->medi : S->mdiag;
   const double a = 0.25 / 1.02, bb = 2.25 * 1.02;
   const double theta = 0.5 * (bb + a), delta = 0.5 * (bb - a), sigma = theta / delta;
   double rho = 1.0 / sigma;
-  double* bufs[2] = {x, S->tP};
-  const int K = iters < 1 ? 1 : iters;
-  for (int k = 0; k < K; ++k) {
-    double c1 = 0.0, c2 = 1.0 / theta;
-    if (k > 0) {
-      double rn = 1.0 / (2.0 * sigma - rho);
-      c1 = rn * rho;
-      c2 = 2.0 * rn / delta;
-      rho = rn;
+  double *xs[2] = {x, S->tP}, *ds[2] = {S->tP2, S->GTz};
+  const int K = iters < 1 ? 1 : iters, launches = (K + MASS_STEPS - 1) / MASS_STEPS;
+  for (int l = 0, k = 0; l < launches; ++l) {
+    MassSteps st;
+    memset(&st, 0, sizeof(st));
+    st.first = l == 0;
+    st.n = std::min(MASS_STEPS, K - k);
+    for (int q = 0; q < st.n; ++q, ++k) {
+      if (k == 0) {
+        st.c2[q] = 1.0 / theta;
+      } else {
+        const double rn = 1.0 / (2.0 * sigma - rho);
+        st.c1[q] = rn * rho;
+        st.c2[q] = 2.0 * rn / delta;
+        rho = rn;
+      }
     }
-    double* xin = bufs[(K - k) % 2];
-    double* xout = bufs[(K - 1 - k) % 2];
-    pdl_launch(k_mass_cheb, std::min(grid_for(n, 256), NB), 256, 0, s, g, w, b, xin, xout, S->tP2, dg, c1, c2, k == 0,
-               k == 0 ? (const double*)(S->sc + U_M1) : nullptr, k == 0 ? zero : nullptr, S->red, S->counter,
-               k == K - 1 ? S->sc + U_M2 : nullptr);
+    const int own = MASS_TILE - 2 * (st.n - (l == 0 ? 1 : 0));
+    const bool last = l == launches - 1;
+    pdl_launch(k_mass_steps, dim3((g.nx + own) / own, (g.nz + own) / own), MASS_TILE * MASS_TILE, 0, s, g, w, b,
+               (const double*)(S->sc + U_M1), (const double*)xs[(launches - l) % 2], xs[(launches - 1 - l) % 2],
+               (const double*)ds[(l + 1) % 2], last ? nullptr : ds[l % 2], dg, st, l == 0 ? zero : nullptr, S->red,
+               S->counter, last ? S->sc + U_M2 : nullptr);
   }
 }
 
@@ -3284,7 +3360,7 @@ struct Schur {
   }
   void tail(bool first, const LoopTest& t, cudaStream_t s) const {
     mass_solve(S, weights(), S->rP, S->wP, sp.mass_iters, first && from_zero ? P : nullptr, s);
-    pdl_launch(k_schur_dots, nb_for(np()), 256, 0, s, np(), S->wP, (const double*)S->rP, first ? 1 : 0, S->red,
+    pdl_launch(k_schur_dots, nb_for(np()), 256, 0, s, np(), S->wP, S->rP, first ? 1 : 0, S->red,
                S->counter, S->sc, t);
     if (!first && sp.history && sp.history_len > 0)
       pdl_launch(k_schur_history, 1, 1, 0, s, (const double*)S->sc, sp.history, sp.history_len);
