@@ -11,8 +11,10 @@
 // The time stepper uses the matrix-free form of the same operator instead (mw_energy_op_*): the
 // Gauss-point coefficients of the element matrices stored once per step, the element products
 // formed on the fly in shared-memory tiles, the right-hand side and the Jacobi diagonal formed by
-// the same kernel -- no element matrices are written or read.
+// the same kernel -- no element matrices are written or read.  Its products form the iteration's vectors
+// as they stage them: a BiCGSTAB iteration is three launches.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -170,7 +172,8 @@ struct BicgEnd {
 MW_D void bicg_condition(const BicgEnd& E) {
   const double rr = E.sc[11];
   if (E.use_h)
-    cudaGraphSetConditional(E.h, (isfinite(rr) && rr > E.rtol * E.rtol * E.sc[10] && E.sc[12] < (double)E.maxit) ? 1u : 0u);
+    cudaGraphSetConditional(
+        E.h, (isfinite(rr) && rr > E.rtol * E.rtol * E.sc[10] && E.sc[12] < (double)E.maxit) ? 1u : 0u);
 }
 
 // The sums of a kernel of KIND (a, and b where it has two) and what follows from them.  Called once,
@@ -549,11 +552,9 @@ constexpr size_t E_SMEM = (size_t)(ENEL * 9 + ELZ * ELX) * sizeof(double) + 16;
 // Without TMA (an operator buffer that is not 16-byte aligned) the coefficients are read from global
 // memory.
 template <int KIND, bool TMA>
-__global__ void __launch_bounds__(E_THREADS, E_CTAS_PER_SM) k_energy_op_apply(const __grid_constant__ CUtensorMap tmP, mw_box b,
-                                                                   EnergyOp op, const double* __restrict__ x,
-                                                                   const double* __restrict__ rhs,
-                                                                   double* __restrict__ y, BicgVecs V, BicgEnd E,
-                                                                   int32_t* flag) {
+__global__ void __launch_bounds__(E_THREADS, E_CTAS_PER_SM)
+    k_energy_op_apply(const __grid_constant__ CUtensorMap tmP, mw_box b, EnergyOp op, const double* __restrict__ x,
+                      const double* __restrict__ rhs, double* __restrict__ y, BicgVecs V, BicgEnd E, int32_t* flag) {
   constexpr bool ITER = KIND == EK_P || KIND == EK_S;
   extern __shared__ __align__(128) double esm[];
   double* sc = esm;                                     // TMA: the tile's coefficients; then the products
@@ -766,18 +767,23 @@ static bool eop_plane_map(CUtensorMap* m, mw_box b, const void* op) {
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Raises a kernel's shared-memory limit once per device (done: a bit per device).
+template <typename F>
+static void smem_limit(F* kernel, size_t bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done.load() >> dev & 1u) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+    done.fetch_or(uint64_t(1) << dev);
+}
+
 // Launches k_energy_op_apply<KIND> on the TMA path when the map could be made.
 template <int KIND>
 static void launch_eop_apply(bool tma, const CUtensorMap& tm, int grid, cudaStream_t s, mw_box b, const EnergyOp& op,
                              const double* x, const double* rhs, double* y, const BicgVecs& V, const BicgEnd& E,
                              int32_t* flag) {
   if (tma) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_energy_op_apply<KIND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)E_SMEM_TMA);
-      attr = true;
-    }
+    static std::atomic<uint64_t> done{0};
+    smem_limit(k_energy_op_apply<KIND, true>, E_SMEM_TMA, done);
     pdl_launch(k_energy_op_apply<KIND, true>, grid, E_THREADS, E_SMEM_TMA, s, tm, b, op, x, rhs, y, V, E, flag);
   } else {
     pdl_launch(k_energy_op_apply<KIND, false>, grid, E_THREADS, E_SMEM, s, tm, b, op, x, rhs, y, V, E, flag);
@@ -814,7 +820,8 @@ __global__ void k_bicg_s(int64_t n, const double* __restrict__ sc, BicgVecs V) {
 // a pass have their loads in flight together; one wave of four CTAs an SM (at three the launch was two
 // waves: 300x200 elements, 15 -> 11 us).
 constexpr int EX_THREADS = 256, EX_CTAS_PER_SM = 4;
-__global__ void __launch_bounds__(EX_THREADS, EX_CTAS_PER_SM) k_bicg_x(int64_t n, BicgVecs V, double* __restrict__ x, BicgEnd E) {
+__global__ void __launch_bounds__(EX_THREADS, EX_CTAS_PER_SM)
+    k_bicg_x(int64_t n, BicgVecs V, double* __restrict__ x, BicgEnd E) {
   pdl_entry();
   const double alpha = bicg_alpha(E.sc), omega = bicg_omega(E.sc);
   const double* __restrict__ p = (int)E.sc[12] & 1 ? V.p[1] : V.p[0];
@@ -952,7 +959,8 @@ static EnergyBufs energy_bufs(mw_box box, void* work, EnergyA A, double rtol, in
   E.grid = std::min(grid_for(n, 256), E_NB);
   E.grid_x = (int)std::min<int64_t>({(n + EX_THREADS - 1) / EX_THREADS, (int64_t)EX_CTAS_PER_SM * num_sms(), E_NB});
   E.flag = reinterpret_cast<int32_t*>(E.sc + 13);
-  E.end = BicgEnd{E.sc, w + 9 * n, reinterpret_cast<unsigned*>(E.sc + 200), rtol, maxit, 0, cudaGraphConditionalHandle(0)};
+  E.end = BicgEnd{E.sc, w + 9 * n, reinterpret_cast<unsigned*>(E.sc + 200), rtol, maxit, 0,
+                  cudaGraphConditionalHandle(0)};
   E.tma = false;
   memset(&E.tm, 0, sizeof(E.tm));
   if (A.op) {
@@ -1147,11 +1155,8 @@ int mw_energy_op_setup(mw_box box, mw_energy_in in, void* op, size_t op_bytes, d
   double* diag = planes + eop_plane_doubles(box);
   uint8_t* fix = reinterpret_cast<uint8_t*>(diag + eop_nodes(box));
   const int64_t ntile = (int64_t)((box.nelx + ETX - 1) / ETX) * ((box.nelz + ETZ - 1) / ETZ);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_energy_op_setup, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E_SMEM_SETUP);
-    attr = true;
-  }
+  static std::atomic<uint64_t> done{0};
+  smem_limit(k_energy_op_setup, E_SMEM_SETUP, done);
   pdl_launch(k_energy_op_setup, (int)std::min<int64_t>(ntile, 8 * num_sms()), ES_THREADS, E_SMEM_SETUP,
              (cudaStream_t)stream, box, in, planes, diag, fix, rhs, eop_view(box, op).flag);
   MW_CHECK_LAUNCH();

@@ -4,9 +4,9 @@
 // :659-1053, least squares :1061-1285, population control :1621-1812).  Interpolation and
 // advection are in advect.cu.
 //
-// Layout: particles are SoA (x, z, r, t: f64; iel: i32; active: u8), one thread per particle,
-// grid-stride loops sized to a multiple of the SM count.  Projections are atomic-free and
-// deterministic: particles are binned by element (counting sort, each bin sorted by particle
+// Layout: particles are SoA (x, z, r, t: f64; iel: i32; active: u8), one thread per particle where
+// particles are independent, groups of lanes per bin where they are summed; grid-stride loops sized to a
+// multiple of the SM count.  Projections are atomic-free and deterministic: particles are binned by element (counting sort, each bin sorted by particle
 // index), so every element and node sums its particles in particle-index order -- the order of
 // the reference's sequential loops.  This file is compiled with -fmad=false so the basis and
 // weight arithmetic rounds exactly as the reference's unfused double-precision code.

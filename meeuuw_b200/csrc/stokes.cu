@@ -6,11 +6,14 @@
 // M_eta-preconditioned form cd_u_eta.py:13-99; the reference solves K with SuperLU (splu), here
 // K^-1 is a multigrid-preconditioned conjugate gradient run on the device.
 //
-// Operator tiles: a CTA owns a TX x TZ tile of elements' nodes; it recomputes a one-element halo
-// on its left/bottom so that every owned node sums all its incident elements itself, in
-// ascending element order, from shared memory.  No atomics, deterministic results.  The element
-// kernel evaluates K u, G p, G^T u at the 3x3 Gauss points from the viscosity at the qpoints and
-// the uniform-box Jacobian (no stored element matrices).
+// The operator and its residuals are op_apply.cu, a level's half of a V-cycle mg_level.cu, the coarse
+// levels that are not nested mg_tail.cu, the hierarchy's set-up mg_setup.cu; here are the vector kernels
+// of the iterations, their graphs, and the element-tile operator (k_apply) that smoothing of degree above
+// two, single Chebyshev steps and the ensemble's clusters use: a CTA owns a TX x TZ tile of elements'
+// nodes and recomputes a one-element halo on its left/bottom.  Everywhere each node sums all its incident
+// elements itself, in ascending element order: no atomics, deterministic results.  The element kernels
+// evaluate K u, G p, G^T u at the 3x3 Gauss points from the viscosity at the qpoints and the
+// uniform-box Jacobian (no stored element matrices).
 //
 // Dirichlet semantics (identical to SpMV with the reference's eliminated COO): fixed velocity
 // dofs are zeroed before the element products; fixed rows return diag(K)_i * u_i; G rows of
@@ -90,8 +93,6 @@ struct ApplyArgs {
   R* xo;
   const double* cheb; // device coefficients {c1, c2}
   const double* cheb0;// AM_CHEB_Z: the first step's pair {0, 1/theta}
-  const R* xc;        // AM_CHEB_P: the coarse correction (interleaved u, w) ...
-  LevelGeo gc;        // ... on this coarse level
 };
 
 // Element contribution of K u_el + G p_el and G^T u_el at the 9 Gauss points: strain rate B u
@@ -2184,6 +2185,7 @@ struct Hierarchy {
   int tail0 = 0;             // first level of the cluster V-cycle tail (0: none)
   int64_t tail_len = 0;      // element products of its largest level (18 per element)
   R* tail_ye = nullptr;      // their global scratch
+  char* tables_end = nullptr;   // end of the transfer tables (from L[0].tj[0] on)
 };
 
 }  // namespace mw
@@ -2287,9 +2289,9 @@ static void plan_levels(Hierarchy<R>& H, const LevelGeo& fine, const mw_stokes_p
 
 
 
-// The transfer of one direction between nf and nc elements on the device tables (host-built; the
-// weights of pw_g and restrict_taps_1d).
-static int fill_transfer(int nf, int nc, int* dj, double* dw) {
+// The transfer of one direction between nf and nc elements as tables in host memory (the weights of pw_g and
+// restrict_taps_1d): pj, ri, rn into hj, pw and rw into hw.
+static int fill_transfer(int nf, int nc, int* hj, double* hw) {
   const int nnf = 2 * nf + 1, nnc = 2 * nc + 1;
   std::vector<int> j(nnf + 2 * nnc);
   std::vector<double> w(3 * (size_t)nnf + RTAPS * (size_t)nnc, 0.0);
@@ -2327,20 +2329,26 @@ static int fill_transfer(int nf, int nc, int* dj, double* dw) {
     j[nnf + J] = first;
     j[nnf + nnc + J] = last - first + 1;
   }
-  if (cudaMemcpy(dj, j.data(), sizeof(int) * j.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(dw, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-    return MW_ERR_CUDA;
+  std::copy(j.begin(), j.end(), hj);
+  std::copy(w.begin(), w.end(), hw);
   return MW_OK;
 }
 
+// Every level's tables, which carve() laid out in one piece, by one copy.
 template <typename R>
 static int fill_transfers(Hierarchy<R>& H) {
+  if (H.nlev < 2) return MW_OK;
+  char* const base = (char*)H.L[0].tj[0];
+  std::vector<double> host((H.tables_end - base) / sizeof(double), 0.0);
+  auto at = [&](void* device) { return (char*)host.data() + ((char*)device - base); };
   for (int l = 0; l + 1 < H.nlev; ++l)
     for (int d = 0; d < 2; ++d) {
       const LevelGeo &f = H.L[l].g, &c = H.L[l + 1].g;
-      if (int rc = fill_transfer(d ? f.nz : f.nx, d ? c.nz : c.nx, H.L[l].tj[d], H.L[l].tw[d])) return rc;
+      if (int rc = fill_transfer(d ? f.nz : f.nx, d ? c.nz : c.nx, (int*)at(H.L[l].tj[d]), (double*)at(H.L[l].tw[d])))
+        return rc;
     }
-  return MW_OK;
+  return cudaMemcpy(base, host.data(), sizeof(double) * host.size(), cudaMemcpyHostToDevice) == cudaSuccess ? MW_OK
+                                                                                                            : MW_ERR_CUDA;
 }
 
 template <typename R>
@@ -2367,12 +2375,15 @@ static void carve(Hierarchy<R>& H, Arena& A, const uint8_t* fine_fix) {
     L.lam2 = (double*)A.take(sizeof(double) * 4);
     L.ev = (R*)A.take(sizeof(R) * L.ndof);
     L.ev_ready = false;
-    for (int d = 0; d < 2 && l + 1 < H.nlev; ++d) {
-      const int nf = d ? L.g.nnz : L.g.nnx, nc = d ? H.L[l + 1].g.nnz : H.L[l + 1].g.nnx;
-      L.tj[d] = (int*)A.take(sizeof(int) * (nf + 2 * nc));
-      L.tw[d] = (double*)A.take(sizeof(double) * (3 * nf + RTAPS * nc));
-    }
   }
+  for (int l = 0; l + 1 < H.nlev; ++l)
+    for (int d = 0; d < 2; ++d) {
+      const LevelGeo &f = H.L[l].g, &c = H.L[l + 1].g;
+      const int nf = d ? f.nnz : f.nnx, nc = d ? c.nnz : c.nnx;
+      H.L[l].tj[d] = (int*)A.take(sizeof(int) * (nf + 2 * nc));
+      H.L[l].tw[d] = (double*)A.take(sizeof(double) * (3 * nf + RTAPS * nc));
+      H.tables_end = (char*)(H.L[l].tw[d] + (3 * nf + RTAPS * nc));
+    }
   H.Ainv = H.dense ? (double*)A.take(sizeof(double) * (size_t)H.nd * H.nd) : nullptr;
   H.tail_ye = H.tail0 ? (R*)A.take(sizeof(R) * H.tail_len) : nullptr;
 }
