@@ -2334,10 +2334,14 @@ static int fill_transfer(int nf, int nc, int* hj, double* hw) {
   return MW_OK;
 }
 
-// Every level's tables, which carve() laid out in one piece, by one copy.
+// Every level's tables, which carve() laid out in one piece, by one copy.  Nested levels have their taps at
+// compile time: a hierarchy of nothing else reads no tables, and its solver is created without waiting for
+// the device (16 us against 89 and a synchronous copy).
 template <typename R>
 static int fill_transfers(Hierarchy<R>& H) {
-  if (H.nlev < 2) return MW_OK;
+  bool nested = true;
+  for (int l = 0; l + 1 < H.nlev; ++l) nested = nested && nested_levels(H.L[l].g, H.L[l + 1].g);
+  if (nested) return MW_OK;
   char* const base = (char*)H.L[0].tj[0];
   std::vector<double> host((H.tables_end - base) / sizeof(double), 0.0);
   auto at = [&](void* device) { return (char*)host.data() + ((char*)device - base); };
