@@ -26,6 +26,10 @@ enum DevSlot {
   I_OUTER = 96, I_INNER, I_STATUS                             // info
 };
 
+// S_*, T_REL and I_* are the outcome of the last solve (mw_stokes_device_info): a call that is no solve
+// leaves them alone.  A residual asked for by itself has scalars of its own, this far from the solve's.
+constexpr int CALL_SCALARS = 128;
+
 // Work caps of one solve on top of the per-loop caps: a stagnating solve ends with status 3 after
 // this many inner (multigrid-PCG) or outer (Schur) iterations in total.
 constexpr double DEV_INNER_BUDGET = 40000, DEV_OUTER_BUDGET = 4000;

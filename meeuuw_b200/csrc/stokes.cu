@@ -1930,13 +1930,12 @@ __global__ void k_pcg_update(int64_t n, const R* __restrict__ p0, const R* __res
   }
 }
 
-// the result in double, and the solve's iteration count
+// the result in double
 template <typename R>
-__global__ void k_pcg_finish(int64_t n, const R* __restrict__ xr, double* __restrict__ x, double* __restrict__ sc) {
+__global__ void k_pcg_finish(int64_t n, const R* __restrict__ xr, double* __restrict__ x) {
   pdl_entry();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] = (double)xr[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) sc[I_INNER] += sc[P_IT];
 }
 
 // ---- the Schur-complement iteration around it (slots U_*): k_pcg_start_grad, the inner loop,
@@ -3236,7 +3235,7 @@ struct Pcg {
                pc[1], S->red, S->counter, S->sc, rtol, maxit, dev ? 1 : 0, hw);
   }
   void finish(double* x, cudaStream_t s) const {
-    pdl_launch(k_pcg_finish<R>, grid_for(n, 256), 256, 0, s, n, (const R*)pc[0], x, S->sc);
+    pdl_launch(k_pcg_finish<R>, grid_for(n, 256), 256, 0, s, n, (const R*)pc[0], x);
   }
 };
 
@@ -3325,13 +3324,17 @@ static void remove_mean(mw_stokes* S, int64_t n, double* x, cudaStream_t s) {
   pdl_launch(k_sub_mean, grid_for(n, 256), 256, 0, s, n, S->sc + 40, x);
 }
 
-// Full saddle residual in FP64: (RV, RP) = (f, h) - [K G; G^T 0] (V, P); T_RV = its sum of squares, T_REL
-// relative to S_BNORM, and what `action` asks for.
-static void true_residual(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
-                          int action, const LoopTest& test, cudaStream_t s) {
+// Full saddle residual in FP64: (RV, RP) = (f, h) - [K G; G^T 0] (V, P); in the scalars sc, T_RV = its sum
+// of squares, T_REL relative to S_BNORM, and what `action` asks for.
+static void residual_into(mw_stokes* S, double* sc, const double* V, const double* P, const double* f,
+                          const double* h, int action, const LoopTest& test, cudaStream_t s) {
   OpArgs<double> a = op_args64(S);
   a.u = V; a.p = P; a.yV = S->RV; a.yP = S->RP; a.bV = f; a.bP = h;
-  op_residual(a, ResidSum{S->red, S->sc, S->counter, action, test}, s);
+  op_residual(a, ResidSum{S->red, sc, S->counter, action, test}, s);
+}
+static void true_residual(mw_stokes* S, const double* V, const double* P, const double* f, const double* h,
+                          int action, const LoopTest& test, cudaStream_t s) {
+  residual_into(S, S->sc, V, P, f, h, action, test, s);
 }
 
 // Inner K solve at the requested precision.
@@ -3829,8 +3832,9 @@ int mw_stokes_residual(mw_stokes* S, const double* V, const double* P, const dou
                        double* RP, double* norm_out, void* stream) {
   if (!f || !h || !pair_aligned(V, 16) || !pair_aligned(f, 16)) return MW_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  true_residual(S, V, P, f, h, RA_NONE, refine_test(mw_solve_params{}, 0, false, 0), s);
-  const double r = std::sqrt(read_scalar(S->sc + T_RV, s));
+  double* sc = S->sc + CALL_SCALARS;                        // the last solve's outcome stays in S->sc
+  residual_into(S, sc, V, P, f, h, RA_NONE, refine_test(mw_solve_params{}, 0, false, 0), s);
+  const double r = std::sqrt(read_scalar(sc + T_RV, s));
   if (RV) cudaMemcpyAsync(RV, S->RV, sizeof(double) * 2 * S->fine.nnx * S->fine.nnz, cudaMemcpyDeviceToDevice, s);
   if (RP) cudaMemcpyAsync(RP, S->RP, sizeof(double) * (S->fine.nx + 1) * (S->fine.nz + 1), cudaMemcpyDeviceToDevice, s);
   if (norm_out) *norm_out = r;
