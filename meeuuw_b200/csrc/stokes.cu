@@ -1353,6 +1353,44 @@ MW_D int restrict_taps_1d(int J, int nf, int nc, int* idx, double* w) {
   return k;
 }
 
+// The tables of Transfer1D: the taps of pw_g and restrict_taps_1d, one direction of one level a row of blocks
+// (tj: pj, ri, rn; tw: pw, rw).  A coarse node's fine nodes lie strictly inside the support of its basis
+// function, at most four fine elements: eight nodes (RTAPS).
+struct TransferFill {
+  int nf, nc;
+  int* tj;
+  double* tw;
+};
+struct TransferFills {
+  TransferFill t[2 * MAXLEV];
+};
+
+__global__ void k_transfer_tables(const __grid_constant__ TransferFills A) {
+  pdl_entry();
+  const TransferFill& T = A.t[blockIdx.y];
+  const int nnf = 2 * T.nf + 1, nnc = 2 * T.nc + 1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nnf; i += gridDim.x * blockDim.x) {
+    int J[3];
+    double w[3] = {0.0, 0.0, 0.0};
+    pw_g(i, T.nf, T.nc, J, w);
+    T.tj[i] = J[0];
+    for (int k = 0; k < 3; ++k) T.tw[3 * i + k] = w[k];
+    if (i >= nnc) continue;
+    int idx[RMAXT];
+    double v[RMAXT], row[RTAPS] = {};
+    const int n = restrict_taps_1d(i, T.nf, T.nc, idx, v);
+    int count = 0;
+    for (int k = 0; k < n; ++k)
+      if (idx[k] - idx[0] < RTAPS) {
+        count = idx[k] - idx[0] + 1;
+        row[count - 1] = v[k];
+      }
+    T.tj[nnf + i] = idx[0];
+    T.tj[nnf + nnc + i] = count;
+    for (int k = 0; k < RTAPS; ++k) T.tw[3 * nnf + RTAPS * i + k] = row[k];
+  }
+}
+
 // The restriction at coarse node n when a dimension is not nested: the same epilogue as
 // restrict_core, the fine residual summed over the general taps (z outer, x inner)
 template <typename R, typename Fetch>
@@ -2184,7 +2222,6 @@ struct Hierarchy {
   int tail0 = 0;             // first level of the cluster V-cycle tail (0: none)
   int64_t tail_len = 0;      // element products of its largest level (18 per element)
   R* tail_ye = nullptr;      // their global scratch
-  char* tables_end = nullptr;   // end of the transfer tables (from L[0].tj[0] on)
 };
 
 }  // namespace mw
@@ -2200,6 +2237,7 @@ struct mw_stokes {
   double *cV, *cP;       // refinement corrections
   double* diag64;        // assembled diag(K) of the fine level, FP64
   bool dirty64 = true, dirty32 = true;
+  bool started = false;  // the workspace's constant parts are written (start_workspace)
   double* etae_w;        // 1/eta_e per element (M_eta weights)
   double* red;           // reduction partials
   double* sc;            // device scalars
@@ -2288,70 +2326,28 @@ static void plan_levels(Hierarchy<R>& H, const LevelGeo& fine, const mw_stokes_p
 
 
 
-// The transfer of one direction between nf and nc elements as tables in host memory (the weights of pw_g and
-// restrict_taps_1d): pj, ri, rn into hj, pw and rw into hw.
-static int fill_transfer(int nf, int nc, int* hj, double* hw) {
-  const int nnf = 2 * nf + 1, nnc = 2 * nc + 1;
-  std::vector<int> j(nnf + 2 * nnc);
-  std::vector<double> w(3 * (size_t)nnf + RTAPS * (size_t)nnc, 0.0);
-  for (int i = 0; i < nnf; ++i) {
-    double* q = &w[3 * (size_t)i];
-    if (nested_1d(nf, nc)) {
-      if (i & 1) {
-        const int E = i / 4;
-        j[i] = 2 * E;
-        q[0] = (i & 3) == 1 ? 0.375 : -0.125; q[1] = 0.75; q[2] = (i & 3) == 1 ? -0.125 : 0.375;
-      } else {
-        j[i] = i / 2;
-        q[0] = 1.0;
-      }
-    } else {
-      int E = (int)(((int64_t)i * nc) / (2LL * nf));
-      if (E > nc - 1) E = nc - 1;
-      const double xi = (double)((int64_t)i * nc - 2LL * nf * E - nf) / (double)nf;
-      j[i] = 2 * E;
-      q[0] = 0.5 * xi * (xi - 1.0); q[1] = (1.0 - xi) * (1.0 + xi); q[2] = 0.5 * xi * (xi + 1.0);
-    }
-  }
-  for (int J = 0; J < nnc; ++J) {           // the transpose: the fine nodes with a weight on J
-    int first = -1, last = -1;
-    const int lo = std::max(0, (int)(((int64_t)(J - 2) * nf) / nc) - 1), hi = std::min(nnf - 1, (int)(((int64_t)(J + 2) * nf) / nc) + 1);
-    for (int i = lo; i <= hi; ++i) {
-      const int o = J - j[i];
-      if (o < 0 || o > 2 || w[3 * (size_t)i + o] == 0.0) continue;
-      if (first < 0) first = i;
-      last = i;
-      if (i - first >= RTAPS) return MW_ERR_BAD_ARG;
-      w[3 * (size_t)nnf + RTAPS * (size_t)J + (i - first)] = w[3 * (size_t)i + o];
-    }
-    if (first < 0) return MW_ERR_BAD_ARG;
-    j[nnf + J] = first;
-    j[nnf + nnc + J] = last - first + 1;
-  }
-  std::copy(j.begin(), j.end(), hj);
-  std::copy(w.begin(), w.end(), hw);
-  return MW_OK;
+template <typename R>
+static bool all_nested(const Hierarchy<R>& H) {
+  for (int l = 0; l + 1 < H.nlev; ++l)
+    if (!nested_levels(H.L[l].g, H.L[l + 1].g)) return false;
+  return true;
 }
 
-// Every level's tables, which carve() laid out in one piece, by one copy.  Nested levels have their taps at
-// compile time: a hierarchy of nothing else reads no tables, and its solver is created without waiting for
-// the device (16 us against 89 and a synchronous copy).
+// Every level's transfer tables in one launch.  Nested levels have their taps at compile time: a hierarchy of
+// nothing else reads no tables.
 template <typename R>
-static int fill_transfers(Hierarchy<R>& H) {
-  bool nested = true;
-  for (int l = 0; l + 1 < H.nlev; ++l) nested = nested && nested_levels(H.L[l].g, H.L[l + 1].g);
-  if (nested) return MW_OK;
-  char* const base = (char*)H.L[0].tj[0];
-  std::vector<double> host((H.tables_end - base) / sizeof(double), 0.0);
-  auto at = [&](void* device) { return (char*)host.data() + ((char*)device - base); };
+static void fill_transfers(const Hierarchy<R>& H, cudaStream_t s) {
+  if (all_nested(H)) return;
+  TransferFills F;
+  memset(&F, 0, sizeof(F));
+  int n = 0;
   for (int l = 0; l + 1 < H.nlev; ++l)
     for (int d = 0; d < 2; ++d) {
       const LevelGeo &f = H.L[l].g, &c = H.L[l + 1].g;
-      if (int rc = fill_transfer(d ? f.nz : f.nx, d ? c.nz : c.nx, (int*)at(H.L[l].tj[d]), (double*)at(H.L[l].tw[d])))
-        return rc;
+      F.t[n++] = TransferFill{d ? f.nz : f.nx, d ? c.nz : c.nx, H.L[l].tj[d], H.L[l].tw[d]};
     }
-  return cudaMemcpy(base, host.data(), sizeof(double) * host.size(), cudaMemcpyHostToDevice) == cudaSuccess ? MW_OK
-                                                                                                            : MW_ERR_CUDA;
+  const int longest = std::max(H.L[0].g.nnx, H.L[0].g.nnz);
+  pdl_launch(k_transfer_tables, dim3((longest + 255) / 256, n), 256, 0, s, F);
 }
 
 template <typename R>
@@ -2385,7 +2381,6 @@ static void carve(Hierarchy<R>& H, Arena& A, const uint8_t* fine_fix) {
       const int nf = d ? f.nnz : f.nnx, nc = d ? c.nnz : c.nnx;
       H.L[l].tj[d] = (int*)A.take(sizeof(int) * (nf + 2 * nc));
       H.L[l].tw[d] = (double*)A.take(sizeof(double) * (3 * nf + RTAPS * nc));
-      H.tables_end = (char*)(H.L[l].tw[d] + (3 * nf + RTAPS * nc));
     }
   H.Ainv = H.dense ? (double*)A.take(sizeof(double) * (size_t)H.nd * H.nd) : nullptr;
   H.tail_ye = H.tail0 ? (R*)A.take(sizeof(R) * H.tail_len) : nullptr;
@@ -3337,8 +3332,25 @@ static void true_residual(mw_stokes* S, const double* V, const double* P, const 
   residual_into(S, S->sc, V, P, f, h, action, test, s);
 }
 
-// Inner K solve at the requested precision.
+// What the workspace holds whatever the viscosity: idle arrival counters and the transfer tables, written on
+// the stream that first uses the solver.  Nothing else orders them: the workspace may be a block that work
+// queued on that stream still writes, and a table or a counter that a kernel reads too early is an index out
+// of range or a sum that never ends.  Recorded uses record it too and leave it to be done again: what is
+// recorded may never run.
+static int start_workspace(mw_stokes* S, cudaStream_t s) {
+  if (S->started) return MW_OK;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) return MW_ERR_CUDA;
+  if (cudaMemsetAsync(S->counter, 0, sizeof(unsigned) * (MAXLEV + 4), s) != cudaSuccess) return MW_ERR_CUDA;
+  if (S->has64) fill_transfers(S->H64, s);
+  if (S->has32) fill_transfers(S->H32, s);
+  if (cudaGetLastError() != cudaSuccess) return MW_ERR_CUDA;
+  S->started = st == cudaStreamCaptureStatusNone;
+  return MW_OK;
+}
+
 static int ensure_hierarchy(mw_stokes* S, int prec, cudaStream_t s) {
+  if (int rc = start_workspace(S, s)) return rc;
   if (prec == MW_F32) {
     if (!S->has32) return MW_ERR_BAD_ARG;
     if (S->dirty32) { int rc = setup_hierarchy<float>(S, S->H32, s); if (rc) return rc; S->dirty32 = false; }
@@ -3349,6 +3361,7 @@ static int ensure_hierarchy(mw_stokes* S, int prec, cudaStream_t s) {
   return MW_OK;
 }
 
+// Inner K solve at the requested precision.
 static int solve_K(mw_stokes* S, int prec, const double* b, double* x, double rtol, int maxit, double* relres,
                    cudaStream_t s) {
   if (prec == MW_F32) return pcg_K<float>(S, S->H32, S->pc32, b, x, rtol, maxit, relres, s);
@@ -3633,8 +3646,6 @@ int mw_stokes_create(mw_box box, mw_stokes_params prm, const uint8_t* bc_fix_V, 
   size_t need = do_layout(S, nullptr, true);
   if (work_bytes < need) { delete S; return MW_ERR_WORKSPACE; }
   do_layout(S, (char*)work, false);
-  if ((S->has64 && fill_transfers(S->H64)) || (S->has32 && fill_transfers(S->H32))) { delete S; return MW_ERR_CUDA; }
-  if (cudaMemset(S->counter, 0, sizeof(unsigned) * (MAXLEV + 4)) != cudaSuccess) { delete S; return MW_ERR_CUDA; }
   *out = S;
   return MW_OK;
 }
@@ -3675,6 +3686,7 @@ int mw_stokes_levels(const mw_stokes* S, int32_t precision) {
 
 int mw_stokes_set_viscosity(mw_stokes* S, const double* etaq, const double* eta_e, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
+  if (int rc = start_workspace(S, s)) return rc;
   const int64_t nel = (int64_t)S->fine.nx * S->fine.nz;
   pdl_launch(k_cast<double>, grid_for(nel * 9, 256), 256, 0, s, nel * 9, etaq, S->etaq64);
   if (S->has32) pdl_launch(k_cast<float>, grid_for(nel * 9, 256), 256, 0, s, nel * 9, etaq, S->etaq32);
@@ -3832,6 +3844,7 @@ int mw_stokes_residual(mw_stokes* S, const double* V, const double* P, const dou
                        double* RP, double* norm_out, void* stream) {
   if (!f || !h || !pair_aligned(V, 16) || !pair_aligned(f, 16)) return MW_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
+  if (int rc = start_workspace(S, s)) return rc;
   double* sc = S->sc + CALL_SCALARS;                        // the last solve's outcome stays in S->sc
   residual_into(S, sc, V, P, f, h, RA_NONE, refine_test(mw_solve_params{}, 0, false, 0), s);
   const double r = std::sqrt(read_scalar(sc + T_RV, s));
