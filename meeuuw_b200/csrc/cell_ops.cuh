@@ -107,13 +107,8 @@ MW_D double2 div2(double2 a, double2 d, double2 y) { return make_double2(div1(a.
 
 // a translation unit's copy of the tables, filled before its first launch
 int ensure_cell_tables() {
-  static bool ready = false;
-  if (ready) return MW_OK;
-  RefTables t;
-  host_ref_tables(&t);
-  if (cudaMemcpyToSymbol(c_k, &t, sizeof(t)) != cudaSuccess) return MW_ERR_CUDA;
-  ready = true;
-  return MW_OK;
+  static OncePerDevice once;
+  return fill_constant(once, c_k, host_ref_tables) ? MW_OK : MW_ERR_CUDA;
 }
 
 }  // namespace

@@ -12,6 +12,7 @@
 #include <utility>
 
 #include "../../include/meeuuw_b200.h"
+#include "once_per_device.h"
 
 #define MW_HD __host__ __device__ __forceinline__
 #define MW_D __device__ __forceinline__
@@ -79,6 +80,34 @@ MW_D void pdl_entry() {
 // predecessor's predecessor is complete and visible.  The level and Krylov kernels load the diagonal,
 // the viscosity, the Dirichlet flags and their tables there (written at least two launches earlier, by
 // the set-up), so that a chain of short launches does not wait for them.
+inline int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+// Raises a kernel's shared-memory limit on the current device (once: that kernel's, of its own).
+template <typename F>
+inline bool raise_smem(OncePerDevice& once, F* kernel, size_t bytes) {
+  return once.run(current_device(), [&] {
+    const bool ok =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  });
+}
+
+// Fills a constant table on the current device (fill(&host) makes its contents) and waits until it is there:
+// the streams that read it need not wait for the one that copies it.
+template <typename T, typename Fill>
+inline bool fill_constant(OncePerDevice& once, T& table, const Fill& fill) {
+  return once.run(current_device(), [&] {
+    T host;
+    fill(&host);
+    return cudaMemcpyToSymbol(table, &host, sizeof(T)) == cudaSuccess &&
+           cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess;
+  });
+}
+
 bool pdl_enabled();        // false when the environment sets MW_PDL=0
 
 template <typename... KArgs, typename... Args>

@@ -14,7 +14,6 @@
 // the same kernel -- no element matrices are written or read.  Its products form the iteration's vectors
 // as they stage them: a BiCGSTAB iteration is three launches.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -767,23 +766,14 @@ static bool eop_plane_map(CUtensorMap* m, mw_box b, const void* op) {
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Raises a kernel's shared-memory limit once per device (done: a bit per device).
-template <typename F>
-static void smem_limit(F* kernel, size_t bytes, std::atomic<uint64_t>& done) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done.load() >> dev & 1u) return;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
-    done.fetch_or(uint64_t(1) << dev);
-}
-
 // Launches k_energy_op_apply<KIND> on the TMA path when the map could be made.
 template <int KIND>
 static void launch_eop_apply(bool tma, const CUtensorMap& tm, int grid, cudaStream_t s, mw_box b, const EnergyOp& op,
                              const double* x, const double* rhs, double* y, const BicgVecs& V, const BicgEnd& E,
                              int32_t* flag) {
   if (tma) {
-    static std::atomic<uint64_t> done{0};
-    smem_limit(k_energy_op_apply<KIND, true>, E_SMEM_TMA, done);
+    static OncePerDevice once;
+    raise_smem(once, k_energy_op_apply<KIND, true>, E_SMEM_TMA);
     pdl_launch(k_energy_op_apply<KIND, true>, grid, E_THREADS, E_SMEM_TMA, s, tm, b, op, x, rhs, y, V, E, flag);
   } else {
     pdl_launch(k_energy_op_apply<KIND, false>, grid, E_THREADS, E_SMEM, s, tm, b, op, x, rhs, y, V, E, flag);
@@ -877,20 +867,12 @@ static std::vector<EnergyGraph> g_energy_graphs;
 static std::mutex g_energy_mutex;
 static cudaStream_t g_energy_stream[64], g_energy_body[64];   // library stream, body-capture stream
 static cudaEvent_t g_energy_ev[64][2];
-static uint64_t g_eref_ready = 0;   // devices whose c_eref is loaded
 
 // The reference-element tables of the matrix-free operator in this device's constant bank (once
 // per device; synchronous, so the first call on a device precedes any stream capture).
 static int ensure_energy_tables() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MW_ERR_CUDA;
-  std::lock_guard<std::mutex> lock(g_energy_mutex);
-  if (g_eref_ready >> dev & 1u) return MW_OK;
-  RefTables T;
-  host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_eref, &T, sizeof(T)) != cudaSuccess) return MW_ERR_CUDA;
-  g_eref_ready |= uint64_t(1) << dev;
-  return MW_OK;
+  static OncePerDevice once;
+  return fill_constant(once, c_eref, host_ref_tables) ? MW_OK : MW_ERR_CUDA;
 }
 
 }  // namespace mw
@@ -1155,8 +1137,8 @@ int mw_energy_op_setup(mw_box box, mw_energy_in in, void* op, size_t op_bytes, d
   double* diag = planes + eop_plane_doubles(box);
   uint8_t* fix = reinterpret_cast<uint8_t*>(diag + eop_nodes(box));
   const int64_t ntile = (int64_t)((box.nelx + ETX - 1) / ETX) * ((box.nelz + ETZ - 1) / ETZ);
-  static std::atomic<uint64_t> done{0};
-  smem_limit(k_energy_op_setup, E_SMEM_SETUP, done);
+  static OncePerDevice once;
+  raise_smem(once, k_energy_op_setup, E_SMEM_SETUP);
   pdl_launch(k_energy_op_setup, (int)std::min<int64_t>(ntile, 8 * num_sms()), ES_THREADS, E_SMEM_SETUP,
              (cudaStream_t)stream, box, in, planes, diag, fix, rhs, eop_view(box, op).flag);
   MW_CHECK_LAUNCH();

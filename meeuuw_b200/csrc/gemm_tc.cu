@@ -394,13 +394,8 @@ static int launch_conv(const CUtensorMap& tx, const CUtensorMap& tw, ConvGeo cg,
                        int32_t* err, cudaStream_t s) {
   dim3 grid((M + GT_BM - 1) / GT_BM, (N + BN - 1) / BN, 1);
   const size_t smem = 1024 + GT_STAGES * (GT_BM * KB * 2 + BN * KB * 2) + 256;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(k_conv3x3_bf16_tc<BN, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return MW_ERR_CUDA;
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  if (!raise_smem(once, k_conv3x3_bf16_tc<BN, KB>, smem)) return MW_ERR_CUDA;
   k_conv3x3_bf16_tc<BN, KB><<<grid, GT_THREADS, smem, s>>>(tx, tw, cg, M, N, ep, err);
   MW_CHECK_LAUNCH();
   return MW_OK;
@@ -413,13 +408,8 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int M, int 
   const int per = (kbt + splits - 1) / splits;   // splits is pre-adjusted so that none is empty
   dim3 grid((M + GT_BM - 1) / GT_BM, (N + BN - 1) / BN, splits);
   const size_t smem = 1024 + GT_STAGES * (GT_BM * GT_BK * 2 + BN * GT_BK * 2) + 256;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(k_gemm_bf16_tc<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return MW_ERR_CUDA;
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  if (!raise_smem(once, k_gemm_bf16_tc<BN>, smem)) return MW_ERR_CUDA;
   k_gemm_bf16_tc<BN><<<grid, GT_THREADS, smem, s>>>(ta, tb, M, N, per, kbt, ep, err);
   MW_CHECK_LAUNCH();
   return MW_OK;

@@ -389,26 +389,14 @@ __global__ void __launch_bounds__(NT, 1) k_mg_tail(const __grid_constant__ MgTai
 }
 
 int tail_limit() {
-  static int limit = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return v;
-  }();
-  return limit;
+  int v = 0;
+  return cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, current_device()) == cudaSuccess ? v : 0;
 }
 
 template <typename R, int DEG>
 bool launch_tail_deg(const MgTailArgs<R>& a, const TailLayout<R>& S, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_mg_tail<R, DEG>, cudaFuncAttributeMaxDynamicSharedMemorySize, tail_limit()) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    attr = true;
-  }
+  static OncePerDevice once;
+  if (!raise_smem(once, k_mg_tail<R, DEG>, tail_limit())) return false;
   pdl_launch(k_mg_tail<R, DEG>, 1, NT, S.total, s, a, S);
   return true;
 }

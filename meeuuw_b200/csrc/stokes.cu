@@ -36,7 +36,6 @@ namespace mw {
 
 // ---------------------------------------------------------------- reference-element tables
 __constant__ RefTables c_ref;
-static bool g_ref_ready = false;
 
 // FP32 kernels take the values as immediates; FP64 ones read them from the constant bank (an FP64
 // immediate would be materialised in registers for every use).  Which terms vanish is decided at
@@ -55,13 +54,10 @@ template <> struct CT<double> {
 };
 
 static int ensure_ref_tables() {
-  if (g_ref_ready) return MW_OK;
-  RefTables T;
-  host_ref_tables(&T);
-  if (cudaMemcpyToSymbol(c_ref, &T, sizeof(T)) != cudaSuccess || mg_ensure_tables() || mg_tail_ensure_tables() ||
+  static OncePerDevice once;
+  if (!fill_constant(once, c_ref, host_ref_tables) || mg_ensure_tables() || mg_tail_ensure_tables() ||
       op_ensure_tables() || setup_ensure_tables())
     return MW_ERR_CUDA;
-  g_ref_ready = true;
   return MW_OK;
 }
 
@@ -2855,17 +2851,13 @@ static void launch_tail(Hierarchy<R>& H, int l0, bool first_done, cudaStream_t s
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const size_t limit = (size_t)optin > 1024 ? (size_t)optin - 1024 : 0;   // static TailLevel copies
   if (smem_on && sm <= limit) {
-    static size_t attr_set = 0;
-    if (sm > attr_set &&
-        cudaFuncSetAttribute(k_vtail_smem<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) == cudaSuccess)
-      attr_set = limit;
-    if (sm <= attr_set) {
+    static OncePerDevice once;
+    if (raise_smem(once, k_vtail_smem<R>, limit)) {
       tail_swaps(H, l0, first_done);          // the host's record of where level l0's x ends up
       A.out_x = H.L[l0].x;
       pdl_launch(k_vtail_smem<R>, 1, tail_threads<R>(), sm, s, A);
       return;
     }
-    cudaGetLastError();
   }
   pdl_launch(k_vtail<R>, TAIL_CLUSTER, tail_threads<R>(), 0, s, A);
   tail_swaps(H, l0, first_done);
