@@ -8,8 +8,8 @@
 //
 // The operator and its residuals are op_apply.cu, a level's half of a V-cycle mg_level.cu, the coarse
 // levels that are not nested mg_tail.cu, the hierarchy's set-up mg_setup.cu; here are the vector kernels
-// of the iterations, their graphs, and the element-tile operator (k_apply) that smoothing of degree above
-// two, single Chebyshev steps and the ensemble's clusters use: a CTA owns a TX x TZ tile of elements'
+// of the iterations, their graphs, and the element-tile operator (apply_tile) that smoothing of degree above
+// two and single Chebyshev steps launch (k_apply) and the ensemble's clusters call: a CTA owns a TX x TZ tile of elements'
 // nodes and recomputes a one-element halo on its left/bottom.  Everywhere each node sums all its incident
 // elements itself, in ascending element order: no atomics, deterministic results.  The element kernels
 // evaluate K u, G p, G^T u at the 3x3 Gauss points from the viscosity at the qpoints and the
@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 
+#include "cell_ops.cuh"
 #include "common.cuh"
 #include "mg_level.cuh"
 #include "mg_setup.cuh"
@@ -37,25 +38,9 @@ namespace mw {
 // ---------------------------------------------------------------- reference-element tables
 __constant__ RefTables c_ref;
 
-// FP32 kernels take the values as immediates; FP64 ones read them from the constant bank (an FP64
-// immediate would be materialised in registers for every use).  Which terms vanish is decided at
-// compile time in both cases (ref_dr / ref_dt of q2_ref.cuh).
-template <typename R> struct CT {
-  template <int Q, int K> MW_D static constexpr R dr() { return (R)RefD<Q, K>::r; }
-  template <int Q, int K> MW_D static constexpr R dt() { return (R)RefD<Q, K>::t; }
-  template <int Q, int K> MW_D static constexpr R np() { constexpr double v = ref_np(Q, K); return (R)v; }
-  template <int Q> MW_D static constexpr R wq() { constexpr double v = ref_wq(Q); return (R)v; }
-};
-template <> struct CT<double> {
-  template <int Q, int K> MW_D static double dr() { return c_ref.dr[Q * 9 + K]; }
-  template <int Q, int K> MW_D static double dt() { return c_ref.dt[Q * 9 + K]; }
-  template <int Q, int K> MW_D static double np() { return c_ref.NP[Q * 4 + K]; }
-  template <int Q> MW_D static double wq() { return c_ref.wq[Q]; }
-};
-
 static int ensure_ref_tables() {
   static OncePerDevice once;
-  if (!fill_constant(once, c_ref, host_ref_tables) || mg_ensure_tables() || mg_tail_ensure_tables() ||
+  if (!fill_constant(once, c_ref, host_ref_tables) || ensure_cell_tables() || mg_ensure_tables() || mg_tail_ensure_tables() ||
       op_ensure_tables() || setup_ensure_tables())
     return MW_ERR_CUDA;
   return MW_OK;
@@ -75,13 +60,13 @@ enum ApplyMode { AM_APPLY = 0, AM_RESID = 1, AM_CHEB = 2, AM_CHEB_Z = 3 };
 
 template <typename R>
 struct ApplyArgs {
-  const R* u;        // velocity (interleaved u,w), may be null
-  const R* p;        // pressure, may be null
+  const R* u;        // velocity (interleaved u,w); AM_CHEB_Z computes it from b
+  const R* p;        // pressure (tiles with pressure)
   const R* eta;      // (nel, 9)
   const uint8_t* fix;// (2*nn)
   const R* diag;     // (2*nn) assembled diag(K)
   R* yV;             // output velocity part (AM_APPLY: K u + G p; AM_RESID: b - (...))
-  R* yP;             // output pressure part: G^T u (AM_RESID: h - G^T u); may be null
+  R* yP;             // output pressure part: G^T u (AM_RESID: h - G^T u) (tiles with pressure)
   const R* bV;       // rhs for residual / Chebyshev
   const R* bP;
   // Chebyshev: d = c1*d + c2*Dinv*r; xo = x + d   (x = u)
@@ -91,110 +76,19 @@ struct ApplyArgs {
   const double* cheb0;// AM_CHEB_Z: the first step's pair {0, 1/theta}
 };
 
-// Element contribution of K u_el + G p_el and G^T u_el at the 9 Gauss points: strain rate B u
-// at each point, stress 2 eta (exx, ezz) and eta (du/dz + dw/dx) with the pressure term, then B^T
-// back onto the nodes (build_matrix_stokes.py:130-157 applied to a vector).  The reference-element
-// tables are __constant__ and every loop is unrolled, so each table value is an immediate
-// constant-bank operand of the FMA; the uniform-box Jacobian enters as sx = 2/hx, sz = 2/hz.
-// HAS_U = false: no velocity (G p only; the strain-rate terms vanish).  NEED_V = false: only the
-// pressure rows are wanted (G^T u), so the B^T scatter and the shear gradients are skipped.
-template <typename R, bool HAS_U = true, bool NEED_V = true>
-MW_D void element_apply(R sx, R sz, R jac, R s, const R* ue, const R* pe, const R* eq, R* ye, R* ype, bool use_p) {
+// K u_el on one element (k_element of cell_ops.cuh) from and to interleaved (u, w) pairs; with PRESSURE, G p_el
+// joins it and G^T u_el goes to ype (build_matrix_stokes.py:130-157 applied to a vector).
+template <bool PRESSURE, typename R>
+MW_D void element_apply(const LevelGeo& g, const R* ue, const R* pe, const R (&eq)[9], R* ye, R* ype) {
+  typedef typename Vec2<R>::T R2;
+  R2 u[9], y[9];
 #pragma unroll
-  for (int k = 0; k < 18; ++k) ye[k] = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) ype[k] = 0;
-  static_for<9>([&](auto qc) {
-    constexpr int Q = qc.value;
-    R dxu = 0, dzw = 0, dzu = 0, dxw = 0;
-    if constexpr (HAS_U) {
-      static_for<9>([&](auto kc) {
-        constexpr int K = kc.value;
-        if constexpr (RefD<Q, K>::r != 0.0) {
-          const R r = CT<R>::template dr<Q, K>();
-          dxu += r * ue[2 * K];
-          if (NEED_V) dxw += r * ue[2 * K + 1];
-        }
-        if constexpr (RefD<Q, K>::t != 0.0) {
-          const R t = CT<R>::template dt<Q, K>();
-          dzw += t * ue[2 * K + 1];
-          if (NEED_V) dzu += t * ue[2 * K];
-        }
-      });
-    }
-    // the shear rate du/dz + dw/dx, its rounding written out: every kernel that applies K rounds alike
-    const R exx = sx * dxu, ezz = sz * dzw, gg = fma(sz, dzu, sx * dxw);
-    const R jw = jac * CT<R>::template wq<Q>();
-    if constexpr (NEED_V) {
-      const R e = eq[Q] * jw;
-      R pq = 0;
-      if (use_p) static_for<4>([&](auto kc) { pq += CT<R>::template np<Q, kc.value>() * pe[kc.value]; });
-      const R sp = s * jw * pq;
-      const R A = (R(2) * e * exx - sp) * sx, B = (R(2) * e * ezz - sp) * sz;
-      const R Cx = e * gg * sx, Cz = e * gg * sz;
-      static_for<9>([&](auto kc) {
-        constexpr int K = kc.value;
-        if constexpr (RefD<Q, K>::r != 0.0) {
-          const R r = CT<R>::template dr<Q, K>();
-          ye[2 * K] += r * A;
-          if (HAS_U) ye[2 * K + 1] += r * Cx;
-        }
-        if constexpr (RefD<Q, K>::t != 0.0) {
-          const R t = CT<R>::template dt<Q, K>();
-          if (HAS_U) ye[2 * K] += t * Cz;
-          ye[2 * K + 1] += t * B;
-        }
-      });
-    }
-    if constexpr (HAS_U) {
-      const R dv = -s * jw * (exx + ezz);
-      static_for<4>([&](auto kc) { ype[kc.value] += CT<R>::template np<Q, kc.value>() * dv; });
-    }
-  });
-}
-
-// FP32 variant on the packed two-lane FMA of sm_100 (__ffma2_rn): a node's (u, w) pair is one
-// operand, so each nonzero basis value costs one instruction for both velocity components, in the
-// gradients and in the B^T scatter.
-template <>
-MW_D void element_apply<float, true, true>(float sx, float sz, float jac, float s, const float* ue, const float* pe,
-                                           const float* eq, float* ye, float* ype, bool use_p) {
-  const float2* u2 = reinterpret_cast<const float2*>(ue);
-  float2 y2[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) y2[k] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) ype[k] = 0.f;
-  static_for<9>([&](auto qc) {
-    constexpr int Q = qc.value;
-    float2 gx = make_float2(0.f, 0.f), gz = make_float2(0.f, 0.f);   // (du/dr, dw/dr), (du/dt, dw/dt)
-    static_for<9>([&](auto kc) {
-      constexpr int K = kc.value;
-      constexpr float r = (float)RefD<Q, K>::r, t = (float)RefD<Q, K>::t;
-      if constexpr (r != 0.f) gx = __ffma2_rn(make_float2(r, r), u2[K], gx);
-      if constexpr (t != 0.f) gz = __ffma2_rn(make_float2(t, t), u2[K], gz);
-    });
-    const float exx = sx * gx.x, ezz = sz * gz.y, gg = fma(sx, gx.y, sz * gz.x);
-    const float jw = jac * CT<float>::wq<Q>();
-    const float e = eq[Q] * jw;
-    float pq = 0.f;
-    if (use_p) static_for<4>([&](auto kc) { pq += CT<float>::np<Q, kc.value>() * pe[kc.value]; });
-    const float sp = s * jw * pq;
-    const float2 ar = make_float2((2.f * e * exx - sp) * sx, e * gg * sx);   // coefficients of dN/dr
-    const float2 at = make_float2(e * gg * sz, (2.f * e * ezz - sp) * sz);   // coefficients of dN/dt
-    static_for<9>([&](auto kc) {
-      constexpr int K = kc.value;
-      constexpr float r = (float)RefD<Q, K>::r, t = (float)RefD<Q, K>::t;
-      if constexpr (r != 0.f) y2[K] = __ffma2_rn(make_float2(r, r), ar, y2[K]);
-      if constexpr (t != 0.f) y2[K] = __ffma2_rn(make_float2(t, t), at, y2[K]);
-    });
-    const float dv = -s * jw * (exx + ezz);
-    static_for<4>([&](auto kc) { ype[kc.value] += CT<float>::np<Q, kc.value>() * dv; });
-  });
+  for (int k = 0; k < 9; ++k) u[k] = pair(ue[2 * k], ue[2 * k + 1]);
+  k_element<PRESSURE>(R(2.0 / g.hx), R(2.0 / g.hz), R(g.hx * g.hz / 4.0), u, eq, y, R(g.s), pe, ype);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    ye[2 * k] = y2[k].x;
-    ye[2 * k + 1] = y2[k].y;
+    ye[2 * k] = y[k].x;
+    ye[2 * k + 1] = y[k].y;
   }
 }
 
@@ -427,17 +321,18 @@ MW_D void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory");
 // reads for the four nodes each owned element emits (b; b, diag, d) are fetched asynchronously
 // while the element products run (FP32 only: the FP64 tile's shared memory stays under the 48 KB
 // static limit without them).
-template <typename R, int MODE>
+template <typename R, int MODE, bool PRESSURE = false>
 struct ApplySmem {
   typedef typename Vec2<R>::T R2;
+  static constexpr int YS = PRESSURE ? 22 : 18;       // results of an element: 18 velocity, 4 pressure
   static constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z;
   static constexpr int NPRE = sizeof(R) == 8 ? 0 : (CHEB ? 3 : (MODE == AM_RESID ? 1 : 0));
   static constexpr int NJ = APPLY_THREADS - TX * TZ;  // spare threads: right column and top row nodes
   __align__(16) R su[LZ * LX * 2];
   __align__(16) R2 spre[NPRE ? NPRE * 4 * TX * TZ : 1];
   __align__(16) R2 sspare[NPRE ? NPRE * 2 * NJ : 1];
-  R sp[PZ * PX];
-  R sye[NEL_T * 22];
+  R sp[PRESSURE ? PZ * PX : 1];
+  R sye[NEL_T * YS];
   uchar2 sfix[LZ * LX];                              // Dirichlet flags of the staged nodes
 };
 
@@ -452,20 +347,20 @@ struct ApplyPtrs {
   uchar2* sfix;
 };
 
-template <typename R, int MODE>
-MW_D ApplyPtrs<R> apply_ptrs(ApplySmem<R, MODE>& sm) {
+template <typename R, int MODE, bool PRESSURE>
+MW_D ApplyPtrs<R> apply_ptrs(ApplySmem<R, MODE, PRESSURE>& sm) {
   return ApplyPtrs<R>{sm.su, sm.spre, sm.sspare, sm.sp, sm.sye, sm.sfix};
 }
 
 // One operator apply over element tile (bx, bz) by the APPLY_THREADS threads of a CTA, in the
 // shared arrays sm.  A CTA that runs several tiles one after another separates them with a
 // __syncthreads() (the next tile's staging overwrites what this one's epilogue reads).
-template <typename R, int MODE>
+template <typename R, int MODE, bool PRESSURE>
 MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, const ApplyPtrs<R>& sm) {
   typedef typename Vec2<R>::T R2;
-  constexpr bool CHEB = ApplySmem<R, MODE>::CHEB;
-  constexpr int NPRE = ApplySmem<R, MODE>::NPRE;
-  constexpr int NJ = ApplySmem<R, MODE>::NJ;
+  typedef ApplySmem<R, MODE, PRESSURE> SM;
+  constexpr bool CHEB = SM::CHEB;
+  constexpr int NPRE = SM::NPRE, NJ = SM::NJ, YS = SM::YS;
   static_assert(2 * TZ + 1 + 2 * TX <= 2 * NJ, "the spare threads take at most two boundary nodes each");
   R* const su = sm.su;
   R2* const spre = sm.spre;
@@ -476,7 +371,6 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   const int ex0 = bx * TX, ez0 = bz * TZ;
   const int lx0 = 2 * ex0 - 2, lz0 = 2 * ez0 - 2;      // lattice origin of the staged nodes
   const int tid = threadIdx.x;
-  const bool use_u = a.u != nullptr, use_p = a.p != nullptr;
   // Chebyshev coefficients, read now so that no epilogue load waits on them
   const double c1 = CHEB ? a.cheb[0] : 0.0;
   const R c2 = CHEB ? R(a.cheb[1]) : R(0);
@@ -484,7 +378,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   // ---- prefetch: the epilogue's node vectors (owned elements), the element viscosities ----
   // slot j of an owned element: 0 centre (2ex+1, 2ez+1), 1 bottom midpoint (2ex+1, 2ez),
   // 2 left midpoint (2ex, 2ez+1), 3 corner (2ex, 2ez)
-  if (NPRE && a.yV && tid < TX * TZ) {
+  if (NPRE && tid < TX * TZ) {
     const int ex = ex0 + tid % TX, ez = ez0 + tid / TX;
     if (ex < g.nx && ez < g.nz) {
 #pragma unroll
@@ -504,7 +398,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   const int oz1 = lastz ? 2 * g.nz + 1 : 2 * (ez0 + TZ);
   const int ncol_v = lastx ? oz1 - 2 * ez0 : 0;
   const int nrow_v = lastz ? (lastx ? 2 * (g.nx - ex0) : 2 * TX) : 0;
-  if (NPRE && a.yV && tid >= TX * TZ && (lastx || lastz)) {
+  if (NPRE && tid >= TX * TZ && (lastx || lastz)) {
 #pragma unroll
     for (int it = 0; it < 2; ++it) {
       const int j = tid - TX * TZ + it * NJ;
@@ -552,16 +446,14 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
       if (ix >= 0 && ix < g.nnx && iz >= 0 && iz < g.nnz) {
         const int64_t n = (int64_t)iz * g.nnx + ix;
         ff = f2[n];
-        if (use_u) {
-          R2 uu = u2[n];
-          v.x = ff.x ? R(0) : uu.x;
-          v.y = ff.y ? R(0) : uu.y;
-        }
+        const R2 uu = u2[n];
+        v.x = ff.x ? R(0) : uu.x;
+        v.y = ff.y ? R(0) : uu.y;
       }
       su2[i] = v;
       sfix[i] = ff;
     }
-    if (use_p)
+    if (PRESSURE)
       for (int i = tid; i < PZ * PX; i += APPLY_THREADS) {
         int jz = i / PX, jx = i % PX;
         int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
@@ -582,7 +474,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
         const R2 bb = reinterpret_cast<const R2*>(a.bV)[n], dg = reinterpret_cast<const R2*>(a.diag)[n];
         sv[k].x = cz * bb.x / dg.x;
         sv[k].y = cz * bb.y / dg.y;
-      } else if (use_u) {
+      } else {
         sv[k] = u2[n];
       }
     }
@@ -592,7 +484,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     const int i = tid + k * APPLY_THREADS;
     const int jz = i / PX, jx = i % PX;
     const int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
-    spv[k] = (use_p && i < PZ * PX && px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz)
+    spv[k] = (PRESSURE && i < PZ * PX && px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz)
                  ? a.p[(int64_t)pz * (g.nx + 1) + px] : R(0);
   }
 #pragma unroll
@@ -609,7 +501,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
 #pragma unroll
   for (int k = 0; k < NSP; ++k) {
     const int i = tid + k * APPLY_THREADS;
-    if (use_p && i < PZ * PX) sp[i] = spv[k];
+    if (PRESSURE && i < PZ * PX) sp[i] = spv[k];
   }
   }
   __syncthreads();
@@ -627,18 +519,13 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
         ue[2 * k] = su[2 * li]; ue[2 * k + 1] = su[2 * li + 1];
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) pe[k] = use_p ? sp[(lez + q1_dz(k)) * PX + lex + q1_dx(k)] : R(0);
-      const R sxe = R(2.0 / g.hx), sze = R(2.0 / g.hz), jace = R(g.hx * g.hz / 4.0), se = R(g.s);
-      if (!use_u)                                   // G p only (the Schur iteration's G d, f - G P)
-        element_apply<R, false, true>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
-      else if (!a.yV)                               // G^T u only
-        element_apply<R, true, false>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
-      else
-        element_apply<R>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
+      for (int k = 0; k < 4; ++k) pe[k] = PRESSURE ? sp[(lez + q1_dz(k)) * PX + lex + q1_dx(k)] : R(0);
+      element_apply<PRESSURE>(g, ue, pe, eq, ye, ype);
 #pragma unroll
-      for (int k = 0; k < 18; ++k) sye[tid * 22 + k] = ye[k];
+      for (int k = 0; k < 18; ++k) sye[tid * YS + k] = ye[k];
+      if (PRESSURE)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) sye[tid * 22 + 18 + k] = ype[k];
+        for (int k = 0; k < 4; ++k) sye[tid * YS + 18 + k] = ype[k];
     }
   }
   cp_async_wait_all();
@@ -659,7 +546,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     const int64_t n = (int64_t)iz * g.nnx + ix;
     const int li = (iz - lz0) * LX + (ix - lx0);
     const uchar2 ff = sfix[li];
-    const bool fixed = (ff.x | ff.y) && use_u;       // calls without a velocity (G p only) pass no diagonal
+    const bool fixed = ff.x | ff.y;
     const bool pre = NPRE && slot >= 0;
     // every load first, none depending on another
     R2 uu = su2[li];                                 // the staged velocity: exact on free dofs
@@ -682,11 +569,8 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     R2 y;
     y.x = y0;
     y.y = y1;
-    if (ff.x | ff.y) {                               // eliminated rows act as K_ii u_i
-      const R2 fy = fixed ? R2{dg.x * uu.x, dg.y * uu.y} : R2{R(0), R(0)};
-      if (ff.x) y.x = fy.x;
-      if (ff.y) y.y = fy.y;
-    }
+    if (ff.x) y.x = dg.x * uu.x;                     // eliminated rows act as K_ii u_i
+    if (ff.y) y.y = dg.y * uu.y;
     if (MODE == AM_APPLY) {
       reinterpret_cast<R2*>(a.yV)[n] = y;
     } else if (MODE == AM_RESID) {
@@ -712,16 +596,16 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     R y0 = 0, y1 = 0;
     if (vza) {
       const int lez = za - (ez0 - 1);
-      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * 22; int k = q2_local_idx(dxa, dza);
+      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * YS; int k = q2_local_idx(dxa, dza);
                  y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * 22; int k = q2_local_idx(0, dza);
+      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * YS; int k = q2_local_idx(0, dza);
                  y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
     }
     if (vzb) {
       const int lez = zb - (ez0 - 1);
-      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * 22; int k = q2_local_idx(dxa, 0);
+      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * YS; int k = q2_local_idx(dxa, 0);
                  y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * 22; int k = q2_local_idx(0, 0);
+      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * YS; int k = q2_local_idx(0, 0);
                  y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
     }
     emit(ix, iz, y0, y1, slot);
@@ -732,10 +616,10 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     const bool l = px >= 1, rr = px < g.nx, bo = pz >= 1, to = pz < g.nz;
     const int lx = px - ex0, lz = pz - ez0;          // tile-local index of element (px, pz) is (lx+1, lz+1)
     R y = 0;
-    if (bo && l) y += sye[((lz) * EX + lx) * 22 + 18 + 2];
-    if (bo && rr) y += sye[((lz) * EX + lx + 1) * 22 + 18 + 3];
-    if (to && l) y += sye[((lz + 1) * EX + lx) * 22 + 18 + 1];
-    if (to && rr) y += sye[((lz + 1) * EX + lx + 1) * 22 + 18 + 0];
+    if (bo && l) y += sye[((lz) * EX + lx) * YS + 18 + 2];
+    if (bo && rr) y += sye[((lz) * EX + lx + 1) * YS + 18 + 3];
+    if (to && l) y += sye[((lz + 1) * EX + lx) * YS + 18 + 1];
+    if (to && rr) y += sye[((lz + 1) * EX + lx + 1) * YS + 18 + 0];
     const int64_t n = (int64_t)pz * (g.nx + 1) + px;
     a.yP[n] = (MODE == AM_RESID) ? a.bP[n] - y : y;
   };
@@ -743,12 +627,12 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     const int lx = tid % TX, lz = tid / TX;          // TX is a power of two
     const int ex = ex0 + lx, ez = ez0 + lz;
     if (ex < g.nx && ez < g.nz) {
-      const R* e00 = sye + ((lz + 1) * EX + lx + 1) * 22;   // element (ex, ez)
-      const R* eL = e00 - 22;                                 // (ex-1, ez)
-      const R* eB = e00 - EX * 22;                            // (ex, ez-1)
-      const R* eBL = eB - 22;                                 // (ex-1, ez-1)
+      const R* e00 = sye + ((lz + 1) * EX + lx + 1) * YS;   // element (ex, ez)
+      const R* eL = e00 - YS;                                 // (ex-1, ez)
+      const R* eB = e00 - EX * YS;                            // (ex, ez-1)
+      const R* eBL = eB - YS;                                 // (ex-1, ez-1)
       const bool hasL = ex > 0, hasB = ez > 0;
-      if (a.yV) {
+      {
         emit(2 * ex + 1, 2 * ez + 1, e00[16], e00[17], 0);   // centre: local node 8
         {                                                     // bottom edge midpoint: 6 of (ex,ez-1), 4
           R y0 = 0, y1 = 0;
@@ -771,7 +655,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
           emit(2 * ex, 2 * ez, y0, y1, 3);
         }
       }
-      if (a.yP) {                                             // pressure node (ex, ez): 2, 3, 1, 0
+      if (PRESSURE) {                                         // pressure node (ex, ez): 2, 3, 1, 0
         R y = 0;
         if (hasB && hasL) y += eBL[18 + 2];
         if (hasB) y += eB[18 + 3];
@@ -785,7 +669,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
     // right column ix = 2 nx (rows of this tile) and top row iz = 2 nz (columns of this tile,
     // the corner taken by the column)
     const int j0 = tid - TX * TZ, nj = NJ;
-    if (a.yV) {
+    {
 #pragma unroll
       for (int it = 0; it < 2; ++it) {                // the nodes whose vectors were prefetched
         const int j = j0 + it * nj;
@@ -795,7 +679,7 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
         }
       }
     }
-    if (a.yP) {
+    if (PRESSURE) {
       const int pz1 = lastz ? g.nz + 1 : ez0 + TZ;
       const int ncol = lastx ? pz1 - ez0 : 0;
       const int nrow = lastz ? (lastx ? g.nx - ex0 : TX) : 0;
@@ -807,362 +691,13 @@ MW_D void apply_tile(const LevelGeo& g, const ApplyArgs<R>& a, int bx, int bz, c
   }
 }
 
-// The operator apply as a kernel, one tile per CTA.  It repeats apply_tile's arithmetic with its
-// body inline and its own static shared arrays: compiled through apply_tile (parameters by value or
-// by reference), the FP64 Chebyshev mode ran 43 % slower and the plain FP64 512x512 step took 106
-// instead of 93 ms (FP32 the same), measured on one GPU; apply_tile serves the kernels that run
-// several tiles per CTA (the ensemble's cluster solve), and its GPU tests check the two against
-// each other through the solves.
+// The operator apply as a kernel, one tile per CTA.
 template <typename R, int MODE>
 __global__ void __launch_bounds__(APPLY_THREADS, sizeof(R) == 4 ? MW_APPLY_MINB : 1)
-k_apply(LevelGeo g, ApplyArgs<R> a) {
+k_apply(const __grid_constant__ LevelGeo g, const __grid_constant__ ApplyArgs<R> a) {
   pdl_entry();
-  typedef typename Vec2<R>::T R2;
-  // node vectors the epilogue reads for the four nodes each owned element emits (b; b, diag, d),
-  // fetched asynchronously while the element products run (FP32; the FP64 kernel's shared memory
-  // is already at the 48 KB static limit)
-  constexpr bool CHEB = MODE == AM_CHEB || MODE == AM_CHEB_Z;
-  constexpr int NPRE = sizeof(R) == 8 ? 0 : (CHEB ? 3 : (MODE == AM_RESID ? 1 : 0));
-  __shared__ __align__(16) R su[LZ * LX * 2];
-  __shared__ __align__(16) R2 spre[(NPRE ? NPRE : 1) * 4 * TX * TZ];
-  constexpr int NJ = APPLY_THREADS - TX * TZ;         // spare threads: right column and top row nodes
-  static_assert(2 * TZ + 1 + 2 * TX <= 2 * NJ, "the spare threads take at most two boundary nodes each");
-  __shared__ __align__(16) R2 sspare[(NPRE ? NPRE : 1) * 2 * NJ];
-  __shared__ R sp[PZ * PX];
-  __shared__ R sye[NEL_T * 22];
-  __shared__ uchar2 sfix[LZ * LX];          // Dirichlet flags of the staged nodes
-  const int ex0 = blockIdx.x * TX, ez0 = blockIdx.y * TZ;
-  const int lx0 = 2 * ex0 - 2, lz0 = 2 * ez0 - 2;      // lattice origin of the staged nodes
-  const int tid = threadIdx.x;
-  const bool use_u = a.u != nullptr, use_p = a.p != nullptr;
-  // Chebyshev coefficients, read now so that no epilogue load waits on them
-  const double c1 = CHEB ? a.cheb[0] : 0.0;
-  const R c2 = CHEB ? R(a.cheb[1]) : R(0);
-  const R cz = MODE == AM_CHEB_Z ? R(a.cheb0[1]) : R(0);
-  // ---- prefetch: the epilogue's node vectors (owned elements), the element viscosities ----
-  // slot j of an owned element: 0 centre (2ex+1, 2ez+1), 1 bottom midpoint (2ex+1, 2ez),
-  // 2 left midpoint (2ex, 2ez+1), 3 corner (2ex, 2ez)
-  if (NPRE && a.yV && tid < TX * TZ) {
-    const int ex = ex0 + tid % TX, ez = ez0 + tid / TX;
-    if (ex < g.nx && ez < g.nz) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int ix = 2 * ex + (j < 2 ? 1 : 0), iz = 2 * ez + ((j & 1) ? 0 : 1);
-        const int64_t n = (int64_t)iz * g.nnx + ix;
-        cp_async_pair<R>(&spre[j * TX * TZ + tid], a.bV + 2 * n);
-        if (NPRE == 3) {
-          cp_async_pair<R>(&spre[(4 + j) * TX * TZ + tid], a.diag + 2 * n);
-          if (MODE == AM_CHEB) cp_async_pair<R>(&spre[(8 + j) * TX * TZ + tid], a.d + 2 * n);
-        }
-      }
-    }
-  }
-  // the spare threads' boundary nodes (at most 2 TZ + 1 + 2 TX = 49, two per spare thread)
-  const bool lastx = ex0 + TX >= g.nx, lastz = ez0 + TZ >= g.nz;
-  const int oz1 = lastz ? 2 * g.nz + 1 : 2 * (ez0 + TZ);
-  const int ncol_v = lastx ? oz1 - 2 * ez0 : 0;
-  const int nrow_v = lastz ? (lastx ? 2 * (g.nx - ex0) : 2 * TX) : 0;
-  if (NPRE && a.yV && tid >= TX * TZ && (lastx || lastz)) {
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const int j = tid - TX * TZ + it * NJ;
-      if (j < ncol_v + nrow_v) {
-        const int ix = j < ncol_v ? 2 * g.nx : 2 * ex0 + (j - ncol_v);
-        const int iz = j < ncol_v ? 2 * ez0 + j : 2 * g.nz;
-        const int64_t n = (int64_t)iz * g.nnx + ix;
-        const int q = tid - TX * TZ;
-        cp_async_pair<R>(&sspare[it * NJ + q], a.bV + 2 * n);
-        if (NPRE == 3) {
-          cp_async_pair<R>(&sspare[(2 + it) * NJ + q], a.diag + 2 * n);
-          if (MODE == AM_CHEB) cp_async_pair<R>(&sspare[(4 + it) * NJ + q], a.d + 2 * n);
-        }
-      }
-    }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  R eq[9];
-  if (tid < NEL_T) {
-    const int ex = ex0 - 1 + tid % EX, ez = ez0 - 1 + tid / EX;
-    if (ex >= 0 && ex < g.nx && ez >= 0 && ez < g.nz) {
-      const R* eg = a.eta + ((int64_t)ez * g.nx + ex) * 9;
-#pragma unroll
-      for (int q = 0; q < 9; ++q) eq[q] = eg[q];
-    }
-  }
-  // ---- stage velocity (masked; one vector load per node), pressure ----
-  // A fixed number of nodes per thread, all loads issued before any shared-memory store, so the
-  // staging costs one memory round trip rather than one per node.
-  const R2* u2 = reinterpret_cast<const R2*>(a.u);
-  const uchar2* f2 = reinterpret_cast<const uchar2*>(a.fix);
-  R2* su2 = reinterpret_cast<R2*>(su);
-  constexpr int NST = (LZ * LX + APPLY_THREADS - 1) / APPLY_THREADS;
-  constexpr int NSP = (PZ * PX + APPLY_THREADS - 1) / APPLY_THREADS;
-  R2 sv[NST];
-  uchar2 sf[NST];
-  R spv[NSP];
-  if constexpr (sizeof(R) == 8) {                    // FP64: one node at a time (fewer live registers)
-    for (int i = tid; i < LZ * LX; i += APPLY_THREADS) {
-      const int lz = i / LX, lx = i - lz * LX;
-      const int ix = lx0 + lx, iz = lz0 + lz;
-      R2 v;
-      v.x = 0; v.y = 0;
-      uchar2 ff = make_uchar2(0, 0);
-      if (ix >= 0 && ix < g.nnx && iz >= 0 && iz < g.nnz) {
-        const int64_t n = (int64_t)iz * g.nnx + ix;
-        ff = f2[n];
-        if (use_u) {
-          R2 uu = u2[n];
-          v.x = ff.x ? R(0) : uu.x;
-          v.y = ff.y ? R(0) : uu.y;
-        }
-      }
-      su2[i] = v;
-      sfix[i] = ff;
-    }
-    if (use_p)
-      for (int i = tid; i < PZ * PX; i += APPLY_THREADS) {
-        int jz = i / PX, jx = i % PX;
-        int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
-        sp[i] = (px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz) ? a.p[(int64_t)pz * (g.nx + 1) + px] : R(0);
-      }
-  } else {
-#pragma unroll
-  for (int k = 0; k < NST; ++k) {
-    const int i = tid + k * APPLY_THREADS;
-    const int lz = i / LX, lx = i - lz * LX;
-    const int ix = lx0 + lx, iz = lz0 + lz;
-    sv[k].x = 0; sv[k].y = 0;
-    sf[k] = make_uchar2(0, 0);
-    if (i < LZ * LX && ix >= 0 && ix < g.nnx && iz >= 0 && iz < g.nnz) {
-      const int64_t n = (int64_t)iz * g.nnx + ix;
-      sf[k] = f2[n];
-      if (MODE == AM_CHEB_Z) {                       // x0 = (1/theta) D^-1 b
-        const R2 bb = reinterpret_cast<const R2*>(a.bV)[n], dg = reinterpret_cast<const R2*>(a.diag)[n];
-        sv[k].x = cz * bb.x / dg.x;
-        sv[k].y = cz * bb.y / dg.y;
-      } else if (use_u) {
-        sv[k] = u2[n];
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) {
-    const int i = tid + k * APPLY_THREADS;
-    const int jz = i / PX, jx = i % PX;
-    const int px = ex0 - 1 + jx, pz = ez0 - 1 + jz;
-    spv[k] = (use_p && i < PZ * PX && px >= 0 && px <= g.nx && pz >= 0 && pz <= g.nz)
-                 ? a.p[(int64_t)pz * (g.nx + 1) + px] : R(0);
-  }
-#pragma unroll
-  for (int k = 0; k < NST; ++k) {
-    const int i = tid + k * APPLY_THREADS;
-    if (i < LZ * LX) {
-      R2 v;
-      v.x = sf[k].x ? R(0) : sv[k].x;
-      v.y = sf[k].y ? R(0) : sv[k].y;
-      su2[i] = v;
-      sfix[i] = sf[k];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) {
-    const int i = tid + k * APPLY_THREADS;
-    if (use_p && i < PZ * PX) sp[i] = spv[k];
-  }
-  }
-  __syncthreads();
-  // ---- element products ----
-  if (tid < NEL_T) {
-    int lex = tid % EX, lez = tid / EX;
-    int ex = ex0 - 1 + lex, ez = ez0 - 1 + lez;
-    if (ex >= 0 && ex < g.nx && ez >= 0 && ez < g.nz) {
-      __align__(16) R ue[18];
-      R pe[4], ye[18], ype[4];
-      const int bx = 2 * lex, bz = 2 * lez;          // staged lattice coords of local node 0
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        int li = (bz + q2_dz(k)) * LX + bx + q2_dx(k);
-        ue[2 * k] = su[2 * li]; ue[2 * k + 1] = su[2 * li + 1];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pe[k] = use_p ? sp[(lez + q1_dz(k)) * PX + lex + q1_dx(k)] : R(0);
-      const R sxe = R(2.0 / g.hx), sze = R(2.0 / g.hz), jace = R(g.hx * g.hz / 4.0), se = R(g.s);
-      if (!use_u)                                   // G p only (the Schur iteration's G d, f - G P)
-        element_apply<R, false, true>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
-      else if (!a.yV)                               // G^T u only
-        element_apply<R, true, false>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
-      else
-        element_apply<R>(sxe, sze, jace, se, ue, pe, eq, ye, ype, use_p);
-#pragma unroll
-      for (int k = 0; k < 18; ++k) sye[tid * 22 + k] = ye[k];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) sye[tid * 22 + 18 + k] = ype[k];
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  // ---- owned nodes: sums over the incident elements in ascending element order ----
-  // Each owned element's thread takes the four nodes of its lower-left quadrant (centre, bottom
-  // and left edge midpoints, lower-left corner) and its lower-left pressure node, with the element
-  // local indices known at compile time; the spare threads take the nodes on the right and top
-  // mesh boundary, which belong to no element's lower-left quadrant.
-  // prefetched value of array k (0 b, 1 diag, 2 d): slots 0-3 are an owned element's nodes,
-  // slots 4-5 a spare thread's two boundary nodes
-  auto pre_at = [&](int k, int slot) -> R2 {
-    return slot < 4 ? spre[(4 * k + slot) * TX * TZ + tid] : sspare[(2 * k + slot - 4) * NJ + (tid - TX * TZ)];
-  };
-  // velocity node epilogue: Dirichlet rows, then the mode's output.  slot >= 0: b, diag, d were
-  // prefetched; slot < 0: read them here.
-  auto emit = [&](int ix, int iz, R y0, R y1, int slot) {
-    const int64_t n = (int64_t)iz * g.nnx + ix;
-    const int li = (iz - lz0) * LX + (ix - lx0);
-    const uchar2 ff = sfix[li];
-    const bool fixed = (ff.x | ff.y) && use_u;       // calls without a velocity (G p only) pass no diagonal
-    const bool pre = NPRE && slot >= 0;
-    // every load first, none depending on another
-    R2 uu = su2[li];                                 // the staged velocity: exact on free dofs
-    R2 dg{R(0), R(0)}, bb{R(0), R(0)}, dd{R(0), R(0)};
-    if (CHEB) dg = pre ? pre_at(1, slot) : reinterpret_cast<const R2*>(a.diag)[n];
-    else if (fixed) dg = reinterpret_cast<const R2*>(a.diag)[n];
-    if (fixed && MODE != AM_CHEB_Z) {                // the fixed components' values (staged as 0);
-      const R2 raw = reinterpret_cast<const R2*>(a.u)[n];   // a free one keeps its staged value
-      if (ff.x) uu.x = raw.x;
-      if (ff.y) uu.y = raw.y;
-    }
-    if (MODE != AM_APPLY) bb = pre ? pre_at(0, slot) : reinterpret_cast<const R2*>(a.bV)[n];
-    if (MODE == AM_CHEB && c1 != 0.0)                // restart steps never read the old direction
-      dd = pre ? pre_at(2, slot) : reinterpret_cast<const R2*>(a.d)[n];
-    if (MODE == AM_CHEB_Z) {                         // the first step's x and d, both x0
-      const R2 x0{cz * bb.x / dg.x, cz * bb.y / dg.y};
-      if (fixed) uu = x0;
-      dd = x0;
-    }
-    R2 y;
-    y.x = y0;
-    y.y = y1;
-    if (ff.x | ff.y) {                               // eliminated rows act as K_ii u_i
-      const R2 fy = fixed ? R2{dg.x * uu.x, dg.y * uu.y} : R2{R(0), R(0)};
-      if (ff.x) y.x = fy.x;
-      if (ff.y) y.y = fy.y;
-    }
-    if (MODE == AM_APPLY) {
-      reinterpret_cast<R2*>(a.yV)[n] = y;
-    } else if (MODE == AM_RESID) {
-      reinterpret_cast<R2*>(a.yV)[n] = R2{bb.x - y.x, bb.y - y.y};
-    } else {   // Chebyshev step: d = c1 d + c2 D^-1 (b - y); x_out = u + d
-      R2 dn{c2 * (bb.x - y.x) / dg.x, c2 * (bb.y - y.y) / dg.y};
-      if (c1 != 0.0) {
-        dn.x += R(c1) * dd.x;
-        dn.y += R(c1) * dd.y;
-      }
-      reinterpret_cast<R2*>(a.d)[n] = dn;
-      reinterpret_cast<R2*>(a.xo)[n] = R2{uu.x + dn.x, uu.y + dn.y};
-    }
-  };
-  // any velocity node of the tile (incident elements found from the node's parity)
-  auto node_generic = [&](int ix, int iz, int slot) {
-    const bool xo = ix & 1, zo = iz & 1;
-    const int xa = xo ? (ix >> 1) : (ix >> 1) - 1, xb = (ix >> 1);
-    const int za = zo ? (iz >> 1) : (iz >> 1) - 1, zb = (iz >> 1);
-    const bool vxa = xa >= 0, vxb = !xo && xb < g.nx;
-    const bool vza = za >= 0, vzb = !zo && zb < g.nz;
-    const int dxa = xo ? 1 : 2, dza = zo ? 1 : 2;   // offsets inside element xa / za; 0 inside xb / zb
-    R y0 = 0, y1 = 0;
-    if (vza) {
-      const int lez = za - (ez0 - 1);
-      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * 22; int k = q2_local_idx(dxa, dza);
-                 y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * 22; int k = q2_local_idx(0, dza);
-                 y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-    }
-    if (vzb) {
-      const int lez = zb - (ez0 - 1);
-      if (vxa) { const R* ye = sye + (lez * EX + xa - (ex0 - 1)) * 22; int k = q2_local_idx(dxa, 0);
-                 y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-      if (vxb) { const R* ye = sye + (lez * EX + xb - (ex0 - 1)) * 22; int k = q2_local_idx(0, 0);
-                 y0 += ye[2 * k]; y1 += ye[2 * k + 1]; }
-    }
-    emit(ix, iz, y0, y1, slot);
-  };
-  // any pressure node of the tile
-  auto pnode_generic = [&](int px, int pz) {
-    // incident elements (pz-1, px-1) k=2, (pz-1, px) k=3, (pz, px-1) k=1, (pz, px) k=0
-    const bool l = px >= 1, rr = px < g.nx, bo = pz >= 1, to = pz < g.nz;
-    const int lx = px - ex0, lz = pz - ez0;          // tile-local index of element (px, pz) is (lx+1, lz+1)
-    R y = 0;
-    if (bo && l) y += sye[((lz) * EX + lx) * 22 + 18 + 2];
-    if (bo && rr) y += sye[((lz) * EX + lx + 1) * 22 + 18 + 3];
-    if (to && l) y += sye[((lz + 1) * EX + lx) * 22 + 18 + 1];
-    if (to && rr) y += sye[((lz + 1) * EX + lx + 1) * 22 + 18 + 0];
-    const int64_t n = (int64_t)pz * (g.nx + 1) + px;
-    a.yP[n] = (MODE == AM_RESID) ? a.bP[n] - y : y;
-  };
-  if (tid < TX * TZ) {
-    const int lx = tid % TX, lz = tid / TX;          // TX is a power of two
-    const int ex = ex0 + lx, ez = ez0 + lz;
-    if (ex < g.nx && ez < g.nz) {
-      const R* e00 = sye + ((lz + 1) * EX + lx + 1) * 22;   // element (ex, ez)
-      const R* eL = e00 - 22;                                 // (ex-1, ez)
-      const R* eB = e00 - EX * 22;                            // (ex, ez-1)
-      const R* eBL = eB - 22;                                 // (ex-1, ez-1)
-      const bool hasL = ex > 0, hasB = ez > 0;
-      if (a.yV) {
-        emit(2 * ex + 1, 2 * ez + 1, e00[16], e00[17], 0);   // centre: local node 8
-        {                                                     // bottom edge midpoint: 6 of (ex,ez-1), 4
-          R y0 = 0, y1 = 0;
-          if (hasB) { y0 += eB[12]; y1 += eB[13]; }
-          y0 += e00[8]; y1 += e00[9];
-          emit(2 * ex + 1, 2 * ez, y0, y1, 1);
-        }
-        {                                                     // left edge midpoint: 5 of (ex-1,ez), 7
-          R y0 = 0, y1 = 0;
-          if (hasL) { y0 += eL[10]; y1 += eL[11]; }
-          y0 += e00[14]; y1 += e00[15];
-          emit(2 * ex, 2 * ez + 1, y0, y1, 2);
-        }
-        {                                                     // lower-left corner: 2, 3, 1, 0
-          R y0 = 0, y1 = 0;
-          if (hasB && hasL) { y0 += eBL[4]; y1 += eBL[5]; }
-          if (hasB) { y0 += eB[6]; y1 += eB[7]; }
-          if (hasL) { y0 += eL[2]; y1 += eL[3]; }
-          y0 += e00[0]; y1 += e00[1];
-          emit(2 * ex, 2 * ez, y0, y1, 3);
-        }
-      }
-      if (a.yP) {                                             // pressure node (ex, ez): 2, 3, 1, 0
-        R y = 0;
-        if (hasB && hasL) y += eBL[18 + 2];
-        if (hasB) y += eB[18 + 3];
-        if (hasL) y += eL[18 + 1];
-        y += e00[18 + 0];
-        const int64_t n = (int64_t)ez * (g.nx + 1) + ex;
-        a.yP[n] = (MODE == AM_RESID) ? a.bP[n] - y : y;
-      }
-    }
-  } else if (lastx || lastz) {
-    // right column ix = 2 nx (rows of this tile) and top row iz = 2 nz (columns of this tile,
-    // the corner taken by the column)
-    const int j0 = tid - TX * TZ, nj = NJ;
-    if (a.yV) {
-#pragma unroll
-      for (int it = 0; it < 2; ++it) {                // the nodes whose vectors were prefetched
-        const int j = j0 + it * nj;
-        if (j < ncol_v + nrow_v) {
-          if (j < ncol_v) node_generic(2 * g.nx, 2 * ez0 + j, 4 + it);
-          else node_generic(2 * ex0 + (j - ncol_v), 2 * g.nz, 4 + it);
-        }
-      }
-    }
-    if (a.yP) {
-      const int pz1 = lastz ? g.nz + 1 : ez0 + TZ;
-      const int ncol = lastx ? pz1 - ez0 : 0;
-      const int nrow = lastz ? (lastx ? g.nx - ex0 : TX) : 0;
-      for (int j = j0; j < ncol + nrow; j += nj) {
-        if (j < ncol) pnode_generic(g.nx, ez0 + j);
-        else pnode_generic(ex0 + (j - ncol), g.nz);
-      }
-    }
-  }
+  __shared__ ApplySmem<R, MODE, false> sm;
+  apply_tile<R, MODE, false>(g, a, blockIdx.x, blockIdx.y, apply_ptrs(sm));
 }
 
 // diag(K): sum over incident elements of the element diagonal, ascending element order; and its
@@ -2446,7 +1981,7 @@ static void div_u(mw_stokes* S, const double* u, double* y, cudaStream_t s) {
   pdl_launch(k_div_u, grid, 128, 0, s, g, u, S->fixV, y);
 }
 
-// y = K x on level l
+// the operator's arguments on level l
 template <typename R>
 static OpArgs<R> op_args(const Level<R>& L, bool planes) {
   OpArgs<R> a;
@@ -2455,13 +1990,6 @@ static OpArgs<R> op_args(const Level<R>& L, bool planes) {
   a.qs = planes ? L.nel : 0;                        // level 0: nine planes; below: one value per element
   a.es = 1;
   return a;
-}
-
-template <typename R>
-static void level_apply(const Level<R>& L, bool planes, const R* x, R* y, cudaStream_t s) {
-  OpArgs<R> a = op_args(L, planes);
-  a.u = x; a.yV = y;
-  op_apply<R>(a, s);
 }
 
 // the FP64 operator on the fine mesh (the caller's viscosity, element by element)
@@ -2536,11 +2064,10 @@ MW_D void tail_apply(const TailLevel<R>& L, const R* u, R* xo, const double* che
   typedef typename Vec2<R>::T R2;
   const LevelGeo& g = L.g;
   const int nel = g.nx * g.nz;
-  const R sxe = R(2.0 / g.hx), sze = R(2.0 / g.hz), jace = R(g.hx * g.hz / 4.0), se = R(g.s);
   for (int e = t0; e < nel; e += nt) {
     const int ex = e % g.nx, ez = e / g.nx;
     __align__(16) R ue[18];
-    R pe[4] = {R(0), R(0), R(0), R(0)}, ye[18], ype[4], eq[9];
+    R ye[18], eq[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const int64_t n = q2_node(ex, ez, k, g.nnx);
@@ -2549,7 +2076,7 @@ MW_D void tail_apply(const TailLevel<R>& L, const R* u, R* xo, const double* che
     }
 #pragma unroll
     for (int q = 0; q < 9; ++q) eq[q] = L.eta[(int64_t)e * 9 + q];
-    element_apply<R>(sxe, sze, jace, se, ue, pe, eq, ye, ype, false);
+    element_apply<false>(g, ue, (const R*)nullptr, eq, ye, (R*)nullptr);
 #pragma unroll
     for (int k = 0; k < 18; ++k) sye[e * 18 + k] = ye[k];
   }

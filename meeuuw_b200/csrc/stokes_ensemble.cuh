@@ -22,8 +22,11 @@ constexpr int ENS_CLUSTER = 8;                     // CTAs per model
 constexpr int ENS_THREADS = APPLY_THREADS;         // one tile apply per CTA at a time
 constexpr int ENS_NT = ENS_CLUSTER * ENS_THREADS;
 constexpr int ENS_WARPS = ENS_THREADS / 32;
+// Resident CTAs per SM the registers are sized for, and model-steps/s of ensembles of 24, 64 and 128 models
+// (64 to 192 squared): two (168 registers) 282, 518, 633; three (128) 274, 508, 741; four (96, the phases'
+// values spilled) 236, 440, 703.
 #ifndef MW_ENS_MINB
-#define MW_ENS_MINB 4                              // resident CTAs per SM the registers are sized for
+#define MW_ENS_MINB 3
 #endif
 
 // one model of the ensemble: its FP32 hierarchy, inner PCG vectors, FP64 fine-level vectors and
@@ -47,14 +50,15 @@ struct EnsParams {
   int max_inner, max_outer, max_refine, mass_iters, use_guess, weighted;
 };
 
-// Shared memory of the cluster solve: the tile apply's arrays (one layout at a time), cluster
+// Shared memory of the cluster solve: the tile apply's arrays (one layout at a time; only the FP64 residual
+// has pressure, so that each layout holds one element product), cluster
 // reduction slots, the G tables and element mass matrix, the model's descriptor.
 union EnsApplySmem {
   ApplySmem<float, AM_APPLY> a0;
   ApplySmem<float, AM_RESID> a1;
   ApplySmem<float, AM_CHEB> a2;
   ApplySmem<float, AM_CHEB_Z> a3;
-  ApplySmem<double, AM_RESID> d1;
+  ApplySmem<double, AM_RESID, true> d1;
 };
 
 struct EnsCtx {
@@ -99,13 +103,13 @@ MW_D void ens_sum(EnsCtx& c, double (&v)[NV]) {
 }
 
 // One operator apply of level g by the cluster: its element tiles dealt to the CTAs in turn.
-template <typename R, int MODE>
+template <typename R, int MODE, bool PRESSURE = false>
 MW_D void ens_apply(EnsCtx& c, const LevelGeo& g, const ApplyArgs<R>& a) {
   const int ntx = (g.nx + TX - 1) / TX, ntz = (g.nz + TZ - 1) / TZ;
-  const ApplyPtrs<R> sm = apply_ptrs(*reinterpret_cast<ApplySmem<R, MODE>*>(c.tile));
+  const ApplyPtrs<R> sm = apply_ptrs(*reinterpret_cast<ApplySmem<R, MODE, PRESSURE>*>(c.tile));
   for (int t = c.rank; t < ntx * ntz; t += ENS_CLUSTER) {
     __syncthreads();
-    apply_tile<R, MODE>(g, a, t % ntx, t / ntx, sm);
+    apply_tile<R, MODE, PRESSURE>(g, a, t % ntx, t / ntx, sm);
   }
   cluster_barrier();
 }
@@ -396,7 +400,7 @@ MW_D double ens_true_residual(EnsCtx& c, const double* V, const double* P, doubl
   memset(&a, 0, sizeof(a));
   a.u = V; a.p = P; a.eta = M.eta64; a.fix = M.fixV; a.diag = M.diag64;
   a.yV = M.RV; a.yP = M.RP; a.bV = M.f; a.bP = M.h;
-  ens_apply<double, AM_RESID>(c, M.g, a);
+  ens_apply<double, AM_RESID, true>(c, M.g, a);
   const int64_t nv = 2LL * M.g.nnx * M.g.nnz, np = (int64_t)(M.g.nx + 1) * (M.g.nz + 1);
   double v2[2] = {0.0, 0.0};
   for (int64_t i = c.t0; i < nv; i += ENS_NT) v2[0] += M.RV[i] * M.RV[i];
