@@ -31,13 +31,16 @@ MW_HD int q2_local(int dx, int dz) {
 }
 
 // One matrix row (element, dof) a thread, EB_S elements a pass, CTAs that stay for many passes.  A point's
-// weighted coefficients are formed once per element, so that an entry of K costs three multiply-adds (two
-// for its diagonal component, one for the other) from one 16-byte load of (dN/dx, dN/dz).  The results
-// take the room of the derivatives and leave as bulk copies.  BLOCKS writes K, G, GT, M, M_eta and H,
-// otherwise [K | G G]; both skip what they do not write.
-// Bounds: the 245 MB written (256^2 elements, FP64) take 37 us; the FP64 multiply-adds about 24, the
-// loads that feed them as much; the phases of a batch overlap only across the three CTAs of an SM:
-// 325 -> 128 us (8 elements a batch, 5 or 6 CTAs: 139, 146; 16 and 2: 139).
+// weighted coefficient is formed once per element; an entry of K then takes one rounded addition a point (the
+// geometric factor 2 o o_j + t t_j of the row's own component is formed before it is weighted: adding its two
+// weighted halves one after the other is one operation fewer and 8 to 15 % further from exact sums).  Rows of
+// both components run the same instructions on derivatives read by component: a branch on it issued every
+// multiply-add twice.  The results take the room of the derivatives and leave as bulk copies.  BLOCKS writes
+// K, G, GT, M, M_eta and H, otherwise [K | G G]; both skip what they do not write.
+// A pass over 256^2 elements in FP64, right-hand sides included: 337 -> 138 us, in FP32 175 -> 88; with BLOCKS
+// 361 -> 188 and 187 -> 125 (a batch a CTA, derivatives and results apart, before).  Bounds: the 245 MB written
+// take 37 us, the FP64 multiply-adds about 30, the loads that feed them as much; the phases of a batch
+// overlap only across the CTAs of an SM.
 template <typename R>
 struct alignas(2 * sizeof(R)) Pair {
   R x, z;
@@ -139,9 +142,10 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       }
     __syncthreads();
 
-    R K[18], G[4], H[4], Mv = 0, f = 0;
+    // the row's entries by node: own[j] in the row's component (column 2 j + c), oth[j] in the other one
+    R own[9], oth[9], G[4], H[4], Mv = 0, f = 0;
 #pragma unroll
-    for (int j = 0; j < 18; ++j) K[j] = 0;
+    for (int j = 0; j < 9; ++j) own[j] = oth[j] = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) { G[k] = 0; H[k] = 0; }
     if (live) {
@@ -149,34 +153,22 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       for (int q = 0; q < 9; ++q) {
         const int eq = el * 9 + q;
         const R w = wq[eq], jxw = wq[L::Q + eq];
-        const Pair<R>* d = dV + el * 81 + q * 9;
-        const Pair<R> di = d[i];
-        // B^T C B (build_matrix_stokes.py:140), C = diag(2, 2, 1): with (o, t) the row's own direction and
-        // the other one, K_own = 2 o o_j + t t_j, K_other = t o_j
-        const R own = c == 0 ? di.x : di.z, oth = c == 0 ? di.z : di.x;
-        const R wo = R(2) * w * own, wt = w * oth;
-        if (c == 0) {
+        // B^T C B (build_matrix_stokes.py:140), C = diag(2, 2, 1): with (o, t) the derivatives in the row's own
+        // direction and the other one, 2 o o_j + t t_j in its own component, t o_j in the other
+        const R* dc = reinterpret_cast<const R*>(dV + el * 81 + q * 9) + c;
+        const R* dt = reinterpret_cast<const R*>(dV + el * 81 + q * 9) + (c ^ 1);
+        const R o = dc[2 * i], t = dt[2 * i], wt = w * t;
 #pragma unroll
-          for (int j = 0; j < 9; ++j) {
-            const Pair<R> dj = d[j];
-            K[2 * j] += wo * dj.x;
-            K[2 * j] += wt * dj.z;
-            K[2 * j + 1] += wt * dj.x;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 9; ++j) {
-            const Pair<R> dj = d[j];
-            K[2 * j + 1] += wo * dj.z;
-            K[2 * j + 1] += wt * dj.x;
-            K[2 * j] += wt * dj.z;
-          }
+        for (int j = 0; j < 9; ++j) {
+          const R oj = dc[2 * j];
+          own[j] += (R(2) * o * oj + t * dt[2 * j]) * w;
+          oth[j] += wt * oj;
         }
         const R n = NV[q * 9 + i];
         f += n * wq[(2 + c) * L::Q + eq];                                // :142-143
-        const R oj = own * jxw;
+        const R ow = o * jxw;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) G[k] -= oj * NP[q * 4 + k];          // :144-146
+        for (int k = 0; k < 4; ++k) G[k] -= ow * NP[q * 4 + k];          // :144-146
         if (BLOCKS) {
           const R nj = n * jxw;
 #pragma unroll
@@ -199,17 +191,23 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       if (fx >> ikk & 1) {
         R kd = 0;
 #pragma unroll
-        for (int j = 0; j < 18; ++j) {
-          if (j == ikk) kd = K[j];
-          else K[j] = 0;
+        for (int j = 0; j < 9; ++j) {
+          if (j == i) kd = own[j];
+          else own[j] = 0;
+          oth[j] = 0;
         }
         frow = kd * (R)fv[ikk];
 #pragma unroll
         for (int k = 0; k < 4; ++k) G[k] = 0;
       } else {
 #pragma unroll
-        for (int j = 0; j < 18; ++j)
-          if (fx >> j & 1) { frow -= K[j] * (R)fv[j]; K[j] = 0; }
+        for (int j = 0; j < 9; ++j) {                      // ascending dofs
+          R e0 = c == 0 ? own[j] : oth[j], e1 = c == 0 ? oth[j] : own[j];
+          if (fx >> (2 * j) & 1) { frow -= e0 * (R)fv[2 * j]; e0 = 0; }
+          if (fx >> (2 * j + 1) & 1) { frow -= e1 * (R)fv[2 * j + 1]; e1 = 0; }
+          own[j] = c == 0 ? e0 : e1;
+          oth[j] = c == 0 ? e1 : e0;
+        }
       }
     }
     __syncthreads();                                       // the derivatives are read: their room is reused
@@ -236,7 +234,7 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       if (live) {
         Pair<R>* o = reinterpret_cast<Pair<R>*>(outs + el * 468 + ikk * 26);    // :268-276
 #pragma unroll
-        for (int j = 0; j < 9; ++j) o[j] = Pair<R>{K[2 * j], K[2 * j + 1]};
+        for (int j = 0; j < 9; ++j) o[j] = c == 0 ? Pair<R>{own[j], oth[j]} : Pair<R>{oth[j], own[j]};
 #pragma unroll
         for (int k = 0; k < 4; ++k) o[9 + k] = Pair<R>{G[k], G[k]};
       }
@@ -245,7 +243,10 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
       R *oG = outs + EB_S * 324, *oGT = oG + EB_S * 72, *oH = oGT + EB_S * 72, *oM = oH + EB_S * 72;
       R* oMe = oM + EB_S * 16;
 #pragma unroll
-      for (int j = 0; j < 18; ++j) oK[j] = K[j];                                // :237-240
+      for (int j = 0; j < 9; ++j) {                                             // :237-240
+        oK[2 * j + c] = own[j];
+        oK[2 * j + (c ^ 1)] = oth[j];
+      }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         oG[el * 72 + ikk * 4 + k] = G[k];                                       // :243-246
