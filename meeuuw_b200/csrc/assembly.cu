@@ -37,8 +37,8 @@ MW_HD int q2_local(int dx, int dz) {
 // both components run the same instructions on derivatives read by component: a branch on it issued every
 // multiply-add twice.  The results take the room of the derivatives and leave as bulk copies.  BLOCKS writes
 // K, G, GT, M, M_eta and H, otherwise [K | G G]; both skip what they do not write.
-// A pass over 256^2 elements in FP64, right-hand sides included: 337 -> 138 us, in FP32 175 -> 88; with BLOCKS
-// 361 -> 188 and 187 -> 125 (a batch a CTA, derivatives and results apart, before).  Bounds: the 245 MB written
+// A pass over 256^2 elements in FP64, right-hand sides included: 337 -> 139 us, in FP32 175 -> 93; with BLOCKS
+// 361 -> 188 and 187 -> 130 (a batch a CTA, derivatives and results apart, before).  Bounds: the 245 MB written
 // take 37 us, the FP64 multiply-adds about 30, the loads that feed them as much; the phases of a batch
 // overlap only across the CTAs of an SM.
 template <typename R>
@@ -51,7 +51,7 @@ struct StokesSmem {                        // R values per CTA, by offset
   static constexpr int Q = EB_S * 9;
   static constexpr int DV = 0;                                   // pairs (dN/dx, dN/dz) of the velocity
   static constexpr int DP = DV + 2 * EB_S * 81;                  // of the pressure
-  static constexpr int W = DP + (BLOCKS ? 2 * EB_S * 36 : 0);    // eta JxW, JxW, rho gx JxW, rho gz JxW
+  static constexpr int W = DP + (BLOCKS ? 2 * EB_S * 36 : 0);    // eta JxW (FP32: eta), JxW, rho gx JxW, rho gz JxW
   static constexpr int J = W + 4 * Q;                            // the four entries of the Jacobian
   static constexpr int IN_END = J + 4 * Q;
   static constexpr int G0 = 0;                                   // rows of G before the elimination
@@ -107,7 +107,7 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
     if (tid < ne * 9) {
       const int64_t g = e0 * 9 + tid;
       const R jxw = (R)in.JxWq[g], eta = (R)in.etaq[g], rj = jxw * (R)in.rhoq[g];
-      wq[tid] = eta * jxw;
+      wq[tid] = sizeof(R) == 8 ? eta * jxw : eta;   // (their product alone may leave FP32's range)
       wq[L::Q + tid] = jxw;
       wq[2 * L::Q + tid] = rj * (R)in.gxq[g];
       wq[3 * L::Q + tid] = rj * (R)in.gzq[g];
@@ -161,8 +161,9 @@ k_assemble_stokes(mw_box b, mw_stokes_in in, int write, int bulk, R* __restrict_
 #pragma unroll
         for (int j = 0; j < 9; ++j) {
           const R oj = dc[2 * j];
-          own[j] += (R(2) * o * oj + t * dt[2 * j]) * w;
-          oth[j] += wt * oj;
+          const R g = R(2) * o * oj + t * dt[2 * j];
+          own[j] += sizeof(R) == 8 ? g * w : g * w * jxw;
+          oth[j] += sizeof(R) == 8 ? wt * oj : wt * oj * jxw;
         }
         const R n = NV[q * 9 + i];
         f += n * wq[(2 + c) * L::Q + eq];                                // :142-143

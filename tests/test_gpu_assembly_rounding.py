@@ -1,4 +1,5 @@
-"""The rounding of the assembled viscous block: nine rounded additions an entry, one a Gauss point."""
+"""The rounding of the assembled viscous block (nine rounded additions an entry, one a Gauss point) and its range
+in FP32."""
 import numpy as np
 import pytest
 import torch
@@ -48,3 +49,13 @@ def test_rounding_of_the_own_component():
             got += float((((K[:, i, c, :, c] - exact) / scale) ** 2).mean())
             nine += float((((model - exact) / scale) ** 2).mean())
     assert got ** 0.5 <= 1.04 * nine ** 0.5, (got ** 0.5, nine ** 0.5)
+
+
+def test_fp32_range():
+    """Entries of some 1e28 from a viscosity whose product with JxW (4e38) is past FP32's largest number; FP32
+    rounds each of about ten operations an entry, of terms up to ten times the entry: 1e-5 of the largest."""
+    etaq = np.exp(np.random.default_rng(1).uniform(-0.1, 0.1, (12, 9))) * 1e28
+    _, K = assemble(4, 3, 3e6, etaq, 0)
+    _, K32 = assemble(4, 3, 3e6, etaq, 1)
+    assert np.isfinite(K32).all()
+    assert np.abs(K32 - K).max() <= 1e-5 * np.abs(K).max()
