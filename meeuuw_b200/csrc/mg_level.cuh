@@ -60,6 +60,7 @@ template <typename R> void mg_up(const MgArgs<R>& a, int deg, bool planes, cudaS
 // The coarse end of a V-cycle in one launch (mg_tail.cu): `n` smoothed levels of at most MG_TAIL_CELLS cells
 // ((nx + 1)(nz + 1)) and the coarsest level's dense inverse.
 constexpr int MG_TAIL_CELLS = 384, MG_TAIL_LEVELS = 5;
+template <typename R> constexpr int mg_tail_degree() { return sizeof(R) == 4 ? MG_MAXDEG : 1; }   // smoothing steps
 template <typename R>
 struct MgTailLevel {
   LevelGeo g;

@@ -406,7 +406,9 @@ bool launch_tail_deg(const MgTailArgs<R>& a, const TailLayout<R>& S, cudaStream_
 template <typename R> bool mg_tail(const MgTailArgs<R>& a, int deg, cudaStream_t s) {
   TailLayout<R> S;
   if (!S.plan(a, tail_limit())) return false;
-  return deg <= 1 ? launch_tail_deg<R, 1>(a, S, s) : launch_tail_deg<R, MG_MAXDEG>(a, S, s);
+  if constexpr (mg_tail_degree<R>() > 1)
+    if (deg > 1) return launch_tail_deg<R, MG_MAXDEG>(a, S, s);
+  return deg <= 1 && launch_tail_deg<R, 1>(a, S, s);
 }
 
 int mg_tail_ensure_tables() { return ensure_cell_tables(); }

@@ -2393,12 +2393,14 @@ static void launch_tail(Hierarchy<R>& H, int l0, bool first_done, cudaStream_t s
 // The cycle from level l down in one launch where every level fits a CTA (mg_tail.cu) and some transfer
 // there is not nested; false when it goes level by level.  One CTA takes 3000 clocks an apply at 20 x 14
 // cells and 1800 at one warp; the level launches spread theirs over several SMs and cost 2.9 us each when
-// nested (64^2: 37 us a cycle by levels, 46 with the tail), 4 to 5 when not (150x97, from 19 x 13: 31 us in
-// the tail, 40 by levels).
+// nested (64^2: 37 us a cycle by levels, 46 with the tail), 4 to 5 when not.  V-cycles in us, by levels and with
+// the tail, on meshes whose tails start at 360, 280, 196 and 100 cells (34x38, 150x97, 26x26, 20x18): FP32 50, 86,
+// 39, 36 and 46, 80, 36, 31; FP64 with one smoothing step 53, 87, 41, 39 and 44, 77, 35, 31.  With two FP64 steps
+// the applies cost one SM more than the launches (67, 116, 51, 50 and 71, 118, 54, 48): by levels.
 template <typename R>
 static bool vcycle_tail(Hierarchy<R>& H, int l, cudaStream_t s) {
   const int n = H.nlev - 1 - l;
-  if (l < 1 || n < 1 || n > MG_TAIL_LEVELS || !H.dense || H.L[l].deg > MG_MAXDEG) return false;
+  if (l < 1 || n < 1 || n > MG_TAIL_LEVELS || !H.dense || H.L[l].deg > mg_tail_degree<R>()) return false;
   if ((int64_t)(H.L[l].g.nx + 1) * (H.L[l].g.nz + 1) > MG_TAIL_CELLS) return false;
   bool nested = true;
   for (int i = l; i + 1 < H.nlev; ++i) nested = nested && nested_levels(H.L[i].g, H.L[i + 1].g);
