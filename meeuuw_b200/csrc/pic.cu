@@ -5,11 +5,11 @@
 // advection are in advect.cu.
 //
 // Layout: particles are SoA (x, z, r, t: f64; iel: i32; active: u8), one thread per particle where
-// particles are independent, groups of lanes per bin where they are summed; grid-stride loops sized to a
-// multiple of the SM count.  Projections are atomic-free and deterministic: particles are binned by element (counting sort, each bin sorted by particle
+// particles are independent, lanes or blocks per piece of the bins where they are summed; grid-stride loops.  Projections are atomic-free and deterministic: particles are binned by element (counting sort, each bin sorted by particle
 // index), so every element and node sums its particles in particle-index order -- the order of
 // the reference's sequential loops.  This file is compiled with -fmad=false so the basis and
 // weight arithmetic rounds exactly as the reference's unfused double-precision code.
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -345,53 +345,49 @@ MW_D double avg_transform(int averaging, double v) {
 // largest value over the warp
 MW_D int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
-// pic_functions.py:603-650 over the sorted bins.  16 lanes an element load and transform 16 particles
-// at a time (coalesced where the bin's particles are neighbours in memory; log10 in parallel), then one
-// lane adds each sum in particle order, so the sums are the sequential loop's.
-// PASSES x 16 elements a block.
-template <int PASSES>
+// pic_functions.py:603-650 over the sorted bins.  A block takes as many elements as hold PART particles on
+// average (a power of two, at most PROJ_ELEMENTS), whose particles are one piece of `order`: all of its
+// threads load and transform them, PART at a time, and then a thread per element and field adds its own in
+// particle order, so the sums are the sequential loop's whatever the bins' sizes.  Geometric means, in us
+// (16 lanes an element; a thread an element): 512^2 elements of 4, 9, 16 particles 15, 23, 31 (33, 35, 41; 12, 17,
+// 45), 256^2 of 9, 25, 64 9, 15, 31 (13, 19, 33; 10, 16, 57), 128^2 of 100 17 (17; 36).  A thread an element keeps a
+// lead on meshes of 512^2 with few particles an element in memory order, and loses it in any other order.
+constexpr int PART = 1024, PROJ_ELEMENTS = 64;
 __global__ void __launch_bounds__(256) k_project_elements(int32_t nel, const int32_t* __restrict__ offsets,
                                                           const int32_t* __restrict__ order,
                                                           const double* __restrict__ rho,
                                                           const double* __restrict__ eta, int averaging,
                                                           double* __restrict__ rho_e, double* __restrict__ eta_e,
                                                           int32_t* err) {
-  constexpr int PE = PASSES * (256 / GROUP);
-  __shared__ double sv[2][256 + 4 * (256 / GROUP)];          // a group's 16 values, the next group 4 banks on
-  __shared__ double ssum[2][PE];
-  __shared__ int scnt[PE];
-  const int lane = threadIdx.x % GROUP, grp = threadIdx.x / GROUP, g0 = grp * (GROUP + 4);
-  for (int64_t e0 = blockIdx.x * (int64_t)PE; e0 < nel; e0 += (int64_t)gridDim.x * PE) {
-    for (int le = grp; le < PE; le += 256 / GROUP) {
-      const int64_t e = e0 + le;
-      const int b0 = e < nel ? offsets[e] : 0, m = e < nel ? offsets[e + 1] - b0 : 0;
-      const int rounds = (warp_max(m) + GROUP - 1) / GROUP;
-      double sum = 0.0;
-      for (int c = 0; c < rounds; ++c) {
-        const int j = c * GROUP + lane;
-        if (j < m) {
-          const int p = order[b0 + j];
-          sv[0][g0 + lane] = rho[p];
-          sv[1][g0 + lane] = avg_transform(averaging, eta[p]);
-        }
-        __syncwarp();
-        if (lane < 2) {
-          const int k1 = min(GROUP, m - c * GROUP);
-          for (int k = 0; k < k1; ++k) sum = sum + sv[lane][g0 + k];
-        }
-        __syncwarp();
-      }
-      if (lane < 2) ssum[lane][le] = sum;
-      if (lane == 0) scnt[le] = m;
-    }
+  static_assert(2 * PROJ_ELEMENTS <= 256, "a thread per element and field");
+  constexpr int PAD = 16;                                    // a gap every 16 values: bins of 16 on all banks
+  __shared__ double sv[2][PART + PART / PAD];
+  __shared__ int so[PROJ_ELEMENTS + 1];
+  const int64_t total = offsets[nel];
+  int shift = 6;                                             // elements of a block: 1 << shift
+  while (shift > 0 && (total << shift) > (int64_t)PART * nel) --shift;
+  const int pe = 1 << shift, tid = threadIdx.x, le = tid & (pe - 1), which = tid >> shift;
+  for (int64_t e0 = blockIdx.x * (int64_t)pe; e0 < nel; e0 += (int64_t)gridDim.x * pe) {
+    if (tid <= pe) so[tid] = offsets[min(e0 + tid, (int64_t)nel)];
     __syncthreads();
-    // the means with every lane at work (the power of ten is the costliest step)
-    const int le = threadIdx.x % PE, which = threadIdx.x / PE;
+    const int b0 = so[le], b1 = so[le + 1], end = so[pe];
+    double sum = 0.0;
+    for (int c0 = so[0]; c0 < end; c0 += PART) {
+      for (int j = c0 + tid; j < min(c0 + PART, end); j += 256) {
+        const int p = order[j], i = j - c0;
+        sv[0][i + i / PAD] = rho[p];
+        sv[1][i + i / PAD] = avg_transform(averaging, eta[p]);
+      }
+      __syncthreads();
+      if (which < 2)
+        for (int i = max(b0, c0) - c0; i < min(b1, c0 + PART) - c0; ++i) sum = sum + sv[which][i + i / PAD];
+      __syncthreads();
+    }
     const int64_t e = e0 + le;
     if (e < nel && which < 2) {
-      const double c = (double)scnt[le], sum = ssum[which][le];
+      const double c = (double)(b1 - b0);
       if (which == 0) {
-        if (scnt[le] == 0) set_flag(err, MW_FLAG_EMPTY_ELEMENT);
+        if (b1 == b0) set_flag(err, MW_FLAG_EMPTY_ELEMENT);
         rho_e[e] = sum / c;
       } else if (averaging == MW_AVG_GEOMETRIC) {
         eta_e[e] = pow(10.0, sum / c);
@@ -401,7 +397,7 @@ __global__ void __launch_bounds__(256) k_project_elements(int32_t nel, const int
         eta_e[e] = sum / c;
       }
     }
-    __syncthreads();
+    __syncthreads();                                         // the offsets are read
   }
 }
 
@@ -1076,16 +1072,9 @@ int mw_project_elements(int32_t nel, const int32_t* offsets, const int32_t* orde
                         const double* eta, int32_t averaging, double* rho_e, double* eta_e, int32_t* err,
                         void* stream) {
   if (nel <= 0 || averaging < 0 || averaging > 2) return MW_ERR_BAD_ARG;
-  // 128 elements a block share the means' transcendental step among full warps (262144 elements: 41 us
-  // against 65 with 16 a block); below four such blocks an SM, 16 a block keep every SM busy (1320
-  // elements: 4 us against 17)
-  cudaStream_t s = (cudaStream_t)stream;
-  if (nel >= 128 * 4 * num_sms())
-    k_project_elements<8><<<grid_all(nel, 128), 256, 0, s>>>(nel, offsets, order, rho, eta, averaging, rho_e, eta_e,
+  const unsigned grid = (unsigned)std::min<int64_t>(nel, 8 * num_sms());
+  k_project_elements<<<grid, 256, 0, (cudaStream_t)stream>>>(nel, offsets, order, rho, eta, averaging, rho_e, eta_e,
                                                              err);
-  else
-    k_project_elements<1><<<grid_all(nel, 16), 256, 0, s>>>(nel, offsets, order, rho, eta, averaging, rho_e, eta_e,
-                                                            err);
   MW_CHECK_LAUNCH();
   return MW_OK;
 }

@@ -1,5 +1,5 @@
-"""Bins around and past the lengths the particle kernels branch on: the sort by rank and by merge exchange, the
-rounds of the nodal projections in all flavours and capacities for fields."""
+"""Bins around and past the lengths the particle kernels branch on: the sort by rank, by merge exchange, the rounds
+of 16 and of 1024 particles of the projections, all nodal flavours, all capacities for fields."""
 import numpy as np
 import pytest
 import torch
@@ -43,6 +43,28 @@ def test_bins_are_sorted(kind, order):
     assert np.array_equal(counts.cpu().numpy(), want)
     assert np.array_equal(offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(want)]))
     assert np.array_equal(perm.cpu().numpy()[: len(iel)], np.argsort(iel, kind="stable"))
+
+
+@pytest.mark.parametrize("nel", [1, 63, 64, 65, 40 * 33, 300 * 260])
+@pytest.mark.parametrize("kind", ["1", "4", "16", "25", "100", "mixed"])
+def test_element_means(kind, nel):
+    """The arithmetic mean is the sequential sum's, bit for bit; the geometric one to 1e-13 (its transform)."""
+    from meeuuw_b200 import ops
+    if nel > 10000 and kind in ("100", "mixed"):
+        nel = 70 * 70
+    iel, _, _, eta, rho = swarm(kind, nel, "shuffled")
+    counts, offsets, perm = bins(iel, nel)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rho_e, eta_e = ops.project_elements(nel, offsets, perm, torch.as_tensor(rho).cuda(), torch.as_tensor(eta).cuda(),
+                                        "geometric", err=err)
+    cnt = np.bincount(iel, minlength=nel)
+    s, l = np.zeros(nel), np.zeros(nel)
+    np.add.at(s, iel, rho)
+    np.add.at(l, iel, np.log10(eta))
+    full = cnt > 0
+    assert np.array_equal(rho_e.cpu().numpy()[full], s[full] / cnt[full])
+    assert np.max(np.abs(eta_e.cpu().numpy()[full] / 10.0 ** (l[full] / cnt[full]) - 1)) < 1e-13
+    assert (int(err.item()) != 0) == (not full.all())
 
 
 @pytest.mark.parametrize("nfield", [1, 2, 3, 5, 8])
