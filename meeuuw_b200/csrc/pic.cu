@@ -567,7 +567,8 @@ template <int NF>
 __global__ void __launch_bounds__(PFX * PFZ) k_project_finish(mw_box b, ProjFields pf,
                                                               const double* __restrict__ part) {
   __shared__ double sc[NF][(PFX + 1) * (PFZ + 1)];
-  const int i0 = blockIdx.x * PFX, j0 = blockIdx.y * PFZ;
+  const int ntx = (b.nelx + PFX - 1) / PFX;                  // (tiles in x alone: a mesh may be taller than the grid's y)
+  const int i0 = (int)(blockIdx.x % ntx) * PFX, j0 = (int)(blockIdx.x / ntx) * PFZ;
   const int nf1 = pf.n + 1;
   const int64_t nnx = 2 * b.nelx + 1;
   for (int c = threadIdx.x; c < (PFX + 1) * (PFZ + 1); c += PFX * PFZ) {
@@ -1097,7 +1098,7 @@ int mw_project_nodes(mw_box box, int32_t flavour, int32_t nfield, const int32_t*
   int64_t nc = (int64_t)(box.nelx + 1) * (box.nelz + 1);
   if (work && work_bytes >= mw_project_nodes_workspace_bytes(box, nfield)) {
     const int64_t nel = (int64_t)box.nelx * box.nelz;
-    const dim3 tiles((box.nelx + PFX - 1) / PFX, (box.nelz + PFZ - 1) / PFZ);
+    const unsigned tiles = (unsigned)((box.nelx + PFX - 1) / PFX) * (unsigned)((box.nelz + PFZ - 1) / PFZ);
     const double* part = (const double*)work;
     auto go = [&](auto cap) {
       constexpr int NF = cap.value;

@@ -85,3 +85,18 @@ def test_node_projections(order, flavour, nfield):
     b = ops.project_nodes(box, flavour, fields, offsets, perm, D(r), D(t), exact_order=True)
     for x, y in zip(a, b):
         assert float((x - y).abs().max() / y.abs().max()) < 1e-13
+
+
+def test_node_projection_of_a_tall_mesh():
+    """A column of more tiles than a launch has in its second dimension."""
+    from meeuuw_b200 import _lib, ops
+    nelx, nelz = 1, 530000
+    iel, r, t, eta, rho = swarm("1", nelx * nelz, "sorted")
+    counts, offsets, perm = bins(iel, nelx * nelz)
+    D = lambda a: torch.as_tensor(a).cuda()
+    fields = [(D(rho), "arithmetic"), (D(eta), "geometric")]
+    box = _lib.box_of(nelx, nelz, 1.0, 1.0 * nelz)
+    a = ops.project_nodes(box, 2, fields, offsets, perm, D(r), D(t))
+    b = ops.project_nodes(box, 2, fields, offsets, perm, D(r), D(t), exact_order=True)
+    for x, y in zip(a, b):
+        assert float((x / y - 1).abs().max()) < 1e-12
