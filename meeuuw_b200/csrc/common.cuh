@@ -65,11 +65,10 @@ inline unsigned grid_all(int64_t n, int threads) {
 // Programmatic dependent launch.  The solver loops are long chains of short kernels on one stream;
 // launched through pdl_launch(), a kernel's CTAs are scheduled while its predecessor is still
 // running, so the launch latency between the two is hidden.  Every kernel started this way runs
-// pdl_entry() before touching global memory: it waits until every prerequisite grid has completed
-// and its writes are visible, then allows the next kernel to be scheduled (for a kernel started the
-// ordinary way both instructions return at once).  Because each kernel waits for the complete
-// predecessor before its first access, the stream order of all reads and writes is unchanged, and
-// at most one waiting grid is resident beside the running one.
+// pdl_entry(): it waits until every prerequisite grid has completed and its writes are visible, then
+// allows the next kernel to be scheduled (for a kernel started the ordinary way both instructions return
+// at once).  A kernel writes, and reads what its predecessor may have written, only after it, so the
+// order of those accesses is the stream's, and at most one waiting grid is resident beside the running one.
 MW_D void pdl_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -80,6 +79,7 @@ MW_D void pdl_entry() {
 // predecessor's predecessor is complete and visible.  The level and Krylov kernels load the diagonal,
 // the viscosity, the Dirichlet flags and their tables there (written at least two launches earlier, by
 // the set-up), so that a chain of short launches does not wait for them.
+
 inline int current_device() {
   int dev = -1;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;

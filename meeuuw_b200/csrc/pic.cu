@@ -58,8 +58,8 @@ __global__ void k_locate(mw_box b, int64_t n, const uint8_t* __restrict__ active
     const uint8_t act = active[i];
     const double xi = x[i], zi = z[i];
     if (!act) { r[i] = 0.0; t[i] = 0.0; iel[i] = 0; continue; }
-    // element_of with the quotients above: int() truncates toward zero; a quotient that does not fit an
-    // int is out of range (the reference would index out of bounds there)
+    // the element: pic_functions.py:29-31; int() truncates toward zero, and a quotient that does not fit an int
+    // is out of range (the reference would index out of bounds there)
     const double qx = quotient_exact(xi, b.hx, ihx), qz = quotient_exact(zi, b.hz, ihz);
     bool ok = qx > -2147483648.0 && qx < 2147483647.0 && qz > -2147483648.0 && qz < 2147483647.0;
     int ex = 0, ez = 0;

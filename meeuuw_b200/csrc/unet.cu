@@ -22,7 +22,7 @@ template <typename I> MW_D void split(I i, I n, I* q, I* r) { *q = i / n; *r = i
 
 // X [B,H,W,C] (bf16) -> col [M = B*H*W, Kp] (bf16), 'same' 3x3 patches, zeros outside; eight K entries a
 // thread, one 16-byte store (an entry a thread with 64-bit index divisions: 104 us for 262144 pixels of two
-// channels, now 47: two-channel pixels are 4-byte loads)
+// channels, now 47; the entries are still loaded one by one)
 template <int V>
 __global__ void __launch_bounds__(256) k_im2col(int B, int H, int W, int C, int Kp, const bf16* __restrict__ X,
                                                 bf16* __restrict__ col) {
