@@ -193,7 +193,7 @@ def run_ours(args):
         launches = int(len(ours) * args.steps)
         kernel_mix = {}
         for nm in ours:
-            k = nm.split("(")[0].replace("void ", "")
+            k = nm.replace("(anonymous namespace)::", "").split("(")[0].replace("void ", "")
             kernel_mix[k] = kernel_mix.get(k, 0) + 1
     except Exception as ex:  # profiler unavailable: leave the claim empty
         kernel_mix = {"error": str(ex)}
@@ -491,7 +491,7 @@ def step1_vs_oracle(torch, weights):
 
 
 def roofline_apply(model, torch):
-    """Average duration of the fine-level FP32 operator apply (k_apply), CUDA events on its stream."""
+    """Average duration of the fine-level FP32 operator apply (k_op_apply), CUDA events on its stream."""
     from meeuuw_b200 import _lib
     S = model.solver
     nv, npp = S.nv, S.np
@@ -522,10 +522,10 @@ def roofline_apply(model, torch):
     peak = peaks.get("hbm_gbs", 6650.0)
     achieved = algo / (us * 1e-6) / 1e9
     # DRAM bytes (read + write) of one launch at 512x512 from an ncu capture of this kernel
-    # (profiles/k_apply_fp32_fk512.txt); other sizes scale with the element count
-    traffic = int(20162560 * nel / 262144)
-    # the Chebyshev smoothing step (mode CHEB, the kernel the V-cycle launches most): reads x, b,
-    # diag, d (2nn f32 each), eta, mask; writes d and x_out (2nn f32 each); no pressure
+    # (profiles/kernels_512.txt); other sizes scale with the element count
+    traffic = int(21169000 * nel / 262144)
+    # a Chebyshev smoothing step by itself (what smoothing of degree above two launches): reads x, b, diag, d
+    # (2nn f32 each), eta, mask; writes d and x_out (2nn f32 each); no pressure
     b = torch.randn(nv, dtype=torch.float32, device="cuda")
     d = torch.zeros_like(b)
     xo = torch.empty_like(b)
@@ -541,7 +541,7 @@ def roofline_apply(model, torch):
     algo_c = 4 * 2 * nn * 4 + 4 * 9 * nel + 2 * nn + 4 * 2 * nn * 2
     cheb = {"kernel": "mw::k_apply<float, AM_CHEB> (fine level)", "us_per_launch": us_c, "algorithmic_bytes": algo_c,
             "achieved": algo_c / (us_c * 1e-6) / 1e9, "frac": algo_c / (us_c * 1e-6) / 1e9 / peak}
-    return {"kernel": "mw::k_apply<float, AM_APPLY> (fine level, 512x512)", "bound": "hbm", "achieved": achieved,
+    return {"kernel": "mw::k_op_apply<float, K u + G p and G^T u> (fine level, 512x512)", "bound": "hbm", "achieved": achieved,
             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic, "us_per_launch": us,
             "algorithmic_bytes": algo, "cheb_mode": cheb,
             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if "hbm_gbs" in peaks else "fallback 6650"}

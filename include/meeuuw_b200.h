@@ -380,7 +380,8 @@ void mw_solve_default_params(mw_solve_params* p);
 size_t mw_stokes_workspace_bytes(mw_box box, mw_stokes_params prm);
 
 /* Create a solver for the box with the velocity Dirichlet mask bc_fix_V (device, Nfem_V bytes,
- * kept by reference).  All device arrays are carved from `work`. */
+ * kept by reference).  All device arrays are carved from `work`, which nothing touches until the first call that
+ * uses the solver, on that call's stream. */
 int mw_stokes_create(mw_box box, mw_stokes_params prm, const uint8_t* bc_fix_V, void* work, size_t work_bytes,
                      mw_stokes** out);
 int mw_stokes_destroy(mw_stokes* S);
@@ -418,7 +419,8 @@ int mw_stokes_level_shape(const mw_stokes* S, int32_t precision, int32_t level, 
 int mw_stokes_solve_K(mw_stokes* S, int32_t precision, const double* b, double* x, double rtol, int32_t maxit,
                       int32_t* iters, double* relres, void* stream);
 
-/* Result of the last solve from its device scalars (synchronises `stream`).  When mw_stokes_solve is
+/* Result of the last solve from its device scalars (synchronises `stream`); residuals, solve_K and other calls
+ * that are no solve leave them alone.  When mw_stokes_solve is
  * called on a stream that is recording a CUDA graph, the solve is recorded into that graph (its
  * loops as conditional nodes), returns MW_OK with a zeroed info, and this call reads the outcome
  * after a replay; converged = rel_residual <= tol. */

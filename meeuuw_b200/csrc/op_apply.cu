@@ -7,8 +7,8 @@
 // element-tile form this replaces staged the velocity and every element's 22 results in shared memory and
 // looked its indices up per node: 1065 warp instructions an element, of which 370 were the product.
 //
-// Measured, (u, p) -> (K u + G p, G^T u), before and now: FP32 512^2 16.5 -> 15.9 us, 128^2 5.0 -> 3.5, 8^2
-// 4.6 -> 3.4; FP64 512^2 40.8 -> 31, 256^2 13.8 -> 10.8.  At 512^2 the packed multiply-adds alone take 5.9 us
+// Measured, (u, p) -> (K u + G p, G^T u), before and now: FP32 512^2 17.5 -> 16.2 us, 128^2 5.3 -> 3.7, 8^2
+// 4.9 -> 3.5; FP64 512^2 42.5 -> 34.4, 256^2 14.3 -> 12.8.  At 512^2 the packed multiply-adds alone take 5.9 us
 // (they issue at half rate); the rest is the load and exchange latency that two tiles an SM leave open.
 #include "cell_ops.cuh"
 #include "op_apply.cuh"
